@@ -48,6 +48,11 @@ struct KernelArgs {
   const struct RotaryPackFusion* rotary_fusion;
 };
 
+// Bytes between the sequences of a batched short-conv step.
+struct ShortConvStepStrides {
+  size_t in_proj, state, output;
+};
+
 typedef int (*Launcher)(const KernelArgs&);
 struct NamedLauncher {
   const char* name;

@@ -5,8 +5,8 @@
 //   llmopt_short_conv_step{,_fused}_f16    one decode token, state updated in place
 //   llmopt_short_conv_prefill{,_init}_f16  the same recurrence over T tokens
 // All arithmetic in fp32, one rounding to half per stored value, as the
-// reference kernels do. These move a few KB per call; launch latency is the
-// bound, so they stay one thread per output element.
+// reference kernels do. These move a few KB per call (a prompt some MB); launch
+// latency is the bound, so they stay one thread per output element or short strip.
 #include "common.cuh"
 
 namespace llmopt {
@@ -59,12 +59,16 @@ __global__ void short_conv_silu_tm_kernel(const __half* __restrict__ input, cons
   output[gid] = __float2half_rn(value / (1.0f + expf(-value)));
 }
 
+// One decode token of gridDim.y sequences, whose rows, states and outputs lie `stride` bytes apart (the weights are shared).
 __global__ void short_conv_step_kernel(const __half* __restrict__ in_proj, __half* __restrict__ conv_state,
                                        const __half* __restrict__ conv_weight, __half* __restrict__ output,
-                                       uint32_t channels) {
+                                       uint32_t channels, ShortConvStepStrides stride) {
   grid_chain_prologue();
   const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= channels) return;
+  in_proj = (const __half*)((const uint8_t*)in_proj + blockIdx.y * stride.in_proj);
+  conv_state = (__half*)((uint8_t*)conv_state + blockIdx.y * stride.state);
+  output = (__half*)((uint8_t*)output + blockIdx.y * stride.output);
   const float x0 = __half2float(in_proj[c]);
   const float x1 = __half2float(in_proj[channels + c]);
   const float x2 = __half2float(in_proj[2 * channels + c]);
@@ -82,23 +86,35 @@ __global__ void short_conv_step_kernel(const __half* __restrict__ in_proj, __hal
   output[c] = __float2half_rn(x1 * conv_out);
 }
 
+// A prompt.  An output reads the gated inputs x0 x2 of its own and the two tokens before it and nothing that another
+// token's output leaves behind, so a thread takes a strip of `strip` tokens of one channel and forms the two products ahead
+// of its strip again: 333 tokens of 1024 channels as one strip per channel (four thread blocks that walk over the prompt,
+// every load waiting for the one before) took 101 us, in strips of eight 3 us.  Eight tokens re-read a quarter more rows,
+// which still are in the cache; shorter strips would re-read more and 148 SMs are filled already.
+constexpr uint32_t kConvStrip = 8;
+
 __global__ void short_conv_prefill_kernel(const __half* __restrict__ in_proj, const __half* __restrict__ conv_weight,
-                                          __half* __restrict__ output, __half* __restrict__ state_out,
-                                          const __half* __restrict__ state_in, uint32_t tokens, uint32_t channels,
-                                          uint32_t has_initial_state) {
+                                          __half* __restrict__ output, __half* state_out, const __half* state_in,
+                                          uint32_t tokens, uint32_t channels, uint32_t strip) {
   grid_chain_prologue();
   const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= channels) return;
+  const uint32_t first = blockIdx.y * strip;
+  const uint32_t last = min(tokens, first + strip);
   const float w0 = __half2float(conv_weight[c * 3 + 0]);
   const float w1 = __half2float(conv_weight[c * 3 + 1]);
   const float w2 = __half2float(conv_weight[c * 3 + 2]);
-  float prev3 = 0.0f, prev2 = 0.0f, prev1 = 0.0f;
-  if (has_initial_state != 0 && state_in != nullptr) {
-    prev3 = __half2float(state_in[c * 3 + 0]);
-    prev2 = __half2float(state_in[c * 3 + 1]);
-    prev1 = __half2float(state_in[c * 3 + 2]);
-  }
-  for (uint32_t t = 0; t < tokens; ++t) {
+  // the gated input `back` places ahead of the strip; ahead of the prompt it is the initial state
+  auto before = [&](uint32_t back) {
+    if (first >= back) {
+      const __half* row = in_proj + (size_t)(first - back) * 3 * channels + c;
+      return __half2float(row[0]) * __half2float(row[2 * channels]);
+    }
+    return state_in != nullptr ? __half2float(state_in[c * 3 + 3 + first - back]) : 0.0f;
+  };
+  float prev3 = before(3), prev2 = before(2), prev1 = before(1);
+#pragma unroll 8
+  for (uint32_t t = first; t < last; ++t) {
     const size_t offset = (size_t)t * 3 * channels + c;
     const float x0 = __half2float(in_proj[offset]);
     const float x1 = __half2float(in_proj[offset + channels]);
@@ -110,9 +126,11 @@ __global__ void short_conv_prefill_kernel(const __half* __restrict__ in_proj, co
     prev2 = prev1;
     prev1 = current;
   }
-  state_out[c * 3 + 0] = __float2half_rn(prev3);
-  state_out[c * 3 + 1] = __float2half_rn(prev2);
-  state_out[c * 3 + 2] = __float2half_rn(prev1);
+  if (last == tokens) {
+    state_out[c * 3 + 0] = __float2half_rn(prev3);
+    state_out[c * 3 + 1] = __float2half_rn(prev2);
+    state_out[c * 3 + 2] = __float2half_rn(prev1);
+  }
 }
 
 }  // namespace
@@ -171,9 +189,42 @@ int launch_short_conv_step(const KernelArgs& args) {
   LLMOPT_REQUIRE(args.lengths[0] >= (size_t)channels * 6 && args.lengths[1] >= (size_t)channels * 6 &&
                      args.lengths[2] >= (size_t)channels * 6 && args.lengths[3] >= (size_t)channels * 2,
                  "buffer is too short");
-  launch_kernel(args, short_conv_step_kernel, dim3((channels + 255) / 256), dim3(256), 0,
+  launch_kernel(args, short_conv_step_kernel, dim3((channels + 255) / 256, 1), dim3(256), 0,
       (const __half*)args.buffers[0], (__half*)args.buffers[1], (const __half*)args.buffers[2], (__half*)args.buffers[3],
-      channels);
+      channels, ShortConvStepStrides{});
+  return check_launch(args);
+}
+
+// The same record of `count` sequences, one after another in a dispatch list, as one launch.  `args` are the first one's,
+// `second` the buffers of the second; every further one has to lie as far behind its predecessor (the caller has compared
+// them).  False where the records could touch each other's data, which a launch would then read or write in another order.
+bool short_conv_steps_stride(const KernelArgs& first, const KernelArgs& second, uint32_t count, ShortConvStepStrides* stride) {
+  if (first.buffer_count != 4 || first.param_bytes != 4 || count > 65535) return false;
+  const size_t channels = param_u32(first, 0);
+  const size_t bytes[4] = {channels * 6, channels * 6, channels * 6, channels * 2};  // of a record in each buffer
+  size_t step[4], extent[4];
+  for (int i = 0; i < 4; ++i) {
+    const intptr_t distance = (const uint8_t*)second.buffers[i] - (const uint8_t*)first.buffers[i];
+    if (first.lengths[i] < bytes[i] || distance < 0 || (i == 2 ? distance != 0 : distance < (intptr_t)bytes[i])) return false;
+    step[i] = (size_t)distance;
+    extent[i] = step[i] * (count - 1) + bytes[i];
+  }
+  for (int i = 0; i < 4; ++i)
+    for (int j = 0; j < i; ++j) {
+      const uint8_t *a = (const uint8_t*)first.buffers[i], *b = (const uint8_t*)first.buffers[j];
+      if (a < b + extent[j] && b < a + extent[i]) return false;
+    }
+  *stride = ShortConvStepStrides{step[0], step[1], step[3]};
+  return true;
+}
+
+// Sixteen sequences of 1024 channels: sixteen launches of 1.3 us behind each other in a plan, together one of 2 us.
+int launch_short_conv_steps(const KernelArgs& args, uint32_t count, const ShortConvStepStrides& stride) {
+  const uint32_t channels = param_u32(args, 0);
+  LLMOPT_REQUIRE(channels > 0, "needs channels > 0");
+  launch_kernel(args, short_conv_step_kernel, dim3((channels + 255) / 256, count), dim3(256), 0,
+      (const __half*)args.buffers[0], (__half*)args.buffers[1], (const __half*)args.buffers[2], (__half*)args.buffers[3],
+      channels, stride);
   return check_launch(args);
 }
 
@@ -194,9 +245,17 @@ int launch_short_conv_prefill(const KernelArgs& args) {
     LLMOPT_REQUIRE(args.lengths[4] >= (size_t)channels * 6, "initial state buffer is too short");
     state_in = (const __half*)args.buffers[4];
   }
-  launch_kernel(args, short_conv_prefill_kernel, dim3((channels + 255) / 256), dim3(256), 0,
+  if (has_initial == 0) state_in = nullptr;
+  // A state updated in place is read by the first strip and written by the last one: a single strip then, whose thread reads
+  // before it writes.  So too for prompts whose strips are more than a grid has rows.
+  const uint8_t *in = (const uint8_t*)state_in, *out = (const uint8_t*)args.buffers[3];
+  const size_t state_bytes = (size_t)channels * 6;
+  const bool in_place = in != nullptr && in < out + state_bytes && out < in + state_bytes;
+  const uint32_t strips = in_place || tokens == 0 ? 1 : (tokens + kConvStrip - 1) / kConvStrip;
+  const uint32_t strip = strips == 1 || strips > 65535 ? tokens : kConvStrip;
+  launch_kernel(args, short_conv_prefill_kernel, dim3((channels + 255) / 256, strips > 65535 ? 1 : strips), dim3(256), 0,
       (const __half*)args.buffers[0], (const __half*)args.buffers[1], (__half*)args.buffers[2], (__half*)args.buffers[3],
-      state_in, tokens, channels, has_initial);
+      state_in, tokens, channels, strip);
   return check_launch(args);
 }
 

@@ -67,6 +67,8 @@ LLMOPT_FAMILY int launch_attention_q8_paged(const KernelArgs&);
 template <bool WEIGHT_F32> LLMOPT_FAMILY int launch_short_conv(const KernelArgs&);
 template <bool WEIGHT_F32> LLMOPT_FAMILY int launch_short_conv_silu_tm(const KernelArgs&);
 LLMOPT_FAMILY int launch_short_conv_step(const KernelArgs&);
+LLMOPT_FAMILY bool short_conv_steps_stride(const KernelArgs& first, const KernelArgs& second, uint32_t count, ShortConvStepStrides* stride);
+LLMOPT_FAMILY int launch_short_conv_steps(const KernelArgs& args, uint32_t count, const ShortConvStepStrides& stride);
 LLMOPT_FAMILY int launch_short_conv_prefill(const KernelArgs&);
 template <bool INPUT_F32> LLMOPT_FAMILY int launch_rms_norm(const KernelArgs&);
 LLMOPT_FAMILY int launch_rotary_qk(const KernelArgs&);
@@ -624,6 +626,41 @@ static int run_rotary_pack_attention(Context* context, const OwnedRecord& rotary
   attention_args.error = &message;
   if (attention.launcher(attention_args) != 0) return set_error(LLMOPT_CUDA_FAILURE, message);
   return LLMOPT_CUDA_OK;
+}
+
+// Plan-capture peephole: the short-conv steps of several sequences, recorded one after another because the step kernel
+// carries one, as one launch.  Returns the number of records it took, 0 when records [index, ...) are no such run, -1 on failure.
+static int run_short_conv_steps(Context* context, const std::vector<OwnedRecord>& records, size_t index) {
+  const OwnedRecord& first = records[index];
+  if (first.is_copy || first.name != "llmopt_short_conv_step_f16" || first.buffers.size() != 4) return 0;
+  auto alike = [&](const OwnedRecord& record) {
+    return !record.is_copy && record.name == first.name && record.params == first.params && record.buffers.size() == 4;
+  };
+  auto distance = [&](size_t place, int buffer) {
+    return records[place].buffers[buffer]->pointer() - records[place - 1].buffers[buffer]->pointer();
+  };
+  size_t end = index + 1;
+  for (; end < records.size() && alike(records[end]); ++end) {
+    bool same = true;
+    for (int buffer = 0; buffer < 4; ++buffer) {
+      same = same && records[end].buffers[buffer]->length == first.buffers[buffer]->length &&
+             distance(end, buffer) == distance(index + 1, buffer);
+    }
+    if (!same) break;
+  }
+  if (end - index < 2) return 0;
+  KernelArgs args = {}, second = {};
+  fill_args(context, first, nullptr, nullptr, &args);
+  fill_args(context, records[index + 1], nullptr, nullptr, &second);
+  std::string message;
+  args.error = &message;
+  ShortConvStepStrides stride;
+  if (!short_conv_steps_stride(args, second, (uint32_t)(end - index), &stride)) return 0;
+  if (launch_short_conv_steps(args, (uint32_t)(end - index), stride) != 0) {
+    set_error(LLMOPT_CUDA_FAILURE, message);
+    return -1;
+  }
+  return (int)(end - index);
 }
 
 static int wait_stream(Context* context, const char* what) {
@@ -1274,6 +1311,12 @@ int llmopt_cuda_prebaked_create_bound(llmopt_cuda_library* library, const llmopt
         if (failure != LLMOPT_CUDA_OK) break;
         continue;
       }
+    }
+    if (const int taken = run_short_conv_steps(context, plan->records, index)) {
+      if (taken < 0) failure = LLMOPT_CUDA_FAILURE;
+      if (failure != LLMOPT_CUDA_OK) break;
+      index += taken - 1;
+      continue;
     }
     if (fuse_pack && index + 1 < plan->records.size()) {
       const int fused_status = run_rotary_pack(context, plan->records[index], plan->records[index + 1]);
