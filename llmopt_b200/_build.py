@@ -14,7 +14,7 @@ OBJECTS = os.path.join(PACKAGE_DIR, "build")
 
 # Kernel families that are enough to serve one kind of model: a host that needs no others can build
 # and load libllmopt_cuda_<family>.so (the runtime registers only the names that were linked in).
-_ATTENTION = ("runtime", "sampling", "dense_linear", "dense_gemm_tc", "sequence_glue", "row_attention", "experts")
+_ATTENTION = ("runtime", "sampling", "dense_linear", "dense_f32", "dense_gemm_tc", "sequence_glue", "row_attention", "experts")
 FAMILIES = {
     "attention": _ATTENTION,  # decoders whose mixers all are attention
     "mixers": _ATTENTION + ("matrix_state",),

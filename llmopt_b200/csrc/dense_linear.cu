@@ -11,8 +11,9 @@
 //    as their B words: no shared-memory staging and full 128-byte lines.  Eight warps split K and
 //    add their sums in warp order.
 //  * bf16, more rows: dense_gemm_tc.cu (tcgen05).
-//  * fp32, and bf16 rows that are no whole 16-byte vectors: CUDA-core kernels (a warp per column for
-//    few rows, 64 x 64 tiles otherwise).
+//  * fp32: dense_f32.cu.
+//  * rows that are no whole 16-byte vectors: CUDA-core kernels (a warp per column for few rows, 64 x 64
+//    tiles otherwise).
 #include <type_traits>
 
 #include "dense_stream.cuh"
@@ -214,7 +215,10 @@ int run_gemv(const KernelArgs& args, DenseProblem p, DenseStore store) {
 template <typename T>
 int run_dense(const KernelArgs& args, const DenseProblem& p, DenseStore store) {
   if (p.m == 0) return 0;
-  if (sizeof(T) == 4) return run_cuda_cores<T>(args, p, store);
+  if (sizeof(T) == 4) {
+    const int status = launch_dense_f32(args, p, store, 0);
+    return status >= 0 ? status : run_cuda_cores<T>(args, p, store);
+  }
   const bool vectors = p.k % 8u == 0 && ((uintptr_t)p.x & 15u) == 0 && ((uintptr_t)p.w & 15u) == 0;
   if (!vectors) return run_cuda_cores<T>(args, p, store);
   if (p.m > 64u) {
@@ -322,10 +326,8 @@ int launch_dense_residual(const KernelArgs& args) {
 
 template <typename T>
 int run_expert_rows(const KernelArgs& args, const DenseProblem& p, DenseStore store, uint32_t tiles) {
-  if (sizeof(T) == 2) {
-    const int status = launch_dense_gemm_tc(args, p, store);
-    if (status >= 0) return status;
-  }
+  const int status = sizeof(T) == 2 ? launch_dense_gemm_tc(args, p, store) : launch_dense_f32(args, p, store, tiles);
+  if (status >= 0) return status;
   constexpr uint32_t kHalves = kExpertTile / 64u;
   LLMOPT_REQUIRE(tiles * kHalves <= 65535u, "too many tiles");
   const dim3 grid((p.n + 63u) / 64u, tiles * kHalves);

@@ -174,6 +174,10 @@ __device__ __forceinline__ void dense_store_pair(const DenseTask<kStorePair>& p,
 // Prompt rows on tcgen05 (bf16); -1 when the shape or the pointers are outside its domain.
 int launch_dense_gemm_tc(const KernelArgs& args, const DenseProblem& problem, DenseStore store);
 
+// fp32, rows of whole 16-byte vectors; with a plan at most `tiles` tiles of it.  -1 when the shape or the pointers are outside
+// its domain.
+int launch_dense_f32(const KernelArgs& args, const DenseProblem& problem, DenseStore store, uint32_t tiles);
+
 // Rows of at most `tiles` tiles of a plan, each with its expert's matrix.
 template <typename T>
 int run_expert_rows(const KernelArgs& args, const DenseProblem& problem, DenseStore store, uint32_t tiles);

@@ -4,6 +4,9 @@ and largest of a range."""
 import numpy as np
 import pytest
 
+import oracle_mixers as plain
+from test_gpu_mixers import close, download, empty, upload
+
 pytestmark = pytest.mark.gpu
 
 
@@ -72,3 +75,28 @@ def test_short_conv_steps_of_a_plan_as_one_launch(runtime, oracle, apart, shared
         return states.contents(), out.contents()
 
     assert run(True) == run(False)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 9, 4), (2, 8, 516), (4, 7, 128), (5, 33, 1028), (8, 16, 260), (9, 65, 36), (32, 64, 32),
+                                   (33, 63, 2052), (64, 128, 1024), (65, 130, 96), (100, 256, 2048), (129, 20, 7168)])
+def test_dense_fp32(runtime, m, n, k):
+    """Vectors of a few columns, tiles and their splits of k.  fp32 sums of k products in parts: an error of a few times
+    2^-24 sqrt(k) of the terms' size, where the result has sqrt(k) of them; 3e-6 of the largest result."""
+    from llmopt_b200 import parameters
+
+    rng = np.random.default_rng(m * 1000 + n)
+    x, w = rng.standard_normal((m, k)).astype(np.float32), (rng.standard_normal((n, k)) / np.sqrt(k)).astype(np.float32)
+    bias = rng.standard_normal(n).astype(np.float32)
+    y = x.astype(np.float64) @ w.T.astype(np.float64) + bias
+    split = n // 2
+    buffers = [upload(runtime, x), upload(runtime, w), upload(runtime, bias), empty(runtime, m * n), empty(runtime, m * n),
+               upload(runtime, np.zeros(m, np.int64)), empty(runtime, 16)]
+    runtime.dispatch("llmopt_dense_linear_f32", buffers=buffers, parameters=parameters.dense_linear(
+        m=m, n=n, k=k, split=split, has_bias=True, epilogue=None))
+    if split:
+        close(download(buffers[3], (m, split)), y[:, :split], 3e-6)
+    close(download(buffers[4], (m, n - split)), y[:, split:], 3e-6)
+    if n % 2 == 0:
+        runtime.dispatch("llmopt_dense_linear_f32", buffers=buffers, parameters=parameters.dense_linear(
+            m=m, n=n, k=k, split=n, has_bias=True, epilogue="silu_pair"))
+        close(download(buffers[3], (m, n // 2)), plain.silu(y[:, 0::2]) * y[:, 1::2], 6e-6)
