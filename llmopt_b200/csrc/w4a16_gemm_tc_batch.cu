@@ -54,6 +54,14 @@ constexpr uint32_t kSplitCounterTiles = 1u << 14;
 // pair's two accumulator columns.
 enum BatchEpilogue { kBatchLinear = 0, kBatchDualSwiglu = 1, kBatchLinearPair = 2, kBatchDualStacked = 3, kBatchSplitF32 = 4 };
 
+// kBatchLinear: further matrices with the same input whose tiles follow the first one's (fused QKV); tile `first` on.
+struct BatchSegment {
+  uint32_t first, n;
+  const uint8_t* packed;
+  const __half* scale;
+  __half* out;
+};
+
 struct BatchProblem {
   uint32_t m, n, k;
   const uint8_t* packed[2];
@@ -64,8 +72,10 @@ struct BatchProblem {
   const __half* aux;  // bias (row stride 0) or residual (row stride n)
   uint32_t aux_row_stride, has_aux;
   uint32_t splits;
-  float* partials;     // [tiles][splits][matrices * 128 rows][NB]
+  float* partials;     // [tiles][splits][matrices][NB / 4][128 rows][4]: lanes (rows) side by side
   uint32_t* counters;  // [tiles], zero between launches
+  uint32_t segments;
+  BatchSegment segment[2];
 };
 
 constexpr uint32_t next_power_of_two(uint32_t value) {
@@ -160,7 +170,22 @@ w4a16_gemm_tc_batch_kernel(const __grid_constant__ CUtensorMap map_x, const Batc
   volatile uint32_t* holder = reinterpret_cast<volatile uint32_t*>(base_pointer + L::kOffsetHolder);  // [tmem, abort, last]
 
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-  const uint32_t tile = blockIdx.x, split = blockIdx.y, n0 = tile * kTileRows;
+  const uint32_t tile = blockIdx.x, split = blockIdx.y;
+  // the matrix this tile belongs to
+  constexpr bool kSegments = EPI == kBatchLinear && !AFFINE;
+  uint32_t first_tile = 0, n = p.n;
+  const uint8_t* own_packed = p.packed[0];
+  const __half* own_scale = p.scale[0];
+  __half* out = p.out;
+  if (kSegments) {
+#pragma unroll
+    for (uint32_t i = 0; i < 2; ++i)
+      if (i < p.segments && tile >= p.segment[i].first) {
+        first_tile = p.segment[i].first, n = p.segment[i].n, out = p.segment[i].out;
+        own_packed = p.segment[i].packed, own_scale = p.segment[i].scale;
+      }
+  }
+  const uint32_t n0 = (tile - first_tile) * kTileRows;
   const uint32_t token0 = blockIdx.z * NB;           // first activation row of this CTA (prompts: several row tiles)
   const uint32_t tile_id = blockIdx.z * gridDim.x + tile;  // index of the output tile for the K-split bookkeeping
   const uint32_t all_k_blocks = p.k / kBK, all_groups = (all_k_blocks + kGroupBlocks - 1u) / kGroupBlocks;
@@ -277,14 +302,14 @@ w4a16_gemm_tc_batch_kernel(const __grid_constant__ CUtensorMap map_x, const Batc
     const uint32_t tile_first_row = n0 + (EPI == kBatchLinearPair ? matrix * kRows : 0u);
     auto row_in_source = [&](uint32_t row) { return kStacked ? (row & (kRows / 2 - 1u)) : row; };
     const uint32_t weight_row = tile_first_row + row_in_source(tile_row);
-    const bool row_present = weight_row < p.n;
+    const bool row_present = weight_row < n;
     const uint32_t groups = p.k / 64;
-    const __half* scale_row = p.scale[source] + (size_t)(row_present ? weight_row : 0u) * groups;
+    const __half* scale_row = (kSegments ? own_scale : p.scale[source]) + (size_t)(row_present ? weight_row : 0u) * groups;
     const uint32_t swizzle = (tile_row & 7u) * 16u;
     const uint32_t lane_base = (quarter * 32u) << 16;     // lane field of this warp's tensor-memory addresses
     bool ok = true;
     // the two group scales of this warp's k-blocks, fetched one group ahead (one 4-byte load where aligned)
-    const bool pair_ok = groups % 2u == 0u && ((uintptr_t)p.scale[source] & 3u) == 0;
+    const bool pair_ok = groups % 2u == 0u && ((uintptr_t)(kSegments ? own_scale : p.scale[source]) & 3u) == 0;
     auto load_scales = [&](uint32_t group) -> __half2 {
       const uint32_t first = kb_begin + group * kGroupBlocks + 2u * duo;
       if (!row_present || first >= groups) return __float2half2_rn(0.0f);
@@ -307,7 +332,7 @@ w4a16_gemm_tc_batch_kernel(const __grid_constant__ CUtensorMap map_x, const Batc
     // row's group) that it converts, four lanes per row, eight rows per instruction.
     const uint32_t copy_row = lane >> 2, copy_chunk = 4u * duo + (lane & 3u);
     const uint32_t row_bytes = p.k / 2, my_groups = (k_blocks + kGroupBlocks - 1u) / kGroupBlocks;
-    const uint8_t* packed = p.packed[source];
+    const uint8_t* packed = kSegments ? own_packed : p.packed[source];
     auto issue_group = [&](uint32_t group) {
       if (group < my_groups) {
         const uint32_t stage = base + L::kOffsetRaw + (group % kRawStages) * L::kRawTile + matrix * (kRows * L::kRowPitch);
@@ -316,7 +341,7 @@ w4a16_gemm_tc_batch_kernel(const __grid_constant__ CUtensorMap map_x, const Batc
 #pragma unroll
         for (uint32_t pass = 0; pass < 4; ++pass) {
           const uint32_t row = quarter * 32u + pass * 8u + copy_row;
-          const uint32_t source_row = min(tile_first_row + row_in_source(row), p.n - 1u);  // absent rows re-read the last one
+          const uint32_t source_row = min(tile_first_row + row_in_source(row), n - 1u);  // absent rows re-read the last one
           const uint8_t* from = packed + (size_t)source_row * row_bytes + (bytes ? byte_at : 0u);
           const uint32_t target = stage + row * L::kRowPitch + ((copy_chunk ^ (row & 7u)) * 16u);
           asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(target), "l"(from), "r"(bytes) : "memory");
@@ -386,6 +411,26 @@ w4a16_gemm_tc_batch_kernel(const __grid_constant__ CUtensorMap map_x, const Batc
 
     // epilogue: a thread owns weight row (lane quarter * 32 + lane) = one output column, and half of
     // the batch columns; lanes of a warp are consecutive output columns, so stores coalesce per batch row
+    constexpr int kHalf = NB / 4;       // batch columns per thread (the four warps of a lane quarter split them)
+    constexpr int kPiece = kHalf < 16 ? kHalf : 16;  // columns handled at a time
+    constexpr int kPieces = kHalf / kPiece;
+    constexpr int kWritten = EPI == kBatchLinearPair ? 2 : 1;  // the pair form writes both of its tiles
+    const uint32_t half_index = sub;
+    // Bias or residual of a piece, requested together and a piece ahead of their use: read one by one beside the stores (which
+    // they may alias, so the compiler keeps their order) 64 of them took 9 us of a CTA's life.
+    __half extra[kWritten][kPiece];
+    auto fetch_extra = [&](int piece) {
+      if (EPI != kBatchLinear && EPI != kBatchLinearPair) return;
+#pragma unroll
+      for (int a = 0; a < kWritten; ++a)
+#pragma unroll
+        for (int i = 0; i < kPiece; ++i) {
+          const uint32_t column = n0 + a * kRows + tile_row, batch_row = token0 + half_index * kHalf + piece * kPiece + i;
+          extra[a][i] = p.has_aux && column < n && batch_row < p.m ? p.aux[(size_t)batch_row * p.aux_row_stride + column]
+                                                                   : __float2half(0.0f);
+        }
+    };
+    fetch_extra(0);
     ok = ok && !*abort_flag && barrier_wait(accumulator_full, 0u);
     if (!ok) give_up();
     {
@@ -402,10 +447,6 @@ w4a16_gemm_tc_batch_kernel(const __grid_constant__ CUtensorMap map_x, const Batc
     }
     if (ok) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      constexpr int kHalf = NB / 4;       // batch columns per thread (the four warps of a lane quarter split them)
-      constexpr int kPiece = kHalf < 16 ? kHalf : 16;  // columns handled at a time
-      constexpr int kPieces = kHalf / kPiece;
-      const uint32_t half_index = sub;
       const uint32_t lane_address = tmem_base + lane_base + half_index * kHalf;
       constexpr int kPerTile = NMAT * kRows * NB;
       auto load_piece = [&](int piece, float (&values)[NMAT][kPiece]) {
@@ -430,45 +471,47 @@ w4a16_gemm_tc_batch_kernel(const __grid_constant__ CUtensorMap map_x, const Batc
           for (int i = 0; i < kPiece; ++i) values[a][i] = __uint_as_float(bits[i]);
         }
       };
-      auto write_piece = [&](int piece, const float (&values)[NMAT][kPiece]) {
+      auto write_piece = [&](int piece, float (&values)[NMAT][kPiece]) {
+        if (p.has_aux && EPI != kBatchDualSwiglu) {
 #pragma unroll
-        for (int a = 0; a < (EPI == kBatchLinearPair ? 2 : 1); ++a) {  // the pair form writes both of its tiles
-          const uint32_t column = n0 + a * kRows + tile_row;           // output column
-          if (column >= p.n) continue;
+          for (int a = 0; a < kWritten; ++a)
+#pragma unroll
+            for (int i = 0; i < kPiece; ++i) values[a][i] += __half2float(extra[a][i]);
+          if (piece + 1 < kPieces) fetch_extra(piece + 1);
+        }
+#pragma unroll
+        for (int a = 0; a < kWritten; ++a) {
+          const uint32_t column = n0 + a * kRows + tile_row;  // output column
+          if (column >= n) continue;
 #pragma unroll
           for (int i = 0; i < kPiece; ++i) {
             const uint32_t batch_row = token0 + half_index * kHalf + piece * kPiece + i;
             if (batch_row >= p.m) break;
-            float value;
-            if (EPI == kBatchDualSwiglu) {
-              const float g = values[0][i];
-              value = (g / (1.0f + __expf(-g))) * values[NMAT - 1][i];  // lib/metal_w4a16_source.ml:571-575
-            } else {
-              value = values[a][i];
-              if (p.has_aux) value += __half2float(p.aux[(size_t)batch_row * p.aux_row_stride + column]);
-            }
+            float value = values[a][i];
+            if (EPI == kBatchDualSwiglu)
+              value = (value / (1.0f + __expf(-value))) * values[NMAT - 1][i];  // lib/metal_w4a16_source.ml:571-575
             if (EPI != kBatchDualSwiglu && p.out_f32 != nullptr)
-              p.out_f32[(size_t)batch_row * p.n + column] = value;  // unrounded partial sum of a row-split product
+              p.out_f32[(size_t)batch_row * n + column] = value;  // unrounded partial sum of a row-split product
             else
-              p.out[(size_t)batch_row * p.n + column] = __float2half_rn(value);
+              out[(size_t)batch_row * n + column] = __float2half_rn(value);
           }
         }
       };
       // stacked gate/up form: the finished values meet in shared memory ([token][tile row], the rings are idle by now)
       float* stash = reinterpret_cast<float*>(base_pointer + L::kOffsetX);
       static_assert(!kStacked || NB * kRows * 4 <= L::kXStages * L::kXStage, "the stash must fit the X ring");
-      auto emit = [&](int piece, const float (&values)[NMAT][kPiece]) {
+      auto emit = [&](int piece, float (&values)[NMAT][kPiece]) {
         if (EPI == kBatchSplitF32) {
           // this thread's 16 columns are two slot tiles: token 4 t + w = column 8 t + w (hi) + column 8 t + 4 + w (lo)
           static_assert(EPI != kBatchSplitF32 || kPiece == 16, "hi and lo of a token must sit in one thread's piece");
           const uint32_t column = n0 + tile_row;
-          if (column < p.n) {
+          if (column < n) {
 #pragma unroll
             for (int t = 0; t < kPiece / 8; ++t)
 #pragma unroll
               for (int w = 0; w < 4; ++w) {
                 const uint32_t token = (half_index * kHalf + piece * kPiece) / 2 + 4 * t + w;
-                if (token < p.m) p.out_f32[(size_t)token * p.n + column] = values[0][8 * t + w] + values[0][8 * t + 4 + w];
+                if (token < p.m) p.out_f32[(size_t)token * n + column] = values[0][8 * t + w] + values[0][8 * t + 4 + w];
               }
           }
         } else if (kStacked) {
@@ -489,6 +532,9 @@ w4a16_gemm_tc_batch_kernel(const __grid_constant__ CUtensorMap map_x, const Batc
       } else {
         // park, count, and go on only as the last split of this tile
         float* mine = p.partials + ((size_t)tile_id * p.splits + split) * kPerTile;
+        // four batch columns of a row; the warp's rows are 512 contiguous bytes (a row's columns side by side make every
+        // access of the warp touch 32 lines: 1024 x 4608, 333 rows, four splits of 256 tokens 70 us instead of 33)
+        auto parked = [&](int a, int column) { return (((size_t)a * (NB / 4) + column / 4) * kRows + tile_row) * 4; };
 #pragma unroll 1
         for (int piece = 0; piece < kPieces; ++piece) {
           float values[NMAT][kPiece];
@@ -497,8 +543,7 @@ w4a16_gemm_tc_batch_kernel(const __grid_constant__ CUtensorMap map_x, const Batc
           for (int a = 0; a < NMAT; ++a)
 #pragma unroll
             for (int i = 0; i < kPiece / 4; ++i)
-              *reinterpret_cast<float4*>(mine + ((size_t)a * kRows + tile_row) * NB + half_index * kHalf + piece * kPiece +
-                                         4 * i) =
+              *reinterpret_cast<float4*>(mine + parked(a, half_index * kHalf + piece * kPiece + 4 * i)) =
                   make_float4(values[a][4 * i], values[a][4 * i + 1], values[a][4 * i + 2], values[a][4 * i + 3]);
         }
         asm volatile("bar.sync 1, 512;" ::: "memory");
@@ -527,8 +572,7 @@ w4a16_gemm_tc_batch_kernel(const __grid_constant__ CUtensorMap map_x, const Batc
 #pragma unroll
                 for (int i = 0; i < kPiece / 4; ++i) {
                   const float4 part = __ldcg(reinterpret_cast<const float4*>(
-                      parts + (size_t)s * kPerTile + ((size_t)a * kRows + tile_row) * NB + half_index * kHalf +
-                      piece * kPiece + 4 * i));
+                      parts + (size_t)s * kPerTile + parked(a, half_index * kHalf + piece * kPiece + 4 * i)));
                   values[a][4 * i] += part.x;
                   values[a][4 * i + 1] += part.y;
                   values[a][4 * i + 2] += part.z;
@@ -545,9 +589,9 @@ w4a16_gemm_tc_batch_kernel(const __grid_constant__ CUtensorMap map_x, const Batc
         for (uint32_t index = first; index < (kRows / 2) * NB; index += kConvertWarps * 32) {
           const uint32_t token = index / (kRows / 2), local = index % (kRows / 2);
           const uint32_t batch_row = token0 + token, column = n0 + local;
-          if (batch_row >= p.m || column >= p.n) continue;
+          if (batch_row >= p.m || column >= n) continue;
           const float g = stash[token * kRows + local], u = stash[token * kRows + kRows / 2 + local];
-          p.out[(size_t)batch_row * p.n + column] = __float2half_rn((g / (1.0f + __expf(-g))) * u);  // lib/metal_w4a16_source.ml:571-575
+          out[(size_t)batch_row * n + column] = __float2half_rn((g / (1.0f + __expf(-g))) * u);  // lib/metal_w4a16_source.ml:571-575
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -577,6 +621,15 @@ EncodeTiled encode_tiled() {
   return function;
 }
 
+// How many CTAs share a tile's k: one CTA per SM at most (a second wave would double the time); each split keeps at least two
+// groups of k-blocks.
+uint32_t batch_splits(uint32_t sms, uint32_t tiles, uint32_t groups) {
+  uint32_t splits = tiles < 1u ? 1u : sms / tiles;
+  if (splits > groups / 2u) splits = groups / 2u;
+  if (splits > 16u) splits = 16u;
+  return splits < 1u || tiles > kSplitCounterTiles ? 1u : splits;
+}
+
 template <int EPI, int NB, bool AFFINE = false>
 int run_batch(const KernelArgs& args, const CUtensorMap& map_x, BatchProblem p) {
   constexpr int NMAT = (EPI == kBatchLinear || EPI == kBatchDualStacked || EPI == kBatchSplitF32) ? 1 : 2;
@@ -587,14 +640,15 @@ int run_batch(const KernelArgs& args, const CUtensorMap& map_x, BatchProblem p) 
     cudaGetLastError();
     return -1;
   }
-  const uint32_t tiles = (p.n + kTileRows - 1) / kTileRows, row_tiles = (p.m + NB - 1) / NB;
+  uint32_t tiles = (p.n + kTileRows - 1) / kTileRows;
+  for (uint32_t i = 0; i < p.segments; ++i) {
+    p.segment[i].first = tiles;
+    tiles += (p.segment[i].n + kTileRows - 1) / kTileRows;
+  }
+  const uint32_t row_tiles = (p.m + NB - 1) / NB;
   const uint32_t sms = (uint32_t)context_sm_count(args.ctx);
   const uint32_t groups = (p.k / kBK + L::kGroupBlocks - 1u) / L::kGroupBlocks;
-  // one CTA per SM at most (a second wave would double the time); each split keeps at least two groups
-  uint32_t splits = sms / (tiles * row_tiles);
-  if (splits > groups / 2u) splits = groups / 2u;
-  if (splits > 16u) splits = 16u;
-  if (splits < 1u || tiles * row_tiles > kSplitCounterTiles) splits = 1u;
+  const uint32_t splits = batch_splits(sms, tiles * row_tiles, groups);
   p.splits = splits;
   if (splits > 1u) {
     constexpr size_t counter_bytes = kSplitCounterTiles * sizeof(uint32_t);
@@ -639,7 +693,7 @@ uint32_t tensor_core_batch_max_rows() {
   return rows;
 }
 
-// Prompts (more than 64 rows) on this kernel: 128-row activation tiles, two weight tiles per CTA.
+// Prompts (more than 64 rows) on this kernel.
 // LLMOPT_CUDA_TC_PROMPT_TMEM=0 sends them to the shared-memory-operand GEMM instead.
 static bool prompt_rows_enabled() {
   static const bool enabled = []() {
@@ -647,6 +701,36 @@ static bool prompt_rows_enabled() {
     return text == nullptr || text[0] != '0';
   }();
   return enabled;
+}
+
+// Tokens per tile of a prompt: the width with the shortest estimate, waves x (start and writeback + k-blocks x time of one) +
+// the adding of splits.  A tile of 256 tokens runs the MMA at its full rate (narrower ones cost three quarters of that for half the
+// work or less), but its k-block and its writeback take longer, and few wide tiles leave SMs idle: 1024 x 1024 for 333 tokens is
+// 16 tiles of 256 (15.5 us) or 48 of 64 (10.2 us), 4096 x 14336 for 2048 tokens 208 us against 488.  The constants (us) are fitted
+// to back-to-back launches at N and K from 576 to 14336 and 72 to 2048 rows; the choice is within 6 % of the best of the four at
+// each of them.
+static uint32_t prompt_tile(const KernelArgs& args, uint32_t m, uint32_t weight_tiles, uint32_t k, bool dual) {
+  struct Width {
+    uint32_t tokens;
+    float start, block, adding;
+  };
+  static const Width kLinear[] = {{32, 5.2f, 0.285f, 2.3f}, {64, 5.4f, 0.29f, 2.8f}, {128, 6.5f, 0.295f, 3.9f}, {256, 7.3f, 0.45f, 6.4f}};
+  // gate and up: two weight tiles of 128 rows beside each other, or 64 rows of each stacked in one tile (twice as many tiles)
+  static const Width kDual[] = {{128, 6.5f, 0.51f, 7.0f}, {256, 7.3f, 0.40f, 6.4f}};
+  const Width* const widths = dual ? kDual : kLinear;
+  const uint32_t sms = (uint32_t)context_sm_count(args.ctx), blocks = k / kBK;
+  uint32_t best = 256u;
+  float shortest = 0.0f;
+  for (uint32_t i = 0; i < (dual ? 2u : 4u); ++i) {
+    const Width& w = widths[i];
+    const uint32_t group = dual && w.tokens == 128u ? 4u : 8u;
+    const uint32_t tiles = weight_tiles * (dual && w.tokens == 256u ? 2u : 1u) * ((m + w.tokens - 1u) / w.tokens);
+    const uint32_t splits = batch_splits(sms, tiles, (blocks + group - 1u) / group);
+    const float time = (float)((tiles * splits + sms - 1u) / sms) * (w.start + (float)blocks / (float)splits * w.block) +
+                       (splits > 1u ? w.adding : 0.0f);
+    if (shortest == 0.0f || time < shortest) best = w.tokens, shortest = time;
+  }
+  return best;
 }
 
 // Decode batches (up to 64 rows) and prompts; returns -1 outside its domain (the caller falls back).
@@ -662,18 +746,7 @@ int launch_w4a16_gemm_tc_batch(const KernelArgs& args, const GemvProblem& proble
   if (problem.m <= 32 && !forced &&
       (epilogue == kEpiQkv || (uint64_t)problem.mat[0].n * problem.k < (24ull << 20)))
     return -1;
-  if (epilogue == kEpiQkv) {
-    for (uint32_t i = 0; i < problem.matrices; ++i) {
-      GemvProblem one = problem;
-      one.mat[0] = problem.mat[i];
-      one.matrices = 1;
-      one.out[0] = problem.out[i];
-      one.has_aux = 0;
-      const int status = launch_w4a16_gemm_tc_batch(args, one, kEpiLinear, false);
-      if (status != 0) return i == 0 ? status : (status < 0 ? 1 : status);
-    }
-    return 0;
-  }
+  if (epilogue == kEpiQkv && (problem.matrices > 3 || problem.has_aux)) return -1;
   if (epilogue == kEpiSplitF32) {
     // the LM head's hi/lo rows: 17..32 rows = up to 64 slot rows, one launch instead of two 16-row passes
     if (affine || prompt || problem.m > 32 || problem.x_rows > 64 || problem.x_rows % 8 != 0 || problem.out_f32 == nullptr ||
@@ -699,21 +772,25 @@ int launch_w4a16_gemm_tc_batch(const KernelArgs& args, const GemvProblem& proble
     p.out_f32 = problem.out_f32;
     return run_batch<kBatchSplitF32, 64>(args, map_x, p);
   }
-  if (epilogue != kEpiLinear && epilogue != kEpiDualSwiglu) return -1;
+  const bool qkv = epilogue == kEpiQkv;
+  if (epilogue != kEpiLinear && epilogue != kEpiDualSwiglu && !qkv) return -1;
+  if (qkv && affine) return -1;
   if (problem.out_f32 != nullptr && (epilogue != kEpiLinear || problem.has_aux)) return -1;
   // the zero-point form: plain products of prompts only (what the shared-memory-operand GEMM covered)
   if (affine && (epilogue != kEpiLinear || !prompt || problem.mat[0].zero == nullptr)) return -1;
-  const uint32_t matrices = epilogue == kEpiDualSwiglu ? 2u : 1u;
+  const uint32_t matrices = epilogue == kEpiDualSwiglu ? 2u : qkv ? problem.matrices : 1u;
   if (((uintptr_t)problem.x & 15u) != 0 || (problem.k / 2) % 16 != 0) return -1;
   for (uint32_t i = 0; i < matrices; ++i)
-    if (((uintptr_t)problem.mat[i].packed & 15u) != 0 || problem.mat[i].n != problem.mat[0].n) return -1;
+    if (((uintptr_t)problem.mat[i].packed & 15u) != 0 || (!qkv && problem.mat[i].n != problem.mat[0].n)) return -1;
   EncodeTiled encode = encode_tiled();
   if (encode == nullptr) return -1;
-  // prompts of 256 rows and more: 256-token tiles (an MMA with N = 256 runs at the tensor pipe's full rate,
-  // narrower ones cost three quarters of that for half the work); LLMOPT_CUDA_TC_PROMPT_WIDE=0 keeps 128
   static const bool wide_prompts = getenv("LLMOPT_CUDA_TC_PROMPT_WIDE") == nullptr || getenv("LLMOPT_CUDA_TC_PROMPT_WIDE")[0] != '0';
-  const bool wide = prompt && wide_prompts && problem.m >= 256;
-  const uint32_t padded = wide ? 256u : prompt ? 128u : problem.m <= 16 ? 16u : problem.m <= 32 ? 32u : 64u;
+  uint32_t weight_tiles = 0;  // of all matrices with the same input
+  for (uint32_t i = 0; i < (qkv ? matrices : 1u); ++i) weight_tiles += (problem.mat[i].n + kRows - 1u) / kRows;
+  const uint32_t padded = prompt ? !wide_prompts ? 128u
+                                   : affine      ? (problem.m >= 256u ? 256u : 128u)
+                                                 : prompt_tile(args, problem.m, weight_tiles, problem.k, epilogue == kEpiDualSwiglu)
+                                 : problem.m <= 16 ? 16u : problem.m <= 32 ? 32u : 64u;
   CUtensorMap map_x;
   const cuuint64_t dims[2] = {problem.k, problem.m};
   const cuuint64_t strides[1] = {(cuuint64_t)problem.k * 2};
@@ -728,24 +805,25 @@ int launch_w4a16_gemm_tc_batch(const KernelArgs& args, const GemvProblem& proble
   p.n = problem.mat[0].n;
   p.k = problem.k;
   for (uint32_t i = 0; i < 2; ++i) {
-    p.packed[i] = problem.mat[i < matrices ? i : 0].packed;
-    p.scale[i] = problem.mat[i < matrices ? i : 0].scale;
-    p.zero[i] = problem.mat[i < matrices ? i : 0].zero;
+    p.packed[i] = problem.mat[i < matrices && !qkv ? i : 0].packed;
+    p.scale[i] = problem.mat[i < matrices && !qkv ? i : 0].scale;
+    p.zero[i] = problem.mat[i < matrices && !qkv ? i : 0].zero;
   }
+  for (uint32_t i = 1; qkv && i < matrices; ++i)
+    p.segment[p.segments++] = BatchSegment{0u, problem.mat[i].n, problem.mat[i].packed, problem.mat[i].scale, problem.out[i]};
   p.out = problem.out[0];
   p.out_f32 = problem.out_f32;
   p.aux = problem.aux0;
   p.aux_row_stride = problem.aux_row_stride;
   p.has_aux = problem.has_aux;
-  if (prompt) {
+  if (prompt && padded >= 128u) {
     if (epilogue == kEpiDualSwiglu)
       return padded == 256 ? run_batch<kBatchDualStacked, 256>(args, map_x, p) : run_batch<kBatchDualSwiglu, 128>(args, map_x, p);
     if (affine) {
       if (padded == 256) return run_batch<kBatchLinear, 256, true>(args, map_x, p);
       return p.n > kRows ? run_batch<kBatchLinearPair, 128, true>(args, map_x, p) : run_batch<kBatchLinear, 128, true>(args, map_x, p);
     }
-    if (padded == 256) return run_batch<kBatchLinear, 256>(args, map_x, p);
-    return p.n > kRows ? run_batch<kBatchLinearPair, 128>(args, map_x, p) : run_batch<kBatchLinear, 128>(args, map_x, p);
+    return padded == 256 ? run_batch<kBatchLinear, 256>(args, map_x, p) : run_batch<kBatchLinear, 128>(args, map_x, p);
   }
   if (epilogue == kEpiDualSwiglu) {
     switch (padded) {

@@ -100,3 +100,36 @@ def test_dense_fp32(runtime, m, n, k):
         runtime.dispatch("llmopt_dense_linear_f32", buffers=buffers, parameters=parameters.dense_linear(
             m=m, n=n, k=k, split=n, has_bias=True, epilogue="silu_pair"))
         close(download(buffers[3], (m, n // 2)), plain.silu(y[:, 0::2]) * y[:, 1::2], 6e-6)
+
+
+@pytest.mark.parametrize("m,k,columns", [(66, 192, (40,)), (257, 1024, (300,)), (300, 4608, (130,)), (700, 512, (1100,)),
+                                         (2049, 64, (129,)), (40, 128, (130, 70, 64)), (72, 576, (576, 192, 192)),
+                                         (300, 1024, (129, 512, 1)), (513, 320, (200, 60, 1000))])
+def test_prompt_tiles_and_fused_projections(runtime, oracle, m, k, columns):
+    """Every width of a prompt's tiles, with and without splits of k, with the residual read ahead; three matrices of unequal
+    sizes as one launch.  The parity bound of the product, 2e-3 of the outputs' scale."""
+    from conftest import assert_close_f16
+    from helpers import random_w4
+    from llmopt_b200 import dispatch
+    from llmopt_b200.cuda_native import Buffer
+
+    rng = np.random.default_rng(m)
+    x = rng.standard_normal((m, k)).astype(np.float16)
+    matrices = [random_w4(rng, n, k) for n in columns]
+    upload_tensor = lambda array, kind="float16": dispatch.Tensor(Buffer.of_array(runtime, array), array.shape, kind)
+    weights = [(upload_tensor(packed, "uint8"), upload_tensor(scale)) for packed, scale in matrices]
+    outputs = [upload_tensor(np.full((m, n), np.nan, np.float16)) for n in columns]
+    context = dispatch.Context(runtime)
+    if len(columns) == 1:
+        residual = rng.standard_normal((m, columns[0])).astype(np.float16)
+        dispatch.dispatch_w4a16_linear(context, input=upload_tensor(x), weight=weights[0][0], scale=weights[0][1],
+                                       output=outputs[0], bias=upload_tensor(residual), bias_row_stride=columns[0])
+        wanted = [oracle.w4a16_linear(x, *matrices[0], residual, columns[0])]
+    else:
+        (q, k_, v) = weights
+        dispatch.dispatch_w4a16_qkv_linear_command(
+            context, input=upload_tensor(x), q_weight=q[0], q_scale=q[1], k_weight=k_[0], k_scale=k_[1], v_weight=v[0], v_scale=v[1],
+            q_output=outputs[0], k_output=outputs[1], v_output=outputs[2])
+        wanted = [oracle.w4a16_linear(x, *pair) for pair in matrices]
+    for output, want in zip(outputs, wanted):
+        assert_close_f16(output.buffer.to_numpy(np.float16, want.shape), want)
