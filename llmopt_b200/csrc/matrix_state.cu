@@ -12,7 +12,7 @@
 // columns, because every slice's CTA needs them and keeps a copy of its own.  A sequence with nothing
 // behind it (past = 0) starts from zero whatever its pool row holds.
 //
-// Scan: a CTA owns kSlice value columns of one head of one sequence and walks over the tokens.  Sixteen lanes
+// Scan: a CTA owns some value columns of one head of one sequence and walks over the tokens.  Sixteen lanes
 // share two columns of S (each lane dim / 16 rows of them, in registers).  Compute warps work on a chunk of tokens in
 // shared memory while producer warps bring in the next chunk (converted to fp32, with the per-token
 // scalars) and write out the previous one's results.  The read-out of the delta rule uses
@@ -28,7 +28,13 @@ constexpr uint32_t kSlice = 32;   // value columns per CTA
 constexpr uint32_t kLanes = 16;   // lanes per column
 constexpr uint32_t kColumns = 2;  // columns per thread
 constexpr uint32_t kColumnWarps = kSlice / kColumns * kLanes / 32;  // 4
-constexpr uint32_t kProducerWarps = 4;
+
+// Columns per CTA of a scan.  The delta rule is bound by a chain per token (a sum over the lanes of a column, then the
+// update), behind which twice the columns hide: 395 us for 2048 tokens and 16 heads of 128 columns, 435 with half a slice.
+// The matrix memory has no such chain and gains from twice the CTAs: 269 us for 8 heads of 256 columns, 344 with a whole
+// slice.  While the producers waited for their loads within each chunk the two took 470 and 349 us.
+template <bool MEMORY> __host__ __device__ constexpr uint32_t scan_columns() { return MEMORY ? kSlice / 2u : kSlice; }
+constexpr uint32_t kLoaderWarps = 8;  // bring in q, k and v and write out; one more warp prepares the tokens' scalars
 
 __host__ __device__ constexpr uint32_t slices_of(uint32_t vdim) { return (vdim + kSlice - 1u) / kSlice; }
 
@@ -318,11 +324,11 @@ struct StateRow {
 };
 
 // One chunk's inputs and results in shared memory.
-template <int R4, int CHUNK>
+template <int R4, int CHUNK, uint32_t COLUMNS>
 struct ScanChunk {
   float q[CHUNK][R4 * kLanes * 4], k[CHUNK][R4 * kLanes * 4];
-  float v[CHUNK][kSlice];
-  float out[CHUNK][kSlice];
+  float v[CHUNK][COLUMNS];
+  float out[CHUNK][COLUMNS];
   float4 scalar[CHUNK];   // delta: decay, beta, k . q; memory: keep, write, exp(-m)
   float norm_dot[CHUNK];  // memory: n . q
 };
@@ -332,8 +338,9 @@ struct ScanChunk {
 template <int CHUNK> struct ScanGroup { static constexpr uint32_t kTokens = CHUNK >= 8 ? 4 : 1; };
 
 template <bool MEMORY> struct ScanThreads {
-  static constexpr uint32_t kCompute = (kColumnWarps + (MEMORY ? 1u : 0u)) * 32u;  // one more warp carries n
-  static constexpr uint32_t kAll = kCompute + kProducerWarps * 32u;
+  static constexpr uint32_t kCompute = (scan_columns<MEMORY>() / kColumns * kLanes / 32u + (MEMORY ? 1u : 0u)) * 32u;  // one more warp carries n
+  static constexpr uint32_t kProducers = (kLoaderWarps + 1u) * 32u;
+  static constexpr uint32_t kAll = kCompute + kProducers;
 };
 
 // Two fp32 numbers in one register pair (Blackwell's packed fp32 arithmetic).
@@ -423,146 +430,159 @@ __global__ void __launch_bounds__(ScanThreads<MEMORY>::kAll) scan_kernel(const T
                                                                          ScanParams p) {
   grid_chain_prologue();
   extern __shared__ __align__(16) unsigned char scan_shared[];
-  typedef ScanChunk<R4, CHUNK> Chunk;
+  constexpr uint32_t kScanColumns = scan_columns<MEMORY>();
+  typedef ScanChunk<R4, CHUNK, kScanColumns> Chunk;
   Chunk* chunks = reinterpret_cast<Chunk*>(scan_shared);
   constexpr uint32_t kCompute = ScanThreads<MEMORY>::kCompute;
-  const uint32_t slice = blockIdx.x, head = blockIdx.y, sequence = blockIdx.z;
+  const uint32_t first_column = blockIdx.x * kScanColumns, head = blockIdx.y, sequence = blockIdx.z;
+  const uint32_t slice = first_column / kSlice;
+  const bool owner = first_column % kSlice == 0;  // stores the slice's n and m
   const uint32_t kv_head = head / (p.heads / p.kv_heads);
   const size_t row0 = (size_t)sequence * p.tokens;
   const bool fresh = past[sequence] == 0;
   float* state = state_pool + (size_t)min(sequence_rows[sequence], p.state_rows - 1u) * p.state_stride;
   const StateRow layout = {p.heads, p.dim, p.vdim};
   const uint32_t chunk_count = (p.tokens + CHUNK - 1u) / CHUNK;
+  // The CTAs of a slice start from the same n and m, which one of them stores at the end: all have read them by then.
+  auto ready = [] {
+    if (MEMORY) cluster_sync();
+    else __syncthreads();
+  };
 
   if (threadIdx.x >= kCompute) {
     // ------------------------------ producers ------------------------------
+    // What a chunk needs is requested while the one before it is stored to shared memory.
     const uint32_t thread = threadIdx.x - kCompute, warp = thread >> 5, lane = thread & 31u;
+    const bool loader = warp < kLoaderWarps;
     const float q_scale = MEMORY ? 1.0f / sqrtf((float)p.dim) : 1.0f;
-    float top = 0.0f;  // memory form: running maximum (warp 0)
-    if (MEMORY && !fresh) top = state[layout.top(head, slice)];
-    const uint32_t value_column = slice * kSlice + lane;
+    float top = 0.0f;  // memory form: running maximum (scalar warp)
+    if (MEMORY && !loader && !fresh) top = state[layout.top(head, slice)];
+    const uint32_t value_column = first_column + lane % kScanColumns;
+    constexpr int kSteps = R4 * (int)kLanes / 8;  // 32-wide pieces of a row
+    constexpr uint32_t kBatch = CHUNK >= kLoaderWarps ? CHUNK / kLoaderWarps : 1;  // tokens per warp and chunk
+    constexpr uint32_t kGroup = ScanGroup<CHUNK>::kTokens;
+    TQ q_raw[kBatch][kSteps], k_raw[kBatch][kSteps], v_raw[kBatch];
+    float first_raw = 0.0f, second_raw = 0.0f;
+    auto request = [&](uint32_t index) {
+      const uint32_t t0 = index * CHUNK, count = min((uint32_t)CHUNK, p.tokens - t0);
+      if (!loader) {
+        const size_t scalar_row = (row0 + t0 + min(lane, count - 1u)) * p.scalar_stride;
+        first_raw = first[scalar_row + p.first_column + head];
+        second_raw = second[scalar_row + p.second_column + head];
+        return;
+      }
+      // loads without branches (absent elements read a present one), so that all of them are in flight at once
+#pragma unroll
+      for (uint32_t b = 0; b < kBatch; ++b) {
+        const size_t row = row0 + t0 + min(warp + b * kLoaderWarps, count - 1u);
+        const TQ* q = query + row * p.q_stride + p.q_column + kv_head * p.dim;
+        const TQ* k = key + row * p.k_stride + p.k_column + kv_head * p.dim;
+#pragma unroll
+        for (int i = 0; i < kSteps; ++i) {
+          const uint32_t c = min(lane + i * 32u, p.dim - 1u);
+          q_raw[b][i] = q[c];
+          k_raw[b][i] = k[c];
+        }
+        v_raw[b] = value[row * p.v_stride + p.v_column + head * p.vdim + min(value_column, p.vdim - 1u)];
+      }
+    };
     auto produce = [&](uint32_t index) {
       Chunk& chunk = chunks[index & 1u];
-      const uint32_t t0 = index * CHUNK, count = min((uint32_t)CHUNK, p.tokens - t0);
-      constexpr int kSteps = R4 * (int)kLanes / 8;  // 32-wide pieces of a row
-      constexpr uint32_t kBatch = kSteps <= 4 ? 4 : 2;  // tokens whose loads are in flight together
-      constexpr uint32_t kGroup = ScanGroup<CHUNK>::kTokens;
+      const uint32_t count = min((uint32_t)CHUNK, p.tokens - index * CHUNK);
       const uint32_t padded = (count + kGroup - 1u) / kGroup * kGroup;
-      for (uint32_t begin = warp; begin < padded; begin += kProducerWarps * kBatch) {
-        // loads without branches (absent elements read a present one), so that all of them are in flight at once
-        TQ q_raw[kBatch][kSteps], k_raw[kBatch][kSteps], v_raw[kBatch];
+      if (loader) {
 #pragma unroll
         for (uint32_t b = 0; b < kBatch; ++b) {
-          const size_t row = row0 + t0 + min(begin + b * kProducerWarps, count - 1u);
-          const TQ* q = query + row * p.q_stride + p.q_column + kv_head * p.dim;
-          const TQ* k = key + row * p.k_stride + p.k_column + kv_head * p.dim;
-#pragma unroll
-          for (int i = 0; i < kSteps; ++i) {
-            const uint32_t c = min(lane + i * 32u, p.dim - 1u);
-            q_raw[b][i] = q[c];
-            k_raw[b][i] = k[c];
-          }
-          v_raw[b] = value[row * p.v_stride + p.v_column + head * p.vdim + min(value_column, p.vdim - 1u)];
-        }
-        float qs[kBatch][kSteps], ks[kBatch][kSteps], vs[kBatch];
-#pragma unroll
-        for (uint32_t b = 0; b < kBatch; ++b) {
-#pragma unroll
-          for (int i = 0; i < kSteps; ++i) {
-            const bool present = lane + i * 32u < p.dim && begin + b * kProducerWarps < count;
-            qs[b][i] = present ? as_float(q_raw[b][i]) * q_scale : 0.0f;
-            ks[b][i] = present ? as_float(k_raw[b][i]) : 0.0f;
-          }
-          vs[b] = value_column < p.vdim ? as_float(v_raw[b]) : 0.0f;
-        }
-#pragma unroll
-        for (uint32_t b = 0; b < kBatch; ++b) {
-          const uint32_t t = begin + b * kProducerWarps;
+          const uint32_t t = warp + b * kLoaderWarps;
           if (t >= padded) break;
           float dot = 0.0f;
 #pragma unroll
           for (int i = 0; i < kSteps; ++i) {
-            chunk.q[t][lane + i * 32u] = qs[b][i];
-            chunk.k[t][lane + i * 32u] = ks[b][i];
-            dot = fmaf(qs[b][i], ks[b][i], dot);
+            const bool present = lane + i * 32u < p.dim && t < count;
+            const float q = present ? as_float(q_raw[b][i]) * q_scale : 0.0f, k = present ? as_float(k_raw[b][i]) : 0.0f;
+            chunk.q[t][lane + i * 32u] = q;
+            chunk.k[t][lane + i * 32u] = k;
+            dot = fmaf(q, k, dot);
           }
-          chunk.v[t][lane] = vs[b];
+          if (lane < kScanColumns) chunk.v[t][lane] = value_column < p.vdim ? as_float(v_raw[b]) : 0.0f;
           if (!MEMORY) {
             dot = warp_sum(dot);
             if (lane == 0) chunk.scalar[t].z = dot;
           }
         }
+        return;
       }
-      if (warp == 0) {
-        const bool present = lane < count;
-        const size_t scalar_row = (row0 + t0 + (present ? lane : 0u)) * p.scalar_stride;
-        float a = present ? first[scalar_row + p.first_column + head] : 0.0f;
-        float b = present ? second[scalar_row + p.second_column + head] : 0.0f;
-        if (MEMORY) {
-          const float log_input = p.gate_cap * tanhf(a / p.gate_cap);
-          const float log_forget = -softplus_f32(-p.gate_cap * tanhf(b / p.gate_cap));
-          // m_t = max(f_t + m_(t-1), i_t): composition (f1, i1) then (f2, i2) = (f1 + f2, max(i1 + f2, i2))
-          float sum = present ? log_forget : 0.0f, best = present ? log_input : -INFINITY;
+      const bool present = lane < count;
+      float a = first_raw, b = second_raw;
+      if (MEMORY) {
+        const float log_input = p.gate_cap * tanhf(a / p.gate_cap);
+        const float log_forget = -softplus_f32(-p.gate_cap * tanhf(b / p.gate_cap));
+        // m_t = max(f_t + m_(t-1), i_t): composition (f1, i1) then (f2, i2) = (f1 + f2, max(i1 + f2, i2))
+        float sum = present ? log_forget : 0.0f, best = present ? log_input : -INFINITY;
 #pragma unroll
-          for (int offset = 1; offset < 32; offset <<= 1) {
-            const float earlier_sum = __shfl_up_sync(0xffffffffu, sum, offset);
-            const float earlier_best = __shfl_up_sync(0xffffffffu, best, offset);
-            if (lane >= (uint32_t)offset) {
-              best = fmaxf(earlier_best + sum, best);
-              sum += earlier_sum;
-            }
+        for (int offset = 1; offset < 32; offset <<= 1) {
+          const float earlier_sum = __shfl_up_sync(0xffffffffu, sum, offset);
+          const float earlier_best = __shfl_up_sync(0xffffffffu, best, offset);
+          if (lane >= (uint32_t)offset) {
+            best = fmaxf(earlier_best + sum, best);
+            sum += earlier_sum;
           }
-          const float m = fmaxf(sum + top, best);
-          float before = __shfl_up_sync(0xffffffffu, m, 1);
-          if (lane == 0) before = top;
-          a = expf(log_forget + before - m);
-          b = expf(log_input - m);
-          if (present) chunk.scalar[lane].z = expf(-m);
-          top = __shfl_sync(0xffffffffu, m, count - 1u);
         }
-        if (lane < padded) {
-          chunk.scalar[lane].x = present ? a : 1.0f;
-          chunk.scalar[lane].y = present ? b : 0.0f;
-        }
+        const float m = fmaxf(sum + top, best);
+        float before = __shfl_up_sync(0xffffffffu, m, 1);
+        if (lane == 0) before = top;
+        a = expf(log_forget + before - m);
+        b = expf(log_input - m);
+        if (present) chunk.scalar[lane].z = expf(-m);
+        top = __shfl_sync(0xffffffffu, m, count - 1u);
+      }
+      if (lane < padded) {
+        chunk.scalar[lane].x = present ? a : 1.0f;
+        chunk.scalar[lane].y = present ? b : 0.0f;
       }
     };
     auto write_out = [&](uint32_t index) {
       const Chunk& chunk = chunks[index & 1u];
       const uint32_t t0 = index * CHUNK, count = min((uint32_t)CHUNK, p.tokens - t0);
-      for (uint32_t t = warp; t < count; t += kProducerWarps) {
-        float o = chunk.out[t][lane];
+      if (!loader) return;
+      for (uint32_t t = thread / kScanColumns; t < count; t += kLoaderWarps * 32u / kScanColumns) {
+        float o = chunk.out[t][lane % kScanColumns];
         if (MEMORY) o /= fmaxf(fabsf(chunk.norm_dot[t]), chunk.scalar[t].z) + 1e-6f;
         if (value_column < p.vdim) out[((row0 + t0 + t) * p.heads + head) * p.vdim + value_column] = o;
       }
     };
+    request(0);
     produce(0);
-    __syncthreads();
+    if (chunk_count > 1u) request(1);
+    ready();
     for (uint32_t index = 0; index < chunk_count; ++index) {
       if (index > 0) {
-        write_out(index - 1u);  // before its buffer is filled again
-        asm volatile("bar.sync 1, %0;" ::"n"(kProducerWarps * 32) : "memory");
+        write_out(index - 1u);
+        // its scalars are filled again next
+        if (MEMORY) asm volatile("bar.sync 1, %0;" ::"n"(ScanThreads<MEMORY>::kProducers) : "memory");
       }
       if (index + 1u < chunk_count) produce(index + 1u);
+      if (index + 2u < chunk_count) request(index + 2u);
       __syncthreads();
     }
     write_out(chunk_count - 1u);
-    if (MEMORY && thread == 0) state[layout.top(head, slice)] = top;
+    if (MEMORY && owner && !loader && lane == 0) state[layout.top(head, slice)] = top;
   } else {
     // ------------------------------ state ------------------------------
     const uint32_t column0 = threadIdx.x / kLanes * kColumns, part = threadIdx.x % kLanes;
-    const bool is_norm = MEMORY && column0 >= kSlice;  // the extra warp: the first column of its first lanes carries n
+    const bool is_norm = MEMORY && column0 >= kScanColumns;  // the extra warp: the first column of its first lanes carries n
     StateColumns<R4> columns;
     auto& active = columns.active;
     auto& s = columns.s;
 #pragma unroll
     for (int j = 0; j < (int)kColumns; ++j) {
-      const uint32_t column = slice * kSlice + column0 + j;
-      active[j] = is_norm ? column0 + j == kSlice : column < p.vdim;
+      const uint32_t column = first_column + column0 + j;
+      active[j] = is_norm ? column0 + j == kScanColumns : column < p.vdim;
       columns.home[j] = state + (is_norm ? layout.norm(head, slice) : layout.matrix(head) + (size_t)(active[j] ? column : 0u) * p.dim);
     }
     const bool vectors = p.dim % 4u == 0 && p.state_stride % 4u == 0;
     columns.load(part, p.dim, vectors, fresh);
-    __syncthreads();
+    ready();
     for (uint32_t index = 0; index < chunk_count; ++index) {
       Chunk& chunk = chunks[index & 1u];
       const uint32_t count = min((uint32_t)CHUNK, p.tokens - index * CHUNK);
@@ -577,7 +597,7 @@ __global__ void __launch_bounds__(ScanThreads<MEMORY>::kAll) scan_kernel(const T
           const ulonglong2* q = reinterpret_cast<const ulonglong2*>(chunk.q[t]) + part;
           const ulonglong2* k = reinterpret_cast<const ulonglong2*>(chunk.k[t]) + part;
           const float4 scalar = chunk.scalar[t];
-          const float2 values = *reinterpret_cast<const float2*>(&chunk.v[t][column0 % kSlice]);
+          const float2 values = *reinterpret_cast<const float2*>(&chunk.v[t][column0 % kScanColumns]);
           const Pair keep2 = pair_of(scalar.x, scalar.x);
           Pair kk[R4 * 2];
 #pragma unroll
@@ -698,7 +718,7 @@ __global__ void __launch_bounds__(ScanThreads<MEMORY>::kAll) scan_kernel(const T
       }
       __syncthreads();
     }
-    columns.store(part, p.dim, vectors);
+    if (!is_norm || owner) columns.store(part, p.dim, vectors);
   }
 }
 
@@ -732,18 +752,23 @@ int launch_scan(const KernelArgs& args) {
       cudaGetLastError();
       return fail(args, "shared memory request was refused");
     }
-    launch_kernel(args, kernel, dim3(slices_of(p.vdim), p.heads, p.sequences), dim3(ScanThreads<MEMORY>::kAll), shared,
-                  (const TQ*)args.buffers[0], (const TQ*)args.buffers[1], (const TQ*)args.buffers[2],
-                  (const float*)args.buffers[3], (const float*)args.buffers[4], (float*)args.buffers[5],
-                  (const uint32_t*)args.buffers[6], (const uint32_t*)args.buffers[7], (float*)args.buffers[8], p);
+    auto launch = [&](auto&& start, uint32_t blocks, auto... cluster) {
+      start(args, kernel, dim3(blocks, p.heads, p.sequences), dim3(ScanThreads<MEMORY>::kAll), shared, cluster...,
+            (const TQ*)args.buffers[0], (const TQ*)args.buffers[1], (const TQ*)args.buffers[2], (const float*)args.buffers[3],
+            (const float*)args.buffers[4], (float*)args.buffers[5], (const uint32_t*)args.buffers[6],
+            (const uint32_t*)args.buffers[7], (float*)args.buffers[8], p);
+    };
+    constexpr uint32_t kScanColumns = scan_columns<MEMORY>(), kPerSlice = kSlice / kScanColumns;
+    if (MEMORY) launch([](auto&&... a) { launch_cluster_kernel(a...); }, slices_of(p.vdim) * kPerSlice, kPerSlice);
+    else launch([](auto&&... a) { launch_kernel(a...); }, (p.vdim + kScanColumns - 1u) / kScanColumns);
     return check_launch(args);
   };
   const uint32_t quads = (p.dim + kLanes * 4u - 1u) / (kLanes * 4u);
   // few tokens: small chunks, so that more CTAs fit on an SM
   auto sized = [&](auto r4) {
     constexpr int R4 = decltype(r4)::value;
-    if (p.tokens <= 4u) return run(scan_kernel<TQ, MEMORY, R4, 4>, 2 * sizeof(ScanChunk<R4, 4>));
-    return run(scan_kernel<TQ, MEMORY, R4, 32>, 2 * sizeof(ScanChunk<R4, 32>));
+    if (p.tokens <= 4u) return run(scan_kernel<TQ, MEMORY, R4, 4>, 2 * sizeof(ScanChunk<R4, 4, scan_columns<MEMORY>()>));
+    return run(scan_kernel<TQ, MEMORY, R4, 32>, 2 * sizeof(ScanChunk<R4, 32, scan_columns<MEMORY>()>));
   };
   if (quads <= 1u) return sized(std::integral_constant<int, 1>());
   if (quads <= 2u) return sized(std::integral_constant<int, 2>());

@@ -366,6 +366,57 @@ def test_matrix_memory(runtime, dtype, heads, dim, vdim, cap, loud):
         close(tops[:, one], top, 1e-5, "m")
 
 
+@pytest.mark.parametrize("form", ["delta", "memory"])
+@pytest.mark.parametrize("tokens", [3, 6, 35])
+def test_scans_of_many_sequences_look_back_only(runtime, form, tokens):
+    """More thread blocks than fit on the chip at once, all from states that came before (n and m are read by two blocks and
+    stored by one); an infinite value reaches no earlier token, also of those whose sums are formed together."""
+    from llmopt_b200 import parameters
+    from llmopt_b200.kv_cache import matrix_state_elements
+
+    rng = np.random.default_rng(tokens)
+    sequences, heads, dim, vdim, memory = 80, 4, 64, 48, form == "memory"
+    qk, vs = heads * dim, heads * vdim
+    stride = matrix_state_elements(heads, dim, vdim, normalized=memory)
+    raw = (rng.standard_normal((sequences, tokens, 2 * qk + vs)) * 0.2).astype(np.float32)
+    gates = rng.uniform(0.1, 0.9, (sequences, tokens, 2 * heads)).astype(np.float32)
+    q, k, v = (raw[..., a:b].reshape(sequences, tokens, heads, -1).astype(np.float64)
+               for a, b in ((0, qk), (qk, 2 * qk), (2 * qk, 2 * qk + vs)))
+    pool = (rng.standard_normal((sequences, stride)) * 0.3).astype(np.float32)
+    matrices = pool[:, :heads * vdim * dim].reshape(sequences, heads, vdim, dim).transpose(0, 1, 3, 2).astype(np.float64)
+    if memory:  # the copies of n and m of a head are alike
+        n, m = rng.standard_normal((sequences, heads, 1, dim)).astype(np.float32), rng.standard_normal((sequences, heads, 1)).astype(np.float32)
+        slices = -(-vdim // 32)
+        pool[:, heads * vdim * dim:heads * (vdim + slices) * dim] = np.repeat(n, slices, 2).reshape(sequences, -1)
+        pool[:, heads * (vdim + slices) * dim:][:, :heads * slices] = np.repeat(m, slices, 2).reshape(sequences, -1)
+    broken = raw.copy()
+    broken[:, tokens - 2, 2 * qk:] = np.inf
+    past, order = upload(runtime, np.full(sequences, 9, np.uint32)), rng.permutation(sequences).astype(np.uint32)
+    results = []
+    for values in (raw, broken):
+        states, out = upload(runtime, pool), empty(runtime, sequences * tokens * vs)
+        projected, scalars, rows = upload(runtime, values), upload(runtime, gates), upload(runtime, order)
+        runtime.dispatch("llmopt_memory_scan_f32" if memory else "llmopt_delta_scan_f32",
+                         buffers=[projected, projected, projected, scalars, scalars, states, past, rows, out],
+                         parameters=parameters.state_scan(
+                             sequences=sequences, tokens=tokens, heads=heads, kv_heads=heads, dim=dim, vdim=vdim, q_stride=2 * qk + vs,
+                             q_column=0, k_stride=2 * qk + vs, k_column=qk, v_stride=2 * qk + vs, v_column=2 * qk,
+                             scalar_stride=2 * heads, first_column=0, second_column=heads, state_rows=sequences, state_stride=stride,
+                             gate_cap=5.0 if memory else 0.0))
+        results.append(download(out, (sequences, tokens, heads, vdim)))
+    for one in range(0, sequences, 7):
+        begin = order[one]
+        if memory:
+            capped = 5.0 * np.tanh(gates[one].astype(np.float64) / 5.0)
+            want, _ = plain.matrix_memory_scan(q[one] * dim ** -0.5, k[one], v[one], capped[:, :heads], plain.log_sigmoid(capped[:, heads:]),
+                                               (matrices[begin], n[begin, :, 0].astype(np.float64), m[begin, :, 0].astype(np.float64)))
+        else:
+            want, _ = plain.delta_scan(q[one], k[one], v[one], gates[one, :, :heads].astype(np.float64),
+                                       gates[one, :, heads:].astype(np.float64), matrices[begin])
+        close(results[0][one], want, 1e-4 if memory else 2e-5, (form, one))
+    assert np.array_equal(results[0][:, :tokens - 2], results[1][:, :tokens - 2])
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_head_norm_gate(runtime, dtype):
     from llmopt_b200 import parameters
