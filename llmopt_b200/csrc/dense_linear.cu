@@ -80,6 +80,72 @@ __global__ void __launch_bounds__(kGemvWarps * 32, NT <= 4 ? 2 : 1) dense_gemv_k
   stream_finish<NT>(p, partial, n0, rank, cluster);
 }
 
+// The same sums, in the same order, for matrices with a tile for every SM and more.  A CTA per tile had three blocks of
+// weights under way while it waited for the activation rows in L2, which came to two thirds of its traffic with 32 rows,
+// and nothing while it stored.  32 rows, k 2048: n 32768 76 -> 36 us, n 14336 (pairs) 38 -> 22, n 5120 (cached) 20.5 -> 16.4.
+template <int NT, DenseStore STORE>
+__global__ void __launch_bounds__(kWideThreads, NT == 1 ? 2 : 1) dense_wide_kernel(const DenseTask<STORE> p) {
+  grid_launch_dependents();
+  extern __shared__ __align__(128) unsigned char wide_shared[];
+  typedef WideShape<NT> Shape;
+  typename Shape::Sums* sums = reinterpret_cast<typename Shape::Sums*>(wide_shared + Shape::kRingBytes);
+  uint4* rows = reinterpret_cast<uint4*>(wide_shared + Shape::kRowsAt);
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, g = lane >> 2, t = lane & 3u;
+  const uint32_t tiles = (p.n + 15u) / 16u, mine = (tiles - blockIdx.x + gridDim.x - 1u) / gridDim.x, blocks = (p.k + 63u) / 64u;
+  auto tile_of = [&](uint32_t index, const bf16*& low, const bf16*& high) {
+    const uint32_t n0 = (blockIdx.x + index * gridDim.x) * 16u;
+    low = reinterpret_cast<const bf16*>(p.w) + (size_t)min(n0 + g, p.n - 1u) * p.k;
+    high = reinterpret_cast<const bf16*>(p.w) + (size_t)min(n0 + g + 8u, p.n - 1u) * p.k;
+  };
+  auto stage_rows = [&]() {
+    grid_dependency_wait();
+    const bf16* x = reinterpret_cast<const bf16*>(p.x);
+    const uint32_t chunks = blocks * 8u;
+    for (uint32_t index = threadIdx.x; index < NT * 8u * chunks; index += kWideThreads) {
+      const uint32_t row = index / chunks, chunk = index - row * chunks;
+      uint4 value = make_uint4(0u, 0u, 0u, 0u);
+      if (row < p.m && chunk * 8u < p.k) value = *reinterpret_cast<const uint4*>(x + (size_t)row * p.k + chunk * 8u);
+      rows[wide_chunk(row, blocks, chunk)] = value;
+    }
+    __syncthreads();
+  };
+  if (warp < kGemvWarps) {
+    // the weights are nobody's output: their first blocks are requested before the predecessor ends
+    WideRing<decltype(tile_of)> ring(wide_shared, tile_of, p.k, mine);
+    stage_rows();
+    for (uint32_t tile = 0; tile < mine; ++tile) {
+      float sum[NT][4];
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sum[nt][i] = 0.0f;
+      for (uint32_t block = warp; block < blocks; block += kGemvWarps) {
+        uint4 a[4];
+        ring.next(a);
+#pragma unroll
+        for (int half = 0; half < 2; ++half)
+#pragma unroll
+          for (int nt = 0; nt < NT; ++nt)
+            stream_multiply(sum[nt], a[half], a[2 + half], rows[wide_chunk(nt * 8u + g, blocks, block * 8u + half * 4u + t)]);
+      }
+      // sums are full (1, 2) and free again (3, 4), two buffers
+      const uint32_t buffer = tile & 1u;
+      if (tile >= 2u) wide_barrier_sync(3u + buffer);
+      stream_collect<NT>(sum, sums[buffer][warp]);
+      wide_barrier_arrive(1u + buffer);
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    return;
+  }
+  stage_rows();
+  for (uint32_t tile = 0; tile < mine; ++tile) {
+    const uint32_t buffer = tile & 1u, n0 = (blockIdx.x + tile * gridDim.x) * 16u;
+    wide_barrier_sync(1u + buffer);
+    wide_finish<NT>(p, sums[buffer], n0, threadIdx.x - kGemvWarps * 32u);
+    if (tile + 2u < mine) wide_barrier_arrive(3u + buffer);
+  }
+}
+
 // One warp per output column (pairs: per two columns), up to eight rows.
 template <typename T, DenseStore STORE>
 __global__ void __launch_bounds__(256) dense_columns_kernel(const DenseTask<STORE> p, uint32_t row0) {
@@ -199,6 +265,20 @@ int run_gemv(const KernelArgs& args, DenseProblem p, DenseStore store) {
   p.cluster = stream_cluster(args, tiles, (p.k + 63u) / 64u);
   return with_store(store, [&](auto constant) {
     constexpr DenseStore STORE = decltype(constant)::value;
+    auto run_wide = [&](auto kernel, uint32_t bytes) {
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(args, "shared memory request was refused");
+      }
+      launch_kernel(args, kernel, dim3(wide_ctas(args, tiles, bytes)), dim3(kWideThreads), bytes, DenseTask<STORE>(p));
+      return check_launch(args);
+    };
+    // a tile for every SM (the sums are then not shared out over clusters either), and the rows beside the rings
+    if (tiles >= (uint32_t)context_sm_count(args.ctx) && p.k <= 32768u) {
+      if (p.m <= 8u && WideShape<1>::bytes(p.k) <= kWideMost) return run_wide(dense_wide_kernel<1, STORE>, WideShape<1>::bytes(p.k));
+      if (p.m > 8u && p.m <= 16u && WideShape<2>::bytes(p.k) <= kWideMost) return run_wide(dense_wide_kernel<2, STORE>, WideShape<2>::bytes(p.k));
+      if (p.m > 16u && p.m <= 32u && WideShape<4>::bytes(p.k) <= kWideMost) return run_wide(dense_wide_kernel<4, STORE>, WideShape<4>::bytes(p.k));
+    }
     auto run = [&](auto kernel) {
       const DenseTask<STORE> task(p);
       if (p.cluster == 1u) launch_kernel(args, kernel, dim3(tiles), dim3(kGemvWarps * 32), 0, task);

@@ -96,6 +96,109 @@ __device__ __forceinline__ void stream_finish(const DenseTask<STORE>& p, float (
   cluster_sync();  // nobody leaves while its sums may be read
 }
 
+// ---- many tiles: persistent CTAs ------------------------------------------------------------------
+// A CTA walks over tiles of 16 weight rows.  Eight warps share out a tile's k-blocks as in the kernels above; the blocks come
+// by cp.async into a ring of the lane that uses them (no other lane reads it, so nothing synchronises), across the ends of
+// tiles.  The activation rows lie in shared memory for all tiles.  Four more warps add the eight sums of one tile and store
+// it while the next is under way.
+constexpr uint32_t kRingDepth = 4, kFinishWarps = 4, kWideThreads = (kGemvWarps + kFinishWarps) * 32;
+constexpr uint32_t kWideMost = 232448;  // bytes of shared memory a CTA can have
+
+__device__ __forceinline__ void ring_copy(uint4* target, const bf16* source, bool present) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(target)), "l"(source),
+               "r"(present ? 16u : 0u)
+               : "memory");
+}
+__device__ __forceinline__ void wide_barrier_sync(uint32_t id) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kWideThreads) : "memory");
+}
+__device__ __forceinline__ void wide_barrier_arrive(uint32_t id) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(kWideThreads) : "memory");
+}
+
+// Shared memory: rings, two tiles' sums, activation rows of whole k-blocks.
+template <int NT>
+struct WideShape {
+  static constexpr uint32_t kRingBytes = kGemvWarps * kRingDepth * 4u * 32u * 16u;
+  typedef float Sums[kGemvWarps][NT * 8][17];
+  static constexpr uint32_t kRowsAt = kRingBytes + 2u * sizeof(Sums);
+  __host__ __device__ static constexpr uint32_t bytes(uint32_t k) { return kRowsAt + NT * 8u * ((k + 63u) / 64u * 128u); }
+};
+// Sixteen-byte chunk `chunk` of a row; odd rows swap the halves of a k-block, so that two rows fill the banks.
+__device__ __forceinline__ uint32_t wide_chunk(uint32_t row, uint32_t blocks, uint32_t chunk) {
+  return row * blocks * 8u + (chunk ^ ((row & 1u) * 4u));
+}
+
+// The ring of one lane.  tile_of(index, low, high) says where the lane's two weight rows of the CTA's tile number `index`
+// begin.
+template <typename Tile>
+struct WideRing {
+  uint4* slots;  // of the lane: piece i of stage s at (4 s + i) * 32
+  const Tile& tile_of;
+  const bf16 *low, *high;
+  uint32_t k, blocks, warp, t, tiles, tile, block, fill, drain;
+  __device__ __forceinline__ WideRing(unsigned char* shared, const Tile& tile_of, uint32_t k, uint32_t tiles)
+      : slots(reinterpret_cast<uint4*>(shared) + (threadIdx.x >> 5) * kRingDepth * 128u + (threadIdx.x & 31u)), tile_of(tile_of), k(k),
+        blocks((k + 63u) / 64u), warp(threadIdx.x >> 5), t(threadIdx.x & 3u), tiles(warp < blocks ? tiles : 0u), tile(0), block(warp),
+        fill(0), drain(0) {
+    if (tile < this->tiles) tile_of(tile, low, high);
+#pragma unroll
+    for (uint32_t i = 0; i + 1u < kRingDepth; ++i) fetch();
+  }
+  __device__ __forceinline__ void fetch() {
+    if (tile < tiles) {
+#pragma unroll
+      for (uint32_t half = 0; half < 2u; ++half) {
+        const uint32_t at = block * 64u + half * 32u + t * 8u;
+        const bool present = at < k;
+        ring_copy(slots + (fill * 4u + half) * 32u, present ? low + at : low, present);
+        ring_copy(slots + (fill * 4u + 2u + half) * 32u, present ? high + at : high, present);
+      }
+      block += kGemvWarps;
+      if (block >= blocks) {
+        block = warp;
+        if (++tile < tiles) tile_of(tile, low, high);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    fill = (fill + 1u) % kRingDepth;
+  }
+  // The next block's pieces: low / high 32 k of the row g, then of row g + 8.
+  __device__ __forceinline__ void next(uint4 (&pieces)[4]) {
+    fetch();  // into the slot that the block before was read from
+    asm volatile("cp.async.wait_group %0;" ::"n"(kRingDepth - 1) : "memory");
+#pragma unroll
+    for (uint32_t i = 0; i < 4u; ++i) pieces[i] = slots[(drain * 4u + i) * 32u];
+    drain = (drain + 1u) % kRingDepth;
+  }
+};
+
+// A tile's eight sums in warp order, stored by the finishing warps' thread number `thread`.
+template <int NT, DenseStore STORE>
+__device__ __forceinline__ void wide_finish(const DenseTask<STORE>& p, const float (&sums)[kGemvWarps][NT * 8][17], uint32_t n0, uint32_t thread) {
+  constexpr uint32_t kStep = STORE == kStorePair ? 2u : 1u;  // columns a thread stores together
+#pragma unroll 2
+  for (uint32_t index = thread * kStep; index < NT * 8u * 16u; index += kFinishWarps * 32u * kStep) {
+    const uint32_t column = index & 15u, row = index >> 4;
+    if (row >= p.m || n0 + column >= p.n) continue;
+    float value[kStep];
+#pragma unroll
+    for (uint32_t i = 0; i < kStep; ++i) {
+      value[i] = 0.0f;
+#pragma unroll
+      for (int part = 0; part < kGemvWarps; ++part) value[i] += sums[part][row][column + i];
+    }
+    stream_store(p, row, n0 + column, value);
+  }
+}
+
+// CTAs for `tiles` tiles: whole rounds of as many as fit, shared out evenly.
+inline uint32_t wide_ctas(const KernelArgs& args, uint32_t tiles, uint32_t bytes) {
+  const uint32_t per_sm = kWideMost / (bytes + 1024u) >= 2u ? 2u : 1u, most = per_sm * (uint32_t)context_sm_count(args.ctx);
+  const uint32_t rounds = (tiles + most - 1u) / most;
+  return (tiles + rounds - 1u) / rounds;
+}
+
 // CTAs per cluster that share out the k-blocks of `tiles` 16-row tiles: at least one CTA per SM, and a warp of a
 // split keeps at least one of the `blocks`.
 inline uint32_t stream_cluster(const KernelArgs& args, uint32_t tiles, uint32_t blocks) {
