@@ -26,10 +26,12 @@
 // are read and converted once per KV head.  The bound is HBM: per key and KV
 // head 2 D bytes of int8 plus 4 D / group bytes of scales.
 //
-// Each CTA (4 warps) owns one split of one (batch, kv head); warps take the
+// Each CTA (4 or 8 warps) owns one split of one (batch, kv head); warps take the
 // tiles of the split round-robin and keep private (max, denominator, O^T);
-// the CTA merges its warps in shared memory and writes one record to scratch;
-// paged_merge_kernel merges the records of all splits and the current token.
+// the CTA merges its warps in shared memory into one record.  Where the splits of a
+// (batch, kv head) are one thread-block cluster, its CTAs read one another's records there,
+// add the current token and write the output; otherwise the records go to scratch and
+// paged_merge_kernel merges them and the current token.
 #include <cstdlib>
 #include "q8_attention.cuh"
 #include "q8_codec.cuh"
@@ -42,6 +44,7 @@ constexpr int kTileKeys = 16;
 constexpr int kWarps = 4;
 constexpr int kResidentCtas = 4;  // per SM, by shared memory and registers (128 per thread)
 constexpr uint32_t kNoSlot = 0xffffffffu;
+constexpr uint32_t kLongestForOneCluster = 3072;  // tokens behind a sequence: three tiles per warp
 constexpr float kLowest = -1.0e30f;  // "no key yet" maximum; keeps the softmax free of inf - inf
 
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t selector) {
@@ -112,7 +115,7 @@ __device__ __forceinline__ void copy_async_wait() {
 
 // Shared-memory shape of one warp's ring.  CP is the copy size: 16 bytes, or 8 for
 // pools whose rows are only 8-byte aligned.
-template <int D, int CP>
+template <int D, int CP, int WARPS>
 struct SplitShape {
   static constexpr int kRowBytes = D + 16;  // the padding spreads the fragment reads over all banks
   static constexpr int kTileBytes = kTileKeys * kRowBytes;
@@ -124,7 +127,7 @@ struct SplitShape {
   static constexpr int kLanesPerKey = D / CP;
   static constexpr int kKeysPerPass = 32 / kLanesPerKey;
   static constexpr int kPasses = kTileKeys / kKeysPerPass;
-  static constexpr int kRingBytes = kWarps * kStages * kStageBytes;
+  static constexpr int kRingBytes = WARPS * kStages * kStageBytes;
 };
 
 // FUSED: the launch also does the rotary embedding and the cache pack of the new token (`fusion`), which
@@ -133,14 +136,17 @@ struct SplitShape {
 // writes of the rotated query / key rows (the merge kernel reads them) and the Q8 pack of the new key and
 // value rows are warp tasks handed out over the CTAs of a (batch, KV head), done while the first tiles are
 // in flight.
-template <int D, int GROUP, int CP, bool FUSED = false>
-__global__ void __launch_bounds__(kWarps * 32, kResidentCtas)
+// `cluster` > 0: the grid's x dimension is one cluster of that many CTAs, which writes `output`.
+template <int D, int GROUP, int CP, bool FUSED, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, kResidentCtas * kWarps / WARPS)
 paged_split_kernel(const __half* __restrict__ query, const uint8_t* __restrict__ pool,
                    const uint32_t* __restrict__ slots, float* __restrict__ scratch, PagedParams p,
                    uint32_t slot_batch_stride, uint32_t splits, const uint32_t* __restrict__ past_cell,
-                   uint32_t pool_tokens, uint32_t* error_word, RotaryPackFusion fusion) {
+                   uint32_t pool_tokens, uint32_t* error_word, RotaryPackFusion fusion, const __half* current_key,
+                   const __half* current_value, __half* output, uint32_t cluster) {
   grid_chain_prologue();
-  using Shape = SplitShape<D, CP>;
+  constexpr int kWarps = WARPS;
+  using Shape = SplitShape<D, CP, WARPS>;
   constexpr int kSteps = D / 16;  // k-steps of QK^T, m-tiles of PV
   constexpr int kStages = Shape::kStages;
   constexpr int groups_per_head = D / GROUP;  // 1, 2 or 4
@@ -452,9 +458,9 @@ paged_split_kernel(const __half* __restrict__ query, const uint8_t* __restrict__
     running_sum[h] += __shfl_xor_sync(0xffffffffu, running_sum[h], 16);
   }
   __syncthreads();
-  float* stage = reinterpret_cast<float*>(ring);  // [warp][16 + 8 * D]
+  float* stage = reinterpret_cast<float*>(ring);  // [warp][16 + 8 * D], then the CTA's own record
   constexpr int kRecord = 16 + 8 * D;
-  static_assert(Shape::kRingBytes >= (int)sizeof(float) * kWarps * kRecord, "merge staging must fit the ring");
+  static_assert(Shape::kRingBytes >= (int)sizeof(float) * (kWarps + 1) * kRecord, "merge staging must fit the ring");
   float* mine = stage + warp * kRecord;
   if (r == 0) {
     mine[2 * c] = running_max[0];
@@ -471,7 +477,8 @@ paged_split_kernel(const __half* __restrict__ query, const uint8_t* __restrict__
       mine[16 + head * D + dim] = out[s][j];
     }
   __syncthreads();
-  float* record = scratch + (((size_t)batch * p.kv_heads + kv_head) * splits + split) * kRecord;
+  float* record = cluster > 0 ? stage + kWarps * kRecord
+                              : scratch + (((size_t)batch * p.kv_heads + kv_head) * splits + split) * kRecord;
   // only the columns of heads that exist are merged and written (the merge kernel reads no others)
   for (uint32_t index = threadIdx.x; index < min(heads_per_kv, 8u) * D; index += kWarps * 32) {
     const uint32_t head = index / D;
@@ -491,6 +498,51 @@ paged_split_kernel(const __half* __restrict__ query, const uint8_t* __restrict__
       record[head] = merged_max <= 0.5f * kLowest ? -INFINITY : merged_max * 0.6931471805599453f;
       record[8 + head] = denominator;
     }
+  }
+  if (cluster == 0u) return;
+
+  // ---- merge the cluster's records and the current token -----------------------
+  // Thread i of the cluster owns elements i, i + threads, ... of [head][D]; a warp's 32 belong to one head.
+  cluster_sync();
+  constexpr int kMost = 8 * D / (2 * kWarps * 32);  // of a thread, in a cluster of two or more
+  const uint32_t elements = min(heads_per_kv, 8u) * D, threads = cluster * kWarps * 32u;
+  float results[kMost];
+#pragma unroll
+  for (int i = 0; i < kMost; ++i) {
+    const uint32_t index = split * kWarps * 32u + threadIdx.x + i * threads;
+    if (index >= elements) break;
+    const uint32_t head = index / D, d = index % D;
+    const size_t query_base = ((size_t)batch * p.query_heads + kv_head * heads_per_kv + head) * D;
+    const size_t current_base = ((size_t)batch * p.kv_heads + kv_head) * D;
+    // the rotated rows may have been written by this launch: not through the read-only path
+    auto half_at = [](const __half* source) {
+      return __half2float(__ushort_as_half(__ldcg(reinterpret_cast<const unsigned short*>(source))));
+    };
+    float dot = 0.0f;
+#pragma unroll
+    for (int part = 0; part < D / 32; ++part)
+      dot = fmaf(half_at(query + query_base + part * 32 + lane), half_at(current_key + current_base + part * 32 + lane), dot);
+    const float current = half_at(current_value + current_base + d);
+    const float score_now = warp_sum(dot) * p.scale;
+    float maximum = score_now;
+    for (uint32_t other = 0; other < cluster; ++other) maximum = fmaxf(maximum, cluster_load(record + head, other));
+    const float now = expf(score_now - maximum);
+    float total = now * current, denominator = now;
+#pragma unroll 4
+    for (uint32_t other = 0; other < cluster; ++other) {
+      const float top = cluster_load(record + head, other);
+      const float weight = top == -INFINITY ? 0.0f : expf(top - maximum);
+      denominator = fmaf(weight, cluster_load(record + 8 + head, other), denominator);
+      total = fmaf(weight, cluster_load(record + 16 + index, other), total);
+    }
+    results[i] = denominator == 0.0f ? 0.0f : total / denominator;
+  }
+  cluster_sync();  // nobody leaves while its record may be read, nor writes while a query row may be
+#pragma unroll
+  for (int i = 0; i < kMost; ++i) {
+    const uint32_t index = split * kWarps * 32u + threadIdx.x + i * threads;
+    if (index < elements)
+      output[((size_t)batch * p.query_heads + kv_head * heads_per_kv) * D + index] = __float2half_rn(results[i]);
   }
 }
 
@@ -574,34 +626,83 @@ paged_merge_kernel(const __half* __restrict__ query, const __half* __restrict__ 
   output[output_base + d] = __float2half_rn(denominator == 0.0f ? 0.0f : result / denominator);
 }
 
-template <int D, int GROUP, int CP>
+// Splits of a (batch, KV head) that form one cluster, and warps per CTA; 0: records and a merge kernel.
+struct ClusterPlan {
+  uint32_t ctas, warps;
+};
+
+template <int D, int GROUP, int CP, int WARPS>
 int launch_split_copy(const KernelArgs& args, const PagedParams& p, uint32_t slot_batch_stride, float* scratch,
-                      uint32_t splits, uint32_t pool_tokens) {
-  auto kernel = args.rotary_fusion ? paged_split_kernel<D, GROUP, CP, true> : paged_split_kernel<D, GROUP, CP, false>;
-  constexpr int ring_bytes = SplitShape<D, CP>::kRingBytes;
+                      uint32_t splits, uint32_t pool_tokens, uint32_t cluster) {
+  auto kernel = args.rotary_fusion ? paged_split_kernel<D, GROUP, CP, true, WARPS> : paged_split_kernel<D, GROUP, CP, false, WARPS>;
+  constexpr int ring_bytes = SplitShape<D, CP, WARPS>::kRingBytes;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ring_bytes) != cudaSuccess) {
     cudaGetLastError();
     return fail(args, "paged attention: the device cannot give one CTA its tile ring");
   }
   const RotaryPackFusion fusion = args.rotary_fusion ? *args.rotary_fusion : RotaryPackFusion{};
-  launch_kernel(args, kernel, dim3(splits, p.kv_heads, p.batches), dim3(kWarps * 32), ring_bytes,
-      (const __half*)args.buffers[0], (const uint8_t*)args.buffers[3], (const uint32_t*)args.buffers[4], scratch, p,
-      slot_batch_stride, splits, args.past_tokens_cell, pool_tokens,
-      args.ctx ? context_device_error(args.ctx) : nullptr, fusion);
+  auto launch = [&](auto&& start, auto... size) {
+    start(args, kernel, dim3(splits, p.kv_heads, p.batches), dim3(WARPS * 32), (size_t)ring_bytes, size...,
+          (const __half*)args.buffers[0], (const uint8_t*)args.buffers[3], (const uint32_t*)args.buffers[4], scratch, p,
+          slot_batch_stride, splits, args.past_tokens_cell, pool_tokens,
+          args.ctx ? context_device_error(args.ctx) : nullptr, fusion, (const __half*)args.buffers[1],
+          (const __half*)args.buffers[2], (__half*)args.buffers[6], cluster);
+  };
+  if (cluster > 0u) launch([](auto&&... a) { launch_cluster_kernel(a...); }, cluster);
+  else launch([](auto&&... a) { launch_kernel(a...); });
   return check_launch(args);
 }
 
 template <int D, int GROUP>
 int launch_split(const KernelArgs& args, const PagedParams& p, uint32_t slot_batch_stride, float* scratch,
-                 uint32_t splits, uint32_t pool_tokens) {
+                 uint32_t splits, uint32_t pool_tokens, ClusterPlan plan) {
   const bool aligned = (p.token_stride % 16 == 0) && (((uintptr_t)args.buffers[3]) % 16 == 0);
-  const int status = aligned ? launch_split_copy<D, GROUP, 16>(args, p, slot_batch_stride, scratch, splits, pool_tokens)
-                             : launch_split_copy<D, GROUP, 8>(args, p, slot_batch_stride, scratch, splits, pool_tokens);
+  if (plan.ctas > 0u) {
+    if (plan.warps == 8u)
+      return aligned ? launch_split_copy<D, GROUP, 16, 8>(args, p, slot_batch_stride, nullptr, plan.ctas, pool_tokens, plan.ctas)
+                     : launch_split_copy<D, GROUP, 8, 8>(args, p, slot_batch_stride, nullptr, plan.ctas, pool_tokens, plan.ctas);
+    return aligned ? launch_split_copy<D, GROUP, 16, 4>(args, p, slot_batch_stride, nullptr, plan.ctas, pool_tokens, plan.ctas)
+                   : launch_split_copy<D, GROUP, 8, 4>(args, p, slot_batch_stride, nullptr, plan.ctas, pool_tokens, plan.ctas);
+  }
+  const int status = aligned ? launch_split_copy<D, GROUP, 16, 4>(args, p, slot_batch_stride, scratch, splits, pool_tokens, 0u)
+                             : launch_split_copy<D, GROUP, 8, 4>(args, p, slot_batch_stride, scratch, splits, pool_tokens, 0u);
   if (status) return status;
   launch_kernel(args, paged_merge_kernel<D>, dim3(p.query_heads, p.batches), dim3(D * kMergeParts), 0,
       (const __half*)args.buffers[0], (const __half*)args.buffers[1], (const __half*)args.buffers[2], scratch,
       (__half*)args.buffers[6], p, splits);
   return check_launch(args);
+}
+
+uint32_t pinned_splits() {
+  // LLMOPT_CUDA_ATTENTION_SPLITS pins the count (within the limit), for tuning
+  static const uint32_t pinned = []() -> uint32_t {
+    const char* text = getenv("LLMOPT_CUDA_ATTENTION_SPLITS");
+    const long value = text ? strtol(text, nullptr, 10) : 0;
+    return value > 0 ? (uint32_t)value : 0u;
+  }();
+  return pinned;
+}
+
+// A cluster saves the merge kernel and the way through scratch, which is 4 to 5 us a layer: 1 sequence x 512 keys x 3 heads of
+// 64 (64 splits before) 10.0 -> 6.7 us, 16 x 1024 x 8 of 64 14.7 -> 13.2, 32 x 2048 x 8 of 128 49.7 -> 41.3.  Few (batch, KV
+// head) pairs take eight CTAs of eight warps; beyond a few tiles per warp (about 2 us each) many short splits are faster
+// again: 8192 keys x 8 heads of 128 24.1 us in clusters, 15.6 as 64 records.  What a plan may grow to decides, not what it
+// was captured at.  More pairs: the cluster size that fills whole waves best; the merge is the same work for all of them.
+ClusterPlan pick_cluster(const KernelArgs& args, const PagedParams& p, uint32_t slot_batch_stride) {
+  if (pinned_splits() != 0u) return {0u, 0u};
+  const size_t slots = args.lengths[4] / 4u, before = (size_t)(p.batches - 1u) * slot_batch_stride;
+  const size_t longest = args.past_tokens_cell ? (slots > before ? slots - before : 0u) : p.past_length;
+  const uint32_t pairs = p.batches * p.kv_heads, sms = (uint32_t)context_sm_count(args.ctx);
+  const uint32_t resident = sms * (uint32_t)kResidentCtas;
+  if (pairs * 8u <= 2u * sms) return longest <= kLongestForOneCluster ? ClusterPlan{8u, 8u} : ClusterPlan{0u, 0u};
+  uint32_t best = 2u;
+  float best_fill = 0.0f;
+  for (uint32_t ctas = 2u; ctas <= 8u; ctas *= 2u) {
+    const uint32_t waves = (pairs * ctas + resident - 1u) / resident;
+    const float fill = (float)(pairs * ctas) / (float)(waves * resident);
+    if (fill > best_fill + 0.01f) best = ctas, best_fill = fill;
+  }
+  return {best, 4u};
 }
 
 }  // namespace
@@ -629,12 +730,7 @@ uint32_t paged_pick_splits(const KernelArgs& args, const PagedParams& p) {
   uint32_t limit = args.past_tokens_cell ? kMaxAttentionSplits : (p.past_length + 63u) / 64u;
   if (limit > kMaxAttentionSplits) limit = kMaxAttentionSplits;
   if (limit == 0) return 1;
-  // LLMOPT_CUDA_ATTENTION_SPLITS pins the count (within the limit), for tuning
-  static const uint32_t pinned = []() -> uint32_t {
-    const char* text = getenv("LLMOPT_CUDA_ATTENTION_SPLITS");
-    const long value = text ? strtol(text, nullptr, 10) : 0;
-    return value > 0 ? (uint32_t)value : 0u;
-  }();
+  const uint32_t pinned = pinned_splits();
   if (pinned != 0u) return pinned < limit ? pinned : limit;
   const uint32_t fill_target = (resident * 85u + 99u) / 100u;
   const uint32_t first = (fill_target + pairs - 1u) / pairs;
@@ -655,19 +751,26 @@ uint32_t paged_pick_splits(const KernelArgs& args, const PagedParams& p) {
   return best;
 }
 
-int launch_paged_attention_split_on(const KernelArgs& args, const PagedParams& p, uint32_t slot_batch_stride,
-                                    float* scratch, uint32_t splits, uint32_t pool_tokens) {
+static int launch_split_as(const KernelArgs& args, const PagedParams& p, uint32_t slot_batch_stride, float* scratch,
+                           uint32_t splits, uint32_t pool_tokens, ClusterPlan plan) {
   LLMOPT_REQUIRE(((uintptr_t)args.buffers[3]) % 8 == 0, "pool must be 8-byte aligned");
   LLMOPT_REQUIRE(((uintptr_t)args.buffers[0]) % 4 == 0, "query must be 4-byte aligned");
   if (p.head_dim == 64)
-    return p.group_size == 64 ? launch_split<64, 64>(args, p, slot_batch_stride, scratch, splits, pool_tokens)
-                              : launch_split<64, 32>(args, p, slot_batch_stride, scratch, splits, pool_tokens);
-  return p.group_size == 64 ? launch_split<128, 64>(args, p, slot_batch_stride, scratch, splits, pool_tokens)
-                            : launch_split<128, 32>(args, p, slot_batch_stride, scratch, splits, pool_tokens);
+    return p.group_size == 64 ? launch_split<64, 64>(args, p, slot_batch_stride, scratch, splits, pool_tokens, plan)
+                              : launch_split<64, 32>(args, p, slot_batch_stride, scratch, splits, pool_tokens, plan);
+  return p.group_size == 64 ? launch_split<128, 64>(args, p, slot_batch_stride, scratch, splits, pool_tokens, plan)
+                            : launch_split<128, 32>(args, p, slot_batch_stride, scratch, splits, pool_tokens, plan);
+}
+
+int launch_paged_attention_split_on(const KernelArgs& args, const PagedParams& p, uint32_t slot_batch_stride,
+                                    float* scratch, uint32_t splits, uint32_t pool_tokens) {
+  return launch_split_as(args, p, slot_batch_stride, scratch, splits, pool_tokens, {0u, 0u});
 }
 
 int launch_paged_attention_split(const KernelArgs& args, const PagedParams& p, uint32_t slot_batch_stride,
                                  uint32_t pool_tokens) {
+  const ClusterPlan plan = pick_cluster(args, p, slot_batch_stride);
+  if (plan.ctas > 0u) return launch_split_as(args, p, slot_batch_stride, nullptr, 0u, pool_tokens, plan);
   const uint32_t splits = paged_pick_splits(args, p);
   const size_t bytes =
       (size_t)p.batches * p.kv_heads * splits * paged_split_record_floats(p.head_dim) * sizeof(float);
