@@ -288,6 +288,9 @@ class DispatchItem:
     barrier_before: bool = False
 
 
+_Three = ctypes.c_int * 3
+
+
 class _RecordArray:
     """Packs DispatchItems into a C array and keeps every referenced object alive."""
 
@@ -301,14 +304,15 @@ class _RecordArray:
             params = ctypes.create_string_buffer(bytes(item.parameters), max(len(item.parameters), 1))
             self._keep.extend([name, handles, params])
             record.name = name
-            record.buffers = ctypes.cast(handles, ctypes.POINTER(ctypes.c_void_p))
+            record.buffers = handles
             record.buffer_count = len(item.buffers)
-            record.parameters = ctypes.cast(params, ctypes.c_void_p)
+            record.parameters = ctypes.addressof(params)
             record.parameter_bytes = len(item.parameters)
-            if any(int(v) > 0x7FFFFFFF for v in tuple(item.grid) + tuple(item.group)):
+            grid, group = [int(v) for v in item.grid], [int(v) for v in item.group]
+            if max(grid + group, default=0) > 0x7FFFFFFF:
                 raise ValueError(f"{item.name}: grid dimension overflows the 32-bit record field")
-            record.grid = (ctypes.c_int * 3)(*[int(v) for v in item.grid])
-            record.group = (ctypes.c_int * 3)(*[int(v) for v in item.group])
+            record.grid = _Three(*grid)
+            record.group = _Three(*group)
             record.barrier_before = int(item.barrier_before)
 
     def __len__(self):

@@ -187,6 +187,10 @@ def _entries() -> list[Entry]:
 
 
 ENTRIES: tuple = tuple(_entries())
+_MATCHES: dict = {}  # (operation, input dtype, output dtype, name or None for any) -> entries
+for _entry in ENTRIES:
+    for _name in (_entry.name, None):
+        _MATCHES.setdefault((_entry.operation, _entry.input_dtype, _entry.output_dtype, _name), []).append(_entry)
 
 
 def find_entry(*, operation: str, input_dtype: str, output_dtype: str, name: Optional[str] = None) -> Entry:
@@ -194,8 +198,7 @@ def find_entry(*, operation: str, input_dtype: str, output_dtype: str, name: Opt
     exactly one entry must match the operation, both dtypes and, if given, the name."""
     if operation not in OPERATIONS:
         raise ValueError(f"unsupported kernel operation: {operation}")
-    matches = [e for e in ENTRIES if e.operation == operation and e.input_dtype == input_dtype
-               and e.output_dtype == output_dtype and (name is None or e.name == name)]
+    matches = _MATCHES.get((operation, input_dtype, output_dtype, name), ())
     if not matches:
         raise LookupError(f"package declares no kernel for operation {operation}" + (f" named {name}" if name else ""))
     if len(matches) > 1:
