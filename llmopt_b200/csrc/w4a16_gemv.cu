@@ -244,6 +244,208 @@ __global__ void __launch_bounds__(256, (NT * NMAT >= 8) ? 1 : 2) w4a16_gemv_kern
   }
 }
 
+// ---- short sums: at most eight rows, K of up to 2048 that is no multiple of 512 --------------------------
+// A launch of a small model moves a few hundred KB: what it costs is the way from its inputs to its outputs.  So a CTA owns
+// one 16-column tile and each of its eight warps at most GROUPS groups of K; their weights are requested ahead of the wait
+// for the previous kernel, the residual ahead of the sums, and a folded RMS norm needs no launch of its own.  K 576, one row, with its
+// norm: Q, K and V 5.6 -> 2.6 us a launch, gate and up 5.9 -> 3.1; without: 4.2 -> 1.8 (one warp in two or four of a CTA per tile, norms apart).
+constexpr uint32_t kShortWarps = 8, kShortGroups = 4;
+
+template <int NMAT, int EPI, int GROUPS>
+__global__ void __launch_bounds__(kShortWarps * 32) w4a16_gemv_short_kernel(const GemvProblem p) {
+  grid_launch_dependents();
+  constexpr int kAcc = NMAT * 4;
+  __shared__ float sums[kShortWarps * GROUPS][kAcc][32];       // of every group, before its scale
+  __shared__ float group_scales[kShortWarps * GROUPS][NMAT][16];
+  __shared__ float inverse_rms[8];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, r = lane >> 2, c = lane & 3u;
+  const uint32_t groups = p.k >> 6, half_k = p.k >> 1;
+  uint32_t matrix = 0, tile = blockIdx.x;
+  if (EPI == kEpiQkv)
+    while (matrix + 1u < p.matrices && tile >= (p.mat[matrix].n + 15u) >> 4) tile -= (p.mat[matrix++].n + 15u) >> 4;
+  const uint32_t n = p.mat[matrix].n;
+  const uint32_t row_a = min(tile * 16u + r, n - 1u), row_b = min(tile * 16u + r + 8u, n - 1u);
+
+  // this warp's groups: warp, warp + 8, ...
+  uint2 words[NMAT][GROUPS][2];
+  __half scales[NMAT][GROUPS][2];
+#pragma unroll
+  for (int a = 0; a < NMAT; ++a) {
+    const GemvMatrix& mat = p.mat[EPI == kEpiQkv ? matrix : a];
+#pragma unroll
+    for (int i = 0; i < GROUPS; ++i) {
+      const uint32_t g = min(warp + i * kShortWarps, groups - 1u);  // a group that is not there is not used
+      words[a][i][0] = __ldg(reinterpret_cast<const uint2*>(mat.packed + (size_t)row_a * half_k + (g << 5) + (c << 3)));
+      words[a][i][1] = __ldg(reinterpret_cast<const uint2*>(mat.packed + (size_t)row_b * half_k + (g << 5) + (c << 3)));
+      scales[a][i][0] = __ldg(mat.scale + (size_t)row_a * groups + g);
+      scales[a][i][1] = __ldg(mat.scale + (size_t)row_b * groups + g);
+    }
+  }
+  grid_dependency_wait();
+
+  // Lane (r, c): row r, k = 64 g + 16 c + [0, 16).
+  const bool present = r < p.x_rows;
+  uint4 x[GROUPS][2];
+#pragma unroll
+  for (int i = 0; i < GROUPS; ++i) {
+    const uint32_t g = warp + i * kShortWarps;
+    x[i][0] = x[i][1] = make_uint4(0u, 0u, 0u, 0u);
+    if (present && g < groups) {
+      const uint4* source = reinterpret_cast<const uint4*>(p.x + (size_t)r * p.k + (g << 6) + (c << 4));
+      x[i][0] = source[0];
+      x[i][1] = source[1];
+    }
+  }
+  // the output of thread (warp < 4, lane): register `warp` of the tile's accumulators
+  const uint32_t out_row = 2u * c + (warp & 1u), out_column = tile * 16u + r + ((warp & 2u) ? 8u : 0u);
+  float residual = 0.0f;
+  if (EPI == kEpiLinear && p.has_aux && warp < 4u && out_row < p.m && out_column < n)
+    residual = __half2float(p.aux0[(size_t)out_row * p.aux_row_stride + out_column]);
+
+  if (p.norm_weight != nullptr) {
+    auto inverse_of = [&](uint32_t row) {  // summed like the stand-alone kernel, 256 elements per warp of it
+      float total = 0.0f;
+#pragma unroll
+      for (uint32_t part = 0; part < GROUPS * 2u; ++part) {
+        if (part * 256u >= p.k) break;
+        const uint32_t at = part * 256u + lane * 8u;
+        float squares = 0.0f;
+        if (at < p.k) {
+          float values[8];
+          load_eight(p.x + (size_t)row * p.k + at, values);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) squares = fmaf(values[e], values[e], squares);
+        }
+        total += warp_sum(squares);
+      }
+      return rsqrtf(total / (float)p.k + p.norm_epsilon);
+    };
+    float inverse;
+    if (p.x_rows == 1u) {  // every warp for itself
+      inverse = inverse_of(0u);
+    } else {
+      if (warp < p.x_rows) {
+        const float own = inverse_of(warp);
+        if (lane == 0) inverse_rms[warp] = own;
+      }
+      __syncthreads();
+      inverse = inverse_rms[present ? r : 0u];
+    }
+#pragma unroll
+    for (int i = 0; i < GROUPS; ++i) {
+      const uint32_t g = warp + i * kShortWarps, at = (g << 6) + (c << 4);
+      if (!present || g >= groups) continue;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        // half((x inv) w) or half((x w) inv), as the stand-alone norm kernels round
+        float w[8];
+        load_eight(p.norm_weight + at + h * 8, w);
+        uint32_t* pairs = reinterpret_cast<uint32_t*>(&x[i][h]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&pairs[e]));
+          const __half2 y = p.norm_weight_first ? __floats2half2_rn((v.x * w[2 * e]) * inverse, (v.y * w[2 * e + 1]) * inverse)
+                                                : __floats2half2_rn((v.x * inverse) * w[2 * e], (v.y * inverse) * w[2 * e + 1]);
+          pairs[e] = *reinterpret_cast<const uint32_t*>(&y);
+        }
+        if (blockIdx.x == 0 && p.norm_out != nullptr) *reinterpret_cast<uint4*>(p.norm_out + (size_t)r * p.k + at + h * 8) = x[i][h];
+      }
+    }
+  }
+
+#pragma unroll
+  for (int i = 0; i < GROUPS; ++i) {
+    const uint32_t g = warp + i * kShortWarps;
+    if (g >= groups) break;
+    const uint4 first = x[i][0], second = x[i][1];
+    uint32_t frag[8];  // pairs (k, k + 4), like the nibbles
+    frag[0] = prmt(first.x, first.z, 0x5410u);
+    frag[1] = prmt(first.x, first.z, 0x7632u);
+    frag[2] = prmt(first.y, first.w, 0x5410u);
+    frag[3] = prmt(first.y, first.w, 0x7632u);
+    frag[4] = prmt(second.x, second.z, 0x5410u);
+    frag[5] = prmt(second.x, second.z, 0x7632u);
+    frag[6] = prmt(second.y, second.w, 0x5410u);
+    frag[7] = prmt(second.y, second.w, 0x7632u);
+#pragma unroll
+    for (int a = 0; a < NMAT; ++a) {
+      float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (int w = 0; w < 2; ++w) {
+        uint32_t bits_a = w == 0 ? words[a][i][0].x : words[a][i][0].y;
+        uint32_t bits_b = w == 0 ? words[a][i][1].x : words[a][i][1].y;
+#pragma unroll
+        for (int step = 0; step < 2; ++step) {
+          uint32_t a_low, a_high, b_low, b_high;
+          nibbles_to_half2<true>(bits_a, a_low, a_high);
+          nibbles_to_half2<true>(bits_b, b_low, b_high);
+          mma_16816(sum, a_low, b_low, a_high, b_high, frag[4 * w + 2 * step], frag[4 * w + 2 * step + 1]);
+          bits_a >>= 8;
+          bits_b >>= 8;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sums[g][a * 4 + j][lane] = sum[j];
+      if (c == 0u) {
+        group_scales[g][a][r] = __half2float(scales[a][i][0]);
+        group_scales[g][a][r + 8u] = __half2float(scales[a][i][1]);
+      }
+    }
+  }
+  __syncthreads();
+  if (warp >= 4u) return;
+  // the groups in order, whichever warp had them
+  float value[NMAT];
+#pragma unroll
+  for (int a = 0; a < NMAT; ++a) {
+    value[a] = 0.0f;
+    for (uint32_t g = 0; g < groups; ++g)
+      value[a] = fmaf(group_scales[g][a][r + ((warp & 2u) ? 8u : 0u)], sums[g][a * 4 + warp][lane], value[a]);
+  }
+  if (EPI == kEpiLinear) {
+    if (out_row >= p.m || out_column >= n) return;
+    const float result = p.has_aux ? value[0] + residual : value[0];
+    if (p.out_f32) p.out_f32[(size_t)out_row * n + out_column] = result;
+    else p.out[0][(size_t)out_row * n + out_column] = __float2half_rn(result);
+    return;
+  }
+  const float partner = EPI == kEpiSplitF32 ? __shfl_xor_sync(0xffffffffu, value[0], 2) : 0.0f;
+  write_position<1, NMAT, EPI>(p, value, partner, matrix, tile, n, 0u, warp, lane);
+}
+
+// Returns -1 for what the kernel does not cover.  Multiples of 512 go to the kernel with a shared-memory pipeline, which
+// absorbs norms as well.
+template <int EPI, int NMAT>
+int launch_short_as(const KernelArgs& args, const GemvProblem& p) {
+  uint32_t tiles = 0;
+  const uint32_t matrices = EPI == kEpiQkv ? p.matrices : 1u;
+  for (uint32_t i = 0; i < matrices; ++i) tiles += (p.mat[i].n + 15u) / 16u;
+  auto run = [&](auto kernel) {
+    launch_kernel(args, kernel, dim3(tiles), dim3(kShortWarps * 32), 0, p);
+    return check_launch(args);
+  };
+  switch ((p.k / 64u + kShortWarps - 1u) / kShortWarps) {
+    case 1: return run(w4a16_gemv_short_kernel<NMAT, EPI, 1>);
+    case 2: return run(w4a16_gemv_short_kernel<NMAT, EPI, 2>);
+    case 3: return run(w4a16_gemv_short_kernel<NMAT, EPI, 3>);
+    default: return run(w4a16_gemv_short_kernel<NMAT, EPI, (int)kShortGroups>);
+  }
+}
+
+int launch_short(const KernelArgs& args, const GemvProblem& p, int epilogue, bool affine) {
+  if (affine || p.x_rows > 8u || p.k % 512u == 0 || p.k > 64u * kShortWarps * kShortGroups) return -1;
+  if (epilogue != kEpiSplitF32 && p.x_rows != p.m) return -1;
+  if (p.norm_weight != nullptr && (epilogue == kEpiSplitF32 || (((uintptr_t)p.norm_weight | (uintptr_t)p.norm_out) & 15u) != 0)) return -1;
+  switch (epilogue) {
+    case kEpiLinear: return launch_short_as<kEpiLinear, 1>(args, p);
+    case kEpiQkv: return launch_short_as<kEpiQkv, 1>(args, p);
+    case kEpiDualSwiglu: return launch_short_as<kEpiDualSwiglu, 2>(args, p);
+    case kEpiTagged: return launch_short_as<kEpiTagged, 1>(args, p);
+    case kEpiSplitF32: return p.x_rows == 8u ? launch_short_as<kEpiSplitF32, 1>(args, p) : -1;
+    default: return -1;
+  }
+}
+
 template <int NT, int NMAT, int EPI, bool AFFINE>
 int launch_one(const KernelArgs& args, const GemvProblem& p) {
   uint32_t total_tiles = 0;
@@ -294,8 +496,13 @@ int launch_w4a16_gemv(const KernelArgs& args, GemvProblem problem, int epilogue,
   }
   if (problem.k_warps == 0) problem.k_warps = pick_k_warps(problem.k);
 
-  // A norm folded into this product: only the pipelined small-batch kernel stages activations in a
-  // form that can absorb it; otherwise run the norm as its own kernel first.
+  {
+    const int status = launch_short(args, problem, epilogue, affine);
+    if (status >= 0) return status;
+  }
+
+  // A norm folded into this product: of the others only the pipelined small-batch kernel stages
+  // activations in a form that can absorb it; otherwise run the norm as its own kernel first.
   if (problem.norm_weight != nullptr) {
     const bool absorbs = !affine && problem.x_rows <= 8 && (size_t)problem.x_rows * problem.k <= 16384 &&
                          epilogue != kEpiSplitF32 && problem.k % 512 == 0;

@@ -133,3 +133,52 @@ def test_prompt_tiles_and_fused_projections(runtime, oracle, m, k, columns):
         wanted = [oracle.w4a16_linear(x, *pair) for pair in matrices]
     for output, want in zip(outputs, wanted):
         assert_close_f16(output.buffer.to_numpy(np.float16, want.shape), want)
+
+
+@pytest.mark.parametrize("rows,k,n", [(1, 64, 1), (1, 576, 200), (8, 576, 33), (3, 1984, 17), (2, 1088, 16), (5, 448, 50)])
+def test_short_sums(runtime, oracle, monkeypatch, rows, k, n):
+    """Few rows and a K that is no multiple of 512: a plain product with a residual, three matrices as one launch, and a plan
+    that folds the RMS norm ahead of a product, whose rows equal the stand-alone norm's byte for byte."""
+    from conftest import assert_close_f16
+    from helpers import random_w4
+    from llmopt_b200 import dispatch, parameters
+    from llmopt_b200.cuda_native import Buffer, DispatchItem, Prebaked
+
+    rng = np.random.default_rng(k + rows)
+    x = rng.standard_normal((rows, k)).astype(np.float16)
+    residual = rng.standard_normal((rows, n)).astype(np.float16)
+    matrices = [random_w4(rng, columns, k) for columns in (n, 5, 40)]
+    tensor = lambda array, kind="float16": dispatch.Tensor(Buffer.of_array(runtime, array), array.shape, kind)
+    weights = [(tensor(packed, "uint8"), tensor(scale)) for packed, scale in matrices]
+    outputs = [tensor(np.full((rows, len(packed)), np.nan, np.float16)) for packed, _ in matrices]
+    context = dispatch.Context(runtime)
+    in_place = tensor(residual)  # the residual's own buffer takes the sum
+    dispatch.dispatch_w4a16_linear(context, input=tensor(x), weight=weights[0][0], scale=weights[0][1], output=in_place,
+                                   bias=in_place, bias_row_stride=n)
+    assert_close_f16(in_place.buffer.to_numpy(np.float16, (rows, n)), oracle.w4a16_linear(x, *matrices[0], residual, n))
+    (q, k_, v) = weights
+    dispatch.dispatch_w4a16_qkv_linear_command(
+        context, input=tensor(x), q_weight=q[0], q_scale=q[1], k_weight=k_[0], k_scale=k_[1], v_weight=v[0], v_scale=v[1],
+        q_output=outputs[0], k_output=outputs[1], v_output=outputs[2])
+    for output, pair in zip(outputs, matrices):
+        assert_close_f16(output.buffer.to_numpy(np.float16, output.shape), oracle.w4a16_linear(x, *pair))
+
+    weight = rng.uniform(0.5, 1.5, size=k).astype(np.float16)
+    results, counts = [], []
+    for fold in ("1", "0"):
+        monkeypatch.setenv("LLMOPT_CUDA_FOLD_NORMS", fold)
+        normed = Buffer.of_array(runtime, np.full((rows, k), np.nan, np.float16))
+        out = Buffer.of_array(runtime, np.full((rows, n), np.nan, np.float16))
+        scales = weights[0][1].buffer
+        plan = Prebaked(runtime, [
+            DispatchItem("llmopt_rms_norm_f16_simd", [Buffer.of_array(runtime, x), Buffer.of_array(runtime, weight), normed],
+                         parameters.rms_norm(rows=rows, width=k, epsilon=1e-5), (256, 1, 1), (256, 1, 1)),
+            DispatchItem("llmopt_w4a16_linear_f16_g64_m4", [normed, weights[0][0].buffer, scales, scales, out],
+                         parameters.u32s([rows, n, k, 0, 0]), (256, 1, 1), (256, 1, 1))], None, None)
+        plan.execute(token=0, past_tokens=0)
+        counts.append(plan.kernel_count())
+        results.append((normed.to_numpy(np.float16, (rows, k)), out.to_numpy(np.float16, (rows, n))))
+    assert counts[0] == counts[1] - 1
+    assert np.array_equal(results[0][0].view(np.uint16), results[1][0].view(np.uint16))
+    assert np.array_equal(results[0][1].view(np.uint16), results[1][1].view(np.uint16))
+    assert_close_f16(results[0][1], oracle.w4a16_linear(results[0][0], *matrices[0]))
