@@ -477,8 +477,9 @@ paged_split_kernel(const __half* __restrict__ query, const uint8_t* __restrict__
       mine[16 + head * D + dim] = out[s][j];
     }
   __syncthreads();
-  float* record = cluster > 0 ? stage + kWarps * kRecord
-                              : scratch + (((size_t)batch * p.kv_heads + kv_head) * splits + split) * kRecord;
+  // two pointers and not one: a store that may be to either memory is slow, and orders the reads of `stage` behind it
+  float* const own = stage + kWarps * kRecord;
+  float* const record = scratch + (((size_t)batch * p.kv_heads + kv_head) * splits + split) * kRecord;
   // only the columns of heads that exist are merged and written (the merge kernel reads no others)
   for (uint32_t index = threadIdx.x; index < min(heads_per_kv, 8u) * D; index += kWarps * 32) {
     const uint32_t head = index / D;
@@ -492,11 +493,20 @@ paged_split_kernel(const __half* __restrict__ query, const uint8_t* __restrict__
       total += weight * stage[w * kRecord + 16 + index];
       denominator += weight * stage[w * kRecord + 8 + head];
     }
-    record[16 + index] = total;
-    if (index % D == 0) {
-      // records carry the maximum in natural units; a split without keys says -inf
-      record[head] = merged_max <= 0.5f * kLowest ? -INFINITY : merged_max * 0.6931471805599453f;
-      record[8 + head] = denominator;
+    // records carry the maximum in natural units; a split without keys says -inf
+    const float natural = merged_max <= 0.5f * kLowest ? -INFINITY : merged_max * 0.6931471805599453f;
+    if (cluster > 0u) {
+      own[16 + index] = total;
+      if (index % D == 0) {
+        own[head] = natural;
+        own[8 + head] = denominator;
+      }
+    } else {
+      record[16 + index] = total;
+      if (index % D == 0) {
+        record[head] = natural;
+        record[8 + head] = denominator;
+      }
     }
   }
   if (cluster == 0u) return;
@@ -525,15 +535,15 @@ paged_split_kernel(const __half* __restrict__ query, const uint8_t* __restrict__
     const float current = half_at(current_value + current_base + d);
     const float score_now = warp_sum(dot) * p.scale;
     float maximum = score_now;
-    for (uint32_t other = 0; other < cluster; ++other) maximum = fmaxf(maximum, cluster_load(record + head, other));
+    for (uint32_t other = 0; other < cluster; ++other) maximum = fmaxf(maximum, cluster_load(own + head, other));
     const float now = expf(score_now - maximum);
     float total = now * current, denominator = now;
 #pragma unroll 4
     for (uint32_t other = 0; other < cluster; ++other) {
-      const float top = cluster_load(record + head, other);
+      const float top = cluster_load(own + head, other);
       const float weight = top == -INFINITY ? 0.0f : expf(top - maximum);
-      denominator = fmaf(weight, cluster_load(record + 8 + head, other), denominator);
-      total = fmaf(weight, cluster_load(record + 16 + index, other), total);
+      denominator = fmaf(weight, cluster_load(own + 8 + head, other), denominator);
+      total = fmaf(weight, cluster_load(own + 16 + index, other), total);
     }
     results[i] = denominator == 0.0f ? 0.0f : total / denominator;
   }
