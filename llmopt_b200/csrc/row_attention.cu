@@ -82,20 +82,24 @@ __device__ __forceinline__ float gate_of(const RowAttentionParams& p, const T* g
 }
 
 // ---- one CTA per (row, head) ---------------------------------------------------------------------
-// Bound by the latency of slot, key and value loads: a warp has the keys of a whole batch in flight and shares the sums
-// over lanes among them, and four warps take every fourth batch.  One key at a time and one warp per head, fp32, 16 heads
-// of 128: 112 us for a row with 100 keys behind it, 66 for a prompt of 100; now 40 and 39 (with the launch).
-template <int SEGMENTS> __host__ __device__ constexpr int row_batch() { return SEGMENTS <= 4 ? 8 : SEGMENTS <= 8 ? 4 : 2; }
-constexpr uint32_t kRowWarps = 4;
+// Bound by the latency of slot, key and value loads: scores of kRowKeys keys are formed side by side, eight keys of a warp in
+// flight, then the weights of all of them, then a thread per column adds the values.  The arithmetic is that of a walk over
+// the keys one after the other (online softmax), to the last bit: decoders that divide by nearly cancelling sums show every
+// change of it.  Such a walk by one warp took 112 us for a row with 100 keys behind it (fp32, 16 heads of 128) and 66 us
+// for a prompt of 100; now 46 and 34,
+// launch included.
+template <int SEGMENTS> __host__ __device__ constexpr int row_batch() { return SEGMENTS <= 8 ? 8 : 4; }
+constexpr uint32_t kRowWarps = 4, kRowThreads = kRowWarps * 32u, kRowKeys = kRowThreads;
 
 template <typename T, int SEGMENTS>
-__global__ void __launch_bounds__(kRowWarps * 32) attention_rows_kernel(const T* query, const T* pool, const uint32_t* table,
+__global__ void __launch_bounds__(kRowThreads) attention_rows_kernel(const T* query, const T* pool, const uint32_t* table,
                                                              const uint32_t* past, const uint32_t* sequence_rows, T* out,
                                                              const T* gate, RowAttentionParams p, uint32_t* error_word) {
   grid_chain_prologue();
-  constexpr int KEYS = row_batch<SEGMENTS>();
+  constexpr int KEYS = row_batch<SEGMENTS>(), COLUMNS = (SEGMENTS * 32 + kRowThreads - 1) / kRowThreads;
   constexpr uint32_t kSpan = 32 / KEYS;  // lanes that end with the same key
-  __shared__ float parts[kRowWarps][SEGMENTS * 32], tops[kRowWarps], totals[kRowWarps];
+  __shared__ uint32_t slots[kRowKeys];
+  __shared__ float scores[kRowKeys], keeps[kRowKeys], weights[kRowKeys], warp_tops[kRowWarps];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, item = blockIdx.x;
   const uint32_t row = item / p.heads, head = item % p.heads, sequence = row / p.tokens;
   const uint32_t kv_head = head / (p.heads / p.kv_heads);
@@ -103,95 +107,97 @@ __global__ void __launch_bounds__(kRowWarps * 32) attention_rows_kernel(const T*
   const Visible<true> visible(p, position, position);
   const uint32_t count = visible.count();
   const KeyRows rows = key_rows(p, table, sequence_rows[sequence]);
-  float q[SEGMENTS], o[SEGMENTS];
+  float q[SEGMENTS], o[COLUMNS];
 #pragma unroll
   for (int s = 0; s < SEGMENTS; ++s) {
     const uint32_t c = lane + s * 32u;
     q[s] = c < p.dim ? as_float(query[(size_t)row * p.query_stride + p.query_column + head * p.dim + c]) : 0.0f;
-    o[s] = 0.0f;
   }
-  const bool sink = p.sink && warp == 0;
-  float top = sink ? 0.0f : kLowest, total = sink && lane == 0 ? 1.0f : 0.0f;  // total: of this lane's keys
-  const uint32_t step = kRowWarps * KEYS;
-  auto slot_of = [&](uint32_t index) { return index < count ? rows(visible.position(index), error_word) : 0u; };
-  uint32_t slots = slot_of(warp * KEYS + lane % KEYS);
-  for (uint32_t begin = warp * KEYS; begin < count; begin += step) {
-    const uint32_t present = min((uint32_t)KEYS, count - begin), now = slots;
-    float k[KEYS][SEGMENTS], v[KEYS][SEGMENTS];
 #pragma unroll
-    for (int j = 0; j < KEYS; ++j) {
-      const uint32_t slot = __shfl_sync(0xffffffffu, now, j);
-      const T* cached = pool + (size_t)slot * p.token_stride;
+  for (int i = 0; i < COLUMNS; ++i) o[i] = 0.0f;
+  float top = p.sink ? 0.0f : kLowest, total = p.sink ? 1.0f : 0.0f;
+  for (uint32_t begin = 0; begin < count; begin += kRowKeys) {
+    const uint32_t present = min(kRowKeys, count - begin);
+    __syncthreads();  // the keys before are read
+    if (threadIdx.x < present) slots[threadIdx.x] = rows(visible.position(begin + threadIdx.x), error_word);
+    __syncthreads();
+    for (uint32_t first = warp * KEYS; first < present; first += kRowWarps * KEYS) {
+      float k[KEYS][SEGMENTS], dots[KEYS];
 #pragma unroll
-      for (int s = 0; s < SEGMENTS; ++s) {
-        const uint32_t c = lane + s * 32u;
-        k[j][s] = j < present && c < p.dim ? as_float(cached[p.key_offset + kv_head * p.dim + c]) : 0.0f;
+      for (int j = 0; j < KEYS; ++j) {
+        const T* cached = pool + (size_t)slots[min(first + j, present - 1u)] * p.token_stride + p.key_offset + kv_head * p.dim;
+#pragma unroll
+        for (int s = 0; s < SEGMENTS; ++s) k[j][s] = as_float(cached[min(lane + s * 32u, p.dim - 1u)]);
       }
 #pragma unroll
-      for (int s = 0; s < SEGMENTS; ++s) {
-        const uint32_t c = lane + s * 32u;
-        v[j][s] = j < present && c < p.vdim ? as_float(cached[p.value_offset + kv_head * p.vdim + c]) : 0.0f;
+      for (int j = 0; j < KEYS; ++j) {
+        dots[j] = 0.0f;
+#pragma unroll
+        for (int s = 0; s < SEGMENTS; ++s)
+          if (lane + s * 32u < p.dim) dots[j] = fmaf(q[s], k[j][s], dots[j]);
+      }
+      // the sum over lanes at distances 16, 8, ..: each exchange halves the keys that a lane keeps, lane l ends with l / kSpan
+#pragma unroll
+      for (int half = KEYS / 2; half > 0; half >>= 1) {
+        const bool upper = (lane & (half * kSpan)) != 0;
+#pragma unroll
+        for (int i = 0; i < half; ++i) {
+          const float sent = upper ? dots[i] : dots[i + half], kept = upper ? dots[i + half] : dots[i];
+          dots[i] = kept + __shfl_xor_sync(0xffffffffu, sent, half * kSpan);
+        }
+      }
+      float score = dots[0];
+#pragma unroll
+      for (uint32_t offset = kSpan / 2; offset > 0; offset >>= 1) score += __shfl_xor_sync(0xffffffffu, score, offset);
+      score *= p.scale;
+      if (p.softcap > 0.0f) score = p.softcap * tanhf(score / p.softcap);
+      if (lane % kSpan == 0 && first + lane / kSpan < present) scores[first + lane / kSpan] = score;
+    }
+    __syncthreads();
+    // the running maximum up to and with this thread's key, and ahead of it
+    const float score = threadIdx.x < present ? scores[threadIdx.x] : -INFINITY;
+    float highest = score;
+#pragma unroll
+    for (uint32_t offset = 1; offset < 32u; offset <<= 1) {
+      const float earlier = __shfl_up_sync(0xffffffffu, highest, offset);
+      if (lane >= offset) highest = fmaxf(earlier, highest);
+    }
+    if (lane == 31u) warp_tops[warp] = highest;
+    float before = __shfl_up_sync(0xffffffffu, highest, 1);
+    __syncthreads();
+    float ahead = top;
+    for (uint32_t w = 0; w < warp; ++w) ahead = fmaxf(ahead, warp_tops[w]);
+    before = lane == 0 ? ahead : fmaxf(ahead, before);
+    const float next = fmaxf(before, score);
+    keeps[threadIdx.x] = expf(before - next);
+    weights[threadIdx.x] = expf(score - next);
+#pragma unroll
+    for (uint32_t w = 0; w < kRowWarps; ++w) top = fmaxf(top, warp_tops[w]);
+    __syncthreads();
+    const T* values[COLUMNS];
+#pragma unroll
+    for (int i = 0; i < COLUMNS; ++i) values[i] = pool + p.value_offset + kv_head * p.vdim + min(threadIdx.x + i * kRowThreads, p.vdim - 1u);
+    constexpr uint32_t kAhead = COLUMNS == 1 ? 16 : 4;
+    for (uint32_t at = 0; at < present; at += kAhead) {
+      float v[kAhead][COLUMNS];
+#pragma unroll
+      for (uint32_t j = 0; j < kAhead; ++j)
+#pragma unroll
+        for (int i = 0; i < COLUMNS; ++i) v[j][i] = as_float(values[i][(size_t)slots[min(at + j, present - 1u)] * p.token_stride]);
+#pragma unroll
+      for (uint32_t j = 0; j < kAhead; ++j) {
+        if (at + j >= present) break;
+        const float keep = keeps[at + j], weight = weights[at + j];
+        total = total * keep + weight;
+#pragma unroll
+        for (int i = 0; i < COLUMNS; ++i) o[i] = o[i] * keep + weight * v[j][i];
       }
     }
-    // the slots of the next batch are on their way while this one's keys are
-    if (begin + step < count) slots = slot_of(begin + step + lane % KEYS);
-    float dots[KEYS];
-#pragma unroll
-    for (int j = 0; j < KEYS; ++j) {
-      dots[j] = 0.0f;
-#pragma unroll
-      for (int s = 0; s < SEGMENTS; ++s) dots[j] = fmaf(q[s], k[j][s], dots[j]);
-    }
-    // each exchange halves the keys that a lane keeps: lane l ends with key l / kSpan
-#pragma unroll
-    for (int half = KEYS / 2; half > 0; half >>= 1) {
-      const bool upper = (lane & (half * kSpan)) != 0;
-#pragma unroll
-      for (int i = 0; i < half; ++i) {
-        const float sent = upper ? dots[i] : dots[i + half], kept = upper ? dots[i + half] : dots[i];
-        dots[i] = kept + __shfl_xor_sync(0xffffffffu, sent, half * kSpan);
-      }
-    }
-    float score = dots[0];
-#pragma unroll
-    for (uint32_t offset = kSpan / 2; offset > 0; offset >>= 1) score += __shfl_xor_sync(0xffffffffu, score, offset);
-    score *= p.scale;
-    if (p.softcap > 0.0f) score = p.softcap * tanhf(score / p.softcap);
-    if (lane / kSpan >= present) score = -INFINITY;
-    float next = fmaxf(top, score);
-#pragma unroll
-    for (uint32_t offset = kSpan; offset < 32u; offset <<= 1) next = fmaxf(next, __shfl_xor_sync(0xffffffffu, next, offset));
-    const float keep = expf(top - next), weight = expf(score - next);
-    top = next;
-    total = total * keep + (lane % kSpan == 0 ? weight : 0.0f);
-#pragma unroll
-    for (int s = 0; s < SEGMENTS; ++s) o[s] *= keep;
-#pragma unroll
-    for (int j = 0; j < KEYS; ++j) {
-      const float one = __shfl_sync(0xffffffffu, weight, j * kSpan);
-#pragma unroll
-      for (int s = 0; s < SEGMENTS; ++s) o[s] = fmaf(one, v[j][s], o[s]);
-    }
   }
-  total = warp_sum(total);
 #pragma unroll
-  for (int s = 0; s < SEGMENTS; ++s) parts[warp][lane + s * 32u] = o[s];
-  if (lane == 0) tops[warp] = top, totals[warp] = total;
-  __syncthreads();
-  float highest = tops[0];
-#pragma unroll
-  for (uint32_t w = 1; w < kRowWarps; ++w) highest = fmaxf(highest, tops[w]);
-  float factor[kRowWarps], sum = 0.0f;
-#pragma unroll
-  for (uint32_t w = 0; w < kRowWarps; ++w) {
-    factor[w] = expf(tops[w] - highest);
-    sum = fmaf(totals[w], factor[w], sum);
-  }
-  for (uint32_t c = threadIdx.x; c < p.vdim; c += kRowWarps * 32u) {
-    float value = 0.0f;
-#pragma unroll
-    for (uint32_t w = 0; w < kRowWarps; ++w) value = fmaf(parts[w][c], factor[w], value);
-    out[(size_t)item * p.vdim + c] = from_float<T>(value / sum * gate_of<true>(p, gate, row, head, c));
+  for (int i = 0; i < COLUMNS; ++i) {
+    const uint32_t c = threadIdx.x + i * kRowThreads;
+    if (c < p.vdim) out[(size_t)item * p.vdim + c] = from_float<T>(o[i] / total * gate_of<true>(p, gate, row, head, c));
   }
 }
 
@@ -695,7 +701,7 @@ int run_rows(const KernelArgs& args, const RowAttentionParams& p) {
   LLMOPT_REQUIRE(items <= 0x7fffffffu, "too many rows");
   const uint32_t widest = p.dim > p.vdim ? p.dim : p.vdim;
   auto run = [&](auto kernel) {
-    launch_kernel(args, kernel, dim3((uint32_t)items), dim3(kRowWarps * 32), 0, (const T*)args.buffers[0],
+    launch_kernel(args, kernel, dim3((uint32_t)items), dim3(kRowThreads), 0, (const T*)args.buffers[0],
                   (const T*)args.buffers[1], (const uint32_t*)args.buffers[2], (const uint32_t*)args.buffers[3],
                   (const uint32_t*)args.buffers[4], (T*)args.buffers[5], (const T*)args.buffers[7], p, context_device_error(args.ctx));
   };
