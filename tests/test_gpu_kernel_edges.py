@@ -80,7 +80,7 @@ def test_short_conv_steps_of_a_plan_as_one_launch(runtime, oracle, apart, shared
 @pytest.mark.parametrize("m,n,k", [(1, 9, 4), (2, 8, 516), (4, 7, 128), (5, 33, 1028), (8, 16, 260), (9, 65, 36), (32, 64, 32),
                                    (33, 63, 2052), (64, 128, 1024), (65, 130, 96), (100, 256, 2048), (129, 20, 7168)])
 def test_dense_fp32(runtime, m, n, k):
-    """Vectors of a few columns, tiles and their splits of k.  fp32 sums of k products in parts: an error of a few times
+    """Streams of a few rows and tiles of every size.  fp32 sums of k products: an error of a few times
     2^-24 sqrt(k) of the terms' size, where the result has sqrt(k) of them; 3e-6 of the largest result."""
     from llmopt_b200 import parameters
 
@@ -100,6 +100,26 @@ def test_dense_fp32(runtime, m, n, k):
         runtime.dispatch("llmopt_dense_linear_f32", buffers=buffers, parameters=parameters.dense_linear(
             m=m, n=n, k=k, split=n, has_bias=True, epilogue="silu_pair"))
         close(download(buffers[3], (m, n // 2)), plain.silu(y[:, 0::2]) * y[:, 1::2], 6e-6)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 18, 4), (3, 40, 1028), (8, 33, 516), (13, 65, 2052), (32, 64, 96), (33, 63, 36),
+                                   (64, 130, 1024), (100, 2048, 260), (100, 7168, 64), (129, 20, 7168)])
+def test_dense_fp32_equals_the_general_kernels(runtime, m, n, k):
+    """Rows off 16-byte boundaries take the general kernels; the others add in the same order, to the last bit."""
+    from llmopt_b200 import parameters
+
+    rng = np.random.default_rng(m + n)
+    x, w, bias = (rng.standard_normal(shape).astype(np.float32) for shape in ((m, k), (n, k), n))
+    shifted = upload(runtime, np.concatenate((np.zeros(1, np.float32), x.reshape(-1)))).view(4, 4 * m * k)
+    results = []
+    for rows in (upload(runtime, x), shifted):
+        out = [empty(runtime, m * n), empty(runtime, m * n)]
+        runtime.dispatch("llmopt_dense_linear_f32", buffers=[
+            rows, upload(runtime, w), upload(runtime, bias), *out, upload(runtime, np.zeros(m, np.int64)), empty(runtime, 16)],
+            parameters=parameters.dense_linear(m=m, n=n, k=k, split=n // 3, has_bias=True, epilogue=None))
+        results.append([download(one, (m, columns)) for one, columns in zip(out, (n // 3, n - n // 3))])
+    for here, general in zip(*results):
+        assert np.array_equal(here, general)
 
 
 @pytest.mark.parametrize("m,k,columns", [(66, 192, (40,)), (257, 1024, (300,)), (300, 4608, (130,)), (700, 512, (1100,)),
