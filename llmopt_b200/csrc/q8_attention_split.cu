@@ -777,9 +777,28 @@ int launch_paged_attention_split_on(const KernelArgs& args, const PagedParams& p
   return launch_split_as(args, p, slot_batch_stride, scratch, splits, pool_tokens, {0u, 0u});
 }
 
+// A cluster writes its part of the output while others still read.  Without clusters the output is written after all reads,
+// so memory that is dead by then may take it (a plan's raw rows behind the rotary record).  Nothing that another cluster reads
+// may lie under the output; rows at the output's own places are read and written by the same cluster.
+static bool output_apart(const KernelArgs& args, const PagedParams& p) {
+  const size_t row = (size_t)p.batches * p.head_dim * 2, query_bytes = row * p.query_heads;
+  const uintptr_t output = (uintptr_t)args.buffers[6];
+  auto under = [&](const void* read, size_t bytes) {
+    return (uintptr_t)read < output + query_bytes && output < (uintptr_t)read + bytes;
+  };
+  const RotaryPackFusion* fusion = args.rotary_fusion;
+  const void* query = fusion ? fusion->q_input : args.buffers[0];
+  if ((uintptr_t)query != output && under(query, query_bytes)) return false;
+  if (under(args.buffers[3], args.lengths[3]) || under(args.buffers[4], args.lengths[4])) return false;
+  if (fusion == nullptr) return true;
+  const size_t trigonometric = (size_t)(fusion->rotary.trig_batches == 1u ? 1u : p.batches) * fusion->rotary.width * 2;
+  return !under(fusion->k_input, row * p.kv_heads) && !under(fusion->cosine, trigonometric) &&
+         !under(fusion->sine, trigonometric) && !under(fusion->slots, (size_t)p.batches * 4);
+}
+
 int launch_paged_attention_split(const KernelArgs& args, const PagedParams& p, uint32_t slot_batch_stride,
                                  uint32_t pool_tokens) {
-  const ClusterPlan plan = pick_cluster(args, p, slot_batch_stride);
+  const ClusterPlan plan = output_apart(args, p) ? pick_cluster(args, p, slot_batch_stride) : ClusterPlan{0u, 0u};
   if (plan.ctas > 0u) return launch_split_as(args, p, slot_batch_stride, nullptr, 0u, pool_tokens, plan);
   const uint32_t splits = paged_pick_splits(args, p);
   const size_t bytes =

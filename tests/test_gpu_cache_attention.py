@@ -512,6 +512,70 @@ def test_plan_hands_rotary_and_pack_to_the_attention_byte_for_byte(runtime, monk
     assert not np.any(np.isnan(plain[4].view(np.float16)))
 
 
+@pytest.mark.parametrize("under", ["raw keys", "cosine", "half of the raw query", "raw query"])
+def test_plan_attention_output_in_memory_of_dead_rows(runtime, under):
+    """The raw rows and the trigonometric rows are dead behind the rotary record, so a plan may keep the attention output in
+    their memory.  More (sequence, KV head) pairs than fit on the chip together: the later ones still read raw rows
+    when the first are done.  The same as with the output in memory of its own (other splits of the keys: the bound
+    of the kernel's parity)."""
+    from llmopt_b200 import dispatch, parameters
+    from llmopt_b200.cuda_native import Batch, Buffer, DispatchItem, Prebaked
+    from llmopt_b200.kv_cache import AttentionLayer, Layout
+
+    rng = np.random.default_rng(31)
+    batch, q_heads, k_heads, dim, group, past = 8, 128, 64, 64, 64, 40
+    layout = Layout([AttentionLayer(k_heads, dim)], group_size=group)
+    region, capacity, segment = layout.attentions[0], past + 1, k_heads * dim
+    raw = [rng.standard_normal((batch, 1, heads, dim)).astype(np.float16) for heads in (q_heads, k_heads)]
+    angle = rng.uniform(0, 6.28, size=(batch, dim))
+    raw += [np.cos(angle).astype(np.float16), np.sin(angle).astype(np.float16)]
+    v = rng.standard_normal((batch, k_heads, dim)).astype(np.float16)
+    pool_bytes = random_pool(rng, batch * capacity, layout.bytes_per_token, layout.token_elements, group)
+    slot_table = np.arange(batch * capacity, dtype=np.uint32).reshape(batch, capacity)
+    out_bytes = batch * q_heads * dim * 2
+
+    def run(place):
+        # one arena: query, keys, cosine, sine, room for an output
+        starts = np.concatenate(([0], np.cumsum([a.nbytes for a in raw])))
+        arena = Buffer.of_array(runtime, np.concatenate([a.reshape(-1) for a in raw] + [np.zeros(2 * out_bytes // 2, np.float16)]))
+        q, k, cos, sin = (arena.view(int(at), a.nbytes) for at, a in zip(starts, raw))
+        at = {"apart": starts[4], "raw keys": starts[1], "cosine": starts[2], "half of the raw query": out_bytes // 2, "raw query": 0}[place]
+        out = arena.view(int(at), out_bytes)
+        pool = Buffer.of_array(runtime, pool_bytes)
+        q_out, k_out = Buffer.create(runtime, raw[0].nbytes), Buffer.create(runtime, raw[1].nbytes)
+        v_in = Buffer.of_array(runtime, v)
+        commands = Batch(runtime)
+        dispatch.dispatch_paged_attention_q8(
+            dispatch.Context(runtime, batch=commands),
+            config=dispatch.PagedAttentionConfig(token_elements=layout.token_elements, key_offset=region.key_offset,
+                                                 value_offset=region.value_offset, group_size=group,
+                                                 token_stride=layout.bytes_per_token, scale=1.0 / np.sqrt(dim)),
+            query=dispatch.Tensor(q_out, (batch, q_heads, 1, dim)), current_key=dispatch.Tensor(k_out, (batch, k_heads, 1, dim)),
+            current_value=dispatch.Tensor(v_in, (batch, k_heads, 1, dim)), pool=dispatch.Tensor(pool, (pool_bytes.size,), "uint8"),
+            slots=dispatch.Tensor(Buffer.of_array(runtime, np.ascontiguousarray(slot_table[:, :past])), (batch, past), "uint32"),
+            output=dispatch.Tensor(out, (batch, 1, q_heads, dim)), slot_batch_stride=past)
+        attention = commands.pending[0]
+        commands.abort()
+        plan = Prebaked(runtime, [
+            DispatchItem("llmopt_rotary_qk_f16_simd_h64", [q, k, cos, sin, q_out, k_out],
+                         parameters.rotary_qk(batches=batch, tokens=1, q_heads=q_heads, k_heads=k_heads, width=dim,
+                                              half_dimension=dim // 2, trig_batches=batch), (256, 1, 1), (256, 1, 1)),
+            DispatchItem("llmopt_cache_pack_attention_q8_pair_simd",
+                         [k_out, v_in, Buffer.of_array(runtime, np.ascontiguousarray(slot_table[:, past])), pool],
+                         parameters.cache_attention_pair(
+                             items=batch, key_segment_offset=region.key_offset, value_segment_offset=region.value_offset,
+                             heads=1, head_dim=segment, group_size=group, token_elements=layout.token_elements,
+                             token_groups=layout.token_groups, token_stride=layout.bytes_per_token, source_items=batch,
+                             source_offset=0), (256, 1, 1), (256, 1, 1)),
+            attention], None, None)
+        plan.execute(token=0, past_tokens=past)
+        return k_out.to_numpy(np.uint16), pool.to_numpy(np.uint8), out.to_numpy(np.float16)
+
+    want, got = run("apart"), run(under)
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+    assert_close_f16(got[2], want[2].astype(np.float64), label=under)
+
+
 def test_plan_refuses_tokens_beyond_its_tables(runtime):
     """A replayed plan indexes device tables with the per-token values it is given: a row binding
     reads row ``past_tokens``, paged attention reads ``past_tokens`` slot entries.  Values beyond
