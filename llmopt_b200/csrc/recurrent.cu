@@ -246,11 +246,21 @@ int launch_short_conv_prefill(const KernelArgs& args) {
     state_in = (const __half*)args.buffers[4];
   }
   if (has_initial == 0) state_in = nullptr;
-  // A state updated in place is read by the first strip and written by the last one: a single strip then, whose thread reads
-  // before it writes.  So too for prompts whose strips are more than a grid has rows.
-  const uint8_t *in = (const uint8_t*)state_in, *out = (const uint8_t*)args.buffers[3];
+  // One strip, whose thread reads ahead of what it writes, where strips would write what others still read: a state
+  // updated in place (read by the first strip, written by the last one), outputs or the state in the memory of the projected
+  // rows (a token's output can take the place of an input of its own channel that is read by then).  So too for prompts whose
+  // strips are more than a grid has rows.
   const size_t state_bytes = (size_t)channels * 6;
-  const bool in_place = in != nullptr && in < out + state_bytes && out < in + state_bytes;
+  auto overlap = [](const void* a, size_t a_bytes, const void* b, size_t b_bytes) {
+    return (uintptr_t)a < (uintptr_t)b + b_bytes && (uintptr_t)b < (uintptr_t)a + a_bytes;
+  };
+  bool in_place = false;
+  for (int written = 2; written < 4; ++written) {
+    const void* target = args.buffers[written];
+    const size_t bytes = written == 2 ? (size_t)tokens * channels * 2 : state_bytes;
+    in_place = in_place || overlap(target, bytes, args.buffers[0], (size_t)tokens * channels * 6) ||
+               (state_in != nullptr && overlap(target, bytes, state_in, state_bytes));
+  }
   const uint32_t strips = in_place || tokens == 0 ? 1 : (tokens + kConvStrip - 1) / kConvStrip;
   const uint32_t strip = strips == 1 || strips > 65535 ? tokens : kConvStrip;
   launch_kernel(args, short_conv_prefill_kernel, dim3((channels + 255) / 256, strips > 65535 ? 1 : strips), dim3(256), 0,

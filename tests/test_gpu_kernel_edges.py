@@ -5,6 +5,7 @@ import numpy as np
 import pytest
 
 import oracle_mixers as plain
+from mixer_models import bf16_round
 from test_gpu_mixers import close, download, empty, upload
 
 pytestmark = pytest.mark.gpu
@@ -43,6 +44,29 @@ def test_short_conv_prompt_in_strips(runtime, oracle, tokens, start):
     got = out.to_numpy(np.float16, (tokens, channels))
     assert np.all(np.abs(got.astype(np.float64) - want) <= 2.0 ** -10 * np.abs(want) + 2.0 ** -12)
     assert np.array_equal(after.to_numpy(np.uint16), state.view(np.uint16).reshape(-1))
+
+
+@pytest.mark.parametrize("tokens,channels", [(1, 64), (9, 300), (200, 1024), (65, 2051)])
+@pytest.mark.parametrize("part", [0, 1, 2])
+def test_short_conv_prompt_over_its_projections(runtime, tokens, channels, part):
+    """Outputs may take the memory of the projected rows, from any of the first row's three parts on: a token's output then
+    lies where an input of the same channel was that is read by then.  The same bits as in memory of their own."""
+    from llmopt_b200 import parameters
+    from llmopt_b200.cuda_native import Buffer
+
+    rng = np.random.default_rng(tokens + part)
+    rows = rng.standard_normal((tokens, 3 * channels)).astype(np.float16)
+    weight = _half(runtime, rng.standard_normal((channels, 3)))
+
+    def run(over):
+        projected, apart = _half(runtime, rows), Buffer.create(runtime, tokens * channels * 2)
+        out = projected.view(part * channels * 2, tokens * channels * 2) if over else apart
+        state = Buffer.create(runtime, channels * 6)
+        runtime.dispatch("llmopt_short_conv_prefill_f16", buffers=[projected, weight, out, state],
+                         parameters=parameters.short_conv_prefill(tokens=tokens, channels=channels, has_initial_state=False))
+        return out.contents(), state.contents()
+
+    assert run(True) == run(False)
 
 
 @pytest.mark.parametrize("apart,shared_state", [(0, False), (16, False), (0, True)])
