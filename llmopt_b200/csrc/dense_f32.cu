@@ -6,9 +6,8 @@
 // Both add the products of an output in the order of the general kernels (dense_linear.cu: lanes 32 apart, and k one after
 // the other), to the last bit: fp32 is what checkpoints are checked with, and decoders that divide by nearly cancelling sums
 // show every change of it.  k shared out over a cluster, with even and odd k as the halves of packed multiply-adds, was faster (2048 x
-// 2048 x 100 rows 32 us) but moved logits by 2.9e-5.  Now, 100 rows, with the time of 64 x 64 tiles and 4-byte loads: 2048 x
-// 2048 and 2048 x 7168 (20 and 8 of them) 111 us on average, 313 and 438 before; 7168 x 2048 126, 1076 before.  With three
-// stages in place of six and eight 198 and 200.
+// 2048 x 100 rows 32 us) but moved logits by 2.9e-5.  Now, 100 rows back to back over cold operands, with the time of 64 x 64
+// tiles and 4-byte loads: n 2048, k 2048 66 us, 305 before; n 2048, k 7168 227, 1075 before; n 7168, k 2048 123, 337 before.
 #include "dense_linear.cuh"
 
 namespace llmopt {
@@ -17,6 +16,7 @@ namespace {
 constexpr uint32_t kDepth = 32;    // k of a stage: a row is one 128-byte line
 constexpr uint32_t kPitch = kDepth + 4;  // floats; eight consecutive rows start in eight different groups of four banks
 constexpr uint32_t kThreads = 128;
+constexpr uint32_t kMostDown = 65535;  // tiles of rows: a grid's second dimension
 
 // 16 bytes to shared memory, zeros where absent.
 __device__ __forceinline__ void copy_vector(float* to, const float* from, bool present) {
@@ -224,8 +224,8 @@ int run(const KernelArgs& args, DenseProblem p, uint32_t tiles) {
   // The tile for which the fullest SM has the least to read from shared memory, which bounds all of them: 16 (TM + TN) cycles per
   // four k and CTA.  One CTA alone on an SM runs at about half the rate.
   const uint32_t sms = (uint32_t)context_sm_count(args.ctx);
-  auto down = [&](uint32_t high) { return p.plan.tiles ? tiles * (kExpertTile / high) : (p.m + high - 1u) / high; };
-  LLMOPT_REQUIRE(down(32u) <= 65535u, "too many rows");
+  auto down = [&](uint32_t high) { return p.plan.tiles ? tiles * (kExpertTile / high) : p.m / high + (p.m % high ? 1u : 0u); };
+  if (down(64u) > kMostDown) return -1;
   auto cost = [&](uint32_t high, uint32_t wide) {
     // the plan's tiles are 128 rows at most and hold m / tiles on average; those without rows end at once
     const uint32_t rows = p.plan.tiles ? p.m / (tiles ? tiles : 1u) : p.m;
@@ -242,7 +242,7 @@ int run(const KernelArgs& args, DenseProblem p, uint32_t tiles) {
     return check_launch(args);
   };
   const uint32_t large = cost(64u, 128u), middle = cost(64u, 64u), small = cost(32u, 64u);
-  if (small <= middle && small <= large) return launch(dense_f32_tile_kernel<4, 4, STORE>, 32u, 64u);
+  if (down(32u) <= kMostDown && small <= middle && small <= large) return launch(dense_f32_tile_kernel<4, 4, STORE>, 32u, 64u);
   if (middle <= large) return launch(dense_f32_tile_kernel<8, 4, STORE>, 64u, 64u);
   return launch(dense_f32_tile_kernel<8, 8, STORE>, 64u, 128u);
 }

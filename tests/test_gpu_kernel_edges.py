@@ -126,6 +126,36 @@ def test_dense_fp32(runtime, m, n, k):
         close(download(buffers[3], (m, n // 2)), plain.silu(y[:, 0::2]) * y[:, 1::2], 6e-6)
 
 
+@pytest.mark.parametrize("m,experts", [(32 * 65535, 0), (32 * 65535 + 1, 0), (64 * 65535, 0), (128 * 16383, 3), (128 * 16384 + 5, 3)])
+def test_dense_fp32_of_millions_of_rows(runtime, m, experts):
+    """More tiles of 32 rows than a grid holds, up to all that it holds of 64: plain, and rows sorted by expert.  Sums of four
+    products of numbers of at most 4 bits: exact."""
+    from llmopt_b200 import parameters
+
+    rng = np.random.default_rng(m % 1000)
+    n, k = 2, 4
+    x = rng.integers(-8, 8, size=(m, k)).astype(np.float32)
+    w = rng.integers(-8, 8, size=(max(experts, 1), n, k)).astype(np.float32)
+    out = empty(runtime, m * n)
+    if experts:
+        bounds = [0, 100, m - 3, m]
+        tiles = [(e, first, min(first + 128, bounds[e + 1])) for e in range(experts) for first in range(bounds[e], bounds[e + 1], 128)]
+        most = m // 128 + experts
+        assert len(tiles) <= most
+        plan = np.zeros((1 + most, 4), np.uint32)
+        plan[0, 0], plan[1:1 + len(tiles), :3] = len(tiles), tiles
+        runtime.dispatch("llmopt_expert_rows_f32", buffers=[
+            upload(runtime, x), upload(runtime, w), upload(runtime, plan), upload(runtime, np.ones(m, np.float32)), out],
+            parameters=parameters.expert_rows(pairs=m, n=n, k=k, experts=experts, paired=False))
+        want = np.concatenate([x[a:b] @ w[e].T for e, (a, b) in enumerate(zip(bounds, bounds[1:]))])
+    else:
+        spare = empty(runtime, 16)
+        runtime.dispatch("llmopt_dense_linear_f32", buffers=[upload(runtime, x), upload(runtime, w), spare, out, spare, spare, spare],
+                         parameters=parameters.dense_linear(m=m, n=n, k=k, split=n))
+        want = x @ w[0].T
+    assert np.array_equal(download(out, (m, n)), want)
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 18, 4), (3, 40, 1028), (8, 33, 516), (13, 65, 2052), (32, 64, 96), (33, 63, 36),
                                    (64, 130, 1024), (100, 2048, 260), (100, 7168, 64), (129, 20, 7168)])
 def test_dense_fp32_equals_the_general_kernels(runtime, m, n, k):
