@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(kGemvWarps * 32, NT <= 4 ? 2 : 1) expert_step_
   uint32_t mine = 0;
   if (!DOWN) {
     const uint32_t first = min(route[at.first + blockIdx.y], pairs);
-    mine = min(route[at.first + blockIdx.y + 1u] - first, rows);
+    mine = min(route[at.first + blockIdx.y + 1u] - first, min(rows, pairs - first));  // whatever the route says
     w += (size_t)min(route[4 + blockIdx.y], experts - 1u) * p.n * p.k;
 #pragma unroll
     for (int nt = 0; nt < (DOWN ? 1 : NT); ++nt) {
@@ -284,6 +284,8 @@ __global__ void __launch_bounds__(kWideThreads, 1) expert_wide_kernel(const Dens
     rows[wide_chunk(row, blocks, chunk)] = value;
   }
   __syncthreads();
+  // no more than there are slots behind the first, whatever the route says
+  auto rows_of = [&](uint32_t place) { return min(firsts[place + 1u] - firsts[place], min(p.m, pairs - firsts[place])); };
   auto tile_of = [&](uint32_t index, const bf16*& low, const bf16*& high) {
     const uint32_t item = blockIdx.x + index * gridDim.x, place = item / per_expert, n0 = (item - place * per_expert) * 16u;
     const bf16* w = reinterpret_cast<const bf16*>(p.w) + (size_t)chosen[place] * p.n * p.k;
@@ -294,7 +296,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) expert_wide_kernel(const Dens
     WideRing<decltype(tile_of)> ring(wide_shared, tile_of, p.k, mine);
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
     for (uint32_t tile = 0; tile < mine; ++tile) {
-      const uint32_t place = (blockIdx.x + tile * gridDim.x) / per_expert, first = firsts[place], count = min(firsts[place + 1u] - first, p.m);
+      const uint32_t place = (blockIdx.x + tile * gridDim.x) / per_expert, first = firsts[place], count = rows_of(place);
       float sum[NT][4];
       uint32_t own[NT];  // the lane's rows of this expert
 #pragma unroll
@@ -327,7 +329,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) expert_wide_kernel(const Dens
     const uint32_t buffer = tile & 1u, item = blockIdx.x + tile * gridDim.x, place = item / per_expert;
     const uint32_t first = firsts[place];
     DenseTask<kStorePair> task = p;
-    task.m = min(firsts[place + 1u] - first, p.m);
+    task.m = rows_of(place);
     task.row_scale = reinterpret_cast<const float*>(route) + at.score + first;
     task.out = reinterpret_cast<bf16*>(p.out) + (size_t)first * (p.n / 2u);
     wide_barrier_sync(1u + buffer);

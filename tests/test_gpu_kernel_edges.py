@@ -256,3 +256,41 @@ def test_short_sums(runtime, oracle, monkeypatch, rows, k, n):
     assert np.array_equal(results[0][0].view(np.uint16), results[1][0].view(np.uint16))
     assert np.array_equal(results[0][1].view(np.uint16), results[1][1].view(np.uint16))
     assert_close_f16(results[0][1], oracle.w4a16_linear(results[0][0], *matrices[0]))
+
+
+# ---- persistent streams (a tile of 16 columns for every SM and more) --------------------------------------
+
+@pytest.mark.parametrize("rows,experts,top,n,k", [(1, 8, 4, 1218, 72), (8, 64, 8, 200, 520), (9, 40, 6, 122, 200), (16, 33, 2, 282, 136),
+                                                  (17, 300, 3, 98, 72), (32, 60, 3, 90, 1000), (32, 16, 2, 1026, 2048),
+                                                  (2, 4, 2, 58, 72), (40, 9, 2, 130, 104)])  # a tile per block
+def test_expert_rows_of_many_tiles(runtime, rows, experts, top, n, k):
+    """Gate and up rows of all chosen experts as one list of tiles, against fp64; a route of any words reads and writes nothing
+    beyond its buffers."""
+    from llmopt_b200 import parameters
+    from llmopt_b200.cuda_native import Buffer
+    from llmopt_b200.feed_forward import route_words
+
+    rng = np.random.default_rng(rows + n)
+    x, w = bf16_round(rng.standard_normal((rows, k))), bf16_round(rng.standard_normal((experts, n, k)) / np.sqrt(k))
+    logits = (rng.standard_normal((rows, experts)) * 3).astype(np.float32)
+    words, pairs = route_words(rows, experts, top), rows * top
+    route = upload(runtime, np.zeros(words, np.uint32))
+    runtime.dispatch("llmopt_route_step_f32", buffers=[upload(runtime, logits), route], parameters=parameters.route(rows=rows, experts=experts, top=top))
+    guard = 64 * n
+    out = Buffer.of_array(runtime, np.full(pairs * n // 2 + guard, 0x7FC0, np.uint16))
+    operands = [upload(runtime, x, "bfloat16"), upload(runtime, w, "bfloat16")]
+    block = parameters.expert_step(rows=rows, n=n, k=k, experts=experts, top=top)
+    runtime.dispatch("llmopt_expert_step_bf16", buffers=[*operands, route, out.view(0, pairs * n)], parameters=block)
+    choices = np.argsort(-logits, axis=1, kind="stable")[:, :top]
+    order = np.argsort(choices.reshape(-1), kind="stable")
+    want = np.empty((pairs, n // 2))
+    for slot, pair in enumerate(order):
+        row, expert = pair // top, choices.reshape(-1)[pair]
+        y = w[expert].astype(np.float64) @ x[row] * plain.sigmoid(np.float64(logits[row, expert]))
+        want[slot] = plain.silu(y[0::2]) * y[1::2]
+    close(download(out, (pairs, n // 2), "bfloat16"), want, 6e-3)
+    for seed in range(3):
+        noise = np.random.default_rng(seed).integers(0, [2 ** 32, 2 * pairs + 2, pairs + 1][seed], size=words, dtype=np.uint32)
+        noise[0] = [2 ** 32 - 1, experts, min(pairs, experts)][seed]
+        runtime.dispatch("llmopt_expert_step_bf16", buffers=[*operands, upload(runtime, noise), out.view(0, pairs * n)], parameters=block)
+    assert np.all(out.to_numpy(np.uint16)[pairs * n // 2:] == 0x7FC0)
