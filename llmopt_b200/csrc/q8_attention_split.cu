@@ -136,14 +136,15 @@ struct SplitShape {
 // writes of the rotated query / key rows (the merge kernel reads them) and the Q8 pack of the new key and
 // value rows are warp tasks handed out over the CTAs of a (batch, KV head), done while the first tiles are
 // in flight.
-// `cluster` > 0: the grid's x dimension is one cluster of that many CTAs, which writes `output`.
-template <int D, int GROUP, int CP, bool FUSED, int WARPS>
+// CLUSTER: the splits of a (batch, KV head) are one cluster, which writes `output`.  A kernel of its own: with the merge behind a
+// run-time argument the launches that leave records took 0.8 us longer (8192 keys x 8 heads of 128).
+template <int D, int GROUP, int CP, bool FUSED, int WARPS, bool CLUSTER>
 __global__ void __launch_bounds__(WARPS * 32, kResidentCtas * kWarps / WARPS)
 paged_split_kernel(const __half* __restrict__ query, const uint8_t* __restrict__ pool,
                    const uint32_t* __restrict__ slots, float* __restrict__ scratch, PagedParams p,
                    uint32_t slot_batch_stride, uint32_t splits, const uint32_t* __restrict__ past_cell,
                    uint32_t pool_tokens, uint32_t* error_word, RotaryPackFusion fusion, const __half* current_key,
-                   const __half* current_value, __half* output, uint32_t cluster) {
+                   const __half* current_value, __half* output) {
   grid_chain_prologue();
   constexpr int kWarps = WARPS;
   using Shape = SplitShape<D, CP, WARPS>;
@@ -458,9 +459,9 @@ paged_split_kernel(const __half* __restrict__ query, const uint8_t* __restrict__
     running_sum[h] += __shfl_xor_sync(0xffffffffu, running_sum[h], 16);
   }
   __syncthreads();
-  float* stage = reinterpret_cast<float*>(ring);  // [warp][16 + 8 * D], then the CTA's own record
+  float* stage = reinterpret_cast<float*>(ring);  // [warp][16 + 8 * D], then (CLUSTER) the CTA's own record
   constexpr int kRecord = 16 + 8 * D;
-  static_assert(Shape::kRingBytes >= (int)sizeof(float) * (kWarps + 1) * kRecord, "merge staging must fit the ring");
+  static_assert(Shape::kRingBytes >= (int)sizeof(float) * (kWarps + (CLUSTER ? 1 : 0)) * kRecord, "merge staging must fit the ring");
   float* mine = stage + warp * kRecord;
   if (r == 0) {
     mine[2 * c] = running_max[0];
@@ -477,9 +478,8 @@ paged_split_kernel(const __half* __restrict__ query, const uint8_t* __restrict__
       mine[16 + head * D + dim] = out[s][j];
     }
   __syncthreads();
-  // two pointers and not one: a store that may be to either memory is slow, and orders the reads of `stage` behind it
-  float* const own = stage + kWarps * kRecord;
-  float* const record = scratch + (((size_t)batch * p.kv_heads + kv_head) * splits + split) * kRecord;
+  float* record = CLUSTER ? stage + kWarps * kRecord
+                          : scratch + (((size_t)batch * p.kv_heads + kv_head) * splits + split) * kRecord;
   // only the columns of heads that exist are merged and written (the merge kernel reads no others)
   for (uint32_t index = threadIdx.x; index < min(heads_per_kv, 8u) * D; index += kWarps * 32) {
     const uint32_t head = index / D;
@@ -493,29 +493,20 @@ paged_split_kernel(const __half* __restrict__ query, const uint8_t* __restrict__
       total += weight * stage[w * kRecord + 16 + index];
       denominator += weight * stage[w * kRecord + 8 + head];
     }
-    // records carry the maximum in natural units; a split without keys says -inf
-    const float natural = merged_max <= 0.5f * kLowest ? -INFINITY : merged_max * 0.6931471805599453f;
-    if (cluster > 0u) {
-      own[16 + index] = total;
-      if (index % D == 0) {
-        own[head] = natural;
-        own[8 + head] = denominator;
-      }
-    } else {
-      record[16 + index] = total;
-      if (index % D == 0) {
-        record[head] = natural;
-        record[8 + head] = denominator;
-      }
+    record[16 + index] = total;
+    if (index % D == 0) {
+      // records carry the maximum in natural units; a split without keys says -inf
+      record[head] = merged_max <= 0.5f * kLowest ? -INFINITY : merged_max * 0.6931471805599453f;
+      record[8 + head] = denominator;
     }
   }
-  if (cluster == 0u) return;
+  if constexpr (!CLUSTER) return;
 
   // ---- merge the cluster's records and the current token -----------------------
   // Thread i of the cluster owns elements i, i + threads, ... of [head][D]; a warp's 32 belong to one head.
   cluster_sync();
   constexpr int kMost = 8 * D / (2 * kWarps * 32);  // of a thread, in a cluster of two or more
-  const uint32_t elements = min(heads_per_kv, 8u) * D, threads = cluster * kWarps * 32u;
+  const uint32_t elements = min(heads_per_kv, 8u) * D, threads = splits * kWarps * 32u;
   float results[kMost];
 #pragma unroll
   for (int i = 0; i < kMost; ++i) {
@@ -535,15 +526,15 @@ paged_split_kernel(const __half* __restrict__ query, const uint8_t* __restrict__
     const float current = half_at(current_value + current_base + d);
     const float score_now = warp_sum(dot) * p.scale;
     float maximum = score_now;
-    for (uint32_t other = 0; other < cluster; ++other) maximum = fmaxf(maximum, cluster_load(own + head, other));
+    for (uint32_t other = 0; other < splits; ++other) maximum = fmaxf(maximum, cluster_load(record + head, other));
     const float now = expf(score_now - maximum);
     float total = now * current, denominator = now;
 #pragma unroll 4
-    for (uint32_t other = 0; other < cluster; ++other) {
-      const float top = cluster_load(own + head, other);
+    for (uint32_t other = 0; other < splits; ++other) {
+      const float top = cluster_load(record + head, other);
       const float weight = top == -INFINITY ? 0.0f : expf(top - maximum);
-      denominator = fmaf(weight, cluster_load(own + 8 + head, other), denominator);
-      total = fmaf(weight, cluster_load(own + 16 + index, other), total);
+      denominator = fmaf(weight, cluster_load(record + 8 + head, other), denominator);
+      total = fmaf(weight, cluster_load(record + 16 + index, other), total);
     }
     results[i] = denominator == 0.0f ? 0.0f : total / denominator;
   }
@@ -641,10 +632,11 @@ struct ClusterPlan {
   uint32_t ctas, warps;
 };
 
-template <int D, int GROUP, int CP, int WARPS>
+template <int D, int GROUP, int CP, int WARPS, bool CLUSTER>
 int launch_split_copy(const KernelArgs& args, const PagedParams& p, uint32_t slot_batch_stride, float* scratch,
-                      uint32_t splits, uint32_t pool_tokens, uint32_t cluster) {
-  auto kernel = args.rotary_fusion ? paged_split_kernel<D, GROUP, CP, true, WARPS> : paged_split_kernel<D, GROUP, CP, false, WARPS>;
+                      uint32_t splits, uint32_t pool_tokens) {
+  auto kernel = args.rotary_fusion ? paged_split_kernel<D, GROUP, CP, true, WARPS, CLUSTER>
+                                   : paged_split_kernel<D, GROUP, CP, false, WARPS, CLUSTER>;
   constexpr int ring_bytes = SplitShape<D, CP, WARPS>::kRingBytes;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ring_bytes) != cudaSuccess) {
     cudaGetLastError();
@@ -656,9 +648,9 @@ int launch_split_copy(const KernelArgs& args, const PagedParams& p, uint32_t slo
           (const __half*)args.buffers[0], (const uint8_t*)args.buffers[3], (const uint32_t*)args.buffers[4], scratch, p,
           slot_batch_stride, splits, args.past_tokens_cell, pool_tokens,
           args.ctx ? context_device_error(args.ctx) : nullptr, fusion, (const __half*)args.buffers[1],
-          (const __half*)args.buffers[2], (__half*)args.buffers[6], cluster);
+          (const __half*)args.buffers[2], (__half*)args.buffers[6]);
   };
-  if (cluster > 0u) launch([](auto&&... a) { launch_cluster_kernel(a...); }, cluster);
+  if constexpr (CLUSTER) launch([](auto&&... a) { launch_cluster_kernel(a...); }, splits);
   else launch([](auto&&... a) { launch_kernel(a...); });
   return check_launch(args);
 }
@@ -669,13 +661,13 @@ int launch_split(const KernelArgs& args, const PagedParams& p, uint32_t slot_bat
   const bool aligned = (p.token_stride % 16 == 0) && (((uintptr_t)args.buffers[3]) % 16 == 0);
   if (plan.ctas > 0u) {
     if (plan.warps == 8u)
-      return aligned ? launch_split_copy<D, GROUP, 16, 8>(args, p, slot_batch_stride, nullptr, plan.ctas, pool_tokens, plan.ctas)
-                     : launch_split_copy<D, GROUP, 8, 8>(args, p, slot_batch_stride, nullptr, plan.ctas, pool_tokens, plan.ctas);
-    return aligned ? launch_split_copy<D, GROUP, 16, 4>(args, p, slot_batch_stride, nullptr, plan.ctas, pool_tokens, plan.ctas)
-                   : launch_split_copy<D, GROUP, 8, 4>(args, p, slot_batch_stride, nullptr, plan.ctas, pool_tokens, plan.ctas);
+      return aligned ? launch_split_copy<D, GROUP, 16, 8, true>(args, p, slot_batch_stride, nullptr, plan.ctas, pool_tokens)
+                     : launch_split_copy<D, GROUP, 8, 8, true>(args, p, slot_batch_stride, nullptr, plan.ctas, pool_tokens);
+    return aligned ? launch_split_copy<D, GROUP, 16, 4, true>(args, p, slot_batch_stride, nullptr, plan.ctas, pool_tokens)
+                   : launch_split_copy<D, GROUP, 8, 4, true>(args, p, slot_batch_stride, nullptr, plan.ctas, pool_tokens);
   }
-  const int status = aligned ? launch_split_copy<D, GROUP, 16, 4>(args, p, slot_batch_stride, scratch, splits, pool_tokens, 0u)
-                             : launch_split_copy<D, GROUP, 8, 4>(args, p, slot_batch_stride, scratch, splits, pool_tokens, 0u);
+  const int status = aligned ? launch_split_copy<D, GROUP, 16, 4, false>(args, p, slot_batch_stride, scratch, splits, pool_tokens)
+                             : launch_split_copy<D, GROUP, 8, 4, false>(args, p, slot_batch_stride, scratch, splits, pool_tokens);
   if (status) return status;
   launch_kernel(args, paged_merge_kernel<D>, dim3(p.query_heads, p.batches), dim3(D * kMergeParts), 0,
       (const __half*)args.buffers[0], (const __half*)args.buffers[1], (const __half*)args.buffers[2], scratch,
