@@ -44,7 +44,6 @@ constexpr int kTileKeys = 16;
 constexpr int kWarps = 4;
 constexpr int kResidentCtas = 4;  // per SM, by shared memory and registers (128 per thread)
 constexpr uint32_t kNoSlot = 0xffffffffu;
-constexpr uint32_t kLongestForOneCluster = 3072;  // tokens behind a sequence: three tiles per warp
 constexpr float kLowest = -1.0e30f;  // "no key yet" maximum; keeps the softmax free of inf - inf
 
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t selector) {
@@ -685,26 +684,37 @@ uint32_t pinned_splits() {
   return pinned;
 }
 
-// A cluster saves the merge kernel and the way through scratch, which is 4 to 5 us a layer: 1 sequence x 512 keys x 3 heads of
-// 64 (64 splits before) 10.0 -> 6.7 us, 16 x 1024 x 8 of 64 14.7 -> 13.2, 32 x 2048 x 8 of 128 49.7 -> 41.3.  Few (batch, KV
-// head) pairs take eight CTAs of eight warps; beyond a few tiles per warp (about 2 us each) many short splits are faster
-// again: 8192 keys x 8 heads of 128 24.1 us in clusters, 15.6 as 64 records.  What a plan may grow to decides, not what it
-// was captured at.  More pairs: the cluster size that fills whole waves best; the merge is the same work for all of them.
+// A cluster saves the merge kernel and the way through scratch; records take as many splits as fill the chip, also in several
+// waves.  What each costs, in keys that one CTA of four warps walks over: its share of the longest sequence times its waves,
+// kWave for each wave, and for records kMerge and kRecord for each.  A CTA of eight warps takes its keys at twice the rate and kWideCta more to
+// begin with.  Clusters fill nine tenths of the chip at most (72 pairs x 8 CTAs take two waves).  The constants are
+// fitted to 22 numbers of pairs from 3 to 512, capacities of 64 to 16384 keys, full, half full and an eighth full, as plans and
+// alone, with heads of 64 and 128: nowhere slower than records alone by more than 3 %, on average 14 % faster.  With 8 heads of
+// 128 a sequence, records -> this rule, us: 1 x 512 6.6 -> 5.3 (plan), 5 x 2048 16.2 -> 14.0, 16 x 2048 26.4 -> 22.7, 32 x 2048
+// 46.6 -> 38.9; where the rule keeps records, records (the best cluster): 1 x 8192 11.5 (17.1), 5 x 8192 29.2 (34.6), 9 x 8192 39.4 (58).
+// What a plan may grow to decides, not what it was captured at.
 ClusterPlan pick_cluster(const KernelArgs& args, const PagedParams& p, uint32_t slot_batch_stride) {
   if (pinned_splits() != 0u) return {0u, 0u};
+  constexpr float kWave = 150.0f, kMerge = 50.0f, kRecord = 0.5f, kWideCta = 24.0f;
   const size_t slots = args.lengths[4] / 4u, before = (size_t)(p.batches - 1u) * slot_batch_stride;
   const size_t longest = args.past_tokens_cell ? (slots > before ? slots - before : 0u) : p.past_length;
-  const uint32_t pairs = p.batches * p.kv_heads, sms = (uint32_t)context_sm_count(args.ctx);
-  const uint32_t resident = sms * (uint32_t)kResidentCtas;
-  if (pairs * 8u <= 2u * sms) return longest <= kLongestForOneCluster ? ClusterPlan{8u, 8u} : ClusterPlan{0u, 0u};
-  uint32_t best = 2u;
-  float best_fill = 0.0f;
-  for (uint32_t ctas = 2u; ctas <= 8u; ctas *= 2u) {
-    const uint32_t waves = (pairs * ctas + resident - 1u) / resident;
-    const float fill = (float)(pairs * ctas) / (float)(waves * resident);
-    if (fill > best_fill + 0.01f) best = ctas, best_fill = fill;
+  const size_t pairs = (size_t)p.batches * p.kv_heads, resident = (size_t)context_sm_count(args.ctx) * kResidentCtas;
+  // outside a plan a short context has few records, which merge at once: 2 x 256 keys x 8 heads 5.7 us, 6.4 as clusters
+  if (args.past_tokens_cell == nullptr && (longest <= 128u || (longest <= 512u && pairs < 40u))) return {0u, 0u};
+  auto waves = [](size_t ctas, size_t room) { return (float)((ctas + room - 1u) / room); };
+  const uint32_t splits = paged_pick_splits(args, p);
+  const float record_waves = waves(pairs * splits, resident);
+  float least = kMerge + kRecord * (float)splits + record_waves * (kWave + (float)longest / (float)splits);
+  ClusterPlan best = {0u, 0u};
+  const ClusterPlan forms[] = {{2u, 4u}, {4u, 4u}, {8u, 4u}, {8u, 8u}};
+  for (const ClusterPlan& form : forms) {
+    const float rate = (float)form.warps / (float)kWarps;
+    const float form_waves = waves(pairs * form.ctas, (size_t)((float)resident * 0.9f / rate));
+    if (form.warps > (uint32_t)kWarps && form_waves > 1.0f) continue;
+    const float cost = form_waves * (kWave + (float)longest / ((float)form.ctas * rate)) + (form.warps > (uint32_t)kWarps ? kWideCta : 0.0f);
+    if (cost < least) least = cost, best = form;
   }
-  return {best, 4u};
+  return best;
 }
 
 }  // namespace

@@ -185,14 +185,14 @@ def test_paged_per_sequence_slot_tables(runtime, oracle):
 
 
 @pytest.mark.parametrize("batches,hq,hkv,dim,group,past", [
-    (1, 8, 1, 64, 32, 0), (1, 16, 2, 128, 32, 1037), (4, 12, 4, 128, 64, 3), (37, 2, 1, 64, 64, 129),  # 8 blocks of 8 warps
-    (6, 64, 8, 64, 32, 100), (38, 1, 1, 128, 64, 17),                                                  # 8 blocks of 4
-    (12, 24, 8, 128, 32, 200), (74, 5, 1, 64, 64, 0),                                                  # 4 blocks
-    (20, 8, 8, 64, 64, 530), (150, 8, 1, 128, 64, 5),                                                  # 2 blocks
-    (1, 4, 1, 64, 64, 3072), (1, 4, 1, 64, 64, 3073),                                                  # the longest, records
+    (1, 8, 1, 64, 32, 0), (1, 16, 2, 128, 32, 1037), (4, 12, 4, 128, 64, 3), (37, 2, 1, 64, 64, 129),
+    (6, 64, 8, 64, 32, 100), (38, 1, 1, 128, 64, 17),
+    (12, 24, 8, 128, 32, 200), (74, 5, 1, 64, 64, 0),
+    (20, 8, 8, 64, 64, 530), (150, 8, 1, 128, 64, 5),
+    (1, 4, 1, 64, 64, 3072), (1, 4, 1, 64, 64, 3073),
 ])
 def test_paged_decode_by_clusters(runtime, oracle, batches, hq, hkv, dim, group, past):
-    """Every number of blocks and warps that share a sequence's keys, with as many heads per block as there are."""
+    """Clusters and records, with as many heads per KV head as there are."""
     got, want, names = _paged(runtime, oracle, batches=batches, hq=hq, hkv=hkv, dim=dim, group=group, past=past,
                               per_sequence=batches > 1 and past > 0, query_scale=3.0, seed=past)
     assert_close_f16(got, want, label=f"paged {names}")

@@ -294,3 +294,28 @@ def test_expert_rows_of_many_tiles(runtime, rows, experts, top, n, k):
         noise[0] = [2 ** 32 - 1, experts, min(pairs, experts)][seed]
         runtime.dispatch("llmopt_expert_step_bf16", buffers=[*operands, upload(runtime, noise), out.view(0, pairs * n)], parameters=block)
     assert np.all(out.to_numpy(np.uint16)[pairs * n // 2:] == 0x7FC0)
+
+
+# ---- paged attention in its forms -----------------------------------------------------------------------
+
+@pytest.mark.parametrize("batch,q_heads,k_heads,dim,group,past", [
+    (1, 8, 2, 128, 64, 3100), (2, 16, 8, 64, 32, 3200),  # records and a merge
+    (2, 16, 8, 128, 32, 900), (3, 8, 8, 64, 64, 1500),   # clusters of 8 blocks of 8 warps
+    (5, 16, 8, 128, 64, 200), (8, 16, 8, 64, 64, 530), (5, 8, 8, 64, 32, 2100),  # 8 of 4
+    (8, 20, 10, 128, 32, 200), (8, 20, 20, 64, 64, 150)])                        # 4 and 2 of 4
+def test_attention_with_rotary_and_pack_in_every_form(runtime, monkeypatch, batch, q_heads, k_heads, dim, group, past):
+    import test_gpu_cache_attention as attention
+
+    attention.test_plan_hands_rotary_and_pack_to_the_attention_byte_for_byte(runtime, monkeypatch, batch, q_heads, k_heads, dim, group, past)
+
+
+@pytest.mark.parametrize("batches,hkv,past", [(3, 8, 600), (3, 8, 1500), (5, 8, 520), (5, 8, 2100), (5, 8, 4500), (10, 8, 2100), (10, 8, 3300),
+                                              (13, 8, 2100), (20, 8, 530), (32, 8, 140)])
+def test_batches_behind_contexts(runtime, oracle, batches, hkv, past):
+    """On both sides of the lines between clusters of 8 x 8, 8 x 4, 4 x 4 and 2 x 4 warps and records."""
+    import test_gpu_cache_attention as attention
+    from conftest import assert_close_f16
+
+    got, want, names = attention._paged(runtime, oracle, batches=batches, hq=2 * hkv, hkv=hkv, dim=64, group=64, past=past, layers=1, layer=0,
+                                        per_sequence=True, query_scale=3.0, seed=past)
+    assert_close_f16(got, want, label=f"paged {names}")
