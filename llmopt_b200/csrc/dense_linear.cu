@@ -5,8 +5,9 @@
 //                                      place, the following sublayer's tanh norm, all in the writeback
 //
 // Kernels behind the names:
-//  * bf16, up to 64 rows (decode): dense_gemv_kernel, weights streamed once from HBM straight into
-//    mma.sync fragments.  The order of the contraction is free, so a lane takes 16 contiguous bytes of
+//  * bf16, up to 64 rows (decode): weights streamed once from HBM straight into mma.sync fragments, by
+//    dense_gemv_kernel (a CTA per 16 columns) or, with many columns and up to 32 rows, dense_wide_kernel
+//    (persistent CTAs).  The order of the contraction is free, so a lane takes 16 contiguous bytes of
 //    a weight row (eight k) as the A words of two MMAs and the same eight k of an activation row
 //    as their B words: no shared-memory staging and full 128-byte lines.  Eight warps split K and
 //    add their sums in warp order.
@@ -84,7 +85,7 @@ __global__ void __launch_bounds__(kGemvWarps * 32, NT <= 4 ? 2 : 1) dense_gemv_k
 // weights under way while it waited for the activation rows in L2, which came to two thirds of its traffic with 32 rows,
 // and nothing while it stored.  32 rows, k 2048: n 32768 76 -> 36 us, n 14336 (pairs) 38 -> 22, n 5120 (cached) 20.5 -> 16.4.
 template <int NT, DenseStore STORE>
-__global__ void __launch_bounds__(kWideThreads, NT == 1 ? 2 : 1) dense_wide_kernel(const DenseTask<STORE> p) {
+__global__ void __launch_bounds__(kWideThreads, WideShape<NT>::kMostPerSm) dense_wide_kernel(const DenseTask<STORE> p) {
   grid_launch_dependents();
   extern __shared__ __align__(128) unsigned char wide_shared[];
   typedef WideShape<NT> Shape;
@@ -100,13 +101,7 @@ __global__ void __launch_bounds__(kWideThreads, NT == 1 ? 2 : 1) dense_wide_kern
   auto stage_rows = [&]() {
     grid_dependency_wait();
     const bf16* x = reinterpret_cast<const bf16*>(p.x);
-    const uint32_t chunks = blocks * 8u;
-    for (uint32_t index = threadIdx.x; index < NT * 8u * chunks; index += kWideThreads) {
-      const uint32_t row = index / chunks, chunk = index - row * chunks;
-      uint4 value = make_uint4(0u, 0u, 0u, 0u);
-      if (row < p.m && chunk * 8u < p.k) value = *reinterpret_cast<const uint4*>(x + (size_t)row * p.k + chunk * 8u);
-      rows[wide_chunk(row, blocks, chunk)] = value;
-    }
+    wide_stage_rows(rows, x, NT * 8u, p.m, p.k, blocks);
     __syncthreads();
   };
   if (warp < kGemvWarps) {
@@ -265,19 +260,28 @@ int run_gemv(const KernelArgs& args, DenseProblem p, DenseStore store) {
   p.cluster = stream_cluster(args, tiles, (p.k + 63u) / 64u);
   return with_store(store, [&](auto constant) {
     constexpr DenseStore STORE = decltype(constant)::value;
-    auto run_wide = [&](auto kernel, uint32_t bytes) {
+    auto run_wide = [&](auto kernel, uint32_t bytes, uint32_t most_per_sm) {
       if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
         cudaGetLastError();
         return fail(args, "shared memory request was refused");
       }
-      launch_kernel(args, kernel, dim3(wide_ctas(args, tiles, bytes)), dim3(kWideThreads), bytes, DenseTask<STORE>(p));
+      launch_kernel(args, kernel, dim3(wide_ctas(args, tiles, bytes, most_per_sm)), dim3(kWideThreads), bytes, DenseTask<STORE>(p));
       return check_launch(args);
     };
-    // a tile for every SM (the sums are then not shared out over clusters either), and the rows beside the rings
-    if (tiles >= (uint32_t)context_sm_count(args.ctx) && p.k <= 32768u) {
-      if (p.m <= 8u && WideShape<1>::bytes(p.k) <= kWideMost) return run_wide(dense_wide_kernel<1, STORE>, WideShape<1>::bytes(p.k));
-      if (p.m > 8u && p.m <= 16u && WideShape<2>::bytes(p.k) <= kWideMost) return run_wide(dense_wide_kernel<2, STORE>, WideShape<2>::bytes(p.k));
-      if (p.m > 16u && p.m <= 32u && WideShape<4>::bytes(p.k) <= kWideMost) return run_wide(dense_wide_kernel<4, STORE>, WideShape<4>::bytes(p.k));
+    // A tile for every SM (the sums are then not shared out over clusters either), and the rows beside the rings.  With k above
+    // 2560 one CTA fits on an SM and two tiles for each are needed: 8 rows, k 7168, n 4736 14.1 us, 15.9 persistent, n 5120 20.5
+    // and 18.5; k 4096 10.0, 10.7, 13.8 and 12.1; k 2048 6.3, 6.0, 9.4 and 7.2.
+    auto wide = [&](auto width) {
+      constexpr int NT = decltype(width)::value;
+      const uint32_t bytes = WideShape<NT>::bytes(p.k);
+      return bytes <= kWideMost ? run_wide(dense_wide_kernel<NT, STORE>, bytes, WideShape<NT>::kMostPerSm) : -1;
+    };
+    const uint32_t sms = (uint32_t)context_sm_count(args.ctx);
+    if (p.m <= 32u && (p.k <= 2560u ? tiles >= sms : p.k <= 32768u && tiles > 2u * sms)) {
+      const int status = p.m <= 8u    ? wide(std::integral_constant<int, 1>())
+                         : p.m <= 16u ? wide(std::integral_constant<int, 2>())
+                                      : wide(std::integral_constant<int, 4>());
+      if (status >= 0) return status;
     }
     auto run = [&](auto kernel) {
       const DenseTask<STORE> task(p);

@@ -120,6 +120,7 @@ __device__ __forceinline__ void wide_barrier_arrive(uint32_t id) {
 template <int NT>
 struct WideShape {
   static constexpr uint32_t kRingBytes = kGemvWarps * kRingDepth * 4u * 32u * 16u;
+  static constexpr uint32_t kMostPerSm = NT == 1 ? 2u : 1u;  // CTAs, by registers
   typedef float Sums[kGemvWarps][NT * 8][17];
   static constexpr uint32_t kRowsAt = kRingBytes + 2u * sizeof(Sums);
   __host__ __device__ static constexpr uint32_t bytes(uint32_t k) { return kRowsAt + NT * 8u * ((k + 63u) / 64u * 128u); }
@@ -127,6 +128,27 @@ struct WideShape {
 // Sixteen-byte chunk `chunk` of a row; odd rows swap the halves of a k-block, so that two rows fill the banks.
 __device__ __forceinline__ uint32_t wide_chunk(uint32_t row, uint32_t blocks, uint32_t chunk) {
   return row * blocks * 8u + (chunk ^ ((row & 1u) * 4u));
+}
+
+// Rows of k elements to shared memory, zeros behind row `m` up to `count` and behind k.  Eight pieces of a thread are under way
+// together: one at a time, 8 rows of k 4096 took 5 us.
+__device__ __forceinline__ void wide_stage_rows(uint4* rows, const bf16* x, uint32_t count, uint32_t m, uint32_t k, uint32_t blocks) {
+  constexpr int kAhead = 8;
+  const uint32_t chunks = blocks * 8u, all = count * chunks;
+  for (uint32_t begin = threadIdx.x; begin < all; begin += kAhead * kWideThreads) {
+    uint4 value[kAhead];
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) {
+      const uint32_t index = begin + i * kWideThreads, row = index / chunks, chunk = index - row * chunks;
+      value[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (index < all && row < m && chunk * 8u < k) value[i] = *reinterpret_cast<const uint4*>(x + (size_t)row * k + chunk * 8u);
+    }
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) {
+      const uint32_t index = begin + i * kWideThreads, row = index / chunks, chunk = index - row * chunks;
+      if (index < all) rows[wide_chunk(row, blocks, chunk)] = value[i];
+    }
+  }
 }
 
 // The ring of one lane.  tile_of(index, low, high) says where the lane's two weight rows of the CTA's tile number `index`
@@ -192,10 +214,11 @@ __device__ __forceinline__ void wide_finish(const DenseTask<STORE>& p, const flo
   }
 }
 
-// CTAs for `tiles` tiles: whole rounds of as many as fit, shared out evenly.
-inline uint32_t wide_ctas(const KernelArgs& args, uint32_t tiles, uint32_t bytes) {
-  const uint32_t per_sm = kWideMost / (bytes + 1024u) >= 2u ? 2u : 1u, most = per_sm * (uint32_t)context_sm_count(args.ctx);
-  const uint32_t rounds = (tiles + most - 1u) / most;
+// CTAs for `tiles` tiles: whole rounds of as many as fit, shared out evenly.  `bytes` of shared memory, at most `most` per SM by
+// registers.
+inline uint32_t wide_ctas(const KernelArgs& args, uint32_t tiles, uint32_t bytes, uint32_t most) {
+  const uint32_t per_sm = most >= 2u && kWideMost / (bytes + 1024u) >= 2u ? 2u : 1u;
+  const uint32_t together = per_sm * (uint32_t)context_sm_count(args.ctx), rounds = (tiles + together - 1u) / together;
   return (tiles + rounds - 1u) / rounds;
 }
 

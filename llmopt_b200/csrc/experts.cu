@@ -276,13 +276,7 @@ __global__ void __launch_bounds__(kWideThreads, 1) expert_wide_kernel(const Dens
     firsts[i] = min(route[at.first + i], pairs);
   }
   for (uint32_t i = threadIdx.x; i < pairs; i += kWideThreads) row_of_slot[i] = (uint8_t)min(route[at.row + i], p.m - 1u);
-  const uint32_t chunks = blocks * 8u;
-  for (uint32_t index = threadIdx.x; index < p.m * chunks; index += kWideThreads) {
-    const uint32_t row = index / chunks, chunk = index - row * chunks;
-    uint4 value = make_uint4(0u, 0u, 0u, 0u);
-    if (chunk * 8u < p.k) value = *reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(p.x) + (size_t)row * p.k + chunk * 8u);
-    rows[wide_chunk(row, blocks, chunk)] = value;
-  }
+  wide_stage_rows(rows, reinterpret_cast<const bf16*>(p.x), p.m, p.m, p.k, blocks);
   __syncthreads();
   // no more than there are slots behind the first, whatever the route says
   auto rows_of = [&](uint32_t place) { return min(firsts[place + 1u] - firsts[place], min(p.m, pairs - firsts[place])); };
@@ -344,18 +338,19 @@ int run_step(const KernelArgs& args, DenseProblem p, const uint32_t* route, cons
   const uint32_t tiles = (p.n + 15u) / 16u, blocks = (p.k + 63u) / 64u;
   p.cluster = stream_cluster(args, DOWN ? tiles : tiles * most, DOWN ? blocks * most : blocks);
   if constexpr (!DOWN) {
-    // a tile for every SM, and the rows beside the rings in shared memory
+    // more than two tiles for every SM, and the rows beside the rings in shared memory (2 rows, 4 choices of 1024 x 512: 256 tiles,
+    // 4.6 us, 5.2 persistent; 4 rows, 512 tiles, 6.2 and 5.8)
     const uint32_t pairs = p.m * top, route_bytes = ((2u * most + 1u) * 4u + pairs + 15u) / 16u * 16u;
     auto run_wide = [&](auto kernel, uint32_t bytes) {
       if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
         cudaGetLastError();
         return fail(args, "shared memory request was refused");
       }
-      launch_kernel(args, kernel, dim3(wide_ctas(args, tiles * most, kWideMost)), dim3(kWideThreads), bytes,
+      launch_kernel(args, kernel, dim3(wide_ctas(args, tiles * most, bytes, 1u)), dim3(kWideThreads), bytes,
                     DenseTask<kStorePair>(p), p.plan.experts, route, at, pairs, most);
       return check_launch(args);
     };
-    if (tiles * most >= (uint32_t)context_sm_count(args.ctx) && p.k <= 32768u) {
+    if (tiles * most > 2u * (uint32_t)context_sm_count(args.ctx) && p.k <= 32768u) {
       if (p.m <= 8u && WideShape<1>::bytes(p.k) + route_bytes <= kWideMost)
         return run_wide(expert_wide_kernel<1>, WideShape<1>::bytes(p.k) + route_bytes);
       if (p.m > 8u && p.m <= 16u && WideShape<2>::bytes(p.k) + route_bytes <= kWideMost)

@@ -260,6 +260,59 @@ def test_short_sums(runtime, oracle, monkeypatch, rows, k, n):
 
 # ---- persistent streams (a tile of 16 columns for every SM and more) --------------------------------------
 
+WIDE = [(1, 2370, 72), (8, 2370, 520), (9, 2370, 72), (16, 2370, 2048), (17, 2370, 520), (32, 2370, 2048),  # one or two tiles per block
+        (8, 15010, 72), (16, 15010, 136), (32, 15010, 72)]                                                 # four and more, the ring crosses their ends
+
+
+@pytest.mark.parametrize("m,n,k", WIDE)
+def test_products_of_many_columns(runtime, m, n, k):
+    """Plain (also an odd number of columns), pair and residual stores against fp64, with the bounds of the same checks at
+    other sizes."""
+    import test_gpu_dalorax as sublayers
+    import test_gpu_mixers as mixers
+
+    mixers.test_dense_linear(runtime, "bfloat16", m, n - 1, k, n // 3)
+    sublayers.test_paired_columns_and_scale(runtime, "bfloat16", m, n, k)
+    sublayers.test_product_that_ends_a_sublayer(runtime, "bfloat16", m, n, k)
+
+
+@pytest.mark.parametrize("m,n,k", WIDE[:6] + [(32, 7300, 136)])
+def test_cache_rows_of_many_columns(runtime, m, n, k):
+    """Columns that go to the output, to a token's key and value row and to fp32 rows, borders off the tiles."""
+    from llmopt_b200 import parameters
+    from llmopt_b200.kv_cache import RowLayout
+
+    rng = np.random.default_rng(m + k)
+    heads, dim, vdim, extra = 3, 24, 40, 5
+    keys, values = heads * dim, heads * vdim
+    own = n - keys - values - extra
+    x, w = bf16_round(rng.standard_normal((m, k))), bf16_round(rng.standard_normal((n, k)) / np.sqrt(k))
+    bias = rng.standard_normal(n).astype(np.float32)
+    layout = RowLayout([(1, 8, 16), (heads, dim, vdim)])
+    region, stride, slots = layout.regions[1], 7, 7 * m + 3
+    table = rng.permutation(slots)[:7 * m].reshape(m, stride).astype(np.uint32)
+    past, which = rng.integers(0, stride, size=m).astype(np.uint32), rng.permutation(m).astype(np.uint32)
+    before = bf16_round(rng.standard_normal((slots, layout.token_elements)))
+    pool, out, out32 = upload(runtime, before, "bfloat16"), empty(runtime, m * own, "bfloat16"), empty(runtime, m * extra)
+    runtime.dispatch("llmopt_dense_cached_bf16", buffers=[
+        upload(runtime, x, "bfloat16"), upload(runtime, w, "bfloat16"), upload(runtime, bias), out, out32, pool, upload(runtime, table),
+        upload(runtime, past), upload(runtime, which)], parameters=parameters.dense_cached(
+            m=m, n=n, k=k, split=own, tokens=1, key_columns=keys, value_columns=values, has_bias=True,
+            token_stride=layout.token_elements, key_offset=region.key_offset, value_offset=region.value_offset, table_stride=stride,
+            table_rows=m, pool_rows=slots))
+    y = x.astype(np.float64) @ w.T.astype(np.float64) + bias
+    close(download(out, (m, own), "bfloat16"), y[:, :own], 6e-3, "rows")
+    close(download(out32, (m, extra)), y[:, n - extra:], 1e-5, "fp32 rows")
+    want = before.astype(np.float64)
+    slot = table[which, past]
+    want[slot, region.key_offset:region.key_offset + keys] = y[:, own:own + keys]
+    want[slot, region.value_offset:region.value_offset + values] = y[:, own + keys:own + keys + values]
+    got = download(pool, before.shape, "bfloat16")
+    close(got, want, 6e-3, "cache")
+    untouched = np.setdiff1d(np.arange(slots), slot)
+    assert np.array_equal(got[untouched], before[untouched])
+
+
 @pytest.mark.parametrize("rows,experts,top,n,k", [(1, 8, 4, 1218, 72), (8, 64, 8, 200, 520), (9, 40, 6, 122, 200), (16, 33, 2, 282, 136),
                                                   (17, 300, 3, 98, 72), (32, 60, 3, 90, 1000), (32, 16, 2, 1026, 2048),
                                                   (2, 4, 2, 58, 72), (40, 9, 2, 130, 104)])  # a tile per block
