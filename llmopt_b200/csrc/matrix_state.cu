@@ -29,12 +29,14 @@ constexpr uint32_t kLanes = 16;   // lanes per column
 constexpr uint32_t kColumns = 2;  // columns per thread
 constexpr uint32_t kColumnWarps = kSlice / kColumns * kLanes / 32;  // 4
 
-// Columns per CTA of a scan.  The delta rule is bound by a chain per token (a sum over the lanes of a column, then the
-// update), behind which twice the columns hide: 395 us for 2048 tokens and 16 heads of 128 columns, 435 with half a slice.
-// The matrix memory has no such chain and gains from twice the CTAs: 269 us for 8 heads of 256 columns, 344 with a whole
-// slice.  While the producers waited for their loads within each chunk the two took 470 and 349 us.
-template <bool MEMORY> __host__ __device__ constexpr uint32_t scan_columns() { return MEMORY ? kSlice / 2u : kSlice; }
-constexpr uint32_t kLoaderWarps = 8;  // bring in q, k and v and write out; one more warp prepares the tokens' scalars
+// A scan comes in two forms (launch_scan says where which is used):
+//  * AHEAD: eight loader warps request a chunk ahead, one more warp prepares the tokens' scalars.  The matrix memory then runs with
+//    half a slice per CTA, two of them a cluster; the delta rule, bound by a chain per token (a sum over the lanes of a
+//    column, then the update), keeps the whole slice, behind which twice the columns hide.
+//  * otherwise four loader warps wait for their loads within each chunk: 288 or 256 threads in place of 384 or 416, so that
+//    more CTAs share an SM.
+template <bool MEMORY, bool AHEAD> __host__ __device__ constexpr uint32_t scan_columns() { return MEMORY && AHEAD ? kSlice / 2u : kSlice; }
+template <bool AHEAD> __host__ __device__ constexpr uint32_t loader_warps() { return AHEAD ? 8u : 4u; }  // bring in q, k and v and write out
 
 __host__ __device__ constexpr uint32_t slices_of(uint32_t vdim) { return (vdim + kSlice - 1u) / kSlice; }
 
@@ -337,9 +339,10 @@ struct ScanChunk {
 // leave the state as it is).
 template <int CHUNK> struct ScanGroup { static constexpr uint32_t kTokens = CHUNK >= 8 ? 4 : 1; };
 
-template <bool MEMORY> struct ScanThreads {
-  static constexpr uint32_t kCompute = (scan_columns<MEMORY>() / kColumns * kLanes / 32u + (MEMORY ? 1u : 0u)) * 32u;  // one more warp carries n
-  static constexpr uint32_t kProducers = (kLoaderWarps + 1u) * 32u;
+template <bool MEMORY, bool AHEAD> struct ScanThreads {
+  static constexpr uint32_t kCompute =
+      (scan_columns<MEMORY, AHEAD>() / kColumns * kLanes / 32u + (MEMORY ? 1u : 0u)) * 32u;  // one more warp carries n
+  static constexpr uint32_t kProducers = (loader_warps<AHEAD>() + (AHEAD ? 1u : 0u)) * 32u;
   static constexpr uint32_t kAll = kCompute + kProducers;
 };
 
@@ -422,18 +425,18 @@ struct StateColumns {
 };
 
 // TQ: element of q, k, v (fp32 for the delta rule, whose unit vectors are fp32).
-template <typename TQ, bool MEMORY, int R4, int CHUNK>
-__global__ void __launch_bounds__(ScanThreads<MEMORY>::kAll) scan_kernel(const TQ* query, const TQ* key, const TQ* value,
-                                                                         const float* first, const float* second,
-                                                                         float* state_pool, const uint32_t* past,
-                                                                         const uint32_t* sequence_rows, float* out,
-                                                                         ScanParams p) {
+template <typename TQ, bool MEMORY, bool AHEAD, int R4, int CHUNK>
+__global__ void __launch_bounds__(ScanThreads<MEMORY, AHEAD>::kAll) scan_kernel(const TQ* query, const TQ* key, const TQ* value,
+                                                                                const float* first, const float* second,
+                                                                                float* state_pool, const uint32_t* past,
+                                                                                const uint32_t* sequence_rows, float* out,
+                                                                                ScanParams p) {
   grid_chain_prologue();
   extern __shared__ __align__(16) unsigned char scan_shared[];
-  constexpr uint32_t kScanColumns = scan_columns<MEMORY>();
+  constexpr uint32_t kScanColumns = scan_columns<MEMORY, AHEAD>(), kLoaderWarps = loader_warps<AHEAD>();
   typedef ScanChunk<R4, CHUNK, kScanColumns> Chunk;
   Chunk* chunks = reinterpret_cast<Chunk*>(scan_shared);
-  constexpr uint32_t kCompute = ScanThreads<MEMORY>::kCompute;
+  constexpr uint32_t kCompute = ScanThreads<MEMORY, AHEAD>::kCompute;
   const uint32_t first_column = blockIdx.x * kScanColumns, head = blockIdx.y, sequence = blockIdx.z;
   const uint32_t slice = first_column / kSlice;
   const bool owner = first_column % kSlice == 0;  // stores the slice's n and m
@@ -445,30 +448,35 @@ __global__ void __launch_bounds__(ScanThreads<MEMORY>::kAll) scan_kernel(const T
   const uint32_t chunk_count = (p.tokens + CHUNK - 1u) / CHUNK;
   // The CTAs of a slice start from the same n and m, which one of them stores at the end: all have read them by then.
   auto ready = [] {
-    if (MEMORY) cluster_sync();
+    if (kScanColumns < kSlice) cluster_sync();
     else __syncthreads();
   };
 
   if (threadIdx.x >= kCompute) {
     // ------------------------------ producers ------------------------------
-    // What a chunk needs is requested while the one before it is stored to shared memory.
+    // AHEAD: what a chunk needs is requested while the one before it is stored to shared memory.
     const uint32_t thread = threadIdx.x - kCompute, warp = thread >> 5, lane = thread & 31u;
-    const bool loader = warp < kLoaderWarps;
+    const bool loader = !AHEAD || warp < kLoaderWarps, preparer = AHEAD ? !loader : warp == 0;  // of rows; of the tokens' scalars
     const float q_scale = MEMORY ? 1.0f / sqrtf((float)p.dim) : 1.0f;
     float top = 0.0f;  // memory form: running maximum (scalar warp)
-    if (MEMORY && !loader && !fresh) top = state[layout.top(head, slice)];
+    if (MEMORY && preparer && !fresh) top = state[layout.top(head, slice)];
     const uint32_t value_column = first_column + lane % kScanColumns;
     constexpr int kSteps = R4 * (int)kLanes / 8;  // 32-wide pieces of a row
-    constexpr uint32_t kBatch = CHUNK >= kLoaderWarps ? CHUNK / kLoaderWarps : 1;  // tokens per warp and chunk
+    constexpr uint32_t kBatch = !AHEAD ? 1 : CHUNK >= kLoaderWarps ? CHUNK / kLoaderWarps : 1;  // AHEAD: tokens per warp and chunk
     constexpr uint32_t kGroup = ScanGroup<CHUNK>::kTokens;
-    TQ q_raw[kBatch][kSteps], k_raw[kBatch][kSteps], v_raw[kBatch];
+    TQ q_next[kBatch][kSteps], k_next[kBatch][kSteps], v_next[kBatch];
     float first_raw = 0.0f, second_raw = 0.0f;
+    auto request_scalars = [&](uint32_t index) {
+      const uint32_t t0 = index * CHUNK, count = min((uint32_t)CHUNK, p.tokens - t0);
+      const size_t scalar_row = (row0 + t0 + min(lane, count - 1u)) * p.scalar_stride;
+      first_raw = first[scalar_row + p.first_column + head];
+      second_raw = second[scalar_row + p.second_column + head];
+    };
     auto request = [&](uint32_t index) {
+      if (!AHEAD) return;
       const uint32_t t0 = index * CHUNK, count = min((uint32_t)CHUNK, p.tokens - t0);
       if (!loader) {
-        const size_t scalar_row = (row0 + t0 + min(lane, count - 1u)) * p.scalar_stride;
-        first_raw = first[scalar_row + p.first_column + head];
-        second_raw = second[scalar_row + p.second_column + head];
+        request_scalars(index);
         return;
       }
       // loads without branches (absent elements read a present one), so that all of them are in flight at once
@@ -480,38 +488,13 @@ __global__ void __launch_bounds__(ScanThreads<MEMORY>::kAll) scan_kernel(const T
 #pragma unroll
         for (int i = 0; i < kSteps; ++i) {
           const uint32_t c = min(lane + i * 32u, p.dim - 1u);
-          q_raw[b][i] = q[c];
-          k_raw[b][i] = k[c];
+          q_next[b][i] = q[c];
+          k_next[b][i] = k[c];
         }
-        v_raw[b] = value[row * p.v_stride + p.v_column + head * p.vdim + min(value_column, p.vdim - 1u)];
+        v_next[b] = value[row * p.v_stride + p.v_column + head * p.vdim + min(value_column, p.vdim - 1u)];
       }
     };
-    auto produce = [&](uint32_t index) {
-      Chunk& chunk = chunks[index & 1u];
-      const uint32_t count = min((uint32_t)CHUNK, p.tokens - index * CHUNK);
-      const uint32_t padded = (count + kGroup - 1u) / kGroup * kGroup;
-      if (loader) {
-#pragma unroll
-        for (uint32_t b = 0; b < kBatch; ++b) {
-          const uint32_t t = warp + b * kLoaderWarps;
-          if (t >= padded) break;
-          float dot = 0.0f;
-#pragma unroll
-          for (int i = 0; i < kSteps; ++i) {
-            const bool present = lane + i * 32u < p.dim && t < count;
-            const float q = present ? as_float(q_raw[b][i]) * q_scale : 0.0f, k = present ? as_float(k_raw[b][i]) : 0.0f;
-            chunk.q[t][lane + i * 32u] = q;
-            chunk.k[t][lane + i * 32u] = k;
-            dot = fmaf(q, k, dot);
-          }
-          if (lane < kScanColumns) chunk.v[t][lane] = value_column < p.vdim ? as_float(v_raw[b]) : 0.0f;
-          if (!MEMORY) {
-            dot = warp_sum(dot);
-            if (lane == 0) chunk.scalar[t].z = dot;
-          }
-        }
-        return;
-      }
+    auto put_scalars = [&](Chunk& chunk, uint32_t count, uint32_t padded) {
       const bool present = lane < count;
       float a = first_raw, b = second_raw;
       if (MEMORY) {
@@ -541,6 +524,87 @@ __global__ void __launch_bounds__(ScanThreads<MEMORY>::kAll) scan_kernel(const T
         chunk.scalar[lane].y = present ? b : 0.0f;
       }
     };
+    auto produce = [&](uint32_t index) {
+      Chunk& chunk = chunks[index & 1u];
+      const uint32_t t0 = index * CHUNK, count = min((uint32_t)CHUNK, p.tokens - t0);
+      const uint32_t padded = (count + kGroup - 1u) / kGroup * kGroup;
+      if constexpr (AHEAD) {
+        if (loader) {
+#pragma unroll
+          for (uint32_t b = 0; b < kBatch; ++b) {
+            const uint32_t t = warp + b * kLoaderWarps;
+            if (t >= padded) break;
+            float dot = 0.0f;
+#pragma unroll
+            for (int i = 0; i < kSteps; ++i) {
+              const bool present = lane + i * 32u < p.dim && t < count;
+              const float q = present ? as_float(q_next[b][i]) * q_scale : 0.0f, k = present ? as_float(k_next[b][i]) : 0.0f;
+              chunk.q[t][lane + i * 32u] = q;
+              chunk.k[t][lane + i * 32u] = k;
+              dot = fmaf(q, k, dot);
+            }
+            if (lane < kScanColumns) chunk.v[t][lane] = value_column < p.vdim ? as_float(v_next[b]) : 0.0f;
+            if (!MEMORY) {
+              dot = warp_sum(dot);
+              if (lane == 0) chunk.scalar[t].z = dot;
+            }
+          }
+          return;
+        }
+        put_scalars(chunk, count, padded);
+        return;
+      }
+      constexpr uint32_t kTogether = kSteps <= 4 ? 4 : 2;  // tokens whose loads are in flight together
+      for (uint32_t begin = warp; begin < padded; begin += kLoaderWarps * kTogether) {
+        // loads without branches (absent elements read a present one), so that all of them are in flight at once
+        TQ q_raw[kTogether][kSteps], k_raw[kTogether][kSteps], v_raw[kTogether];
+#pragma unroll
+        for (uint32_t b = 0; b < kTogether; ++b) {
+          const size_t row = row0 + t0 + min(begin + b * kLoaderWarps, count - 1u);
+          const TQ* q = query + row * p.q_stride + p.q_column + kv_head * p.dim;
+          const TQ* k = key + row * p.k_stride + p.k_column + kv_head * p.dim;
+#pragma unroll
+          for (int i = 0; i < kSteps; ++i) {
+            const uint32_t c = min(lane + i * 32u, p.dim - 1u);
+            q_raw[b][i] = q[c];
+            k_raw[b][i] = k[c];
+          }
+          v_raw[b] = value[row * p.v_stride + p.v_column + head * p.vdim + min(value_column, p.vdim - 1u)];
+        }
+        float qs[kTogether][kSteps], ks[kTogether][kSteps], vs[kTogether];
+#pragma unroll
+        for (uint32_t b = 0; b < kTogether; ++b) {
+#pragma unroll
+          for (int i = 0; i < kSteps; ++i) {
+            const bool present = lane + i * 32u < p.dim && begin + b * kLoaderWarps < count;
+            qs[b][i] = present ? as_float(q_raw[b][i]) * q_scale : 0.0f;
+            ks[b][i] = present ? as_float(k_raw[b][i]) : 0.0f;
+          }
+          vs[b] = value_column < p.vdim ? as_float(v_raw[b]) : 0.0f;
+        }
+#pragma unroll
+        for (uint32_t b = 0; b < kTogether; ++b) {
+          const uint32_t t = begin + b * kLoaderWarps;
+          if (t >= padded) break;
+          float dot = 0.0f;
+#pragma unroll
+          for (int i = 0; i < kSteps; ++i) {
+            chunk.q[t][lane + i * 32u] = qs[b][i];
+            chunk.k[t][lane + i * 32u] = ks[b][i];
+            dot = fmaf(qs[b][i], ks[b][i], dot);
+          }
+          chunk.v[t][lane] = vs[b];
+          if (!MEMORY) {
+            dot = warp_sum(dot);
+            if (lane == 0) chunk.scalar[t].z = dot;
+          }
+        }
+      }
+      if (warp == 0) {
+        request_scalars(index);
+        put_scalars(chunk, count, padded);
+      }
+    };
     auto write_out = [&](uint32_t index) {
       const Chunk& chunk = chunks[index & 1u];
       const uint32_t t0 = index * CHUNK, count = min((uint32_t)CHUNK, p.tokens - t0);
@@ -559,14 +623,14 @@ __global__ void __launch_bounds__(ScanThreads<MEMORY>::kAll) scan_kernel(const T
       if (index > 0) {
         write_out(index - 1u);
         // its scalars are filled again next
-        if (MEMORY) asm volatile("bar.sync 1, %0;" ::"n"(ScanThreads<MEMORY>::kProducers) : "memory");
+        if (MEMORY || !AHEAD) asm volatile("bar.sync 1, %0;" ::"n"(ScanThreads<MEMORY, AHEAD>::kProducers) : "memory");
       }
       if (index + 1u < chunk_count) produce(index + 1u);
       if (index + 2u < chunk_count) request(index + 2u);
       __syncthreads();
     }
     write_out(chunk_count - 1u);
-    if (MEMORY && owner && !loader && lane == 0) state[layout.top(head, slice)] = top;
+    if (MEMORY && owner && preparer && lane == 0) state[layout.top(head, slice)] = top;
   } else {
     // ------------------------------ state ------------------------------
     const uint32_t column0 = threadIdx.x / kLanes * kColumns, part = threadIdx.x % kLanes;
@@ -747,28 +811,44 @@ int launch_scan(const KernelArgs& args) {
                  "buffer is too short");
   LLMOPT_REQUIRE(p.sequences <= 65535u && p.heads <= 65535u, "too many sequences or heads");
   if (rows == 0) return 0;
-  auto run = [&](auto kernel, size_t shared) {
+  auto run = [&](auto kernel, size_t shared, uint32_t threads, uint32_t per_slice) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared) != cudaSuccess) {
       cudaGetLastError();
       return fail(args, "shared memory request was refused");
     }
-    auto launch = [&](auto&& start, uint32_t blocks, auto... cluster) {
-      start(args, kernel, dim3(blocks, p.heads, p.sequences), dim3(ScanThreads<MEMORY>::kAll), shared, cluster...,
+    auto launch = [&](auto&& start, auto... cluster) {
+      start(args, kernel, dim3(slices_of(p.vdim) * per_slice, p.heads, p.sequences), dim3(threads), shared, cluster...,
             (const TQ*)args.buffers[0], (const TQ*)args.buffers[1], (const TQ*)args.buffers[2], (const float*)args.buffers[3],
             (const float*)args.buffers[4], (float*)args.buffers[5], (const uint32_t*)args.buffers[6],
             (const uint32_t*)args.buffers[7], (float*)args.buffers[8], p);
     };
-    constexpr uint32_t kScanColumns = scan_columns<MEMORY>(), kPerSlice = kSlice / kScanColumns;
-    if (MEMORY) launch([](auto&&... a) { launch_cluster_kernel(a...); }, slices_of(p.vdim) * kPerSlice, kPerSlice);
-    else launch([](auto&&... a) { launch_kernel(a...); }, (p.vdim + kScanColumns - 1u) / kScanColumns);
+    if (per_slice > 1u) launch([](auto&&... a) { launch_cluster_kernel(a...); }, per_slice);
+    else launch([](auto&&... a) { launch_kernel(a...); });
     return check_launch(args);
   };
   const uint32_t quads = (p.dim + kLanes * 4u - 1u) / (kLanes * 4u);
+  // Ahead where that is faster, us, in brackets otherwise: matrix memory, dim 256, 2048 tokens, 64 slices 429 (601), 256 slices 1699 (1203):
+  // its two CTAs a slice need an SM each.  Delta rule, 2048 tokens, dim 128 394 (472), dim 64 324 (302), dim 192 as fast, dim 256
+  // 789 (594, where its registers spill); of four tokens the chunks are too short for it: dim 128 x 64 sequences 24 (20).
+  const size_t slices = (size_t)slices_of(p.vdim) * p.heads * p.sequences;
+  const bool ahead = MEMORY ? 2u * slices <= (size_t)context_sm_count(args.ctx) : quads == 2u && p.tokens > 4u;
+  auto form = [&](auto r4, auto constant, auto chunk) {
+    constexpr int R4 = decltype(r4)::value, CHUNK = decltype(chunk)::value;
+    constexpr bool AHEAD = decltype(constant)::value;
+    constexpr uint32_t kScanColumns = scan_columns<MEMORY, AHEAD>();
+    return run(scan_kernel<TQ, MEMORY, AHEAD, R4, CHUNK>, 2 * sizeof(ScanChunk<R4, CHUNK, kScanColumns>), ScanThreads<MEMORY, AHEAD>::kAll,
+               kSlice / kScanColumns);
+  };
   // few tokens: small chunks, so that more CTAs fit on an SM
   auto sized = [&](auto r4) {
-    constexpr int R4 = decltype(r4)::value;
-    if (p.tokens <= 4u) return run(scan_kernel<TQ, MEMORY, R4, 4>, 2 * sizeof(ScanChunk<R4, 4, scan_columns<MEMORY>()>));
-    return run(scan_kernel<TQ, MEMORY, R4, 32>, 2 * sizeof(ScanChunk<R4, 32, scan_columns<MEMORY>()>));
+    constexpr std::integral_constant<int, 4> few;
+    constexpr std::integral_constant<int, 32> many;
+    if constexpr (MEMORY) {
+      if (ahead) return p.tokens <= 4u ? form(r4, std::true_type(), few) : form(r4, std::true_type(), many);
+    } else if constexpr (decltype(r4)::value == 2) {
+      if (ahead) return form(r4, std::true_type(), many);
+    }
+    return p.tokens <= 4u ? form(r4, std::false_type(), few) : form(r4, std::false_type(), many);
   };
   if (quads <= 1u) return sized(std::integral_constant<int, 1>());
   if (quads <= 2u) return sized(std::integral_constant<int, 2>());

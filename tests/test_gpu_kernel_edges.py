@@ -349,6 +349,40 @@ def test_expert_rows_of_many_tiles(runtime, rows, experts, top, n, k):
     assert np.all(out.to_numpy(np.uint16)[pairs * n // 2:] == 0x7FC0)
 
 
+# ---- rules that look at how much there is to do: the same bits alone and among many ----------------------
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("dim,vdim", [(40, 40), (128, 70), (160, 96), (256, 33)])
+@pytest.mark.parametrize("tokens", [4, 70])
+def test_matrix_memory_alone_and_among_many(runtime, dtype, dim, vdim, tokens):
+    """One sequence (half slices) and forty alike (whole ones): the same read-outs and states."""
+    from llmopt_b200 import parameters
+    from llmopt_b200.kv_cache import matrix_state_elements
+    from test_gpu_mixers import suffix
+
+    rng = np.random.default_rng(dim + tokens)
+    heads, results = 3, []
+    width, stride = heads * (2 * dim + vdim), matrix_state_elements(heads, dim, vdim, normalized=True)
+    slices = -(-vdim // 32)
+    raw, gates = rng.standard_normal((tokens, width)) * 0.5, rng.standard_normal((tokens, 2 * heads)).astype(np.float32)
+    state = (rng.standard_normal(stride) * 0.3).astype(np.float32)
+    norms = heads * vdim * dim  # the copies of n and m of a head are alike
+    state[norms:norms + heads * slices * dim] = np.repeat(rng.standard_normal((heads, 1, dim)), slices, 1).reshape(-1)
+    state[norms + heads * slices * dim:][:heads * slices] = np.repeat(rng.standard_normal(heads), slices)
+    for sequences in (1, 40):
+        pool, out = upload(runtime, np.tile(state, (sequences, 1))), empty(runtime, sequences * tokens * heads * vdim)
+        projected, scalars = upload(runtime, np.tile(raw, (sequences, 1)), dtype), upload(runtime, np.tile(gates, (sequences, 1)))
+        runtime.dispatch("llmopt_memory_scan_" + suffix(dtype), buffers=[
+            projected, projected, projected, scalars, scalars, pool, upload(runtime, np.full(sequences, 5, np.uint32)),
+            upload(runtime, np.arange(sequences, dtype=np.uint32)), out], parameters=parameters.state_scan(
+                sequences=sequences, tokens=tokens, heads=heads, kv_heads=heads, dim=dim, vdim=vdim, q_stride=width, q_column=0,
+                k_stride=width, k_column=heads * dim, v_stride=width, v_column=2 * heads * dim, scalar_stride=2 * heads, first_column=0,
+                second_column=heads, state_rows=sequences, state_stride=stride, gate_cap=6.0))
+        results.append((download(out, (sequences, tokens, heads, vdim)), download(pool, (sequences, stride))))
+    for alone, among in zip(*results):
+        assert np.all(np.isfinite(alone)) and all(np.array_equal(alone[0], one) for one in among)
+
+
 # ---- paged attention in its forms -----------------------------------------------------------------------
 
 @pytest.mark.parametrize("batch,q_heads,k_heads,dim,group,past", [
