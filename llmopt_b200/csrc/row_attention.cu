@@ -471,20 +471,16 @@ __global__ void __launch_bounds__(128, prompt_ctas(DK, EXTENDED)) attention_prom
 
 // ---- decode --------------------------------------------------------------------------------------
 constexpr uint32_t kWarpKeys = 16, kDecodeWarps = 4, kMostSplits = 64;
-// Tiles in a warp's ring.  With 128-wide heads two leave room for a third CTA on an SM, so that the usual split counts are
-// one wave: 8 sequences x 2048 keys x 4 key heads 27.9 -> 19.9 us, 32 x 1028 45.4 -> 32.4 (three tiles, two CTAs, before).
-__host__ __device__ constexpr uint32_t decode_stages(int DK) { return DK == 128 ? 2u : 3u; }
-
 // Record of one split: 16 maxima, 16 denominators, 16 x DV sums.
 template <int DV>
 __host__ __device__ constexpr uint32_t record_floats() { return 32u + 16u * DV; }
 
-template <int DK, int DV, bool EXTENDED>
+template <int DK, int DV, bool EXTENDED, uint32_t STAGES>
 __global__ void __launch_bounds__(128) attention_decode_kernel(const bf16* query, const bf16* pool, const uint32_t* table,
                                                                const uint32_t* past_lengths, const uint32_t* sequence_rows,
                                                                bf16* out, const bf16* gate, uint32_t* counters, float* records,
                                                                RowAttentionParams p, uint32_t* error_word) {
-  constexpr uint32_t kDecodeStages = decode_stages(DK);
+  constexpr uint32_t kDecodeStages = STAGES;  // tiles in a warp's ring
   grid_chain_prologue();
   extern __shared__ __align__(16) unsigned char attention_shared[];
   const uint32_t padded = DK > 0 ? DK : round16(p.dim), k_stride = padded + 8u, v_stride = DV + 8u;
@@ -731,17 +727,17 @@ int run_prompt(const KernelArgs& args, const RowAttentionParams& p) {
   return check_launch(args);
 }
 
-template <int DK, int DV, bool EXTENDED>
-int run_decode(const KernelArgs& args, const RowAttentionParams& p) {
+template <int DK, int DV, bool EXTENDED, uint32_t STAGES>
+int run_decode_stages(const KernelArgs& args, const RowAttentionParams& p) {
   const uint32_t padded = DK > 0 ? DK : round16(p.dim);
-  uint32_t bytes = (16u * (padded + 8u) + kDecodeWarps * decode_stages(DK) * kWarpKeys * (padded + 8u + DV + 8u)) * 2u;
+  uint32_t bytes = (16u * (padded + 8u) + kDecodeWarps * STAGES * kWarpKeys * (padded + 8u + DV + 8u)) * 2u;
   const uint32_t merge = kDecodeWarps * record_floats<DV>() * 4u;
   if (bytes < merge) bytes = merge;
   const size_t heads = (size_t)p.sequences * p.kv_heads, counters = (heads * 4 + 255) / 256 * 256;
   LLMOPT_REQUIRE(p.splits <= kMostSplits, "at most 64 splits");
   LLMOPT_REQUIRE(p.splits == 1u || args.lengths[6] >= counters + heads * p.splits * record_floats<DV>() * 4,
                  "split scratch is too short");
-  auto kernel = attention_decode_kernel<DK, DV, EXTENDED>;
+  auto kernel = attention_decode_kernel<DK, DV, EXTENDED, STAGES>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
     cudaGetLastError();
     return -1;
@@ -752,6 +748,18 @@ int run_decode(const KernelArgs& args, const RowAttentionParams& p) {
                 (uint32_t*)args.buffers[6],
                 (float*)((uint8_t*)args.buffers[6] + counters), p, context_device_error(args.ctx));
   return check_launch(args);
+}
+
+// With 128-wide heads a ring of two tiles leaves room for a third CTA on an SM, a ring of three keeps more under way.  Two where
+// that saves a wave: 8 sequences x 2048 keys x 4 key heads, 416 CTAs, 19.9 us with two and 27.9 with three; 32 x 2048 x 8, 256
+// CTAs, 112 and 92.
+template <int DK, int DV, bool EXTENDED>
+int run_decode(const KernelArgs& args, const RowAttentionParams& p) {
+  if constexpr (DK == 128) {
+    const size_t ctas = (size_t)p.splits * p.kv_heads * p.sequences, sms = (size_t)context_sm_count(args.ctx);
+    if ((ctas + 3u * sms - 1u) / (3u * sms) < (ctas + 2u * sms - 1u) / (2u * sms)) return run_decode_stages<DK, DV, EXTENDED, 2>(args, p);
+  }
+  return run_decode_stages<DK, DV, EXTENDED, 3>(args, p);
 }
 
 template <int DK, int DV>
