@@ -15,7 +15,10 @@
 //    splits in split order.
 //  * bf16, more rows (prompts): 64 query tokens of one head per CTA, 64-key tiles double-buffered with
 //    cp.async, online softmax in fp32, P rounded to bfloat16 for P V.
-//  * fp32, and head sizes that are no whole 16-byte vectors: one CTA per (row, head), whose warps split the keys.
+//  * fp32, and head sizes that are no whole 16-byte vectors: one CTA per (row, head), whose warps split the keys, or, with many
+//    rows, one warp.
+#include <type_traits>
+
 #include "element.cuh"
 
 namespace llmopt {
@@ -198,6 +201,57 @@ __global__ void __launch_bounds__(kRowThreads) attention_rows_kernel(const T* qu
   for (int i = 0; i < COLUMNS; ++i) {
     const uint32_t c = threadIdx.x + i * kRowThreads;
     if (c < p.vdim) out[(size_t)item * p.vdim + c] = from_float<T>(o[i] / total * gate_of<true>(p, gate, row, head, c));
+  }
+}
+
+// ---- one warp per (row, head) --------------------------------------------------------------------
+// The same arithmetic, a warp walking over the keys one after the other: with enough rows and heads to fill the chip the
+// latencies hide behind other warps, and nothing is exchanged within a CTA.
+template <typename T, int SEGMENTS>
+__global__ void __launch_bounds__(128) attention_walk_kernel(const T* query, const T* pool, const uint32_t* table,
+                                                             const uint32_t* past, const uint32_t* sequence_rows, T* out,
+                                                             const T* gate, RowAttentionParams p, uint32_t* error_word) {
+  grid_chain_prologue();
+  const uint32_t lane = threadIdx.x & 31u, item = blockIdx.x * 4u + (threadIdx.x >> 5);
+  if (item >= p.sequences * p.tokens * p.heads) return;
+  const uint32_t row = item / p.heads, head = item % p.heads, sequence = row / p.tokens;
+  const uint32_t kv_head = head / (p.heads / p.kv_heads);
+  const uint32_t position = past[sequence] + row % p.tokens;
+  const Visible<true> visible(p, position, position);
+  const KeyRows rows = key_rows(p, table, sequence_rows[sequence]);
+  float q[SEGMENTS], o[SEGMENTS];
+#pragma unroll
+  for (int s = 0; s < SEGMENTS; ++s) {
+    const uint32_t c = lane + s * 32u;
+    q[s] = c < p.dim ? as_float(query[(size_t)row * p.query_stride + p.query_column + head * p.dim + c]) : 0.0f;
+    o[s] = 0.0f;
+  }
+  float top = p.sink ? 0.0f : kLowest, total = p.sink ? 1.0f : 0.0f;
+  for (uint32_t index = 0; index < visible.count(); ++index) {
+    const T* cached = pool + (size_t)rows(visible.position(index), error_word) * p.token_stride;
+    const T* k = cached + p.key_offset + kv_head * p.dim;
+    const T* v = cached + p.value_offset + kv_head * p.vdim;
+    float score = 0.0f;
+#pragma unroll
+    for (int s = 0; s < SEGMENTS; ++s) {
+      const uint32_t c = lane + s * 32u;
+      if (c < p.dim) score = fmaf(q[s], as_float(k[c]), score);
+    }
+    score = warp_sum(score) * p.scale;
+    if (p.softcap > 0.0f) score = p.softcap * tanhf(score / p.softcap);
+    const float next = fmaxf(top, score), keep = expf(top - next), weight = expf(score - next);
+    top = next;
+    total = total * keep + weight;
+#pragma unroll
+    for (int s = 0; s < SEGMENTS; ++s) {
+      const uint32_t c = lane + s * 32u;
+      if (c < p.vdim) o[s] = o[s] * keep + weight * as_float(v[c]);
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < SEGMENTS; ++s) {
+    const uint32_t c = lane + s * 32u;
+    if (c < p.vdim) out[(size_t)item * p.vdim + c] = from_float<T>(o[s] / total * gate_of<true>(p, gate, row, head, c));
   }
 }
 
@@ -694,17 +748,30 @@ __global__ void __launch_bounds__(128) attention_decode_kernel(const bf16* query
 template <typename T>
 int run_rows(const KernelArgs& args, const RowAttentionParams& p) {
   const size_t items = (size_t)p.sequences * p.tokens * p.heads;
-  LLMOPT_REQUIRE(items <= 0x7fffffffu, "too many rows");
   const uint32_t widest = p.dim > p.vdim ? p.dim : p.vdim;
-  auto run = [&](auto kernel) {
-    launch_kernel(args, kernel, dim3((uint32_t)items), dim3(kRowThreads), 0, (const T*)args.buffers[0],
+  // Rows and heads per SM up to which a CTA for each is faster than a warp for each; from there on warps hide one another's
+  // latencies.  The rows of a prompt differ in length, so that the longest walks bound it and the line lies higher.  fp32, 16 heads,
+  // a CTA and a warp each, us: heads of 128, 150 keys, 80 sequences 146 and 178, 200 sequences 286 and 182; a prompt of 200 tokens
+  // 92 and 115, of 800 1184 and 800; heads of 256, 1000 tokens 1850 and 2100, 2048 tokens 7380 and 7030.
+  const uint32_t tokens = p.tokens;
+  const uint32_t per_sm = widest <= 64u    ? min(15u + tokens / 10u, 38u)
+                          : widest <= 128u ? min(11u + tokens / 14u, 29u)
+                                           : min(24u + tokens / 2u, 170u);
+  const bool walk = items > (size_t)per_sm * (size_t)context_sm_count(args.ctx);
+  auto launch = [&](auto kernel, size_t ctas) {
+    launch_kernel(args, kernel, dim3((uint32_t)ctas), dim3(kRowThreads), 0, (const T*)args.buffers[0],
                   (const T*)args.buffers[1], (const uint32_t*)args.buffers[2], (const uint32_t*)args.buffers[3],
                   (const uint32_t*)args.buffers[4], (T*)args.buffers[5], (const T*)args.buffers[7], p, context_device_error(args.ctx));
   };
-  if (widest <= 64u) run(attention_rows_kernel<T, 2>);
-  else if (widest <= 128u) run(attention_rows_kernel<T, 4>);
-  else if (widest <= 256u) run(attention_rows_kernel<T, 8>);
-  else if (widest <= 512u) run(attention_rows_kernel<T, 16>);
+  auto run = [&](auto segments) {
+    constexpr int SEGMENTS = decltype(segments)::value;
+    if (walk) launch(attention_walk_kernel<T, SEGMENTS>, (items + kRowWarps - 1u) / kRowWarps);
+    else launch(attention_rows_kernel<T, SEGMENTS>, items);
+  };
+  if (widest <= 64u) run(std::integral_constant<int, 2>());
+  else if (widest <= 128u) run(std::integral_constant<int, 4>());
+  else if (widest <= 256u) run(std::integral_constant<int, 8>());
+  else if (widest <= 512u) run(std::integral_constant<int, 16>());
   else return fail(args, "head sizes above 512 are not supported");
   return check_launch(args);
 }

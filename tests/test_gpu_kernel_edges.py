@@ -351,6 +351,39 @@ def test_expert_rows_of_many_tiles(runtime, rows, experts, top, n, k):
 
 # ---- rules that look at how much there is to do: the same bits alone and among many ----------------------
 
+@pytest.mark.parametrize("dtype,heads,kv_heads,dim,vdim,tokens,many,splits", [
+    ("float32", 16, 4, 20, 24, 9, 60, 1), ("float32", 16, 8, 128, 100, 3, 200, 1), ("float32", 8, 1, 256, 512, 2, 2000, 1),
+    ("bfloat16", 16, 4, 18, 10, 7, 90, 1),                                                       # a block or a warp per row and head
+    ("bfloat16", 16, 4, 128, 128, 1, 8, 13), ("bfloat16", 8, 8, 128, 128, 2, 40, 1), ("bfloat16", 8, 8, 128, 128, 1, 64, 1)])  # rings
+def test_row_attention_alone_and_among_many(runtime, dtype, heads, kv_heads, dim, vdim, tokens, many, splits):
+    """The first sequence alone and with others that make the dispatch choose another kernel or ring; a window and a cap on the way."""
+    from llmopt_b200 import parameters
+    from test_gpu_mixers import suffix
+
+    rng = np.random.default_rng(dim + many)
+    past = rng.integers(0, 400, size=many).astype(np.uint32)
+    past[0] = 301
+    stride, token_stride = 400 + tokens, kv_heads * (dim + vdim)
+    pool_rows = 3000
+    pool = upload(runtime, rng.standard_normal((pool_rows, token_stride)), dtype)
+    table = upload(runtime, rng.integers(0, pool_rows, size=(many, stride)).astype(np.uint32))
+    query = rng.standard_normal((many * tokens, heads * dim))
+    for options in ({}, dict(window=70, keep_first=3, softcap=9.0)):
+        results = []
+        for sequences in (1, many):
+            out = empty(runtime, sequences * tokens * heads * vdim, dtype)
+            scratch = upload(runtime, np.zeros(4096 + sequences * kv_heads * splits * (32 + 16 * 256), np.float32))
+            q = upload(runtime, query[:sequences * tokens], dtype)
+            runtime.dispatch("llmopt_row_attention_" + suffix(dtype), buffers=[
+                q, pool, table, upload(runtime, past), upload(runtime, np.arange(many, dtype=np.uint32)), out, scratch, q],
+                parameters=parameters.row_attention(
+                    sequences=sequences, tokens=tokens, heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, token_stride=token_stride,
+                    key_offset=0, value_offset=kv_heads * dim, table_stride=stride, table_rows=many, pool_rows=pool_rows, sink=bool(options),
+                    splits=splits, scale=dim ** -0.5, **options))
+            results.append(download(out, (sequences, tokens, heads, vdim), dtype)[0])
+        assert np.all(np.isfinite(results[0])) and np.array_equal(*results)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("dim,vdim", [(40, 40), (128, 70), (160, 96), (256, 33)])
 @pytest.mark.parametrize("tokens", [4, 70])
