@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(kGemvWarps * 32, NT <= 4 ? 2 : 1) dense_gemv_k
 
 // The same sums, in the same order, for matrices with a tile for every SM and more.  A CTA per tile had three blocks of
 // weights under way while it waited for the activation rows in L2, which came to two thirds of its traffic with 32 rows,
-// and nothing while it stored.  32 rows, k 2048: n 32768 76 -> 36 us, n 14336 (pairs) 38 -> 22, n 5120 (cached) 20.5 -> 16.4.
+// and nothing while it stored.  32 rows, k 2048, over cold weights: n 32768 64 -> 34 us, n 14336 (pairs) 31 -> 20, n 5120 18 -> 11.5.
 template <int NT, DenseStore STORE>
 __global__ void __launch_bounds__(kWideThreads, WideShape<NT>::kMostPerSm) dense_wide_kernel(const DenseTask<STORE> p) {
   grid_launch_dependents();

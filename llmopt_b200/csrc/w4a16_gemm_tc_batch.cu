@@ -45,8 +45,8 @@ constexpr int kThreads = (2 + kConvertWarps) * 32;
 constexpr uint32_t kSplitCounterTiles = 1u << 14;
 
 // kBatchLinear: one 128-row weight tile per CTA; kBatchDualSwiglu: the gate and the up tile of the same rows;
-// kBatchLinearPair: two neighbouring 128-row tiles of ONE matrix (the prompt form: the activation tile is
-// read once for 256 output columns); kBatchDualStacked: ONE tile whose lanes 0..63 are 64 gate rows and
+// kBatchLinearPair: two neighbouring 128-row tiles of ONE matrix (zero-point prompts below 256 rows: the activation
+// tile is read once for 256 output columns); kBatchDualStacked: ONE tile whose lanes 0..63 are 64 gate rows and
 // lanes 64..127 the same 64 up rows, so that gate/up prompts also run 256 tokens wide with one accumulator
 // (the halves meet in shared memory for silu(gate) * up).
 // kBatchSplitF32: one weight tile; the activation rows are fp32 values given as exact hi/lo half pairs in
@@ -670,7 +670,8 @@ int run_batch(const KernelArgs& args, const CUtensorMap& map_x, BatchProblem p) 
 // Rows from which decode batches take this kernel (below it the small-M GEMV wins);
 // LLMOPT_CUDA_TC_BATCH_MIN_ROWS overrides it, 0 disables the kernel.  Measured at the Llama-8B shapes
 // (us in a back-to-back run over 32 operand sets, pipelined GEMV -> this kernel): 32 rows: gate/up 54.1 ->
-// 36.7, down 35.2 -> 30.4, o_proj 11.2 -> 14.7, QKV (three launches here) 15.4 -> 42; 16 rows: gate/up
+// 36.7, down 35.2 -> 30.4, o_proj 11.2 -> 14.7, QKV (4096 + 2 x 1024 columns,
+// one launch here) 14.9 -> 15.1; 16 rows: gate/up
 // 36.0 -> 35.4, down 17.2 -> 26.6.  So from 17 rows the large matrices take it, the small ones from 33.
 uint32_t tensor_core_batch_min_rows() {
   static const uint32_t rows = []() -> uint32_t {
