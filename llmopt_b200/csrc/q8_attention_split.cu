@@ -686,16 +686,16 @@ uint32_t pinned_splits() {
 
 // A cluster saves the merge kernel and the way through scratch; records take as many splits as fill the chip, also in several
 // waves.  What each costs, in keys that one CTA of four warps walks over: its share of the longest sequence times its waves,
-// kWave for each wave, and for records kMerge and kRecord for each.  A CTA of eight warps takes its keys at twice the rate and kWideCta more to
-// begin with.  Clusters fill nine tenths of the chip at most (72 pairs x 8 CTAs take two waves).  The constants are
-// fitted to 22 numbers of pairs from 3 to 512, capacities of 64 to 16384 keys, full, half full and an eighth full, as plans and
-// alone, with heads of 64 and 128: nowhere slower than records alone by more than 3 %, on average 14 % faster.  With 8 heads of
-// 128 a sequence, records -> this rule, us: 1 x 512 6.6 -> 5.3 (plan), 5 x 2048 16.2 -> 14.0, 16 x 2048 26.4 -> 22.7, 32 x 2048
+// kWave for each wave (of kMostWaves; more overlap), and for records kMerge and kRecord for each.  A CTA of eight warps takes its
+// keys at twice the rate and kWideCta more to begin with.  Clusters fill nine tenths of the chip at most (72 pairs x 8 CTAs take two
+// waves).  The constants are fitted to 23 numbers of pairs from 3 to 512, capacities of 64 to 16384 keys, full, half full and an
+// eighth full, as plans and alone, with heads of 64 and 128: nowhere slower than records alone by more than 3 %, on average 13 %
+// faster.  With 8 heads of 128 a sequence, records -> this rule, us: 1 x 512 6.6 -> 5.8 (plan), 5 x 2048 16.2 -> 14.0, 16 x 2048 26.4 -> 22.7, 32 x 2048
 // 46.6 -> 38.9; where the rule keeps records, records (the best cluster): 1 x 8192 11.5 (17.1), 5 x 8192 29.2 (34.6), 9 x 8192 39.4 (58).
 // What a plan may grow to decides, not what it was captured at.
 ClusterPlan pick_cluster(const KernelArgs& args, const PagedParams& p, uint32_t slot_batch_stride) {
   if (pinned_splits() != 0u) return {0u, 0u};
-  constexpr float kWave = 150.0f, kMerge = 50.0f, kRecord = 0.5f, kWideCta = 24.0f;
+  constexpr float kWave = 120.0f, kMerge = 50.0f, kRecord = 0.5f, kWideCta = 24.0f, kMostWaves = 3.0f;
   const size_t slots = args.lengths[4] / 4u, before = (size_t)(p.batches - 1u) * slot_batch_stride;
   const size_t longest = args.past_tokens_cell ? (slots > before ? slots - before : 0u) : p.past_length;
   const size_t pairs = (size_t)p.batches * p.kv_heads, resident = (size_t)context_sm_count(args.ctx) * kResidentCtas;
@@ -704,14 +704,15 @@ ClusterPlan pick_cluster(const KernelArgs& args, const PagedParams& p, uint32_t 
   auto waves = [](size_t ctas, size_t room) { return (float)((ctas + room - 1u) / room); };
   const uint32_t splits = paged_pick_splits(args, p);
   const float record_waves = waves(pairs * splits, resident);
-  float least = kMerge + kRecord * (float)splits + record_waves * (kWave + (float)longest / (float)splits);
+  auto cost_of = [&](float count, float share) { return fminf(count, kMostWaves) * kWave + count * share; };
+  float least = kMerge + kRecord * (float)splits + cost_of(record_waves, (float)longest / (float)splits);
   ClusterPlan best = {0u, 0u};
   const ClusterPlan forms[] = {{2u, 4u}, {4u, 4u}, {8u, 4u}, {8u, 8u}};
   for (const ClusterPlan& form : forms) {
     const float rate = (float)form.warps / (float)kWarps;
     const float form_waves = waves(pairs * form.ctas, (size_t)((float)resident * 0.9f / rate));
     if (form.warps > (uint32_t)kWarps && form_waves > 1.0f) continue;
-    const float cost = form_waves * (kWave + (float)longest / ((float)form.ctas * rate)) + (form.warps > (uint32_t)kWarps ? kWideCta : 0.0f);
+    const float cost = cost_of(form_waves, (float)longest / ((float)form.ctas * rate)) + (form.warps > (uint32_t)kWarps ? kWideCta : 0.0f);
     if (cost < least) least = cost, best = form;
   }
   return best;
