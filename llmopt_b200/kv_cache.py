@@ -172,12 +172,15 @@ class SequenceTable:
         need = (wanted + self.page - 1) // self.page
         if need - have > len(self._free_pages):
             raise ValueError("the cache has no free pages")
-        for index in range(have, need):
-            page = self._free_pages.pop()
-            self._pages[row].append(page)
-            first = index * self.page
-            for position in range(first, min(first + self.page, self.stride)):
-                self.table[row, position] = page * self.page + position - first
+        if need > have:
+            import numpy as np
+
+            pages = self._free_pages[:have - need - 1:-1]  # the last ones first
+            del self._free_pages[have - need:]
+            self._pages[row].extend(pages)
+            slots = np.asarray(pages, np.uint32)[:, None] * np.uint32(self.page) + np.arange(self.page, dtype=np.uint32)
+            first, end = have * self.page, min(need * self.page, self.stride)
+            self.table[row, first:end] = slots.reshape(-1)[:end - first]
         return range(min(have * self.page, self.stride), min(need * self.page, self.stride))
 
     def advance(self, row: int, tokens: int) -> None:

@@ -26,6 +26,7 @@ from .residual import RESIDUALS
 from .safetensors_archive import as_bfloat16_bits, as_float32
 
 ARGMAX_PARTS = 32
+KEPT_LOGITS_ROWS = 64  # rows of a prompt's logits whose buffer the engine keeps
 
 
 def _draw_seed(seed: int, *counters: int) -> int:
@@ -110,6 +111,7 @@ class MixerEngine:
         self._trig: Dict[object, Buffer] = {}
         self._prompt_plans: "OrderedDict[int, tuple]" = OrderedDict()
         self._decode_plans: Dict[int, tuple] = {}
+        self._prompt_logits: Tuple[int, Optional[Buffer], Optional[Buffer]] = (0, None, None)
         self.residual = RESIDUALS[config.norm](self, weights)
         self.token_side = self.upload_matrix(weights["side.embed"]) if config.token_side else None
         self.layers = [_Layer(self, index, weights) for index in range(len(config.layers))]
@@ -235,6 +237,18 @@ class MixerEngine:
             self._decode_plans[sequences] = (plan, graph, logits, picked)
         return self._decode_plans[sequences]
 
+    def _prompt_outputs(self, rows: int) -> Tuple[Buffer, Buffer]:
+        """(places, logits) of ``rows`` rows of a prompt.  Freeing device memory stalls the device and takes longer the more a
+        program holds, 0.7 to 20 ms a prompt, so up to ``KEPT_LOGITS_ROWS`` rows stay with the engine; more (a program that
+        scores a whole text) live for the call."""
+        kept, chosen, logits = self._prompt_logits
+        if rows > kept:
+            room = 1 << (rows - 1).bit_length() if rows <= KEPT_LOGITS_ROWS else rows
+            chosen, logits = self.empty_bytes(max(room * 4, 16)), self.empty_bytes(room * self.config.vocabulary * 4)
+            if rows <= KEPT_LOGITS_ROWS:
+                self._prompt_logits = (room, chosen, logits)
+        return chosen, logits
+
     def _prompt_plan(self, tokens: int):
         """(plan, packed dispatch list) of ``tokens`` rows of one sequence."""
         if tokens not in self._prompt_plans:
@@ -316,8 +330,8 @@ class MixerEngine:
         commands.dispatch_recorded(records)
         logits = None
         if len(want):
-            logits = self.empty_bytes(len(want) * self.config.vocabulary * 4)
-            chosen = Buffer.of_array(self.runtime, np.ascontiguousarray(want, np.uint32))
+            chosen, logits = self._prompt_outputs(len(want))
+            chosen.write(0, np.ascontiguousarray(want, np.uint32))
             kept, plan.items = plan.items, []
             self._record_logits(plan.step, chosen, len(want), logits)
             for item in plan.items:
@@ -325,7 +339,10 @@ class MixerEngine:
             plan.items = kept
         commands.commit()
         self.sequences.advance(sequence, len(tokens))
-        return None if logits is None else logits.to_numpy(np.float32, (len(want), self.config.vocabulary))
+        if logits is None:
+            return None
+        vocabulary = self.config.vocabulary
+        return logits.view(0, len(want) * vocabulary * 4).to_numpy(np.float32, (len(want), vocabulary))
 
     # ---- the interface of the decode engine -------------------------------------------------------------
     def _row(self, sequence: int) -> int:
