@@ -1,13 +1,14 @@
 // Dense linear layer in fp32 (CUDA cores, no TF32) where weight and activation rows are whole 16-byte vectors:
 //  * up to 32 rows: dense_f32_stream_kernel, bound by the weight stream.  A warp takes two columns and up to eight rows and
 //    keeps up to 32 loads of weights in flight.
-//  * more rows: dense_f32_tile_kernel, bound by reads of shared memory.  Operands come by cp.async in k-major rows as they lie
-//    in memory; a thread reads four k of a row at once.
+//  * more rows: dense_f32_tile_kernel, bound by the multiply-adds and the reads of shared memory side by side (0.55 to 0.6 of the fp32
+//    rate where all SMs are busy).  Operands come by cp.async.
 // Both add the products of an output in the order of the general kernels (dense_linear.cu: lanes 32 apart, and k one after
 // the other), to the last bit: fp32 is what checkpoints are checked with, and decoders that divide by nearly cancelling sums
 // show every change of it.  k shared out over a cluster, with even and odd k as the halves of packed multiply-adds, was faster (2048 x
-// 2048 x 100 rows 32 us) but moved logits by 2.9e-5.  Now, 100 rows back to back over cold operands, with the time of 64 x 64
-// tiles and 4-byte loads: n 2048, k 2048 66 us, 305 before; n 2048, k 7168 227, 1075 before; n 7168, k 2048 123, 337 before.
+// 2048 x 100 rows 32 us) but moved logits by 2.9e-5.  Pairs of rows keep the order.  Back to back over cold operands, before (scalar
+// multiply-adds, 16 bytes of either operand in four cycles a read, two CTAs on one SM while others idle) and now, us: 100 rows n 2048 k
+// 2048 66, 41; n 2048 k 7168 226, 133; n 7168 k 2048 123, 111; n 9248 k 2048 123, 110; 333 rows n 7168 k 2048 445, 290.
 #include "dense_linear.cuh"
 
 namespace llmopt {
@@ -15,27 +16,48 @@ namespace {
 
 constexpr uint32_t kDepth = 32;    // k of a stage: a row is one 128-byte line
 constexpr uint32_t kPitch = kDepth + 4;  // floats; eight consecutive rows start in eight different groups of four banks
-constexpr uint32_t kThreads = 128;
+constexpr uint32_t kOnePerSm = 117u * 1024u;  // bytes of shared memory of which an SM has no two
 constexpr uint32_t kMostDown = 65535;  // tiles of rows: a grid's second dimension
 
-// 16 bytes to shared memory, zeros where absent.
+// 16 or 4 bytes to shared memory, zeros where absent.
 __device__ __forceinline__ void copy_vector(float* to, const float* from, bool present) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from),
                "r"(present ? 16u : 0u)
                : "memory");
 }
-// Stages of 32 k: what two CTAs of an SM have room for.  A sum is not split, so a CTA walks over all of k and a stage takes as
-// long as its way from memory unless many are under way.
-__host__ __device__ constexpr uint32_t tile_stages(int TM, int TN) { return TM * TN <= 16 ? 8u : TM * TN <= 32 ? 6u : 4u; }
+__device__ __forceinline__ void copy_one(float* to, const float* from, bool present) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from),
+               "r"(present ? 4u : 0u)
+               : "memory");
+}
+// Two sums at once: the halves are rounded one by one, as fmaf does.
+__device__ __forceinline__ void multiply_add_pair(unsigned long long& sum, unsigned long long two, float one) {
+  asm("{.reg .b64 both;\n\tmov.b64 both, {%2, %2};\n\tfma.rn.f32x2 %0, %1, both, %0;}" : "+l"(sum) : "l"(two), "f"(one));
+}
 
-// A tile of 8 TM rows x 16 TN columns; thread (mi, ni) of 8 x 16 owns rows mi + 8 i and columns ni + 16 j.  Every sum walks
-// over all of k in order; four k of an operand are one read.
-template <int TM, int TN, DenseStore STORE>
-__global__ void __launch_bounds__(kThreads, 2) dense_f32_tile_kernel(const DenseTask<STORE> p, const DensePlan plan) {
-  constexpr uint32_t kRows = 8 * TM, kColumns = 16 * TN, kStages = tile_stages(TM, TN);
-  constexpr uint32_t kStageFloats = (kRows + kColumns) * kPitch;
+// DOWN x ACROSS threads; thread (mi, ni) owns rows TM mi .. TM mi + TM - 1 and columns ni + j ACROSS.  Every sum walks over all
+// of k in order.  Weights lie as in memory, four k of a column are one read; rows are transposed on their way in, so that one read
+// holds two pairs of them: packed multiply-adds take half the issue slots, and the copies of a weight to both halves go
+// where those are free.
+template <int TM, int TN, int DOWN, int ACROSS>
+struct Tile {
+  static constexpr uint32_t kThreads = DOWN * ACROSS, kRows = TM * DOWN, kColumns = TN * ACROSS;
+  static constexpr uint32_t kRowPitch = kRows + 4, kStageFloats = kDepth * kRowPitch + kColumns * kPitch;
+  // A sum is not split, so a CTA walks over all of k and a stage takes as long as its way from memory unless many are under way:
+  // what two CTAs of an SM have room for, one of the largest tiles.
+  static constexpr uint32_t kStages = kRows == 32u ? 8u : kColumns == 64u ? 6u : 8u;
+  static constexpr uint32_t kBytes = kStages * kStageFloats * sizeof(float);
+  static constexpr uint32_t kPerSm = kBytes <= 114u * 1024u ? 2u : 1u;
+};
+
+template <int TM, int TN, int DOWN, int ACROSS, DenseStore STORE>
+__global__ void __launch_bounds__(Tile<TM, TN, DOWN, ACROSS>::kThreads, Tile<TM, TN, DOWN, ACROSS>::kPerSm)
+    dense_f32_tile_kernel(const DenseTask<STORE> p, const DensePlan plan) {
+  typedef Tile<TM, TN, DOWN, ACROSS> Shape;
+  constexpr uint32_t kThreads = Shape::kThreads, kWarps = kThreads / 32u;
+  constexpr uint32_t kRows = Shape::kRows, kColumns = Shape::kColumns, kStages = Shape::kStages, kRowPitch = Shape::kRowPitch;
   constexpr uint32_t kSumPitch = kColumns + 4;
-  static_assert(kRows * kSumPitch <= kStages * kStageFloats, "the sums take the stages' place");
+  static_assert(kRows * kSumPitch * sizeof(float) <= Shape::kBytes, "the sums take the stages' place");
   extern __shared__ __align__(16) float stages[];
   const uint32_t n0 = blockIdx.x * kColumns;
   const float* x = reinterpret_cast<const float*>(p.x);
@@ -54,75 +76,88 @@ __global__ void __launch_bounds__(kThreads, 2) dense_f32_tile_kernel(const Dense
     w += (size_t)tile.expert * p.n * p.k;
   }
   const uint32_t blocks = (p.k + kDepth - 1u) / kDepth;
-  const uint32_t lane_k = (threadIdx.x & 7u) * 4u, lane_row = threadIdx.x >> 3;  // of the copies
-  auto copy_x = [&](uint32_t block) {
-    float* const to = stages + block % kStages * kStageFloats;
-    const uint32_t k = block * kDepth + lane_k;
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  auto copy_x = [&](uint32_t block) {  // a warp's copy: four rows, eight k of each, to 32 banks
+    float* const to = stages + block % kStages * Shape::kStageFloats;
 #pragma unroll
-    for (uint32_t row = lane_row; row < kRows; row += 16u) {
-      const bool present = k < p.k && m0 + row < row_end;
-      copy_vector(to + row * kPitch + lane_k, present ? x + (size_t)(m0 + row) * p.k + k : x, present);
+    for (uint32_t part = 0; part < kRows / kWarps; ++part) {
+      const uint32_t row = (warp + part * kWarps) / 4u * 4u + (lane >> 3), k = warp % 4u * 8u + (lane & 7u);
+      const bool present = block * kDepth + k < p.k && m0 + row < row_end;
+      copy_one(to + k * kRowPitch + row, present ? x + (size_t)(m0 + row) * p.k + block * kDepth + k : x, present);
     }
   };
   auto copy_w = [&](uint32_t block) {
-    float* const to = stages + block % kStages * kStageFloats + kRows * kPitch;
-    const uint32_t k = block * kDepth + lane_k;
+    float* const to = stages + block % kStages * Shape::kStageFloats + kDepth * kRowPitch;
+    const uint32_t lane_k = (threadIdx.x & 7u) * 4u, k = block * kDepth + lane_k;
 #pragma unroll
-    for (uint32_t row = lane_row; row < kColumns; row += 16u) {
+    for (uint32_t row = threadIdx.x >> 3; row < kColumns; row += kThreads / 8u) {
       const bool present = k < p.k && n0 + row < p.n;
       copy_vector(to + row * kPitch + lane_k, present ? w + (size_t)(n0 + row) * p.k + k : w, present);
     }
   };
   // the weights are nobody's output: their first stages may be requested before the predecessor ends
 #pragma unroll
-  for (uint32_t s = 0; s + 1u < kStages; ++s)
+  for (uint32_t s = 0; s < kStages; ++s)
     if (s < blocks) copy_w(s);
   grid_dependency_wait();
 #pragma unroll
-  for (uint32_t s = 0; s + 1u < kStages; ++s) {
+  for (uint32_t s = 0; s < kStages; ++s) {
     if (s < blocks) copy_x(s);
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-  const uint32_t mi = (lane >> 3) + 4u * (warp & 1u), ni = (lane & 7u) + 8u * (warp >> 1);
-  float sum[TM][TN];
+  // A read of 16 bytes a lane takes two cycles instead of four where lanes one apart, or lanes two apart, read the same: bit 0 of
+  // the lane only chooses among rows, bit 1 only among columns.
+  constexpr uint32_t kWarpsDown = DOWN / 4u;
+  const uint32_t mi = (lane & 1u) + (lane >> 1 & 2u) + warp % kWarpsDown * 4u;
+  const uint32_t ni = (lane >> 1 & 1u) + (lane >> 2 & 6u) + warp / kWarpsDown * 8u;
+  unsigned long long sum[TM / 2][TN];  // rows 2 i and 2 i + 1
 #pragma unroll
-  for (int i = 0; i < TM; ++i)
+  for (int i = 0; i < TM / 2; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) sum[i][j] = 0.0f;
+    for (int j = 0; j < TN; ++j) sum[i][j] = 0ull;
+  float4 b[2][TN];  // four k each: those that are multiplied, and the next ones on their way
+  ulonglong2 a[2][4][TM / 4];
+  auto read = [&](int side, uint32_t block, uint32_t k) {
+    const float* const xs = stages + block % kStages * Shape::kStageFloats + k * kRowPitch + mi * TM;
+    const float* const ws = stages + block % kStages * Shape::kStageFloats + kDepth * kRowPitch + ni * kPitch + k;
+#pragma unroll
+    for (int j = 0; j < TN; ++j) b[side][j] = *reinterpret_cast<const float4*>(ws + j * ACROSS * kPitch);
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+#pragma unroll
+      for (int i = 0; i < TM / 4; ++i) a[side][q][i] = *reinterpret_cast<const ulonglong2*>(xs + q * kRowPitch + i * 4);
+  };
+  asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 1) : "memory");
+  __syncthreads();
+  read(0, 0, 0);
   for (uint32_t block = 0; block < blocks; ++block) {
-    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
-    __syncthreads();  // this stage has arrived, and the one before it is read
-    if (block + kStages - 1u < blocks) {
-      copy_w(block + kStages - 1u);
-      copy_x(block + kStages - 1u);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    const float* const xs = stages + block % kStages * kStageFloats + mi * kPitch;
-    const float* const ws = stages + block % kStages * kStageFloats + (kRows + ni) * kPitch;
 #pragma unroll
     for (uint32_t k = 0; k < kDepth; k += 4u) {
-      float4 a[TM], b[TN];
+      const int side = k / 4u & 1u;
+      if (k + 4u < kDepth) {
+        read(side ^ 1, block, k + 4u);
+      } else {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+        __syncthreads();  // the next stage has arrived, and this one is read
+        if (block + kStages < blocks) {
+          copy_w(block + kStages);
+          copy_x(block + kStages);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        read(side ^ 1, block + 1u, 0);  // past the last block: what an earlier one left, multiplied by nobody
+      }
 #pragma unroll
-      for (int j = 0; j < TN; ++j) b[j] = *reinterpret_cast<const float4*>(ws + j * 16 * kPitch + k);
+      for (int q = 0; q < 4; ++q)
 #pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4*>(xs + i * 8 * kPitch + k);
+        for (int j = 0; j < TN; ++j) {
+          const float4& four = b[side][j];
+          const float weight = q == 0 ? four.x : q == 1 ? four.y : q == 2 ? four.z : four.w;
 #pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) sum[i][j] = fmaf(a[i].x, b[j].x, sum[i][j]);
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) sum[i][j] = fmaf(a[i].y, b[j].y, sum[i][j]);
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) sum[i][j] = fmaf(a[i].z, b[j].z, sum[i][j]);
-#pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) sum[i][j] = fmaf(a[i].w, b[j].w, sum[i][j]);
+          for (int i = 0; i < TM / 4; ++i) {
+            multiply_add_pair(sum[2 * i][j], a[side][q][i].x, weight);
+            multiply_add_pair(sum[2 * i + 1][j], a[side][q][i].y, weight);
+          }
+        }
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -131,7 +166,9 @@ __global__ void __launch_bounds__(kThreads, 2) dense_f32_tile_kernel(const Dense
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) sums[(mi + 8u * i) * kSumPitch + ni + 16u * j] = sum[i][j];
+    for (int j = 0; j < TN; ++j)
+      sums[(mi * TM + i) * kSumPitch + ni + j * ACROSS] =
+          __uint_as_float(i & 1 ? (uint32_t)(sum[i / 2][j] >> 32) : (uint32_t)sum[i / 2][j]);
   __syncthreads();
   for (uint32_t index = threadIdx.x; index < kRows * kColumns / 2u; index += kThreads) {
     const uint32_t row = index / (kColumns / 2u), column = index % (kColumns / 2u) * 2u;
@@ -221,30 +258,35 @@ int run(const KernelArgs& args, DenseProblem p, uint32_t tiles) {
     else launch_kernel(args, dense_f32_stream_kernel<8, STORE>, dim3(columns, (p.m + 7u) / 8u), dim3(256), 0, task);
     return check_launch(args);
   }
-  // The tile for which the fullest SM has the least to read from shared memory, which bounds all of them: 16 (TM + TN) cycles per
-  // four k and CTA.  One CTA alone on an SM runs at about half the rate.
+  // The tile with which the fullest SM is done first.  Measured per 2048 k: a tile of 32 x 64 alone on its SM 40 us, two side by side 60;
+  // 64 x 64 68 and 128; 64 x 128, which has an SM to itself, 107.
   const uint32_t sms = (uint32_t)context_sm_count(args.ctx);
   auto down = [&](uint32_t high) { return p.plan.tiles ? tiles * (kExpertTile / high) : p.m / high + (p.m % high ? 1u : 0u); };
   if (down(64u) > kMostDown) return -1;
-  auto cost = [&](uint32_t high, uint32_t wide) {
+  auto cost = [&](uint32_t high, uint32_t wide, uint32_t alone, uint32_t beside) {
     // the plan's tiles are 128 rows at most and hold m / tiles on average; those without rows end at once
     const uint32_t rows = p.plan.tiles ? p.m / (tiles ? tiles : 1u) : p.m;
     const uint32_t full = p.plan.tiles ? tiles * ((rows + high - 1u) / high) : down(high);
     const uint32_t most = ((p.n + wide - 1u) / wide * full + sms - 1u) / sms;
-    return (most < 2u ? 2u : most) * (high / 8u + wide / 16u);
+    return (size_t)(most / 2u) * beside + (most % 2u) * alone;
   };
-  auto launch = [&](auto kernel, uint32_t high, uint32_t wide) {
-    const size_t shared = (size_t)tile_stages((int)high / 8, (int)wide / 16) * (high + wide) * kPitch * sizeof(float);
+  auto launch = [&](auto kernel, auto shape) {
+    typedef decltype(shape) Shape;
+    const dim3 grid((p.n + Shape::kColumns - 1u) / Shape::kColumns, down(Shape::kRows));
+    // Where every CTA finds an SM of its own none shares one: CTAs that start beside the last ones of the launch before double up
+    // (2048 x 2048 x 100 rows 59 us, 41 this way).
+    const uint32_t bytes = (size_t)grid.x * grid.y <= sms && Shape::kBytes < kOnePerSm ? kOnePerSm : Shape::kBytes;
     // per device and kernel; cheap beside the launch, and remembered nowhere
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared) != cudaSuccess)
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
       return fail(args, "shared memory could not be raised");
-    launch_kernel(args, kernel, dim3((p.n + wide - 1u) / wide, down(high)), dim3(kThreads), shared, task, p.plan);
+    launch_kernel(args, kernel, grid, dim3(Shape::kThreads), bytes, task, p.plan);
     return check_launch(args);
   };
-  const uint32_t large = cost(64u, 128u), middle = cost(64u, 64u), small = cost(32u, 64u);
-  if (down(32u) <= kMostDown && small <= middle && small <= large) return launch(dense_f32_tile_kernel<4, 4, STORE>, 32u, 64u);
-  if (middle <= large) return launch(dense_f32_tile_kernel<8, 4, STORE>, 64u, 64u);
-  return launch(dense_f32_tile_kernel<8, 8, STORE>, 64u, 128u);
+  const size_t large = cost(64u, 128u, 107u, 214u), middle = cost(64u, 64u, 68u, 128u), small = cost(32u, 64u, 40u, 60u);
+  if (down(32u) <= kMostDown && small <= middle && small <= large)
+    return launch(dense_f32_tile_kernel<4, 4, 8, 16, STORE>, Tile<4, 4, 8, 16>());
+  if (middle <= large) return launch(dense_f32_tile_kernel<4, 4, 16, 16, STORE>, Tile<4, 4, 16, 16>());
+  return launch(dense_f32_tile_kernel<8, 4, 8, 32, STORE>, Tile<8, 4, 8, 32>());
 }
 
 }  // namespace
