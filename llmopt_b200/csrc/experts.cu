@@ -137,6 +137,9 @@ int launch_route_step(const KernelArgs& args) {
 // contraction: a warp adds an expert's sums to those of the rows that chose it when it goes on to the next.  Otherwise x
 // is [row][k] and blockIdx.y picks the expert.
 // The first eight rows of an expert travel through the stages with the weights, further ones are loaded when it is their turn.
+// With an expert's 28 blocks shared out over 16 warps nearly every block begins another expert, so what bounds it besides the
+// stream is what that costs: places are counted on instead of divided out, and sums of rows that an expert does not have are not
+// looked at.  16 experts of 2048 x 1792, two a row, over cold weights: 32 rows 40.2 -> 27.3 us, 8 rows 21.4 -> 17.8, one 9.7 -> 8.4.
 template <int NT, bool DOWN>
 __global__ void __launch_bounds__(kGemvWarps * 32, NT <= 4 ? 2 : 1) expert_step_kernel(DenseTask<DOWN ? kStoreResidual : kStorePair> p, uint32_t experts, const uint32_t* route, Route at, uint32_t pairs) {
   const uint32_t cluster = p.cluster;
@@ -184,20 +187,43 @@ __global__ void __launch_bounds__(kGemvWarps * 32, NT <= 4 ? 2 : 1) expert_step_
   };
   const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
   uint4 a[kGemvStages][4], b[kGemvStages][2];
-  auto fetch = [&](int stage, uint32_t index) {
-    const bool present = index < blocks;
-    const uint32_t place = DOWN && present ? index / per_expert : 0u, block = index - place * per_expert;
-    const bf16* matrix = DOWN && present ? w + (size_t)chosen[place] * p.n * p.k : w;
-    stream_fetch(a[stage], matrix + (size_t)low * p.k, matrix + (size_t)high * p.k, present ? p.k : 0u, block);
-    const bf16* row = present ? row_of(place, 0) : nullptr;
+  // A warp takes every `stride`th block of the contraction: expert `place`, its block `block`, one step after the other.
+  struct Walk {
+    uint32_t place, block;
+  };
+  auto step = [&](Walk& at, uint32_t by) {  // true on a new expert
+    at.block += by;
+    bool moved = false;
+    if constexpr (DOWN)
+      for (; at.block >= per_expert; at.block -= per_expert, ++at.place) moved = true;
+    return moved;
+  };
+  const bf16 *row_low = w + (size_t)low * p.k, *row_high = w + (size_t)high * p.k, *x_row = nullptr;
+  auto enter = [&](uint32_t place) {
+    if (DOWN && place >= used) return;
+    if (DOWN) {
+      const bf16* matrix = w + (size_t)chosen[place] * p.n * p.k;
+      row_low = matrix + (size_t)low * p.k, row_high = matrix + (size_t)high * p.k;
+    }
+    x_row = row_of(place, 0);
+  };
+  Walk ahead = {0u, 0u};
+  step(ahead, rank * kGemvWarps + warp);
+  enter(ahead.place);
+  auto fetch = [&](int stage) {
+    const bool present = DOWN ? ahead.place < used : ahead.block < blocks;
+    const uint32_t block = ahead.block;
+    stream_fetch(a[stage], row_low, row_high, present ? p.k : 0u, block);
+    const bf16* row = present ? x_row : nullptr;
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       const uint32_t k = block * 64u + half * 32u + t * 8u;
       b[stage][half] = row != nullptr && k < p.k ? *reinterpret_cast<const uint4*>(row + k) : zero;
     }
+    if (step(ahead, stride)) enter(ahead.place);
   };
 #pragma unroll
-  for (int s = 0; s < kGemvStages; ++s) fetch(s, rank * kGemvWarps + warp + s * stride);
+  for (int s = 0; s < kGemvStages; ++s) fetch(s);
   float sum[NT][4];
   auto clear = [&]() {
 #pragma unroll
@@ -209,23 +235,32 @@ __global__ void __launch_bounds__(kGemvWarps * 32, NT <= 4 ? 2 : 1) expert_step_
   auto flush = [&](uint32_t place) {
     const uint32_t first = firsts[DOWN ? place : 0], count = count_of(place);
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
+    for (int nt = 0; nt < NT; ++nt) {
+      if (nt > 0 && nt * 8u >= count) break;  // most experts have a tile's rows at most
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint32_t c = nt * 8u + 2u * t + (i & 1);
-        if (c < count) partial[warp][row_of_slot[DOWN ? first + c : 0]][g + (i >> 1) * 8] += sum[nt][i];
+      for (int i = 0; i < 2; ++i) {
+        const uint32_t c = nt * 8u + 2u * t + i;
+        if (c < count) {
+          float* const row = partial[warp][row_of_slot[DOWN ? first + c : 0]];
+          row[g] += sum[nt][i];
+          row[g + 8u] += sum[nt][2 + i];
+        }
       }
+    }
     __syncwarp();
     clear();
   };
   clear();
+  Walk now = {0u, 0u};
+  step(now, rank * kGemvWarps + warp);
   uint32_t current = 0;
   for (uint32_t first = rank * kGemvWarps + warp; first < blocks; first += kGemvStages * stride) {
 #pragma unroll
     for (int s = 0; s < kGemvStages; ++s) {
       const uint32_t index = first + s * stride;
       if (index < blocks) {
-        const uint32_t place = DOWN ? index / per_expert : 0u, block = index - place * per_expert;
+        const uint32_t place = now.place, block = now.block;
+        step(now, stride);
         if (DOWN && place != current) {
           flush(current);
           current = place;
@@ -245,7 +280,7 @@ __global__ void __launch_bounds__(kGemvWarps * 32, NT <= 4 ? 2 : 1) expert_step_
           }
         }
       }
-      fetch(s, index + kGemvStages * stride);
+      fetch(s);
     }
   }
   if (!DOWN) stream_collect<NT>(sum, partial[warp]);
