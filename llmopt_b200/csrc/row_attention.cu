@@ -13,8 +13,9 @@
 //    the query heads of a group ride in the 16 rows of one MMA tile, four warps walk over 16-key tiles
 //    with private cp.async rings.  The last CTA of a (sequence, key/value head) to arrive merges the
 //    splits in split order.
-//  * bf16, more rows (prompts): 64 query tokens of one head per CTA, 64-key tiles double-buffered with
-//    cp.async, online softmax in fp32, P rounded to bfloat16 for P V.
+//  * bf16, more rows (prompts): 64 query tokens of one head per CTA, 64- or 32-key tiles double-buffered with
+//    cp.async, online softmax in fp32, P rounded to bfloat16 for P V.  Where windowed prompts leave the chip idle three groups
+//    of warps share a CTA's keys.
 //  * fp32, and head sizes that are no whole 16-byte vectors: one CTA per (row, head), whose warps split the keys, or, with many
 //    rows, one warp.
 #include <type_traits>
@@ -46,12 +47,16 @@ constexpr float kBoundedCap = 40.0f;  // e^40 and e^-40, and sums of many of the
 struct KeyRows {  // rows of one sequence
   const uint32_t* slots;
   uint32_t limit, pool_rows;
-  // pool row of key `position`; an index outside the table or the pool reads row 0 and is reported
-  __device__ __forceinline__ uint32_t operator()(uint32_t position, uint32_t* error_word) const {
-    const uint32_t slot = position < limit ? slots[position] : pool_rows;
+  // What the table says about key `position`, without waiting for it, and the pool row that this is; an index outside the table or
+  // the pool reads row 0 and is reported.
+  __device__ __forceinline__ uint32_t listed(uint32_t position) const { return position < limit ? slots[position] : pool_rows; }
+  __device__ __forceinline__ uint32_t checked(uint32_t slot, uint32_t* error_word) const {
     if (slot < pool_rows) return slot;
     if (error_word) atomicExch(error_word, 1u);
     return 0u;
+  }
+  __device__ __forceinline__ uint32_t operator()(uint32_t position, uint32_t* error_word) const {
+    return checked(listed(position), error_word);
   }
 };
 __device__ __forceinline__ KeyRows key_rows(const RowAttentionParams& p, const uint32_t* table, uint32_t row) {
@@ -402,26 +407,31 @@ __device__ __forceinline__ void scores(float (&score)[KEYS / 8][4], const uint32
 
 // ---- prompts -------------------------------------------------------------------------------------
 constexpr uint32_t kQueryTile = 64;
-// Keys per tile, and CTAs per SM to compile for (0: no bound): with smaller tiles a third CTA fits, which hides more of the
-// longer way from a score to its weight.
+// Keys per tile, groups of four warps that take turns with the tiles, and CTAs per SM to compile for (0: no bound).  What bounds the
+// kernel is the way from a score to its weight, which other warps hide (mma.sync alone would take a quarter of the time), and the CTAs
+// that start late: the longest go first over all heads, slots are looked up a tile ahead.  2048 tokens, 16 heads of 128, before
+// and now: 155 and 97 us, with windows 137 and 109.
 __host__ __device__ constexpr uint32_t key_tile(int DK, bool EXTENDED) { return EXTENDED && DK == 128 ? 32u : 64u; }
-constexpr int prompt_ctas(int DK, bool EXTENDED) { return DK != 128 ? 0 : EXTENDED ? 3 : 2; }
+constexpr int prompt_ctas(int DK, bool EXTENDED, uint32_t GROUPS) { return DK != 128 ? 0 : GROUPS > 1u ? 1 : EXTENDED ? 3 : 2; }
 
-template <int DK, int DV, bool EXTENDED>
-__global__ void __launch_bounds__(128, prompt_ctas(DK, EXTENDED)) attention_prompt_kernel(const bf16* query, const bf16* pool, const uint32_t* table,
+template <int DK, int DV, bool EXTENDED, uint32_t GROUPS>
+__global__ void __launch_bounds__(128 * GROUPS, prompt_ctas(DK, EXTENDED, GROUPS)) attention_prompt_kernel(const bf16* query, const bf16* pool, const uint32_t* table,
                                                                const uint32_t* past_lengths, const uint32_t* sequence_rows,
                                                                bf16* out, const bf16* gate, RowAttentionParams p, uint32_t* error_word) {
   constexpr uint32_t kKeyTile = key_tile(DK, EXTENDED), kPerKey = 128u / kKeyTile;  // threads that fetch a key
+  constexpr uint32_t kGroups = GROUPS, kThreads = 128u * kGroups;
   grid_chain_prologue();
   extern __shared__ __align__(16) unsigned char attention_shared[];
   const uint32_t padded = DK > 0 ? DK : round16(p.dim), k_stride = padded + 8u, v_stride = DV + 8u;
   bf16* q_tile = reinterpret_cast<bf16*>(attention_shared);
-  bf16* k_tiles = q_tile + kQueryTile * k_stride;
+  const uint32_t group = kGroups > 1u ? threadIdx.x >> 7 : 0u, thread = threadIdx.x & 127u;
+  bf16* k_tiles = q_tile + kQueryTile * k_stride + group * 2u * kKeyTile * (k_stride + v_stride);
   bf16* v_tiles = k_tiles + 2u * kKeyTile * k_stride;
-  // the last query tiles see the most keys: they are scheduled first
-  const uint32_t q0 = (gridDim.x - 1u - blockIdx.x) * kQueryTile, head = blockIdx.y, sequence = blockIdx.z;
+  // the last query tiles see the most keys: they are scheduled first, over all heads
+  const uint32_t place = blockIdx.y * gridDim.x + blockIdx.x, head = place % p.heads, sequence = blockIdx.z;
+  const uint32_t q0 = (gridDim.x - 1u - place / p.heads) * kQueryTile;
   const uint32_t kv_head = head / (p.heads / p.kv_heads);
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, r = lane >> 2, c = lane & 3u;
+  const uint32_t warp = thread >> 5, lane = threadIdx.x & 31u, r = lane >> 2, c = lane & 3u;
   const uint32_t past = past_lengths[sequence];
   const KeyRows rows = key_rows(p, table, sequence_rows[sequence]);
   const uint32_t key_end = past + min(q0 + kQueryTile, p.tokens);
@@ -429,18 +439,32 @@ __global__ void __launch_bounds__(128, prompt_ctas(DK, EXTENDED)) attention_prom
   const Visible<EXTENDED> visible(p, past + q0, key_end - 1u);
   const uint32_t kept_tiles = (visible.kept + kKeyTile - 1u) / kKeyTile;
   const uint32_t skipped = max(visible.begin / kKeyTile, kept_tiles) - kept_tiles;
-  const uint32_t tiles = (key_end + kKeyTile - 1u) / kKeyTile - skipped;
-  auto first_key = [&](uint32_t tile) { return (tile < kept_tiles ? tile : tile + skipped) * kKeyTile; };
+  const uint32_t all_tiles = (key_end + kKeyTile - 1u) / kKeyTile - skipped;
+  const uint32_t tiles = (all_tiles + kGroups - 1u - group) / kGroups;  // of this group: every kGroups-th
+  auto first_key = [&](uint32_t turn) {
+    const uint32_t tile = turn * kGroups + group;
+    return (tile < kept_tiles ? tile : tile + skipped) * kKeyTile;
+  };
+  auto group_sync = [&]() {
+    if (kGroups == 1u) __syncthreads();
+    else asm volatile("bar.sync %0, 128;" ::"r"(1u + group) : "memory");
+  };
   const uint32_t k_chunks = padded / 8u, v_chunks = DV / 8u;
+  const uint32_t key = thread / kPerKey, share = thread % kPerKey;  // of the copies
 
+  auto slot_of = [&](uint32_t tile) {
+    const uint32_t position = first_key(tile) + key;
+    return tile < tiles && position < key_end ? rows.listed(position) : 0u;
+  };
+  uint32_t slot = slot_of(0);  // of the tile that is fetched next
   auto fetch_tile = [&](uint32_t tile) {
     if (tile < tiles) {
       bf16* k_tile = k_tiles + (tile & 1u) * kKeyTile * k_stride;
       bf16* v_tile = v_tiles + (tile & 1u) * kKeyTile * v_stride;
       // a few threads per key row: one slot look-up, a share of the chunks each
-      const uint32_t key = threadIdx.x / kPerKey, share = threadIdx.x % kPerKey, position = first_key(tile) + key;
-      const bool present = position < key_end;
-      const bf16* cached = pool + (size_t)(present ? rows(position, error_word) : 0u) * p.token_stride;
+      const bool present = first_key(tile) + key < key_end;
+      const bf16* cached = pool + (size_t)(present ? rows.checked(slot, error_word) : 0u) * p.token_stride;
+      slot = slot_of(tile + 1u);  // used a tile from now
       const bf16* k = cached + p.key_offset + kv_head * p.dim;
       const bf16* v = cached + p.value_offset + kv_head * p.vdim;
       for (uint32_t chunk = share; chunk < k_chunks; chunk += kPerKey) {
@@ -454,15 +478,16 @@ __global__ void __launch_bounds__(128, prompt_ctas(DK, EXTENDED)) attention_prom
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  fetch_tile(0);
-  for (uint32_t index = threadIdx.x; index < kQueryTile * k_chunks; index += 128u) {
+  for (uint32_t index = threadIdx.x; index < kQueryTile * k_chunks; index += kThreads) {
     const uint32_t row = index / k_chunks, chunk = index % k_chunks;
-    uint4 data = make_uint4(0u, 0u, 0u, 0u);
-    if (q0 + row < p.tokens && chunk * 8u < p.dim)
-      data = *reinterpret_cast<const uint4*>(query + ((size_t)sequence * p.tokens + q0 + row) * p.query_stride +
-                                             p.query_column + head * p.dim + chunk * 8u);
-    *reinterpret_cast<uint4*>(q_tile + row * k_stride + chunk * 8u) = data;
+    const bool there = q0 + row < p.tokens && chunk * 8u < p.dim;
+    copy_async_16(q_tile + row * k_stride + chunk * 8u,
+                  there ? query + ((size_t)sequence * p.tokens + q0 + row) * p.query_stride + p.query_column + head * p.dim + chunk * 8u : pool,
+                  there ? 16u : 0u);
   }
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  fetch_tile(0);
+  asm volatile("cp.async.wait_group 1;" ::: "memory");  // the queries; their way hides behind the first look-up
   __syncthreads();
   const bf16* q_rows = q_tile + warp * 16u * k_stride;
   uint32_t q_frag[DK > 0 ? DK / 16 : 1][4];
@@ -479,7 +504,7 @@ __global__ void __launch_bounds__(128, prompt_ctas(DK, EXTENDED)) attention_prom
     const uint32_t k0 = first_key(tile);
     fetch_tile(tile + 1u);  // into the other buffer, which the previous iteration's last barrier released
     asm volatile("cp.async.wait_group 1;" ::: "memory");
-    __syncthreads();
+    group_sync();
     float score[kKeyTile / 8][4];
     scores<kKeyTile, DK>(score, q_frag, q_rows, k_tiles + (tile & 1u) * kKeyTile * k_stride, k_stride, padded / 16u, lane);
     const uint32_t first_row = past + q0 + warp * 16u;  // of this warp
@@ -493,9 +518,69 @@ __global__ void __launch_bounds__(128, prompt_ctas(DK, EXTENDED)) attention_prom
         score[j][i] = all_visible || sees<EXTENDED>(p, past + token, key) ? score_of(score[j][i]) : -INFINITY;
       }
     state.absorb(score, v_tiles + (tile & 1u) * kKeyTile * v_stride, v_stride, lane);
-    __syncthreads();  // every warp is done with this buffer before the next iteration's fetch refills it
+    group_sync();  // every warp is done with this buffer before the next iteration's fetch refills it
   }
   asm volatile("cp.async.wait_all;" ::: "memory");
+  // The sums of thread t of a group and its part: columns 8 t + 2 c and the one after it, row r + 8 h.  With several groups each
+  // finishes its share of the t: a gate's exponential and division are a long chain.
+  constexpr int kShare = (DV / 8 + (int)kGroups - 1) / (int)kGroups;
+  const int first_t = kGroups > 1u ? (int)group * kShare : 0;
+  auto column_of = [&](int t) { return 8u * (uint32_t)(first_t + t) + 2u * c; };
+  // all gates are requested before the first is needed: a load after each store was 14 us of a prompt's attention
+  bf16 gates[EXTENDED ? 2 : 1][EXTENDED ? kShare : 1][2];
+  if (EXTENDED && p.gate_stride) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const size_t row = (size_t)sequence * p.tokens + min(row_low + h * 8u, p.tokens - 1u);
+      const bf16* const source = gate + row * p.gate_stride + p.gate_column + head * p.vdim;
+#pragma unroll
+      for (int t = 0; t < kShare; ++t)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) gates[EXTENDED ? h : 0][EXTENDED ? t : 0][i] = source[min(column_of(t) + i, p.vdim - 1u)];
+    }
+  }
+  float sums[kShare][4];
+  if constexpr (kGroups > 1u) {  // what the groups have, added in their order; the rings are free
+    constexpr uint32_t kValues = 4u + DV / 2u;  // of a thread
+    float* const shared_values = reinterpret_cast<float*>(q_tile);
+    auto value_of = [&](uint32_t other, uint32_t i) -> float& { return shared_values[(other * kValues + i) * 128u + thread]; };
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < 2; ++h) value_of(group, h) = state.top[h], value_of(group, 2 + h) = state.total[h];
+#pragma unroll
+    for (int t = 0; t < DV / 8; ++t)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) value_of(group, 4 + 4 * t + i) = state.out[t][i];
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < kShare; ++t)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sums[t][i] = 0.0f;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float top = kLowest, total = 0.0f;
+#pragma unroll
+      for (uint32_t other = 0; other < kGroups; ++other) top = fmaxf(top, value_of(other, h));
+#pragma unroll
+      for (uint32_t other = 0; other < kGroups; ++other) {
+        const float weight = exp2_approx(value_of(other, h) - top);  // 1 where no maximum is taken off
+        total += value_of(other, 2 + h) * weight;
+#pragma unroll
+        for (int t = 0; t < kShare; ++t)
+          if (first_t + t < DV / 8) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) sums[t][2 * h + i] += value_of(other, 4 + 4 * (first_t + t) + 2 * h + i) * weight;
+          }
+      }
+      state.top[h] = top;
+      state.total[h] = total;
+    }
+  } else {
+#pragma unroll
+    for (int t = 0; t < kShare; ++t)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sums[t][i] = state.out[t][i];
+  }
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     float total = state.total[h];
@@ -510,15 +595,16 @@ __global__ void __launch_bounds__(128, prompt_ctas(DK, EXTENDED)) attention_prom
     scale /= total;
     const uint32_t token = row_low + h * 8u;
     if (token >= p.tokens) continue;
-    const size_t row = (size_t)sequence * p.tokens + token;
-    bf16* target = out + (row * p.heads + head) * p.vdim;
+    bf16* target = out + (((size_t)sequence * p.tokens + token) * p.heads + head) * p.vdim;
 #pragma unroll
-    for (int t = 0; t < DV / 8; ++t) {
-      const uint32_t column = 8u * t + 2u * c;
-      if (column < p.vdim)  // vdim is a multiple of eight
-        *reinterpret_cast<__nv_bfloat162*>(target + column) =
-            __floats2bfloat162_rn(state.out[t][2 * h] * scale * gate_of<EXTENDED>(p, gate, row, head, column),
-                                  state.out[t][2 * h + 1] * scale * gate_of<EXTENDED>(p, gate, row, head, column + 1u));
+    for (int t = 0; t < kShare; ++t) {
+      float factor[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        factor[i] = EXTENDED && p.gate_stride ? sigmoid_f32(as_float(gates[EXTENDED ? h : 0][EXTENDED ? t : 0][i])) : 1.0f;
+      if (first_t + t < DV / 8 && column_of(t) < p.vdim)  // vdim is a multiple of eight
+        *reinterpret_cast<__nv_bfloat162*>(target + column_of(t)) =
+            __floats2bfloat162_rn(sums[t][2 * h] * scale * factor[0], sums[t][2 * h + 1] * scale * factor[1]);
     }
   }
 }
@@ -555,13 +641,23 @@ __global__ void __launch_bounds__(128) attention_decode_kernel(const bf16* query
   const uint32_t tiles = (end - begin + stretch - 1u) / stretch;  // of this warp
   const uint32_t k_chunks = padded / 8u, v_chunks = DV / 8u;
 
+  const uint32_t key = lane >> 1, half = lane & 1u;  // of the copies
+  auto index_of = [&](uint32_t tile) { return begin + tile * stretch + warp * kWarpKeys + key; };
+  auto slot_of = [&](uint32_t tile) {
+    return index_of(tile) < end ? rows.listed(visible.position(index_of(tile))) : 0u;
+  };
+  uint32_t slots[kDecodeStages];  // of the tiles that are fetched next
+#pragma unroll
+  for (uint32_t s = 0; s < kDecodeStages; ++s) slots[s] = slot_of(s);
   auto fetch_tile = [&](uint32_t tile) {
     if (tile < tiles) {
       bf16* k_tile = ring + (tile % kDecodeStages) * stage_elements;
       bf16* v_tile = k_tile + kWarpKeys * k_stride;
-      const uint32_t key = lane >> 1, half = lane & 1u, index = begin + tile * stretch + warp * kWarpKeys + key;
-      const bool present = index < end;
-      const bf16* cached = pool + (size_t)(present ? rows(visible.position(index), error_word) : 0u) * p.token_stride;
+      const bool present = index_of(tile) < end;
+      const bf16* cached = pool + (size_t)(present ? rows.checked(slots[0], error_word) : 0u) * p.token_stride;
+#pragma unroll
+      for (uint32_t s = 0; s + 1u < kDecodeStages; ++s) slots[s] = slots[s + 1u];
+      slots[kDecodeStages - 1u] = slot_of(tile + kDecodeStages);
       const bf16* k = cached + p.key_offset + kv_head * p.dim;
       const bf16* v = cached + p.value_offset + kv_head * p.vdim;
       for (uint32_t chunk = half; chunk < k_chunks; chunk += 2u) {
@@ -776,22 +872,37 @@ int run_rows(const KernelArgs& args, const RowAttentionParams& p) {
   return check_launch(args);
 }
 
-template <int DK, int DV, bool EXTENDED>
-int run_prompt(const KernelArgs& args, const RowAttentionParams& p) {
+template <int DK, int DV, bool EXTENDED, uint32_t GROUPS>
+int run_prompt_groups(const KernelArgs& args, const RowAttentionParams& p) {
   const uint32_t padded = DK > 0 ? DK : round16(p.dim);
-  constexpr uint32_t kKeyTile = key_tile(DK, EXTENDED);
-  const uint32_t bytes = ((kQueryTile + 2u * kKeyTile) * (padded + 8u) + 2u * kKeyTile * (DV + 8u)) * 2u;
-  auto kernel = attention_prompt_kernel<DK, DV, EXTENDED>;
+  constexpr uint32_t kKeyTile = key_tile(DK, EXTENDED), kGroups = GROUPS;
+  const uint32_t bytes = (kQueryTile * (padded + 8u) + kGroups * 2u * kKeyTile * (padded + 8u + DV + 8u)) * 2u;
+  static_assert(kGroups == 1u || kGroups * (4u + DV / 2u) * 512u <= (kQueryTile * (DK + 8u) + kGroups * 2u * kKeyTile * (DK + DV + 16u)) * 2u,
+                "the groups' results take the tiles' place");
+  auto kernel = attention_prompt_kernel<DK, DV, EXTENDED, GROUPS>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
     cudaGetLastError();
     return -1;
   }
-  launch_kernel(args, kernel, dim3((p.tokens + kQueryTile - 1u) / kQueryTile, p.heads, p.sequences), dim3(128), bytes,
+  launch_kernel(args, kernel, dim3((p.tokens + kQueryTile - 1u) / kQueryTile, p.heads, p.sequences), dim3(128u * kGroups), bytes,
                 (const bf16*)args.buffers[0], (const bf16*)args.buffers[1], (const uint32_t*)args.buffers[2],
                 (const uint32_t*)args.buffers[3], (const uint32_t*)args.buffers[4], (bf16*)args.buffers[5],
                 (const bf16*)args.buffers[7], p,
                 context_device_error(args.ctx));
   return check_launch(args);
+}
+
+template <int DK, int DV, bool EXTENDED>
+int run_prompt(const KernelArgs& args, const RowAttentionParams& p) {
+  // Up to three query tiles and heads per SM, which is what fits at once with one group each, the longest of them bound the kernel,
+  // and three groups walk over its keys together; beyond, CTAs that take turns hide one another's beginnings and ends.  16 heads of
+  // 128, window 1024, one group and three, us: 60 tokens 13.3 and 9.8, 333 37.7 and 19.8, 777 74.8 and 36.0, 1300 107 and 74,
+  // 1600 109 and 91, 2048 (512 CTAs) 109 and 120.
+  if constexpr (EXTENDED && DK == 128) {
+    const size_t ctas = (size_t)((p.tokens + kQueryTile - 1u) / kQueryTile) * p.heads * p.sequences;
+    if (ctas <= (size_t)3u * context_sm_count(args.ctx)) return run_prompt_groups<DK, DV, EXTENDED, 3>(args, p);
+  }
+  return run_prompt_groups<DK, DV, EXTENDED, 1>(args, p);
 }
 
 template <int DK, int DV, bool EXTENDED, uint32_t STAGES>

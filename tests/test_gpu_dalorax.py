@@ -286,6 +286,18 @@ def test_windows_in_portions(runtime, dtype, name, window, keep_first):
     bench.check(0, total, label="whole")
 
 
+@pytest.mark.parametrize("softcap", [None, 4.0])
+@pytest.mark.parametrize("heads,first,total", [(4, 0, 20), (4, 0, 33), (8, 100, 300), (48, 0, 640), (47, 1, 641)])
+def test_prompts_whose_keys_are_shared_out(runtime, heads, first, total, softcap):
+    """Heads of 128: three groups of warps share the keys of few query tiles (one and two key tiles leave groups without any),
+    and one walks over all of them where there are many."""
+    rng = np.random.default_rng(total)
+    q, k, v = (bf16_round(rng.standard_normal((total, n, 128))) for n in (heads, 1, 1))
+    bench = WindowBench(runtime, "bfloat16", q, k, v, scale=0.13, window=150, keep_first=3, softcap=softcap,
+                        gates=bf16_round(rng.standard_normal((total, heads, 128))))
+    bench.check(first, total)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("window,keep_first", [(40, 6), (64, 0), (129, 64), (16, 17), (300, 1)])
 def test_a_key_just_inside_and_just_outside(runtime, dtype, window, keep_first):
