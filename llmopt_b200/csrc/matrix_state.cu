@@ -29,14 +29,19 @@ constexpr uint32_t kLanes = 16;   // lanes per column
 constexpr uint32_t kColumns = 2;  // columns per thread
 constexpr uint32_t kColumnWarps = kSlice / kColumns * kLanes / 32;  // 4
 
-// A scan comes in two forms (launch_scan says where which is used):
-//  * AHEAD: eight loader warps request a chunk ahead, one more warp prepares the tokens' scalars.  The matrix memory then runs with
-//    half a slice per CTA, two of them a cluster; the delta rule, bound by a chain per token (a sum over the lanes of a
-//    column, then the update), keeps the whole slice, behind which twice the columns hide.
-//  * otherwise four loader warps wait for their loads within each chunk: 288 or 256 threads in place of 384 or 416, so that
+// A scan comes in three forms (launch_scan says where which is used):
+//  * kWaits: four loader warps wait for their loads within each chunk: 288 or 256 threads in place of 384 or more, so that
 //    more CTAs share an SM.
-template <bool MEMORY, bool AHEAD> __host__ __device__ constexpr uint32_t scan_columns() { return MEMORY && AHEAD ? kSlice / 2u : kSlice; }
-template <bool AHEAD> __host__ __device__ constexpr uint32_t loader_warps() { return AHEAD ? 8u : 4u; }  // bring in q, k and v and write out
+//  * kAhead: eight loader warps request a chunk ahead, one more warp prepares the tokens' scalars.  The matrix memory then runs with
+//    half a slice per CTA, two of them a cluster.
+//  * kSpread (delta rule), as kAhead with half a slice per CTA and one column per thread: what bounds a token is its chain (a sum over
+//    the lanes of a column, then the update) and the instructions of the warps beside it, of which an SM now has half.
+enum ScanForm { kWaits, kAhead, kSpread };
+template <bool MEMORY, ScanForm FORM> __host__ __device__ constexpr uint32_t scan_columns() {
+  return FORM == kSpread || (MEMORY && FORM == kAhead) ? kSlice / 2u : kSlice;
+}
+template <ScanForm FORM> __host__ __device__ constexpr uint32_t thread_columns() { return FORM == kSpread ? 1u : kColumns; }
+template <ScanForm FORM> __host__ __device__ constexpr uint32_t loader_warps() { return FORM == kWaits ? 4u : 8u; }  // bring in q, k and v and write out
 
 __host__ __device__ constexpr uint32_t slices_of(uint32_t vdim) { return (vdim + kSlice - 1u) / kSlice; }
 
@@ -339,10 +344,10 @@ struct ScanChunk {
 // leave the state as it is).
 template <int CHUNK> struct ScanGroup { static constexpr uint32_t kTokens = CHUNK >= 8 ? 4 : 1; };
 
-template <bool MEMORY, bool AHEAD> struct ScanThreads {
+template <bool MEMORY, ScanForm FORM> struct ScanThreads {
   static constexpr uint32_t kCompute =
-      (scan_columns<MEMORY, AHEAD>() / kColumns * kLanes / 32u + (MEMORY ? 1u : 0u)) * 32u;  // one more warp carries n
-  static constexpr uint32_t kProducers = (loader_warps<AHEAD>() + (AHEAD ? 1u : 0u)) * 32u;
+      (scan_columns<MEMORY, FORM>() / thread_columns<FORM>() * kLanes / 32u + (MEMORY ? 1u : 0u)) * 32u;  // one more warp carries n
+  static constexpr uint32_t kProducers = (loader_warps<FORM>() + (FORM == kWaits ? 0u : 1u)) * 32u;
   static constexpr uint32_t kAll = kCompute + kProducers;
 };
 
@@ -369,22 +374,22 @@ __device__ __forceinline__ float pair_sum(Pair a) {
   return low + high;
 }
 
-// A lane's share of kColumns columns of a state: four rows every kLanes * 4.  Rows beyond dim hold some finite
+// A lane's share of COLUMNS columns of a state: four rows every kLanes * 4.  Rows beyond dim hold some finite
 // value, which meets only zeros of q and k and is not stored.
-template <int R4>
+template <int R4, int COLUMNS = (int)kColumns>
 struct StateColumns {
-  float* home[kColumns];
-  bool active[kColumns];
-  Pair s[kColumns][R4 * 2];
+  float* home[COLUMNS];
+  bool active[COLUMNS];
+  Pair s[COLUMNS][R4 * 2];
   __device__ __forceinline__ void load(uint32_t part, uint32_t dim, bool vectors, bool fresh) {
     if (fresh) {
 #pragma unroll
-      for (int j = 0; j < (int)kColumns; ++j)
+      for (int j = 0; j < COLUMNS; ++j)
 #pragma unroll
         for (int i = 0; i < R4 * 2; ++i) s[j][i] = 0ull;
     } else if (vectors) {
 #pragma unroll
-      for (int j = 0; j < (int)kColumns; ++j)
+      for (int j = 0; j < COLUMNS; ++j)
 #pragma unroll
         for (int i = 0; i < R4; ++i) {
           const ulonglong2 four = *reinterpret_cast<const ulonglong2*>(home[j] + min(i * kLanes * 4u + part * 4u, dim - 4u));
@@ -393,7 +398,7 @@ struct StateColumns {
         }
     } else {
 #pragma unroll
-      for (int j = 0; j < (int)kColumns; ++j)
+      for (int j = 0; j < COLUMNS; ++j)
 #pragma unroll
         for (int i = 0; i < R4 * 2; ++i) {
           const uint32_t c = (i >> 1) * (kLanes * 4u) + part * 4u + (i & 1) * 2u;
@@ -403,7 +408,7 @@ struct StateColumns {
   }
   __device__ __forceinline__ void store(uint32_t part, uint32_t dim, bool vectors) const {
 #pragma unroll
-    for (int j = 0; j < (int)kColumns; ++j) {
+    for (int j = 0; j < COLUMNS; ++j) {
       if (!active[j]) continue;
 #pragma unroll
       for (int i = 0; i < R4; ++i) {
@@ -425,18 +430,20 @@ struct StateColumns {
 };
 
 // TQ: element of q, k, v (fp32 for the delta rule, whose unit vectors are fp32).
-template <typename TQ, bool MEMORY, bool AHEAD, int R4, int CHUNK>
-__global__ void __launch_bounds__(ScanThreads<MEMORY, AHEAD>::kAll) scan_kernel(const TQ* query, const TQ* key, const TQ* value,
+template <typename TQ, bool MEMORY, ScanForm FORM, int R4, int CHUNK>
+__global__ void __launch_bounds__(ScanThreads<MEMORY, FORM>::kAll) scan_kernel(const TQ* query, const TQ* key, const TQ* value,
                                                                                 const float* first, const float* second,
                                                                                 float* state_pool, const uint32_t* past,
                                                                                 const uint32_t* sequence_rows, float* out,
                                                                                 ScanParams p) {
   grid_chain_prologue();
   extern __shared__ __align__(16) unsigned char scan_shared[];
-  constexpr uint32_t kScanColumns = scan_columns<MEMORY, AHEAD>(), kLoaderWarps = loader_warps<AHEAD>();
+  constexpr bool AHEAD = FORM != kWaits;
+  constexpr uint32_t kScanColumns = scan_columns<MEMORY, FORM>(), kLoaderWarps = loader_warps<FORM>();
+  constexpr int kOwn = (int)thread_columns<FORM>();  // columns of a thread
   typedef ScanChunk<R4, CHUNK, kScanColumns> Chunk;
   Chunk* chunks = reinterpret_cast<Chunk*>(scan_shared);
-  constexpr uint32_t kCompute = ScanThreads<MEMORY, AHEAD>::kCompute;
+  constexpr uint32_t kCompute = ScanThreads<MEMORY, FORM>::kCompute;
   const uint32_t first_column = blockIdx.x * kScanColumns, head = blockIdx.y, sequence = blockIdx.z;
   const uint32_t slice = first_column / kSlice;
   const bool owner = first_column % kSlice == 0;  // stores the slice's n and m
@@ -448,7 +455,7 @@ __global__ void __launch_bounds__(ScanThreads<MEMORY, AHEAD>::kAll) scan_kernel(
   const uint32_t chunk_count = (p.tokens + CHUNK - 1u) / CHUNK;
   // The CTAs of a slice start from the same n and m, which one of them stores at the end: all have read them by then.
   auto ready = [] {
-    if (kScanColumns < kSlice) cluster_sync();
+    if (MEMORY && kScanColumns < kSlice) cluster_sync();
     else __syncthreads();
   };
 
@@ -623,7 +630,7 @@ __global__ void __launch_bounds__(ScanThreads<MEMORY, AHEAD>::kAll) scan_kernel(
       if (index > 0) {
         write_out(index - 1u);
         // its scalars are filled again next
-        if (MEMORY || !AHEAD) asm volatile("bar.sync 1, %0;" ::"n"(ScanThreads<MEMORY, AHEAD>::kProducers) : "memory");
+        if (MEMORY || !AHEAD) asm volatile("bar.sync 1, %0;" ::"n"(ScanThreads<MEMORY, FORM>::kProducers) : "memory");
       }
       if (index + 1u < chunk_count) produce(index + 1u);
       if (index + 2u < chunk_count) request(index + 2u);
@@ -633,13 +640,13 @@ __global__ void __launch_bounds__(ScanThreads<MEMORY, AHEAD>::kAll) scan_kernel(
     if (MEMORY && owner && preparer && lane == 0) state[layout.top(head, slice)] = top;
   } else {
     // ------------------------------ state ------------------------------
-    const uint32_t column0 = threadIdx.x / kLanes * kColumns, part = threadIdx.x % kLanes;
+    const uint32_t column0 = threadIdx.x / kLanes * (uint32_t)kOwn, part = threadIdx.x % kLanes;
     const bool is_norm = MEMORY && column0 >= kScanColumns;  // the extra warp: the first column of its first lanes carries n
-    StateColumns<R4> columns;
+    StateColumns<R4, kOwn> columns;
     auto& active = columns.active;
     auto& s = columns.s;
 #pragma unroll
-    for (int j = 0; j < (int)kColumns; ++j) {
+    for (int j = 0; j < kOwn; ++j) {
       const uint32_t column = first_column + column0 + j;
       active[j] = is_norm ? column0 + j == kScanColumns : column < p.vdim;
       columns.home[j] = state + (is_norm ? layout.norm(head, slice) : layout.matrix(head) + (size_t)(active[j] ? column : 0u) * p.dim);
@@ -653,15 +660,17 @@ __global__ void __launch_bounds__(ScanThreads<MEMORY, AHEAD>::kAll) scan_kernel(
       constexpr int G = ScanGroup<CHUNK>::kTokens;
 #pragma unroll 1
       for (uint32_t t0 = 0; t0 < count; t0 += G) {
-        float partial[G][kColumns];  // this lane's share of the tokens' read-outs
-        float update[G][kColumns];   // delta rule
+        float partial[G][kOwn];  // this lane's share of the tokens' read-outs
+        float update[G][kOwn];   // delta rule
 #pragma unroll
         for (int g = 0; g < G; ++g) {
           const uint32_t t = t0 + g;
           const ulonglong2* q = reinterpret_cast<const ulonglong2*>(chunk.q[t]) + part;
           const ulonglong2* k = reinterpret_cast<const ulonglong2*>(chunk.k[t]) + part;
           const float4 scalar = chunk.scalar[t];
-          const float2 values = *reinterpret_cast<const float2*>(&chunk.v[t][column0 % kScanColumns]);
+          float values[kOwn];
+          if constexpr (kOwn == 2) *reinterpret_cast<float2*>(values) = *reinterpret_cast<const float2*>(&chunk.v[t][column0 % kScanColumns]);
+          else values[0] = chunk.v[t][column0 % kScanColumns];
           const Pair keep2 = pair_of(scalar.x, scalar.x);
           Pair kk[R4 * 2];
 #pragma unroll
@@ -670,17 +679,19 @@ __global__ void __launch_bounds__(ScanThreads<MEMORY, AHEAD>::kAll) scan_kernel(
             kk[2 * i] = four.x;
             kk[2 * i + 1] = four.y;
           }
-          Pair sums[kColumns][2];
+          Pair sums[kOwn][2];
 #pragma unroll
-          for (int j = 0; j < (int)kColumns; ++j) sums[j][0] = sums[j][1] = 0ull;
+          for (int j = 0; j < kOwn; ++j) sums[j][0] = sums[j][1] = 0ull;
           if (MEMORY) {
-            const float write = scalar.y;
-            const float target[kColumns] = {is_norm ? write : write * values.x, write * values.y};
+            const float weight = scalar.y;
+            float target[kOwn];
+#pragma unroll
+            for (int j = 0; j < kOwn; ++j) target[j] = is_norm && j == 0 ? weight : weight * values[j];
 #pragma unroll
             for (int i = 0; i < R4; ++i) {
               const ulonglong2 qq = q[i * kLanes];
 #pragma unroll
-              for (int j = 0; j < (int)kColumns; ++j) {
+              for (int j = 0; j < kOwn; ++j) {
                 const Pair write2 = pair_of(target[j], target[j]);
                 s[j][2 * i] = pair_fma(kk[2 * i], write2, pair_mul(s[j][2 * i], keep2));
                 s[j][2 * i + 1] = pair_fma(kk[2 * i + 1], write2, pair_mul(s[j][2 * i + 1], keep2));
@@ -689,38 +700,38 @@ __global__ void __launch_bounds__(ScanThreads<MEMORY, AHEAD>::kAll) scan_kernel(
               }
             }
 #pragma unroll
-            for (int j = 0; j < (int)kColumns; ++j) partial[g][j] = pair_sum(sums[j][0]) + pair_sum(sums[j][1]);
+            for (int j = 0; j < kOwn; ++j) partial[g][j] = pair_sum(sums[j][0]) + pair_sum(sums[j][1]);
           } else {
-            float with_key[kColumns];
+            float with_key[kOwn];
 #pragma unroll
             for (int i = 0; i < R4; ++i)
 #pragma unroll
-              for (int j = 0; j < (int)kColumns; ++j) {
+              for (int j = 0; j < kOwn; ++j) {
                 sums[j][0] = pair_fma(s[j][2 * i], kk[2 * i], sums[j][0]);
                 sums[j][1] = pair_fma(s[j][2 * i + 1], kk[2 * i + 1], sums[j][1]);
               }
 #pragma unroll
-            for (int j = 0; j < (int)kColumns; ++j) {
+            for (int j = 0; j < kOwn; ++j) {
               with_key[j] = pair_sum(sums[j][0]) + pair_sum(sums[j][1]);
               sums[j][0] = sums[j][1] = 0ull;
             }
 #pragma unroll
             for (int offset = 1; offset < (int)kLanes; offset <<= 1)
 #pragma unroll
-              for (int j = 0; j < (int)kColumns; ++j) with_key[j] += __shfl_xor_sync(0xffffffffu, with_key[j], offset);
+              for (int j = 0; j < kOwn; ++j) with_key[j] += __shfl_xor_sync(0xffffffffu, with_key[j], offset);
 #pragma unroll
             for (int i = 0; i < R4; ++i) {
               const ulonglong2 qq = q[i * kLanes];
 #pragma unroll
-              for (int j = 0; j < (int)kColumns; ++j) {
+              for (int j = 0; j < kOwn; ++j) {
                 sums[j][0] = pair_fma(s[j][2 * i], qq.x, sums[j][0]);
                 sums[j][1] = pair_fma(s[j][2 * i + 1], qq.y, sums[j][1]);
               }
             }
-            update[g][0] = scalar.y * (values.x - scalar.x * with_key[0]);
-            update[g][1] = scalar.y * (values.y - scalar.x * with_key[1]);
 #pragma unroll
-            for (int j = 0; j < (int)kColumns; ++j) {
+            for (int j = 0; j < kOwn; ++j) update[g][j] = scalar.y * (values[j] - scalar.x * with_key[j]);
+#pragma unroll
+            for (int j = 0; j < kOwn; ++j) {
               partial[g][j] = pair_sum(sums[j][0]) + pair_sum(sums[j][1]);
               const Pair update2 = pair_of(update[g][j], update[g][j]);
 #pragma unroll
@@ -728,18 +739,19 @@ __global__ void __launch_bounds__(ScanThreads<MEMORY, AHEAD>::kAll) scan_kernel(
             }
           }
         }
-        if (G == 4) {
-          // eight sums over a column's lanes: each exchange halves what a lane keeps, so that lane `part` ends with
-          // value part / (kLanes / 8); the lanes that hold the same value then add what they have
-          float v[8], u[8];
+        if constexpr (G == 4) {
+          // eight sums (four, with one column) over a column's lanes: each exchange halves what a lane keeps, so that lane `part` ends
+          // with value part / (kLanes / kSums); the lanes that hold the same value then add what they have
+          constexpr int kSums = G * kOwn;
+          float v[kSums], u[kSums];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            v[i] = partial[i / 2 % G][i % 2];
-            u[i] = MEMORY ? 0.0f : update[i / 2 % G][i % 2];
+          for (int i = 0; i < kSums; ++i) {
+            v[i] = partial[i / kOwn][i % kOwn];
+            u[i] = MEMORY ? 0.0f : update[i / kOwn][i % kOwn];
           }
 #pragma unroll
-          for (int half = 4; half > 0; half >>= 1) {
-            const uint32_t distance = half * (kLanes / 8u);
+          for (int half = kSums / 2; half > 0; half >>= 1) {
+            const uint32_t distance = half * (kLanes / kSums);
             const bool upper = (part & distance) != 0;
 #pragma unroll
             for (int i = 0; i < half; ++i) {
@@ -749,10 +761,10 @@ __global__ void __launch_bounds__(ScanThreads<MEMORY, AHEAD>::kAll) scan_kernel(
             }
           }
 #pragma unroll
-          for (uint32_t distance = kLanes / 16u; distance > 0; distance >>= 1)
+          for (uint32_t distance = kLanes / kSums / 2u; distance > 0; distance >>= 1)
             v[0] += __shfl_xor_sync(0xffffffffu, v[0], distance);
-          const uint32_t which = part / (kLanes / 8u), t = t0 + which / 2u, j = which % 2u;
-          if (part % (kLanes / 8u) != 0) {
+          const uint32_t which = part / (kLanes / kSums), t = t0 + which / kOwn, j = which % kOwn;
+          if (part % (kLanes / kSums) != 0) {
             // another lane writes this value
           } else if (MEMORY) {
             if (!is_norm) chunk.out[t][column0 + j] = v[0];
@@ -763,19 +775,20 @@ __global__ void __launch_bounds__(ScanThreads<MEMORY, AHEAD>::kAll) scan_kernel(
           }
         } else {
 #pragma unroll
-          for (int j = 0; j < (int)kColumns; ++j)
+          for (int j = 0; j < kOwn; ++j)
 #pragma unroll
             for (int offset = 1; offset < (int)kLanes; offset <<= 1)
               partial[0][j] += __shfl_xor_sync(0xffffffffu, partial[0][j], offset);
           if (part == 0) {
-            if (MEMORY) {
-              if (!is_norm) *reinterpret_cast<float2*>(&chunk.out[t0][column0]) = make_float2(partial[0][0], partial[0][1]);
-              else if (active[0]) chunk.norm_dot[t0] = partial[0][0];
-            } else {
-              const float4 scalar = chunk.scalar[t0];
-              *reinterpret_cast<float2*>(&chunk.out[t0][column0]) =
-                  make_float2(fmaf(update[0][0], scalar.z, scalar.x * partial[0][0]),
-                              fmaf(update[0][1], scalar.z, scalar.x * partial[0][1]));
+#pragma unroll
+            for (int j = 0; j < kOwn; ++j) {
+              if (MEMORY) {
+                if (!is_norm) chunk.out[t0][column0 + j] = partial[0][j];
+                else if (active[0] && j == 0) chunk.norm_dot[t0] = partial[0][0];
+              } else {
+                const float4 scalar = chunk.scalar[t0];
+                chunk.out[t0][column0 + j] = fmaf(update[0][j], scalar.z, scalar.x * partial[0][j]);
+              }
             }
           }
         }
@@ -822,7 +835,7 @@ int launch_scan(const KernelArgs& args) {
             (const float*)args.buffers[4], (float*)args.buffers[5], (const uint32_t*)args.buffers[6],
             (const uint32_t*)args.buffers[7], (float*)args.buffers[8], p);
     };
-    if (per_slice > 1u) launch([](auto&&... a) { launch_cluster_kernel(a...); }, per_slice);
+    if (MEMORY && per_slice > 1u) launch([](auto&&... a) { launch_cluster_kernel(a...); }, per_slice);
     else launch([](auto&&... a) { launch_kernel(a...); });
     return check_launch(args);
   };
@@ -830,25 +843,31 @@ int launch_scan(const KernelArgs& args) {
   // Ahead where that is faster, us, in brackets otherwise: matrix memory, dim 256, 2048 tokens, 64 slices 429 (601), 256 slices 1699 (1203):
   // its two CTAs a slice need an SM each.  Delta rule, 2048 tokens, dim 128 394 (472), dim 64 324 (302), dim 192 as fast, dim 256
   // 789 (594, where its registers spill); of four tokens the chunks are too short for it: dim 128 x 64 sequences 24 (20).
+  // Spread where each half slice has an SM of its own, 16 heads of 128: 9 tokens 5.2 -> 4.9, 60 14.6 -> 12.0, 2048 395 -> 305.  (The
+  // matrix memory gains nothing from it: 275 for 268.)
   const size_t slices = (size_t)slices_of(p.vdim) * p.heads * p.sequences;
-  const bool ahead = MEMORY ? 2u * slices <= (size_t)context_sm_count(args.ctx) : quads == 2u && p.tokens > 4u;
+  const bool apart = 2u * slices <= (size_t)context_sm_count(args.ctx);  // each half slice on an SM of its own
+  const bool ahead = MEMORY ? apart : quads == 2u && p.tokens > 4u;
   auto form = [&](auto r4, auto constant, auto chunk) {
     constexpr int R4 = decltype(r4)::value, CHUNK = decltype(chunk)::value;
-    constexpr bool AHEAD = decltype(constant)::value;
-    constexpr uint32_t kScanColumns = scan_columns<MEMORY, AHEAD>();
-    return run(scan_kernel<TQ, MEMORY, AHEAD, R4, CHUNK>, 2 * sizeof(ScanChunk<R4, CHUNK, kScanColumns>), ScanThreads<MEMORY, AHEAD>::kAll,
+    constexpr ScanForm FORM = decltype(constant)::value;
+    constexpr uint32_t kScanColumns = scan_columns<MEMORY, FORM>();
+    return run(scan_kernel<TQ, MEMORY, FORM, R4, CHUNK>, 2 * sizeof(ScanChunk<R4, CHUNK, kScanColumns>), ScanThreads<MEMORY, FORM>::kAll,
                kSlice / kScanColumns);
   };
   // few tokens: small chunks, so that more CTAs fit on an SM
   auto sized = [&](auto r4) {
     constexpr std::integral_constant<int, 4> few;
     constexpr std::integral_constant<int, 32> many;
+    constexpr std::integral_constant<ScanForm, kWaits> waits;
+    constexpr std::integral_constant<ScanForm, kAhead> request_ahead;
     if constexpr (MEMORY) {
-      if (ahead) return p.tokens <= 4u ? form(r4, std::true_type(), few) : form(r4, std::true_type(), many);
+      if (ahead) return p.tokens <= 4u ? form(r4, request_ahead, few) : form(r4, request_ahead, many);
     } else if constexpr (decltype(r4)::value == 2) {
-      if (ahead) return form(r4, std::true_type(), many);
+      if (ahead && apart) return form(r4, std::integral_constant<ScanForm, kSpread>(), many);
+      if (ahead) return form(r4, request_ahead, many);
     }
-    return p.tokens <= 4u ? form(r4, std::false_type(), few) : form(r4, std::false_type(), many);
+    return p.tokens <= 4u ? form(r4, waits, few) : form(r4, waits, many);
   };
   if (quads <= 1u) return sized(std::integral_constant<int, 1>());
   if (quads <= 2u) return sized(std::integral_constant<int, 2>());

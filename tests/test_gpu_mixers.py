@@ -417,6 +417,43 @@ def test_scans_of_many_sequences_look_back_only(runtime, form, tokens):
     assert np.array_equal(results[0][:, :tokens - 2], results[1][:, :tokens - 2])
 
 
+@pytest.mark.parametrize("dim,vdim,tokens", [(128, 128, 5), (128, 128, 37), (68, 17, 64), (100, 70, 33), (128, 33, 100)])
+def test_delta_scan_alone_and_among_many(runtime, dim, vdim, tokens):
+    """A sequence alone has half a slice and one column per thread, among many a whole slice and two: the same to the last bit."""
+    from llmopt_b200 import parameters
+    from llmopt_b200.kv_cache import matrix_state_elements
+
+    rng = np.random.default_rng(dim + vdim)
+    sequences, heads = 80, 2
+    qk, vs = heads * dim, heads * vdim
+    stride = matrix_state_elements(heads, dim, vdim, normalized=False)
+    raw = (rng.standard_normal((sequences, tokens, 2 * qk + vs)) * 0.1).astype(np.float32)
+    gates = rng.uniform(0.1, 0.9, (sequences, tokens, 2 * heads)).astype(np.float32)
+    pool = (rng.standard_normal((sequences, stride)) * 0.3).astype(np.float32)
+
+    def scan(chosen):
+        count = len(chosen)
+        states, out = upload(runtime, pool), empty(runtime, count * tokens * vs)
+        projected, scalars = upload(runtime, raw[chosen]), upload(runtime, gates[chosen])
+        past = upload(runtime, np.full(count, 9, np.uint32))
+        runtime.dispatch("llmopt_delta_scan_f32",
+                         buffers=[projected, projected, projected, scalars, scalars, states, past, upload(runtime, chosen), out],
+                         parameters=parameters.state_scan(
+                             sequences=count, tokens=tokens, heads=heads, kv_heads=heads, dim=dim, vdim=vdim, q_stride=2 * qk + vs,
+                             q_column=0, k_stride=2 * qk + vs, k_column=qk, v_stride=2 * qk + vs, v_column=2 * qk,
+                             scalar_stride=2 * heads, first_column=0, second_column=heads, state_rows=sequences, state_stride=stride))
+        return download(out, (count, tokens, heads, vdim)), download(states, (sequences, stride))
+
+    outputs, states = scan(np.arange(sequences, dtype=np.uint32))
+    for one in (0, 79):
+        output, state = scan(np.array([one], np.uint32))
+        assert np.array_equal(output[0], outputs[one]) and np.array_equal(state[one], states[one])
+    q, k, v = (raw[0][:, a:b].reshape(tokens, heads, -1).astype(np.float64) for a, b in ((0, qk), (qk, 2 * qk), (2 * qk, 2 * qk + vs)))
+    matrices = pool[0, :heads * vdim * dim].reshape(heads, vdim, dim).transpose(0, 2, 1).astype(np.float64)
+    want, _ = plain.delta_scan(q, k, v, gates[0, :, :heads].astype(np.float64), gates[0, :, heads:].astype(np.float64), matrices)
+    close(outputs[0], want, 2e-5, "alone")
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_head_norm_gate(runtime, dtype):
     from llmopt_b200 import parameters
