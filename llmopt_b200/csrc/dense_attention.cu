@@ -102,8 +102,9 @@ __global__ void __launch_bounds__(128) dense_attention_mma_kernel(const __half* 
   Row* q_tile = reinterpret_cast<Row*>(dense_shared);                 // [kQueryTile]
   Row* k_tiles = q_tile + kQueryTile;                                  // [2][KT]
   Row* v_tiles = k_tiles + 2 * KT;                                     // [2][KT]
-  // the last query tiles see the most keys under a causal mask: they are scheduled first
-  const uint32_t q0 = (gridDim.x - 1u - blockIdx.x) * kQueryTile, head = blockIdx.y, batch = blockIdx.z;
+  // the last query tiles see the most keys under a causal mask: they are scheduled first, over all heads (2048 tokens x 32 heads of
+  // 128: 174 -> 143 us)
+  const uint32_t q0 = (gridDim.y - 1u - blockIdx.y) * kQueryTile, head = blockIdx.x, batch = blockIdx.z;
   const uint32_t kv_head = head / (p.heads / p.kv_heads);
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, r = lane >> 2, c = lane & 3u;
   constexpr int kChunks = D / 8;  // 16-byte chunks per row
@@ -343,9 +344,10 @@ int launch_attention_dense(const KernelArgs& args) {
     const size_t mask_elements = (size_t)p.mask_batches * p.mask_heads * p.q_len * p.k_len;
     LLMOPT_REQUIRE(args.lengths[3] >= mask_elements * (p.mask_dtype == 2 ? 2 : 1), "mask buffer is too short");
   }
-  const bool aligned = (((uintptr_t)args.buffers[0] | (uintptr_t)args.buffers[1] | (uintptr_t)args.buffers[2]) & 15u) == 0 &&
+  const bool aligned = p.q_len <= 65535u * kQueryTile &&  // a grid's second dimension
+                       (((uintptr_t)args.buffers[0] | (uintptr_t)args.buffers[1] | (uintptr_t)args.buffers[2]) & 15u) == 0 &&
                        ((uintptr_t)args.buffers[4] & 3u) == 0;
-  const dim3 grid((p.q_len + kQueryTile - 1) / kQueryTile, p.heads, p.batches);
+  const dim3 grid(p.heads, (p.q_len + kQueryTile - 1) / kQueryTile, p.batches);
   auto shared_bytes = [](uint32_t dim, uint32_t keys) { return (size_t)(kQueryTile + 4 * keys) * (dim + 8) * sizeof(__half); };
   if (aligned && p.dim == 64) {
     auto kernel = dense_attention_mma_kernel<64, 64>;

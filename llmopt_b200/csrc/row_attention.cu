@@ -428,8 +428,7 @@ __global__ void __launch_bounds__(128 * GROUPS, prompt_ctas(DK, EXTENDED, GROUPS
   bf16* k_tiles = q_tile + kQueryTile * k_stride + group * 2u * kKeyTile * (k_stride + v_stride);
   bf16* v_tiles = k_tiles + 2u * kKeyTile * k_stride;
   // the last query tiles see the most keys: they are scheduled first, over all heads
-  const uint32_t place = blockIdx.y * gridDim.x + blockIdx.x, head = place % p.heads, sequence = blockIdx.z;
-  const uint32_t q0 = (gridDim.x - 1u - place / p.heads) * kQueryTile;
+  const uint32_t q0 = (gridDim.y - 1u - blockIdx.y) * kQueryTile, head = blockIdx.x, sequence = blockIdx.z;
   const uint32_t kv_head = head / (p.heads / p.kv_heads);
   const uint32_t warp = thread >> 5, lane = threadIdx.x & 31u, r = lane >> 2, c = lane & 3u;
   const uint32_t past = past_lengths[sequence];
@@ -884,7 +883,7 @@ int run_prompt_groups(const KernelArgs& args, const RowAttentionParams& p) {
     cudaGetLastError();
     return -1;
   }
-  launch_kernel(args, kernel, dim3((p.tokens + kQueryTile - 1u) / kQueryTile, p.heads, p.sequences), dim3(128u * kGroups), bytes,
+  launch_kernel(args, kernel, dim3(p.heads, (p.tokens + kQueryTile - 1u) / kQueryTile, p.sequences), dim3(128u * kGroups), bytes,
                 (const bf16*)args.buffers[0], (const bf16*)args.buffers[1], (const uint32_t*)args.buffers[2],
                 (const uint32_t*)args.buffers[3], (const uint32_t*)args.buffers[4], (bf16*)args.buffers[5],
                 (const bf16*)args.buffers[7], p,
@@ -894,6 +893,7 @@ int run_prompt_groups(const KernelArgs& args, const RowAttentionParams& p) {
 
 template <int DK, int DV, bool EXTENDED>
 int run_prompt(const KernelArgs& args, const RowAttentionParams& p) {
+  if (p.tokens > 65535u * kQueryTile) return -1;  // a grid's second dimension
   // Up to three query tiles and heads per SM, which is what fits at once with one group each, the longest of them bound the kernel,
   // and three groups walk over its keys together; beyond, CTAs that take turns hide one another's beginnings and ends.  16 heads of
   // 128, window 1024, one group and three, us: 60 tokens 13.3 and 9.8, 333 37.7 and 19.8, 777 74.8 and 36.0, 1300 107 and 74,
