@@ -8,8 +8,9 @@
 //   ki <= qi + past_length; mask dtype 2: f16, a value >= 0 keeps the key, other dtypes: a
 //   nonzero byte keeps it (llmopt_attention_allowed, lib/metal_attention_source.ml:257-274).
 //
-// Two kernels behind the names:
-//  * D in {64, 128}: a flash-attention forward pass on mma.sync.m16n8k16: one CTA per 64 queries
+// Kernels behind the names:
+//  * D in {64, 128} without a mask: dense_attention_tc.cu, on tcgen05.
+//  * D in {64, 128} otherwise: a flash-attention forward pass on mma.sync.m16n8k16: one CTA per 64 queries
 //    of one (batch, head), four warps of 16 query rows; K and V tiles staged in padded shared
 //    memory; S = Q K^T with K rows as the col-major B operand (ldmatrix), online softmax in
 //    fp32 per row (units of log2 e), P rounded to half before P V like the reference's SIMD
@@ -17,17 +18,10 @@
 //  * any other head size: one warp per (batch, head, query) walking the keys with a
 //    single-pass online softmax in fp32.
 // The work is O(q k D) on small prefill lengths; it is not on the HBM-bound decode path.
-#include "common.cuh"
+#include "dense_attention.cuh"
 
 namespace llmopt {
 namespace {
-
-struct DenseParams {  // lib/metal_parameters.ml:95-117
-  uint32_t batches, heads, q_len, k_len, dim, mask_batches, mask_heads, causal;
-  float scale;
-  uint32_t kv_heads, token_first_output, past_length, token_first_value, mask_dtype;
-};
-static_assert(sizeof(DenseParams) == 56, "parameter block is 56 bytes");
 
 __device__ __forceinline__ bool key_allowed(const DenseParams& p, const uint8_t* mask, uint32_t batch, uint32_t head,
                                             uint32_t qi, uint32_t ki) {
@@ -102,8 +96,7 @@ __global__ void __launch_bounds__(128) dense_attention_mma_kernel(const __half* 
   Row* q_tile = reinterpret_cast<Row*>(dense_shared);                 // [kQueryTile]
   Row* k_tiles = q_tile + kQueryTile;                                  // [2][KT]
   Row* v_tiles = k_tiles + 2 * KT;                                     // [2][KT]
-  // the last query tiles see the most keys under a causal mask: they are scheduled first, over all heads (2048 tokens x 32 heads of
-  // 128: 174 -> 143 us)
+  // the last query tiles see the most keys under a causal mask: they are scheduled first, over all heads
   const uint32_t q0 = (gridDim.y - 1u - blockIdx.y) * kQueryTile, head = blockIdx.x, batch = blockIdx.z;
   const uint32_t kv_head = head / (p.heads / p.kv_heads);
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, r = lane >> 2, c = lane & 3u;
@@ -343,6 +336,10 @@ int launch_attention_dense(const KernelArgs& args) {
     LLMOPT_REQUIRE(p.mask_heads > 0, "mask_heads must be positive with a mask");
     const size_t mask_elements = (size_t)p.mask_batches * p.mask_heads * p.q_len * p.k_len;
     LLMOPT_REQUIRE(args.lengths[3] >= mask_elements * (p.mask_dtype == 2 ? 2 : 1), "mask buffer is too short");
+  }
+  {
+    const int status = launch_attention_dense_tc(args, p);
+    if (status >= 0) return status;
   }
   const bool aligned = p.q_len <= 65535u * kQueryTile &&  // a grid's second dimension
                        (((uintptr_t)args.buffers[0] | (uintptr_t)args.buffers[1] | (uintptr_t)args.buffers[2]) & 15u) == 0 &&

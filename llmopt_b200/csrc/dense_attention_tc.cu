@@ -1,0 +1,397 @@
+// Dense fp16 attention of prompts on the 5th-generation tensor cores (dense_attention.cu has the contract): heads of 64 or 128,
+// causal or not, without a mask.
+//
+// A CTA owns 128 queries of one head and walks over tiles of 128 keys.  One thread brings Q, K and V by TMA (128-byte swizzle)
+// and issues tcgen05.mma: S = Q K^T into tensor memory (128 columns), later O += P V (D columns).  Warps of rows read S and write
+// P = exp2(S - top) over it as fp16 pairs, the A operand of P V in tensor memory; V is the B operand as it lies in memory,
+// dimensions contiguous.  O stays in tensor memory; it is scaled only when a row's maximum has grown by more than 2^kSlack since it
+// was last scaled: weights of up to 2^kSlack are as exact in fp16, and the denominator adds what P V uses.
+//
+// What bounds a tile is the chain from S to P (16 exponentials a cycle and SM are its floor), so two of them run side by side,
+// in one of two forms:
+//  * ALONE: one CTA per SM, two threads per row, and the next tile's scores multiplied beside this tile's exponentials;
+//  * otherwise two CTAs share an SM, a thread per row.
+// Up to two and a half CTAs per SM the first is faster, where rows are short in tiles or CTAs few: us with 64 x 64 tiles on mma.sync,
+// two per SM, ALONE: 9 heads of 64, 60 tokens 7.4, 8.8, 6.4; 300 9.5, 11.7, 7.9; 2048 47.6, 39.7, 25.2; 16 heads of 128, 2048
+// tokens 75.6, 48.5, 30.4; 32 heads 1000 tokens 45, 26.1, 19.8; 1400 - , 34.7, 33.2; 1650 - , 38.1, 43.2; 2048 143, 51.0, 60.6.
+// K and V two tiles deep changed nothing: their way hides behind the exponentials.
+//
+// Rows beyond a head's keys or queries are zero-filled by TMA.  Every wait on an mbarrier is bounded; a wait that runs out raises
+// the context's device error word, and the CTA lets its copies land, frees its tensor memory and returns.
+#include <cuda.h>
+
+#include "dense_attention.cuh"
+#include "w4a16_tc_device.cuh"
+
+namespace llmopt {
+using namespace tc;
+
+uint32_t* context_device_error(Context* ctx);
+
+namespace {
+
+constexpr uint32_t kTile = 128;      // queries, and keys of a tile
+constexpr uint32_t kBlockBytes = kTile * 128;  // 64 dimensions of 128 rows
+constexpr float kSlack = 8.0f;
+constexpr float kLowest = -1.0e30f;
+
+template <int D, bool ALONE>
+struct Shape {
+  static constexpr uint32_t kHalves = ALONE ? 2 : 1, kRowWarps = 4 * kHalves, kThreads = (kRowWarps + 1) * 32;
+  static constexpr uint32_t kKeys = kTile / kHalves;  // of a thread
+  static constexpr uint32_t kScores = ALONE ? 2 : 1;  // tiles of scores in tensor memory
+  static constexpr uint32_t kColumns = ALONE ? 512 : 256;
+  static constexpr uint32_t kBlocks = D / 64;
+  static constexpr uint32_t kTileBytes = kBlocks * kBlockBytes;
+  static constexpr uint32_t kK = kTileBytes, kV = 2 * kTileBytes, kBarriers = 3 * kTileBytes;
+  static constexpr uint32_t kHolder = kBarriers + 8 * 8;
+  static constexpr uint32_t kExchange = kHolder + 16;  // [parity][half][row] floats
+  static constexpr uint32_t kUsed = kExchange + (ALONE ? 4 * kTile * 4 : 0) + 1024;  // slack: 1024-byte alignment of the tiles
+  // no more CTAs find room on an SM than there is tensor memory for
+  static constexpr uint32_t kLeast = (ALONE ? 117u : 80u) * 1024u, kSharedBytes = kUsed > kLeast ? kUsed : kLeast;
+};
+
+__device__ __forceinline__ float exp2_fast(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ void tma_load_4d(uint32_t destination, const CUtensorMap* map, int32_t x, int32_t row, int32_t head,
+                                            int32_t batch, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+      ::"r"(destination), "l"(map), "r"(bar), "r"(x), "r"(row), "r"(head), "r"(batch)
+      : "memory");
+}
+__device__ __forceinline__ void mma_f16_weights(uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t instruction, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(instruction), "r"(accumulate), "r"(0u)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_store_16(uint32_t address, const uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      ::"r"(address), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
+        "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_store_32(uint32_t address, const uint32_t (&v)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+      ::"r"(address), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
+        "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]),
+        "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
+        "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_wait_load() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_wait_store() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// B operand whose rows (k) are 128 bytes of 64 columns (n): 128-byte swizzle, eight rows 1024 bytes apart, the next 64 columns
+// kBlockBytes on.
+__device__ __forceinline__ uint64_t value_descriptor(uint32_t shared_address) {
+  uint64_t descriptor = 0;
+  descriptor |= (uint64_t)((shared_address & 0x3ffffu) >> 4);
+  descriptor |= (uint64_t)(kBlockBytes >> 4) << 16;  // leading byte offset
+  descriptor |= (uint64_t)(1024 >> 4) << 32;         // stride byte offset
+  descriptor |= (uint64_t)1 << 46;
+  descriptor |= (uint64_t)2 << 61;
+  return descriptor;
+}
+
+template <int D, bool ALONE>
+__global__ void __launch_bounds__(Shape<D, ALONE>::kThreads, ALONE ? 1 : 2)
+dense_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                          const __grid_constant__ CUtensorMap map_v, __half* output, DenseParams p, uint32_t* error_word) {
+  using S = Shape<D, ALONE>;
+  extern __shared__ unsigned char shared_raw[];
+  grid_chain_prologue();
+  const uint32_t base = (smem_u32(shared_raw) + 1023u) & ~1023u;
+  unsigned char* base_pointer = shared_raw + (base - smem_u32(shared_raw));
+  const uint32_t q_full = base + S::kBarriers, k_full = q_full + 8, v_full = q_full + 16;
+  const uint32_t weights_full = q_full + 24, sums_full = q_full + 32, scores_full = q_full + 40;  // scores_full: one per tile in tensor memory
+  volatile uint32_t* holder = reinterpret_cast<volatile uint32_t*>(base_pointer + S::kHolder);
+  volatile uint32_t* abort_flag = holder + 1;
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+  // the last query tiles see the most keys under a causal mask: they are scheduled first, over all heads
+  const uint32_t q0 = (gridDim.y - 1u - blockIdx.y) * kTile, head = blockIdx.x, batch = blockIdx.z;
+  const uint32_t key_end = p.causal ? min(p.k_len, min(q0 + kTile, p.q_len) + p.past_length) : p.k_len;
+  const uint32_t tiles = (key_end + kTile - 1u) / kTile;
+
+  if (threadIdx.x == 0) {
+    barrier_init(q_full, 1);  // the expect_tx arrivals; complete by byte count
+    barrier_init(k_full, 1);
+    barrier_init(v_full, 1);
+    for (uint32_t i = 0; i < S::kScores; ++i) barrier_init(scores_full + i * 8, 1);  // one tcgen05.commit
+    barrier_init(weights_full, S::kRowWarps);  // one arrival per warp of rows
+    barrier_init(sums_full, 1);    // one tcgen05.commit
+    *abort_flag = 0u;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == S::kRowWarps) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(base + S::kHolder), "r"(S::kColumns)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t scores = *holder, sums = scores + S::kScores * kTile;  // columns of tensor memory
+  auto give_up = [&]() {
+    *abort_flag = 1u;
+    if (error_word) atomicExch(error_word, 1u);
+  };
+
+  if (warp == S::kRowWarps) {
+    if (lane == 0) {
+      const int32_t kv_head = (int32_t)(head / (p.heads / p.kv_heads));
+      uint32_t k_issued = 0, v_issued = 0;
+      auto load = [&](const CUtensorMap* map, uint32_t target, uint32_t row, int32_t of_head, uint32_t bar) {
+        barrier_expect_tx(bar, S::kTileBytes);
+#pragma unroll
+        for (uint32_t block = 0; block < S::kBlocks; ++block)
+          tma_load_4d(base + target + block * kBlockBytes, map, (int32_t)(block * 64u), (int32_t)row, of_head, (int32_t)batch, bar);
+      };
+      load(&map_q, 0, q0, (int32_t)head, q_full);
+      load(&map_k, S::kK, 0, kv_head, k_full), ++k_issued;
+      load(&map_v, S::kV, 0, kv_head, v_full), ++v_issued;
+      auto multiply = [&](uint32_t tile) {  // S = Q K^T
+        if (*abort_flag || !barrier_wait(k_full, tile & 1u)) return false;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t which = tile % S::kScores;
+#pragma unroll
+        for (uint32_t j = 0; j < D / 16; ++j) {
+          const uint32_t at = j / 4u * kBlockBytes + j % 4u * 32u;
+          mma_f16(scores + which * kTile, operand_descriptor(base + at), operand_descriptor(base + S::kK + at), j > 0 ? 1u : 0u,
+                  instruction_descriptor(kTile, kTile));
+        }
+        mma_commit(scores_full + which * 8u);
+        return true;
+      };
+      bool ok = barrier_wait(q_full, 0) && multiply(0);
+      for (uint32_t tile = 0; tile < tiles && ok; ++tile) {
+        const uint32_t which = tile % S::kScores;
+        ok = barrier_wait(scores_full + which * 8u, tile / S::kScores & 1u);  // K is read
+        if (!ok) break;
+        if (tile + 1u < tiles) {
+          load(&map_k, S::kK, (tile + 1u) * kTile, kv_head, k_full), ++k_issued;
+          if (ALONE) ok = multiply(tile + 1u);  // beside this tile's exponentials; its place was last read by P V of the tile before
+        }
+        ok = ok && !*abort_flag && barrier_wait(v_full, tile & 1u) && barrier_wait(weights_full, tile & 1u);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (uint32_t j = 0; j < kTile / 16; ++j) {
+          const uint32_t half = j * 16u / S::kKeys, weights = scores + which * kTile + half * S::kKeys + (j * 16u - half * S::kKeys) / 2u;
+          // bit 16: the B operand's columns are contiguous
+          mma_f16_weights(sums, weights, value_descriptor(base + S::kV + j * 2048u), instruction_descriptor(kTile, D) | (1u << 16),
+                          (tile > 0 || j > 0) ? 1u : 0u);
+        }
+        mma_commit(sums_full);
+        ok = barrier_wait(sums_full, tile & 1u);  // V and the weights are read
+        if (ok && tile + 1u < tiles) {
+          load(&map_v, S::kV, (tile + 1u) * kTile, kv_head, v_full), ++v_issued;
+          if (!ALONE) ok = multiply(tile + 1u);
+        }
+      }
+      if (!ok || *abort_flag) {  // the copies already started must land first
+        give_up();
+        barrier_wait(q_full, 0);
+        barrier_wait(k_full, (k_issued - 1u) & 1u);
+        barrier_wait(v_full, (v_issued - 1u) & 1u);
+      }
+    }
+  } else {
+    const uint32_t row = threadIdx.x % kTile, half = threadIdx.x / kTile;  // of this thread
+    const uint32_t lanes = (warp % 4u * 32u) << 16, query = q0 + row;
+    float* const exchange = reinterpret_cast<float*>(base_pointer + S::kExchange);
+    auto of_row = [&](uint32_t parity, uint32_t of_half) -> float& { return exchange[(parity * 2u + of_half) * kTile + row]; };
+    auto halves_sync = [] { asm volatile("bar.sync 1, 256;" ::: "memory"); };
+    const float scale = p.scale * 1.4426950408889634f;
+    float top = kLowest, total = 0.0f;  // in units of log2 e
+    bool ok = true;
+    for (uint32_t tile = 0; tile < tiles; ++tile) {
+      const uint32_t which = tile % S::kScores, k0 = tile * kTile + half * S::kKeys;
+      const uint32_t mine = scores + which * kTile + half * S::kKeys + lanes;
+      ok = ok && !*abort_flag && barrier_wait(scores_full + which * 8u, tile / S::kScores & 1u);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) {
+        if (ALONE) halves_sync();  // the other half may be waiting there
+        continue;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      // keys below `seen` are visible to this row; all of them to the whole warp where `whole`
+      const uint32_t limit = p.causal ? min(p.k_len, query + p.past_length + 1u) : p.k_len, seen = limit > k0 ? limit - k0 : 0u;
+      const bool whole = __all_sync(0xffffffffu, seen >= S::kKeys);
+      uint32_t raw[S::kKeys / 32u][32];
+#pragma unroll
+      for (uint32_t part = 0; part < S::kKeys / 32u; ++part) tmem_load_32(mine + part * 32u, raw[part]);
+      tmem_wait_load();
+      float four[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      if (whole) {
+#pragma unroll
+        for (uint32_t i = 0; i < S::kKeys; ++i) four[i & 3] = fmaxf(four[i & 3], __uint_as_float(raw[i / 32][i % 32]));
+      } else {
+#pragma unroll
+        for (uint32_t i = 0; i < S::kKeys; ++i)
+          if (i < seen) four[i & 3] = fmaxf(four[i & 3], __uint_as_float(raw[i / 32][i % 32]));
+      }
+      float most = fmaxf(fmaxf(four[0], four[1]), fmaxf(four[2], four[3])) * scale;  // scale is positive
+      if (ALONE) {
+        of_row(tile & 1u, half) = most;
+        halves_sync();
+        most = fmaxf(most, of_row(tile & 1u, half ^ 1u));
+      }
+      const bool grown = most > top + kSlack;
+      if (__any_sync(0xffffffffu, grown)) {
+        const float keep = grown ? exp2_fast(top - most) : 1.0f;
+        if (grown) top = most;
+        total *= keep;
+        if (tile > 0) {
+          if (ALONE) {  // P V of the tile before may still be under way
+            ok = __all_sync(0xffffffffu, barrier_wait(sums_full, (tile - 1u) & 1u));
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          }
+#pragma unroll 1
+          for (uint32_t part = half * (D / 32u / S::kHalves); part < (half + 1u) * (D / 32u / S::kHalves); ++part) {
+            uint32_t held[32];
+            tmem_load_32(sums + lanes + part * 32u, held);
+            tmem_wait_load();
+#pragma unroll
+            for (int i = 0; i < 32; ++i) held[i] = __float_as_uint(__uint_as_float(held[i]) * keep);
+            tmem_store_32(sums + lanes + part * 32u, held);
+          }
+        }
+      }
+#pragma unroll
+      for (uint32_t part = 0; part < S::kKeys / 32u; ++part) {
+        uint32_t weights[16];
+        float two[2] = {0.0f, 0.0f};
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          float low = exp2_fast(fmaf(__uint_as_float(raw[part][2 * i]), scale, -top));
+          float high = exp2_fast(fmaf(__uint_as_float(raw[part][2 * i + 1]), scale, -top));
+          if (!whole) {
+            low = part * 32u + 2u * i < seen ? low : 0.0f;
+            high = part * 32u + 2u * i + 1u < seen ? high : 0.0f;
+          }
+          const __half2 pair = __floats2half2_rn(low, high);
+          const float2 rounded = __half22float2(pair);
+          two[0] += rounded.x;
+          two[1] += rounded.y;
+          weights[i] = *reinterpret_cast<const uint32_t*>(&pair);
+        }
+        total += two[0] + two[1];
+        tmem_store_16(mine + part * 16u, weights);  // over scores that are in registers
+      }
+      tmem_wait_store();
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) barrier_arrive(weights_full);
+    }
+    if (ALONE) {
+      of_row(tiles & 1u, half) = total;
+      halves_sync();
+      total = of_row(tiles & 1u, 0) + of_row(tiles & 1u, 1);
+    }
+    ok = ok && !*abort_flag && barrier_wait(sums_full, (tiles - 1u) & 1u);
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) give_up();
+    if (ok) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const float inverse = total == 0.0f ? 0.0f : 1.0f / total;
+      __half* const target = output + (p.token_first_output ? (((size_t)batch * p.q_len + query) * p.heads + head) * D
+                                                            : (((size_t)batch * p.heads + head) * p.q_len + query) * D);
+#pragma unroll 1
+      for (uint32_t part = half * (D / 32u / S::kHalves); part < (half + 1u) * (D / 32u / S::kHalves); ++part) {
+        uint32_t raw[32];
+        tmem_load_32(sums + lanes + part * 32u, raw);
+        tmem_wait_load();
+        if (query < p.q_len) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            uint32_t words[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const __half2 pair = __floats2half2_rn(__uint_as_float(raw[i * 8 + j * 2]) * inverse, __uint_as_float(raw[i * 8 + j * 2 + 1]) * inverse);
+              words[j] = *reinterpret_cast<const uint32_t*>(&pair);
+            }
+            *reinterpret_cast<uint4*>(target + part * 32u + i * 8) = make_uint4(words[0], words[1], words[2], words[3]);
+          }
+        }
+        __syncwarp();  // tcgen05.ld needs the whole warp
+      }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    }
+  }
+
+  __syncthreads();
+  if (warp == S::kRowWarps) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(scores), "r"(S::kColumns) : "memory");
+  }
+}
+
+// cuTensorMapEncodeTiled, resolved through the runtime so that the library does not link libcuda.
+typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// Rows of `dim` fp16 in boxes of 64 x 128: [batch][head][row], or [batch][row][head] (token first).
+bool make_map(CUtensorMap* map, const void* base, uint64_t dim, uint64_t rows, uint64_t heads, uint64_t batches, bool token_first) {
+  static EncodeTiled encode = []() -> EncodeTiled {
+    void* pointer = nullptr;
+    cudaDriverEntryPointQueryResult result;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &pointer, cudaEnableDefault, &result) != cudaSuccess ||
+        result != cudaDriverEntryPointSuccess)
+      return nullptr;
+    return reinterpret_cast<EncodeTiled>(pointer);
+  }();
+  if (encode == nullptr) return false;
+  const cuuint64_t dims[4] = {dim, rows, heads, batches};
+  const cuuint64_t strides[3] = {(token_first ? heads : 1u) * dim * 2u, (token_first ? 1u : rows) * dim * 2u, rows * heads * dim * 2u};
+  const cuuint32_t box[4] = {64, kTile, 1, 1}, element_strides[4] = {1, 1, 1, 1};
+  return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void*>(base), dims, strides, box, element_strides,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int D, bool ALONE>
+int run(const KernelArgs& args, const DenseParams& p) {
+  using S = Shape<D, ALONE>;
+  CUtensorMap map_q, map_k, map_v;
+  if (!make_map(&map_q, args.buffers[0], D, p.q_len, p.heads, p.batches, false) ||
+      !make_map(&map_k, args.buffers[1], D, p.k_len, p.kv_heads, p.batches, false) ||
+      !make_map(&map_v, args.buffers[2], D, p.k_len, p.kv_heads, p.batches, p.token_first_value != 0))
+    return -1;
+  auto kernel = dense_attention_tc_kernel<D, ALONE>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSharedBytes) != cudaSuccess) {
+    cudaGetLastError();
+    return -1;
+  }
+  launch_kernel(args, kernel, dim3(p.heads, (p.q_len + kTile - 1u) / kTile, p.batches), dim3(S::kThreads), S::kSharedBytes, map_q, map_k,
+                map_v, (__half*)args.buffers[4], p, args.ctx ? context_device_error(args.ctx) : nullptr);
+  return check_launch(args);
+}
+
+}  // namespace
+
+int launch_attention_dense_tc(const KernelArgs& args, const DenseParams& p) {
+  if (!(p.scale > 0.0f)) return -1;  // the largest score is that of the largest product
+  if (args.ctx == nullptr || p.mask_batches != 0 || p.batches > 65535u || p.q_len > 65535u * kTile || (p.dim != 64u && p.dim != 128u)) return -1;
+  if (p.causal && (uint64_t)p.q_len + p.past_length > 0xffffffffull) return -1;
+  for (int i = 0; i < 5; ++i)
+    if (i != 3 && ((uintptr_t)args.buffers[i] & 15u)) return -1;
+  const size_t ctas = (size_t)p.heads * ((p.q_len + kTile - 1u) / kTile) * p.batches;
+  const bool alone = 2u * ctas <= 5u * (size_t)context_sm_count(args.ctx);
+  if (p.dim == 64u) return alone ? run<64, true>(args, p) : run<64, false>(args, p);
+  return alone ? run<128, true>(args, p) : run<128, false>(args, p);
+}
+
+}  // namespace llmopt

@@ -44,6 +44,29 @@ def test_dense_attention_matches_oracle(runtime, oracle, b, h, kvh, ql, kl, d, c
     assert_close_f16(got, want, label=f"dense attention d={d} q={ql} k={kl}")
 
 
+@pytest.mark.parametrize("b,h,kvh,ql,kl,d,causal,tfo,tfv,growth", [
+    (1, 3, 1, 128, 128, 64, True, True, False, 0.0),    # one whole tile
+    (1, 2, 2, 127, 129, 128, True, False, True, 0.0),   # one row less, one key more
+    (1, 4, 2, 385, 385, 64, True, True, False, 0.02),   # maxima that grow by less and by more than what is put up with
+    (2, 2, 1, 1, 300, 128, True, True, True, 0.05),     # a single query
+    (1, 2, 1, 260, 130, 64, False, True, False, 0.3),   # fewer keys than queries
+    (1, 1, 1, 200, 90, 128, True, True, False, 0.0),    # causal, keys that end before the queries
+    (2, 48, 16, 520, 520, 64, True, True, False, 0.02),  # more tiles than SMs: two thread blocks share one
+    (3, 40, 8, 390, 517, 128, True, True, True, 0.02),
+])
+def test_dense_attention_tiles_of_128(runtime, oracle, b, h, kvh, ql, kl, d, causal, tfo, tfv, growth):
+    rng = np.random.default_rng(22)
+    q = rng.standard_normal((b, h, ql, d)).astype(np.float16)
+    places = 1.0 + growth * np.arange(kl)
+    k = (rng.standard_normal((b, kvh, kl, d)) * np.minimum(places, 12.0)[:, None]).astype(np.float16)
+    v = rng.standard_normal((b, kl, kvh, d) if tfv else (b, kvh, kl, d)).astype(np.float16)
+    scale = float(np.float32(1.0 / np.sqrt(d)))
+    got = _attention(runtime, q, k, v, causal=causal, scale=scale, token_first_output=tfo)
+    want = oracle.attention_dense(q, k, v, None, causal=int(causal), scale=scale, kv_heads=kvh,
+                                  token_first_output=int(tfo), past_length=max(0, kl - ql), token_first_value=int(tfv))
+    assert_close_f16(got, want, label=f"dense attention d={d} q={ql} k={kl}")
+
+
 @pytest.mark.parametrize("kind", ["bool", "float16"])
 def test_dense_attention_masks(runtime, oracle, kind):
     rng = np.random.default_rng(21)
