@@ -282,6 +282,12 @@ int run(const KernelArgs& args, DenseProblem p, uint32_t tiles) {
     launch_kernel(args, kernel, grid, dim3(Shape::kThreads), bytes, task, p.plan);
     return check_launch(args);
   };
+  // Narrow products and few rows: tiles of 32 x 16 or 32 x 32 where each has an SM to itself; a thread's sums are what a step over k
+  // takes time for.  k 2048, 100 rows n 256 45 -> 28 us; 40 rows n 2048 41 -> 30.  (Two of 32 x 32 beside one another are slower than
+  // one of 32 x 64: 98 for 59 with 100 rows.)
+  const size_t tall = down(32u);
+  if (tall <= kMostDown && (p.n + 15u) / 16u * tall <= sms) return launch(dense_f32_tile_kernel<4, 1, 8, 16, STORE>, Tile<4, 1, 8, 16>());
+  if (tall <= kMostDown && (p.n + 31u) / 32u * tall <= sms) return launch(dense_f32_tile_kernel<4, 2, 8, 16, STORE>, Tile<4, 2, 8, 16>());
   const size_t large = cost(64u, 128u, 107u, 214u), middle = cost(64u, 64u, 68u, 128u), small = cost(32u, 64u, 40u, 60u);
   if (down(32u) <= kMostDown && small <= middle && small <= large)
     return launch(dense_f32_tile_kernel<4, 4, 8, 16, STORE>, Tile<4, 4, 8, 16>());

@@ -76,6 +76,27 @@ def test_dense_linear(runtime, dtype, m, n, k, split):
             close(download(buffers[4], (m, n - split)), want[:, split:], 1e-5, epilogue)
 
 
+@pytest.mark.parametrize("m,n,k", [(33, 16, 40), (64, 250, 300), (100, 256, 1024), (40, 2048, 64), (100, 1100, 100), (149 * 32, 16, 64)])
+def test_fp32_products_in_tiles_of_every_width(runtime, m, n, k):
+    """Few tiles are narrow ones; the sums of any width run over k in order: those of more columns are the same to the last bit."""
+    from llmopt_b200 import parameters
+
+    rng = np.random.default_rng(m + n)
+    wide = 5200
+    x, w = rng.standard_normal((m, k)).astype(np.float32), (rng.standard_normal((wide, k)) / np.sqrt(k)).astype(np.float32)
+    nothing = empty(runtime, 16)
+    results = []
+    for columns in (n, wide):
+        out = empty(runtime, m * columns)
+        runtime.dispatch("llmopt_dense_linear_f32",
+                         buffers=[upload(runtime, x), upload(runtime, w[:columns]), nothing, nothing, out, nothing, nothing],
+                         parameters=parameters.dense_linear(m=m, n=columns, k=k, split=0, has_bias=False, epilogue=None, table_rows=0,
+                                                            table_stride=0, table_offset=0))
+        results.append(download(out, (m, columns)))
+    assert np.array_equal(results[0], results[1][:, :n])
+    close(results[0], x.astype(np.float64) @ w[:n].T.astype(np.float64), 1e-5, "narrow")
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("width", [97, 104, 192, 1028, 4096, 8192, 9000])
 def test_residual_norm(runtime, dtype, width):
