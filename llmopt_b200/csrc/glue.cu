@@ -53,6 +53,42 @@ __global__ void rotary_qk_kernel(const __half* __restrict__ q_input, const __hal
   }
 }
 
+// Rows whose two halves are whole 16-byte vectors, as prompts have them: eight columns of either half per thread, rows in the order
+// of the inputs.  Bound by memory; an element per lane, each read twice, took 22 us for 2048 tokens of 40 heads of 128, now 6.5.
+__global__ void __launch_bounds__(256) rotary_qk_vector_kernel(const __half* __restrict__ q_input, const __half* __restrict__ k_input,
+                                                               const __half* __restrict__ cosine, const __half* __restrict__ sine,
+                                                               __half* __restrict__ q_output, __half* __restrict__ k_output,
+                                                               RotaryQkParams p) {
+  grid_chain_prologue();
+  const uint32_t pieces = p.half_dimension / 8u, heads = p.q_heads + p.k_heads;
+  const uint32_t index = blockIdx.x * blockDim.x + threadIdx.x, row = index / pieces, column = index % pieces * 8u;
+  if (row >= p.batches * heads * p.tokens) return;
+  const uint32_t any_head = row % heads, batch = row / heads / p.tokens, token = row / heads % p.tokens;
+  const bool is_q = any_head < p.q_heads;
+  const uint32_t head = is_q ? any_head : any_head - p.q_heads, own = is_q ? p.q_heads : p.k_heads;
+  const __half* input = (is_q ? q_input : k_input) + (((size_t)batch * p.tokens + token) * own + head) * p.width + column;
+  __half* output = (is_q ? q_output : k_output) + (((size_t)batch * own + head) * p.tokens + token) * p.width + column;
+  const size_t trig = ((size_t)(p.trig_batches == 1 ? 0 : batch) * p.tokens + token) * p.width + column;
+  struct Eight {
+    __half2 two[4];
+  };
+  auto load = [](const __half* source) {
+    const uint4 raw = *reinterpret_cast<const uint4*>(source);
+    return *reinterpret_cast<const Eight*>(&raw);
+  };
+  const Eight low = load(input), high = load(input + p.half_dimension);
+  const Eight cos_low = load(cosine + trig), cos_high = load(cosine + trig + p.half_dimension);
+  const Eight sin_low = load(sine + trig), sin_high = load(sine + trig + p.half_dimension);
+  Eight out_low, out_high;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {  // *_rn: each operation rounds on its own, never contracted into an fma
+    out_low.two[i] = __hadd2_rn(__hmul2_rn(low.two[i], cos_low.two[i]), __hmul2_rn(__hneg2(high.two[i]), sin_low.two[i]));
+    out_high.two[i] = __hadd2_rn(__hmul2_rn(high.two[i], cos_high.two[i]), __hmul2_rn(low.two[i], sin_high.two[i]));
+  }
+  *reinterpret_cast<uint4*>(output) = *reinterpret_cast<const uint4*>(&out_low);
+  *reinterpret_cast<uint4*>(output + p.half_dimension) = *reinterpret_cast<const uint4*>(&out_high);
+}
+
 struct EmbeddingParams {  // lib/metal_tensor_source.ml:237
   uint32_t tokens, vocabulary, width;
 };
@@ -67,6 +103,16 @@ __global__ void embedding_kernel(const long long* __restrict__ indices, const __
   output[gid] = (index >= 0 && index < (long long)p.vocabulary)
                     ? weight[(size_t)index * p.width + dimension]
                     : __float2half_rn(0.0f);
+}
+
+// Rows of whole 16-byte vectors: 2048 tokens of 4096 36 -> 6.9 us.
+__global__ void __launch_bounds__(256) embedding_vector_kernel(const long long* __restrict__ indices, const uint4* __restrict__ weight,
+                                                               uint4* __restrict__ output, EmbeddingParams p) {
+  grid_chain_prologue();
+  const uint32_t pieces = p.width / 8u, gid = blockIdx.x * blockDim.x + threadIdx.x;
+  if (gid >= p.tokens * pieces) return;
+  const long long index = indices[gid / pieces];
+  output[gid] = index >= 0 && index < (long long)p.vocabulary ? weight[(size_t)index * pieces + gid % pieces] : make_uint4(0u, 0u, 0u, 0u);
 }
 
 __global__ void chain_token_kernel(const uint32_t* __restrict__ argmax_in, long long* __restrict__ token_out) {
@@ -155,6 +201,14 @@ int launch_rotary_qk(const KernelArgs& args) {
   LLMOPT_REQUIRE(args.lengths[2] >= trig * 2 && args.lengths[3] >= trig * 2, "cosine/sine buffer is too short");
   const uint32_t rows = p.batches * (p.q_heads + p.k_heads) * p.tokens;
   if (rows == 0) return 0;
+  bool vectors = p.width == 2u * p.half_dimension && p.half_dimension % 8u == 0 && (size_t)rows * (p.half_dimension / 8u) <= 0xffffff00u;
+  for (int i = 0; i < 6; ++i) vectors = vectors && ((uintptr_t)args.buffers[i] & 15u) == 0;
+  if (vectors) {
+    launch_kernel(args, rotary_qk_vector_kernel, dim3((uint32_t)(((size_t)rows * (p.half_dimension / 8u) + 255) / 256)), dim3(256), 0,
+        (const __half*)args.buffers[0], (const __half*)args.buffers[1], (const __half*)args.buffers[2],
+        (const __half*)args.buffers[3], (__half*)args.buffers[4], (__half*)args.buffers[5], p);
+    return check_launch(args);
+  }
   launch_kernel(args, rotary_qk_kernel, dim3((rows + 7) / 8), dim3(256), 0,
       (const __half*)args.buffers[0], (const __half*)args.buffers[1], (const __half*)args.buffers[2],
       (const __half*)args.buffers[3], (__half*)args.buffers[4], (__half*)args.buffers[5], p);
@@ -170,6 +224,11 @@ int launch_embedding_f16(const KernelArgs& args) {
   LLMOPT_REQUIRE(args.lengths[0] >= (size_t)p.tokens * 8 && args.lengths[1] >= (size_t)p.vocabulary * p.width * 2 &&
                      args.lengths[2] >= elements * 2, "buffer is too short");
   if (elements == 0) return 0;
+  if (p.width % 8u == 0 && (((uintptr_t)args.buffers[1] | (uintptr_t)args.buffers[2]) & 15u) == 0) {
+    launch_kernel(args, embedding_vector_kernel, dim3((uint32_t)((elements / 8 + 255) / 256)), dim3(256), 0,
+        (const long long*)args.buffers[0], (const uint4*)args.buffers[1], (uint4*)args.buffers[2], p);
+    return check_launch(args);
+  }
   launch_kernel(args, embedding_kernel, dim3((uint32_t)((elements + 255) / 256)), dim3(256), 0,
       (const long long*)args.buffers[0], (const __half*)args.buffers[1], (__half*)args.buffers[2], p);
   return check_launch(args);

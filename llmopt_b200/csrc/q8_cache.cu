@@ -48,6 +48,43 @@ __global__ void pack_attention_kernel(const __half* __restrict__ source, const u
                  scales + p.segment_offset / p.group_size + local_group, lane);
 }
 
+// Groups of 32 or 64 in whole 16-byte vectors: eight values per lane, a group in four or eight lanes.  An element or two per lane
+// took 11.3 us for 2048 tokens of 8 heads of 128, this 4.2.
+template <uint32_t GROUP>
+__global__ void __launch_bounds__(256) pack_attention_vector_kernel(const __half* __restrict__ source, const uint32_t* __restrict__ slots,
+                                                                    uint8_t* __restrict__ pool, AttentionCacheParams p, PoolBound bound) {
+  grid_chain_prologue();
+  constexpr uint32_t kLanes = GROUP / 8u;
+  const uint32_t part = threadIdx.x % kLanes, logical_group = (blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
+  const uint32_t groups_per_head = p.head_dim / GROUP, segment_groups = p.heads * groups_per_head;
+  const bool present = logical_group < p.items * segment_groups;  // whole groups; their lanes take part in the exchange all the same
+  const uint32_t item = present ? logical_group / segment_groups : 0u, local_group = present ? logical_group % segment_groups : 0u;
+  const uint32_t head = local_group / groups_per_head, group_in_head = local_group % groups_per_head;
+  const uint4 raw = *reinterpret_cast<const uint4*>(
+      source + ((size_t)head * p.source_items + p.source_offset + item) * p.head_dim + group_in_head * GROUP + part * 8u);
+  const __half2* const halves = reinterpret_cast<const __half2*>(&raw);
+  float values[8], maximum = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 two = __half22float2(halves[i]);
+    values[2 * i] = two.x;
+    values[2 * i + 1] = two.y;
+    maximum = fmaxf(maximum, fmaxf(fabsf(two.x), fabsf(two.y)));
+  }
+#pragma unroll
+  for (uint32_t offset = kLanes / 2u; offset > 0; offset >>= 1) maximum = fmaxf(maximum, __shfl_xor_sync(0xffffffffu, maximum, offset));
+  const uint32_t slot = slots[item];
+  if (!present || !slot_in_pool(slot, bound, part)) return;
+  const __half stored = group_scale(maximum);
+  const float scale = __half2float(stored);
+  uint32_t words[2] = {0u, 0u};
+#pragma unroll
+  for (int i = 0; i < 8; ++i) words[i / 4] |= (uint32_t)(uint8_t)quantized_value(values[i], scale) << (8 * (i % 4));
+  uint8_t* const row = pool + (size_t)slot * p.token_stride;
+  *reinterpret_cast<uint2*>(row + p.segment_offset + local_group * GROUP + part * 8u) = make_uint2(words[0], words[1]);
+  if (part == 0) reinterpret_cast<__half*>(row + p.token_elements)[p.segment_offset / GROUP + local_group] = stored;
+}
+
 __global__ void pack_attention_pair_kernel(const __half* __restrict__ key_source,
                                            const __half* __restrict__ value_source,
                                            const uint32_t* __restrict__ slots, uint8_t* __restrict__ pool,
@@ -277,6 +314,15 @@ int launch_cache_pack_attention_q8(const KernelArgs& args) {
                  "segment or its scales lie outside the token row");
   const uint32_t groups = p.items * p.heads * (p.head_dim / p.group_size);
   if (groups == 0) return 0;
+  const bool vectors = (((uintptr_t)args.buffers[0] & 15u) | ((uintptr_t)args.buffers[2] & 7u)) == 0 && p.token_stride % 8u == 0 &&
+                       p.segment_offset % 8u == 0 && p.items > 0 && groups <= 0x1fffff00u;
+  if (vectors && (p.group_size == 32u || p.group_size == 64u)) {
+    const uint32_t lanes = p.group_size / 8u;
+    auto kernel = p.group_size == 32u ? pack_attention_vector_kernel<32> : pack_attention_vector_kernel<64>;
+    launch_kernel(args, kernel, dim3((groups * lanes + 255u) / 256u), dim3(256), 0, (const __half*)args.buffers[0],
+                  (const uint32_t*)args.buffers[1], (uint8_t*)args.buffers[2], p, pool_bound(args, 2, p.token_stride));
+    return check_launch(args);
+  }
   launch_kernel(args, pack_attention_kernel, dim3((groups + 7) / 8), dim3(256), 0,
       (const __half*)args.buffers[0], (const uint32_t*)args.buffers[1], (uint8_t*)args.buffers[2], p,
       pool_bound(args, 2, p.token_stride));

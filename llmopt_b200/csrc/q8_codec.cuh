@@ -27,8 +27,16 @@ struct RotaryQkParams {  // lib/metal_normalization_source.ml:760-763
   uint32_t batches, tokens, q_heads, k_heads, width, half_dimension, trig_batches;
 };
 
-// One warp quantises one group: scale = half(max == 0 ? 1 : max / 127) (fp32 division), q =
-// clamp(rint(x / float(scale)), -127, 127) with IEEE division and round-half-even.
+// scale = half(max == 0 ? 1 : max / 127) (fp32 division), q = clamp(rint(x / float(scale)), -127, 127) with IEEE division and
+// round-half-even.
+__device__ __forceinline__ __half group_scale(float maximum) {
+  return __float2half_rn(maximum == 0.0f ? 1.0f : __fdiv_rn(maximum, 127.0f));
+}
+__device__ __forceinline__ int8_t quantized_value(float value, float scale) {
+  return (int8_t)max(-127, min(127, (int)rintf(__fdiv_rn(value, scale))));
+}
+
+// One warp quantises one group.
 __device__ __forceinline__ void quantize_group(const __half* __restrict__ source, uint32_t group_size,
                                                int8_t* __restrict__ values, __half* __restrict__ scale_out,
                                                uint32_t lane) {
@@ -36,13 +44,9 @@ __device__ __forceinline__ void quantize_group(const __half* __restrict__ source
   for (uint32_t index = lane; index < group_size; index += 32)
     maximum = fmaxf(maximum, fabsf(__half2float(source[index])));
   maximum = warp_max(maximum);
-  const __half stored = __float2half_rn(maximum == 0.0f ? 1.0f : __fdiv_rn(maximum, 127.0f));
+  const __half stored = group_scale(maximum);
   const float scale = __half2float(stored);
-  for (uint32_t index = lane; index < group_size; index += 32) {
-    int quantized = (int)rintf(__fdiv_rn(__half2float(source[index]), scale));
-    quantized = max(-127, min(127, quantized));
-    values[index] = (int8_t)quantized;
-  }
+  for (uint32_t index = lane; index < group_size; index += 32) values[index] = quantized_value(__half2float(source[index]), scale);
   if (lane == 0) *scale_out = stored;
 }
 

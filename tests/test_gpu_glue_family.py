@@ -231,3 +231,51 @@ def test_a_package_declaring_every_entry_validates_against_the_library(runtime):
         sp.Package("compiled-graph", "model.metallib",
                    [kernel_abi.Entry("llmopt_no_such_kernel", kernel_abi.LINEAR, "float16", "float16")]
                    ).validate_declared_functions(runtime)
+
+
+def _shifted(runtime, array, shift):
+    """The array in a view that begins ``shift`` bytes into its buffer."""
+    raw = np.concatenate([np.zeros(shift, np.uint8), np.ascontiguousarray(array).view(np.uint8).reshape(-1)])
+    buffer = _buf(runtime, raw)
+    return buffer.view(shift, raw.size - shift)
+
+
+@pytest.mark.parametrize("tokens,q_heads,k_heads,width,group", [(1, 3, 1, 64, 32), (5, 9, 3, 64, 64), (37, 2, 1, 128, 32), (130, 4, 2, 128, 64),
+                                                                (3, 1, 1, 96, 32)])
+def test_whole_vectors_and_single_elements_agree(runtime, tokens, q_heads, k_heads, width, group):
+    """Rotary embedding, cache pack and embedding take whole 16-byte vectors where addresses allow it and elements elsewhere."""
+    rng = np.random.default_rng(tokens)
+    half = lambda *shape: rng.standard_normal(shape).astype(np.float16)
+    q, k, cosine, sine = half(tokens, q_heads, width), half(tokens, k_heads, width), half(tokens, width), half(tokens, width)
+    table, ids = half(50, width), rng.integers(-1, 51, tokens).astype(np.int64)
+    elements = k_heads * width
+    stride = (elements + 2 * (elements // group) + 15) // 16 * 16
+    slots = rng.permutation(tokens + 3)[:tokens].astype(np.uint32)
+    k[0, 0] = 0.0  # a group without a scale of its own
+    results = []
+    for shift in (0, 2):
+        put = lambda array: _shifted(runtime, array, shift)
+        room = lambda shape: put(np.zeros(shape, np.float16))
+        q_out, k_out, rows = room(q.shape), room(k.shape), room((tokens, width))
+        runtime.dispatch("llmopt_rotary_qk_f16_simd_h64", buffers=[put(q), put(k), put(cosine), put(sine), q_out, k_out],
+                         parameters=np.array([1, tokens, q_heads, k_heads, width, width // 2, 1], np.uint32).tobytes())
+        pool = _buf(runtime, np.zeros((tokens + 3) * stride, np.uint8))
+        runtime.dispatch("llmopt_cache_pack_attention_q8", buffers=[put(k.transpose(1, 0, 2)), _buf(runtime, slots), pool],
+                         parameters=np.array([tokens, 0, k_heads, width, group, elements, elements // group, stride, tokens, 0],
+                                             np.uint32).tobytes())
+        runtime.dispatch("llmopt_embedding_f16", buffers=[_buf(runtime, ids), put(table), rows],
+                         parameters=np.array([tokens, 50, width], np.uint32).tobytes())
+        results.append([q_out.to_numpy(np.uint16, q.shape), k_out.to_numpy(np.uint16, k.shape), rows.to_numpy(np.float16, (tokens, width)),
+                        pool.to_numpy(np.uint8, (tokens + 3, stride))])
+    for whole, single in zip(*results):
+        assert np.array_equal(whole, single)
+    known = (ids >= 0) & (ids < 50)
+    assert np.array_equal(results[0][2], np.where(known[:, None], table[np.clip(ids, 0, 49)], np.float16(0)))
+    turned = np.concatenate([-q[..., width // 2:], q[..., :width // 2]], -1)
+    want = (q * cosine[:, None] + turned * sine[:, None]).transpose(1, 0, 2)  # each operation rounded to half
+    assert np.array_equal(results[0][0].view(np.float16).reshape(q_heads, tokens, width), want)
+    largest = np.abs(k.reshape(tokens, -1, group).astype(np.float32)).max(-1)
+    scale = np.where(largest == 0, np.float32(1), largest / np.float32(127)).astype(np.float16)
+    quantised = np.clip(np.rint(k.reshape(tokens, -1, group).astype(np.float32) / scale[..., None].astype(np.float32)), -127, 127)
+    assert np.array_equal(results[0][3][slots, :elements].view(np.int8), quantised.reshape(tokens, -1).astype(np.int8))
+    assert np.array_equal(results[0][3][slots, elements:elements + 2 * scale.shape[1]].view(np.float16), scale)
