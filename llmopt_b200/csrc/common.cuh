@@ -46,6 +46,7 @@ struct KernelArgs {
   const FusedNorm* fused_norm;  // null unless the plan builder folded a norm into this dispatch
   // null unless the plan builder handed the rotary + cache pack of the new token to this (attention) dispatch
   const struct RotaryPackFusion* rotary_fusion;
+  bool apart;  // this launch starts when its predecessor has ended, also where overlap is allowed
 };
 
 // Bytes between the sequences of a batched short-conv step.
@@ -105,7 +106,7 @@ inline void launch_kernel(const KernelArgs& launch, void (*kernel)(Params...), d
   attribute[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attribute[0].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attribute;
-  config.numAttrs = context_overlap(launch.ctx) ? 1 : 0;
+  config.numAttrs = context_overlap(launch.ctx) && !launch.apart ? 1 : 0;
   cudaLaunchKernelEx(&config, kernel, static_cast<Args&&>(args)...);
 }
 
@@ -125,7 +126,7 @@ inline void launch_cluster_kernel(const KernelArgs& launch, void (*kernel)(Param
   attribute[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attribute[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attribute;
-  config.numAttrs = context_overlap(launch.ctx) ? 2 : 1;
+  config.numAttrs = context_overlap(launch.ctx) && !launch.apart ? 2 : 1;
   cudaLaunchKernelEx(&config, kernel, static_cast<Args&&>(args)...);
 }
 

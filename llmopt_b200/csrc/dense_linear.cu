@@ -285,8 +285,14 @@ int run_gemv(const KernelArgs& args, DenseProblem p, DenseStore store) {
     }
     auto run = [&](auto kernel) {
       const DenseTask<STORE> task(p);
-      if (p.cluster == 1u) launch_kernel(args, kernel, dim3(tiles), dim3(kGemvWarps * 32), 0, task);
-      else launch_cluster_kernel(args, kernel, dim3(tiles * p.cluster), dim3(kGemvWarps * 32), 0, p.cluster, task);
+      // These start when their predecessor has ended.  Let in early they took longer than they saved, and so did the launch before
+      // them, in steps of both designs of decoders at every number of rows, us: width 2048 recurrent 8 rows 578 -> 535, 32 rows
+      // 1190 -> 1105, windowed one row 340 -> 298, 8 rows 565 -> 500; width 4096 windowed 8 rows 1335 -> 1010, 32 rows 2850 -> 1990,
+      // recurrent one row 850 -> 694.  It is not that early ones share an SM: kept apart by shared memory they stay slow.
+      KernelArgs launch = args;
+      launch.apart = true;
+      if (p.cluster == 1u) launch_kernel(launch, kernel, dim3(tiles), dim3(kGemvWarps * 32), 0, task);
+      else launch_cluster_kernel(launch, kernel, dim3(tiles * p.cluster), dim3(kGemvWarps * 32), 0, p.cluster, task);
       return check_launch(args);
     };
     if (p.m <= 8u) return run(dense_gemv_kernel<1, STORE>);

@@ -398,8 +398,12 @@ int run_step(const KernelArgs& args, DenseProblem p, const uint32_t* route, cons
     const dim3 grid(tiles * p.cluster, DOWN ? 1u : most);
     const DenseTask<DOWN ? kStoreResidual : kStorePair> task(p);
     const uint32_t experts = p.plan.experts, pairs = p.m * top;
-    if (p.cluster == 1u) launch_kernel(args, kernel, grid, dim3(kGemvWarps * 32), 0, task, experts, route, at, pairs);
-    else launch_cluster_kernel(args, kernel, grid, dim3(kGemvWarps * 32), 0, p.cluster, task, experts, route, at, pairs);
+    // Down rows start when the gate and up rows have ended: in a step of 32 rows (16 experts of 2048 x 1792) they took 62 us after
+    // those when they were let in early, 26 this way.
+    KernelArgs launch = args;
+    launch.apart = DOWN;
+    if (p.cluster == 1u) launch_kernel(launch, kernel, grid, dim3(kGemvWarps * 32), 0, task, experts, route, at, pairs);
+    else launch_cluster_kernel(launch, kernel, grid, dim3(kGemvWarps * 32), 0, p.cluster, task, experts, route, at, pairs);
     return check_launch(args);
   };
   if (p.m <= 8u) return run(expert_step_kernel<1, DOWN>);
