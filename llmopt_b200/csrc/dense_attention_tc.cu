@@ -290,6 +290,10 @@ dense_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
         total += two[0] + two[1];
         tmem_store_16(mine + part * 16u, weights);  // over scores that are in registers
       }
+      // A wait names a phase by its parity, so nobody may be two phases behind: with two tiles of scores a row could be done with this
+      // tile before P V of the one before has begun (V late), which would end the wait for the last P V too early, and run
+      // `weights_full` past the thread that waits for it.  tests/test_barrier_order_cpu.py goes through every order.
+      if (ALONE && tile > 0) ok = barrier_wait(sums_full, (tile - 1u) & 1u) && ok;
       tmem_wait_store();
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
