@@ -17,7 +17,7 @@
 // K and V two tiles deep changed nothing: their way hides behind the exponentials.
 //
 // Rows beyond a head's keys or queries are zero-filled by TMA.  Every wait on an mbarrier is bounded; a wait that runs out raises
-// the context's device error word, and the CTA lets its copies land, frees its tensor memory and returns.
+// the context's device error word, and the CTA lets its copies land and its products end, frees its tensor memory and returns.
 #include <cuda.h>
 
 #include "dense_attention.cuh"
@@ -151,7 +151,7 @@ dense_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
   if (warp == S::kRowWarps) {
     if (lane == 0) {
       const int32_t kv_head = (int32_t)(head / (p.heads / p.kv_heads));
-      uint32_t k_issued = 0, v_issued = 0;
+      uint32_t k_issued = 0, v_issued = 0, scores_issued = 0, sums_issued = 0;
       auto load = [&](const CUtensorMap* map, uint32_t target, uint32_t row, int32_t of_head, uint32_t bar) {
         barrier_expect_tx(bar, S::kTileBytes);
 #pragma unroll
@@ -171,7 +171,7 @@ dense_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
           mma_f16(scores + which * kTile, operand_descriptor(base + at), operand_descriptor(base + S::kK + at), j > 0 ? 1u : 0u,
                   instruction_descriptor(kTile, kTile));
         }
-        mma_commit(scores_full + which * 8u);
+        mma_commit(scores_full + which * 8u), ++scores_issued;
         return true;
       };
       bool ok = barrier_wait(q_full, 0) && multiply(0);
@@ -193,18 +193,20 @@ dense_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
           mma_f16_weights(sums, weights, value_descriptor(base + S::kV + j * 2048u), instruction_descriptor(kTile, D) | (1u << 16),
                           (tile > 0 || j > 0) ? 1u : 0u);
         }
-        mma_commit(sums_full);
+        mma_commit(sums_full), ++sums_issued;
         ok = barrier_wait(sums_full, tile & 1u);  // V and the weights are read
         if (ok && tile + 1u < tiles) {
           load(&map_v, S::kV, (tile + 1u) * kTile, kv_head, v_full), ++v_issued;
           if (!ALONE) ok = multiply(tile + 1u);
         }
       }
-      if (!ok || *abort_flag) {  // the copies already started must land first
+      if (!ok || *abort_flag) {  // what is under way must end before shared and tensor memory are given back
         give_up();
         barrier_wait(q_full, 0);
         barrier_wait(k_full, (k_issued - 1u) & 1u);
         barrier_wait(v_full, (v_issued - 1u) & 1u);
+        if (scores_issued) barrier_wait(scores_full + (scores_issued - 1u) % S::kScores * 8u, (scores_issued - 1u) / S::kScores & 1u);
+        if (sums_issued) barrier_wait(sums_full, (sums_issued - 1u) & 1u);
       }
     }
   } else {

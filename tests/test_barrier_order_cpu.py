@@ -43,10 +43,25 @@ def rows(tiles, score_tiles, waits):
     yield "wait", "sums", tiles - 1
 
 
-def orders(tiles, score_tiles, waits):
-    """What can go wrong, over all orders: waits that pass too early ("early"), and sides that wait for good ("stuck").  A copy or
-    product is asynchronous: it is under way until some later point; products end in the order of their issue."""
-    programs = list(issuer(tiles, score_tiles)), list(rows(tiles, score_tiles, waits))
+def giving_up(tiles, score_tiles, steps):
+    """The issuer whose wait after ``steps`` of its steps has run out: it waits once more for the last of each kind that it issued."""
+    done = list(issuer(tiles, score_tiles))[:steps]
+    count = lambda kind, which=None: sum(step[0] == kind and which in (None, step[1]) for step in done)
+    yield from done
+    yield "wait", "q", 0
+    yield "wait", "k", count("copy", "k")
+    yield "wait", "v", count("copy", "v")
+    if count("scores"):
+        yield "wait", ("s", (count("scores") - 1) % score_tiles), (count("scores") - 1) // score_tiles
+    if count("sums"):
+        yield "wait", "sums", count("sums") - 1
+
+
+def orders(programs, score_tiles):
+    """What can go wrong, over all orders: waits that pass too early ("early"), sides that wait for good ("stuck"), and an issuer that
+    ends before what it issued ("left").  A copy or product is asynchronous: it is under way until some later point; products
+    end in the order of their issue."""
+    programs = [list(program) for program in programs]
     wrong, seen = set(), set()
     start = ((0, 0), (("k", 0), ("q", 0), ("s", 0), ("s1", 0), ("sums", 0), ("v", 0), ("weights", 0)), frozenset("qkv"), ())
     name = lambda which: which if isinstance(which, str) else ("s", "s1")[which[1]]
@@ -81,6 +96,8 @@ def orders(tiles, score_tiles, waits):
                 following.append((after, counts, copies, products + ("sums",)))
             else:
                 following.append((after, moved(which), copies, products))
+        if places[0] == len(programs[0]) and (copies or products):
+            wrong.add("left")
         if not following and any(place < len(program) for place, program in zip(places, programs)):
             wrong.add("stuck")
         pending.extend(following)
@@ -90,10 +107,19 @@ def orders(tiles, score_tiles, waits):
 @pytest.mark.parametrize("tiles", [1, 2, 3, 4, 5, 6])
 @pytest.mark.parametrize("score_tiles", [1, 2])
 def test_no_wait_ends_early_and_none_lasts(tiles, score_tiles):
-    assert orders(tiles, score_tiles, waits=True) == set()
+    assert orders((issuer(tiles, score_tiles), rows(tiles, score_tiles, True)), score_tiles) == set()
 
 
 @pytest.mark.parametrize("tiles", [2, 3, 4])
 def test_the_model_sees_rows_that_do_not_wait(tiles):
     """Without the rows' wait for P V of the tile before (a late V is enough) the last wait ends early and the issuer gets stuck."""
-    assert orders(tiles, 2, waits=False) == {"early", "stuck"}
+    assert orders((issuer(tiles, 2), rows(tiles, 2, False)), 2) == {"early", "stuck"}
+
+
+@pytest.mark.parametrize("tiles", [1, 2, 3, 4])
+@pytest.mark.parametrize("score_tiles", [1, 2])
+def test_nothing_is_under_way_when_the_issuer_has_given_up(tiles, score_tiles):
+    program = list(issuer(tiles, score_tiles))
+    for steps, step in enumerate(program):
+        if step[0] == "wait":  # rows may go on or give up as well: only the issuer's end counts
+            assert orders((giving_up(tiles, score_tiles, steps), rows(tiles, score_tiles, True)), score_tiles) <= {"stuck"}
