@@ -35,6 +35,11 @@ constexpr uint32_t kBlockBytes = kTile * 128;  // 64 dimensions of 128 rows
 constexpr float kSlack = 8.0f;
 constexpr float kLowest = -1.0e30f;
 
+// Keys that some query sees; beyond, memory need not hold numbers, and TMA puts zeros there.
+__host__ __device__ inline uint32_t seen_by_any(const DenseParams& p) {
+  return p.causal && p.k_len > p.past_length && p.k_len - p.past_length > p.q_len ? p.q_len + p.past_length : p.k_len;
+}
+
 template <int D, bool ALONE>
 struct Shape {
   static constexpr uint32_t kHalves = ALONE ? 2 : 1, kRowWarps = 4 * kHalves, kThreads = (kRowWarps + 1) * 32;
@@ -105,10 +110,50 @@ __device__ __forceinline__ uint64_t value_descriptor(uint32_t shared_address) {
   return descriptor;
 }
 
+// P V multiplies a weight of zero with the value of a masked key, which makes NaN of an infinity or a NaN there.  A warp computes such
+// a row's dimensions first .. first + 32 * PARTS - 1 once more, from its visible keys alone and in the manner of the general kernel;
+// the queries are still in shared memory.  Nothing is done where the masked keys of its last tile are numbers: the row's own result it is.
+template <int D, int PARTS>
+__device__ __noinline__ void walk_row(const unsigned char* q_tile, uint32_t row, const __half* keys, const __half* values, size_t value_stride,
+                                      uint32_t seen, uint32_t multiplied, uint32_t first, float scale, __half* target) {
+  const uint32_t lane = threadIdx.x & 31u;
+  bool masked = false;
+  for (uint32_t key = seen; key < multiplied; ++key)
+#pragma unroll
+    for (int i = 0; i < PARTS; ++i)
+      masked |= !(fabsf(__half2float(values[key * value_stride + first + i * 32 + lane])) < INFINITY);
+  if (!__any_sync(0xffffffffu, masked)) return;
+  float q[D / 32], result[PARTS] = {}, top = -INFINITY, total = 0.0f;
+#pragma unroll
+  for (int i = 0; i < D / 32; ++i) {  // 128-byte swizzle
+    const uint32_t d = i * 32 + lane, at = d / 64u * kBlockBytes + row * 128u + ((d % 64u * 2u) ^ (row % 8u * 16u));
+    q[i] = __half2float(*reinterpret_cast<const __half*>(q_tile + at));
+  }
+  for (uint32_t key = 0; key < seen; ++key) {
+    float dot = 0.0f;
+#pragma unroll
+    for (int i = 0; i < D / 32; ++i) dot = fmaf(q[i], __half2float(keys[(size_t)key * D + i * 32 + lane]), dot);
+    const float score = warp_sum(dot) * scale, next = fmaxf(top, score);
+    const float keep = top == -INFINITY ? 0.0f : expf(top - next), weight = expf(score - next);
+    bool lost = true;  // every result is NaN and stays it
+#pragma unroll
+    for (int i = 0; i < PARTS; ++i) {
+      result[i] = result[i] * keep + weight * __half2float(values[key * value_stride + first + i * 32 + lane]);
+      lost = lost && isnan(result[i]);
+    }
+    total = total * keep + weight;
+    top = next;
+    if (__all_sync(0xffffffffu, lost)) break;
+  }
+#pragma unroll
+  for (int i = 0; i < PARTS; ++i) target[first + i * 32 + lane] = __float2half_rn(total == 0.0f ? 0.0f : result[i] / total);
+}
+
 template <int D, bool ALONE>
 __global__ void __launch_bounds__(Shape<D, ALONE>::kThreads, ALONE ? 1 : 2)
 dense_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                          const __grid_constant__ CUtensorMap map_v, __half* output, DenseParams p, uint32_t* error_word) {
+                          const __grid_constant__ CUtensorMap map_v, const __half* key, const __half* value, __half* output, DenseParams p,
+                          uint32_t* error_word) {
   using S = Shape<D, ALONE>;
   extern __shared__ unsigned char shared_raw[];
   grid_chain_prologue();
@@ -312,6 +357,7 @@ dense_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
     if (ok) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const float inverse = total == 0.0f ? 0.0f : 1.0f / total;
+      bool finite = true;
       __half* const target = output + (p.token_first_output ? (((size_t)batch * p.q_len + query) * p.heads + head) * D
                                                             : (((size_t)batch * p.heads + head) * p.q_len + query) * D);
 #pragma unroll 1
@@ -325,13 +371,25 @@ dense_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
             uint32_t words[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-              const __half2 pair = __floats2half2_rn(__uint_as_float(raw[i * 8 + j * 2]) * inverse, __uint_as_float(raw[i * 8 + j * 2 + 1]) * inverse);
+              const float low = __uint_as_float(raw[i * 8 + j * 2]) * inverse, high = __uint_as_float(raw[i * 8 + j * 2 + 1]) * inverse;
+              finite = finite && fabsf(low) < INFINITY && fabsf(high) < INFINITY;
+              const __half2 pair = __floats2half2_rn(low, high);
               words[j] = *reinterpret_cast<const uint32_t*>(&pair);
             }
             *reinterpret_cast<uint4*>(target + part * 32u + i * 8) = make_uint4(words[0], words[1], words[2], words[3]);
           }
         }
         __syncwarp();  // tcgen05.ld needs the whole warp
+      }
+      for (uint32_t left = __ballot_sync(0xffffffffu, !finite); left != 0; left &= left - 1u) {
+        barrier_wait(q_full, 0);  // over long ago; this thread has not waited for it yet
+        const uint32_t at = row - lane + (uint32_t)__ffs(left) - 1u, kv_head = head / (p.heads / p.kv_heads);
+        const uint32_t seen = p.causal ? min(p.k_len, q0 + at + p.past_length + 1u) : p.k_len, multiplied = min(seen_by_any(p), tiles * kTile);
+        const size_t head_row = (size_t)batch * p.kv_heads + kv_head;
+        const __half* const values = value + (p.token_first_value ? ((size_t)batch * p.k_len * p.kv_heads + kv_head) * D : head_row * p.k_len * D);
+        const int64_t along = p.token_first_output ? (int64_t)p.heads * D : D;  // from one row of the output to the next
+        walk_row<D, D / 32 / S::kHalves>(base_pointer, at, key + head_row * p.k_len * D, values, p.token_first_value ? (size_t)p.kv_heads * D : D,
+                                         seen, multiplied, half * (D / S::kHalves), p.scale, target + ((int64_t)at - (int64_t)row) * along);
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     }
@@ -349,8 +407,8 @@ typedef CUresult (*EncodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, v
                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
-// Rows of `dim` fp16 in boxes of 64 x 128: [batch][head][row], or [batch][row][head] (token first).
-bool make_map(CUtensorMap* map, const void* base, uint64_t dim, uint64_t rows, uint64_t heads, uint64_t batches, bool token_first) {
+// The first `seen` of `rows` rows of `dim` fp16 in boxes of 64 x 128: [batch][head][row], or [batch][row][head] (token first).
+bool make_map(CUtensorMap* map, const void* base, uint64_t dim, uint64_t rows, uint64_t seen, uint64_t heads, uint64_t batches, bool token_first) {
   static EncodeTiled encode = []() -> EncodeTiled {
     void* pointer = nullptr;
     cudaDriverEntryPointQueryResult result;
@@ -360,7 +418,7 @@ bool make_map(CUtensorMap* map, const void* base, uint64_t dim, uint64_t rows, u
     return reinterpret_cast<EncodeTiled>(pointer);
   }();
   if (encode == nullptr) return false;
-  const cuuint64_t dims[4] = {dim, rows, heads, batches};
+  const cuuint64_t dims[4] = {dim, seen, heads, batches};
   const cuuint64_t strides[3] = {(token_first ? heads : 1u) * dim * 2u, (token_first ? 1u : rows) * dim * 2u, rows * heads * dim * 2u};
   const cuuint32_t box[4] = {64, kTile, 1, 1}, element_strides[4] = {1, 1, 1, 1};
   return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void*>(base), dims, strides, box, element_strides,
@@ -372,9 +430,9 @@ template <int D, bool ALONE>
 int run(const KernelArgs& args, const DenseParams& p) {
   using S = Shape<D, ALONE>;
   CUtensorMap map_q, map_k, map_v;
-  if (!make_map(&map_q, args.buffers[0], D, p.q_len, p.heads, p.batches, false) ||
-      !make_map(&map_k, args.buffers[1], D, p.k_len, p.kv_heads, p.batches, false) ||
-      !make_map(&map_v, args.buffers[2], D, p.k_len, p.kv_heads, p.batches, p.token_first_value != 0))
+  if (!make_map(&map_q, args.buffers[0], D, p.q_len, p.q_len, p.heads, p.batches, false) ||
+      !make_map(&map_k, args.buffers[1], D, p.k_len, seen_by_any(p), p.kv_heads, p.batches, false) ||
+      !make_map(&map_v, args.buffers[2], D, p.k_len, seen_by_any(p), p.kv_heads, p.batches, p.token_first_value != 0))
     return -1;
   auto kernel = dense_attention_tc_kernel<D, ALONE>;
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::kSharedBytes) != cudaSuccess) {
@@ -382,7 +440,7 @@ int run(const KernelArgs& args, const DenseParams& p) {
     return -1;
   }
   launch_kernel(args, kernel, dim3(p.heads, (p.q_len + kTile - 1u) / kTile, p.batches), dim3(S::kThreads), S::kSharedBytes, map_q, map_k,
-                map_v, (__half*)args.buffers[4], p, args.ctx ? context_device_error(args.ctx) : nullptr);
+                map_v, (const __half*)args.buffers[1], (const __half*)args.buffers[2], (__half*)args.buffers[4], p, args.ctx ? context_device_error(args.ctx) : nullptr);
   return check_launch(args);
 }
 

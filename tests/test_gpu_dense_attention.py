@@ -67,6 +67,51 @@ def test_dense_attention_tiles_of_128(runtime, oracle, b, h, kvh, ql, kl, d, cau
     assert_close_f16(got, want, label=f"dense attention d={d} q={ql} k={kl}")
 
 
+@pytest.mark.parametrize("b,h,kvh,ql,kl,past,d,causal,tfo,tfv", [
+    (1, 3, 1, 128, 128, 0, 64, 1, 1, 0),
+    (1, 2, 2, 300, 363, 63, 128, 1, 1, 1),
+    (2, 2, 1, 131, 400, 40, 64, 1, 0, 1),      # keys that no query sees yet: room of a cache
+    (1, 1, 1, 1, 260, 100, 128, 1, 1, 0),
+    (1, 2, 1, 70, 90, 0, 64, 0, 1, 0),         # every key is seen
+    (1, 130, 26, 300, 330, 30, 128, 1, 0, 0),  # two thread blocks share an SM
+    (1, 130, 26, 300, 400, 30, 64, 1, 1, 1),
+])
+def test_values_of_masked_keys_do_not_show(runtime, b, h, kvh, ql, kl, past, d, causal, tfo, tfv):
+    """Infinities and NaN behind keys that a query does not see leave its results as they are with numbers there, and results that do
+    see them are no numbers in the same places; keys behind the last query's need not even be initialised."""
+    from llmopt_b200 import parameters
+
+    rng = np.random.default_rng(23)
+    q, k = rng.standard_normal((b, h, ql, d)).astype(np.float16), rng.standard_normal((b, kvh, kl, d)).astype(np.float16)
+    v = rng.standard_normal((b, kl, kvh, d) if tfv else (b, kvh, kl, d)).astype(np.float16)
+    poisoned_k, poisoned_v = k.copy(), v.copy()
+    by_key = poisoned_v.swapaxes(1, 2) if tfv else poisoned_v  # [b, kvh, kl, d], a view
+    by_key[..., kl // 2, 5], by_key[..., kl * 3 // 4, d - 1], by_key[..., kl - 1, :d // 4] = np.inf, np.nan, -np.inf
+    if causal and kl > ql + past:
+        poisoned_k[..., ql + past:, :], by_key[..., ql + past:, :] = np.nan, np.nan
+
+    def run(keys, values):
+        out = _tensor(runtime, np.full((b, h, ql, d), np.nan, np.float16))
+        query = _tensor(runtime, q)
+        runtime.dispatch(f"llmopt_attention_f16_simd_h{d}",
+                         buffers=[query.buffer, _tensor(runtime, keys).buffer, _tensor(runtime, values).buffer, query.buffer, out.buffer],
+                         parameters=parameters.attention(batches=b, heads=h, query_length=ql, key_length=kl, head_dimension=d,
+                                                         mask_batches=0, mask_heads=0, causal=bool(causal), scale=d ** -0.5, kv_heads=kvh,
+                                                         token_first_output=tfo, past_length=past, token_first_value=tfv, mask_dtype=0))
+        got = out.buffer.to_numpy(np.float16, (b, ql, h, d) if tfo else (b, h, ql, d))
+        return got.swapaxes(1, 2) if tfo else got
+
+    clean, got = run(k, v), run(poisoned_k, poisoned_v)
+    seen = np.minimum(np.arange(ql) + past + 1, kl) if causal else np.full(ql, kl)
+    strange = np.zeros((b, kvh, ql, d), bool)  # a dimension of a query that sees such a value
+    for key, dimension in np.argwhere(~np.isfinite(by_key).all((0, 1))):
+        strange[:, :, seen > key, dimension] = True
+    strange = np.repeat(strange, h // kvh, axis=1)
+    assert np.isfinite(clean).all() and not np.isfinite(got[strange]).any()
+    # two roundings to half, of the result and of the weights: 2^-11 of a sum of at most 5 each
+    assert np.abs(got[~strange].astype(np.float64) - clean[~strange]).max() <= 10 * 2.0 ** -11
+
+
 @pytest.mark.parametrize("kind", ["bool", "float16"])
 def test_dense_attention_masks(runtime, oracle, kind):
     rng = np.random.default_rng(21)
