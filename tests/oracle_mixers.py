@@ -254,14 +254,15 @@ def capped(score, cap):
     return cap * np.tanh(score / cap) if cap else score
 
 
-def masked_attention(q, k, v, seen, scale, cap=None):
-    """q [T, H, dim], k [S, G, dim], v [S, G, vdim], seen [T, S]."""
+def masked_attention(q, k, v, seen, scale, cap=None, sink=False):
+    """q [T, H, dim], k [S, G, dim], v [S, G, vdim], seen [T, S]; ``sink``: one more score of zero in the denominator."""
     group = q.shape[1] // k.shape[1]
     out = np.zeros((*q.shape[:2], v.shape[2]))
     for h in range(q.shape[1]):
         score = np.where(seen, capped((q[:, h] @ k[:, h // group].T) * scale, cap), -np.inf)
-        weight = np.exp(score - score.max(axis=1, keepdims=True))
-        out[:, h] = weight / weight.sum(axis=1, keepdims=True) @ v[:, h // group]
+        top = np.maximum(score.max(axis=1, keepdims=True), 0.0 if sink else -np.inf)
+        weight = np.exp(score - top)
+        out[:, h] = weight / (weight.sum(axis=1, keepdims=True) + (np.exp(-top) if sink else 0.0)) @ v[:, h // group]
     return out
 
 

@@ -213,7 +213,7 @@ class WindowBench:
     """The attention kernel alone over scattered slots.  The whole sequence's keys and values lie in the cache from the
     start, so that a look into the future shows."""
 
-    def __init__(self, runtime, dtype, q, k, v, *, scale, window=None, keep_first=0, softcap=None, gates=None, weights32=True, seed=0):
+    def __init__(self, runtime, dtype, q, k, v, *, scale, window=None, keep_first=0, softcap=None, gates=None, weights32=True, sink=False, seed=0):
         from llmopt_b200.kv_cache import RowLayout
 
         rng = np.random.default_rng(seed)
@@ -233,11 +233,11 @@ class WindowBench:
         self.size = dict(heads=self.heads, kv_heads=self.kv_heads, dim=self.dim, vdim=self.vdim,
                          token_stride=layout.token_elements, key_offset=region.key_offset, value_offset=region.value_offset,
                          table_stride=tokens, table_rows=3, pool_rows=slots, scale=scale, softcap=softcap or 0.0,
-                         window=window or 0, keep_first=keep_first, sink=False, weights32=weights32)
+                         window=window or 0, keep_first=keep_first, sink=sink, weights32=weights32)
         places = np.arange(tokens)
         mask = {"size": window, "keep_first": keep_first} if window else None
         self.want = plain.masked_attention(*(a.astype(np.float64) for a in (q, k, v)), plain.visible_keys(places, places, mask), scale,
-                                           softcap)
+                                           softcap, sink)
         if gates is not None:
             self.want = self.want * plain.sigmoid(gates.astype(np.float64))
 
@@ -296,6 +296,20 @@ def test_prompts_whose_keys_are_shared_out(runtime, heads, first, total, softcap
     bench = WindowBench(runtime, "bfloat16", q, k, v, scale=0.13, window=150, keep_first=3, softcap=softcap,
                         gates=bf16_round(rng.standard_normal((total, heads, 128))))
     bench.check(first, total)
+
+
+@pytest.mark.parametrize("softcap", [None, 4.0])
+@pytest.mark.parametrize("heads,first,total", [(4, 0, 20), (4, 0, 33), (8, 100, 300), (48, 0, 640)])
+def test_a_sink_beside_keys_that_are_shared_out(runtime, heads, first, total, softcap):
+    """The sink enters after the groups' maxima have met: with all scores far below zero it takes nearly everything."""
+    rng = np.random.default_rng(total)
+    q = bf16_round(0.1 + np.abs(rng.standard_normal((total, heads, 128))) * 0.3)
+    k, v = bf16_round(-np.abs(rng.standard_normal((total, 1, 128))) * 0.5), bf16_round(1.0 + rng.random((total, 1, 128)))
+    for sign in (1.0, -1.0):  # far below and far above zero
+        for sink in (True, False):
+            bench = WindowBench(runtime, "bfloat16", q, k * sign, v, scale=0.3, window=150, keep_first=3, softcap=softcap, sink=sink,
+                                gates=bf16_round(rng.standard_normal((total, heads, 128))))
+            bench.check(first, total, label=f"{sign} {sink}")
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
