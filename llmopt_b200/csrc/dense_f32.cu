@@ -275,9 +275,11 @@ int run(const KernelArgs& args, DenseProblem p, uint32_t tiles) {
     const dim3 grid((p.n + Shape::kColumns - 1u) / Shape::kColumns, down(Shape::kRows));
     // Where every CTA finds an SM of its own none shares one: CTAs that start beside the last ones of the launch before double up
     // (2048 x 2048 x 100 rows 59 us, 41 this way).
-    const uint32_t bytes = (size_t)grid.x * grid.y <= sms && Shape::kBytes < kOnePerSm ? kOnePerSm : Shape::kBytes;
-    // per device and kernel; cheap beside the launch, and remembered nowhere
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
+    constexpr uint32_t kMostBytes = Shape::kBytes > kOnePerSm ? Shape::kBytes : kOnePerSm;
+    const uint32_t bytes = (size_t)grid.x * grid.y <= sms ? kMostBytes : Shape::kBytes;
+    // Per device and kernel; cheap beside the launch, and remembered nowhere.  Always the most: another thread may be between this call
+    // and its launch.
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMostBytes) != cudaSuccess)
       return fail(args, "shared memory could not be raised");
     launch_kernel(args, kernel, grid, dim3(Shape::kThreads), bytes, task, p.plan);
     return check_launch(args);

@@ -97,6 +97,43 @@ def test_fp32_products_in_tiles_of_every_width(runtime, m, n, k):
     close(results[0], x.astype(np.float64) @ w[:n].T.astype(np.float64), 1e-5, "narrow")
 
 
+def test_fp32_products_of_two_threads():
+    """One kernel of 128 and of 296 thread blocks, launched by two threads with a runtime of their own: what a launch asks an SM for is
+    nobody else's."""
+    import threading
+
+    from llmopt_b200 import parameters
+    from llmopt_b200.cuda_native import Batch, DispatchItem, Runtime
+
+    start, wrong = threading.Barrier(2), []
+
+    def work(m, n, k):
+        try:
+            runtime = Runtime(0)
+            rng = np.random.default_rng(m)
+            x, w = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
+            out, nothing = empty(runtime, m * n), empty(runtime, 16)
+            item = DispatchItem("llmopt_dense_linear_f32", [upload(runtime, x), upload(runtime, w), nothing, nothing, out, nothing, nothing],
+                                parameters.dense_linear(m=m, n=n, k=k, split=0, has_bias=False, epilogue=None, table_rows=0,
+                                                        table_stride=0, table_offset=0))
+            start.wait()
+            for _ in range(30):
+                commands = Batch(runtime)
+                for _ in range(100):
+                    commands.dispatch_item(item)
+                commands.commit()
+            close(download(out, (m, n)), x.astype(np.float64) @ w.T.astype(np.float64), 1e-5, str(m))
+        except Exception as error:  # an assertion of another thread would go unnoticed
+            wrong.append((m, repr(error)))
+
+    threads = [threading.Thread(target=work, args=shape) for shape in ((100, 2048, 32), (40, 9472, 32))]
+    for thread in threads:
+        thread.start()
+    for thread in threads:
+        thread.join()
+    assert wrong == []
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("width", [97, 104, 192, 1028, 4096, 8192, 9000])
 def test_residual_norm(runtime, dtype, width):
