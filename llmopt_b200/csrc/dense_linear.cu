@@ -261,7 +261,8 @@ int run_gemv(const KernelArgs& args, DenseProblem p, DenseStore store) {
   return with_store(store, [&](auto constant) {
     constexpr DenseStore STORE = decltype(constant)::value;
     auto run_wide = [&](auto kernel, uint32_t bytes, uint32_t most_per_sm) {
-      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
+      // the most that any launch of it asks for: another thread's may be under way
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWideMost) != cudaSuccess) {
         cudaGetLastError();
         return fail(args, "shared memory request was refused");
       }

@@ -377,7 +377,8 @@ int run_step(const KernelArgs& args, DenseProblem p, const uint32_t* route, cons
     // 4.6 us, 5.2 persistent; 4 rows, 512 tiles, 6.2 and 5.8)
     const uint32_t pairs = p.m * top, route_bytes = ((2u * most + 1u) * 4u + pairs + 15u) / 16u * 16u;
     auto run_wide = [&](auto kernel, uint32_t bytes) {
-      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
+      // the most that any launch of it asks for: another thread's may be under way
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWideMost) != cudaSuccess) {
         cudaGetLastError();
         return fail(args, "shared memory request was refused");
       }

@@ -871,15 +871,20 @@ int run_rows(const KernelArgs& args, const RowAttentionParams& p) {
   return check_launch(args);
 }
 
+// Head size up to which tensor cores are used.  The limit of a kernel's shared memory is set for it whatever a launch asks for:
+// another thread's may be under way.
+constexpr uint32_t kWidestHead = 256;
+
 template <int DK, int DV, bool EXTENDED, uint32_t GROUPS>
 int run_prompt_groups(const KernelArgs& args, const RowAttentionParams& p) {
   const uint32_t padded = DK > 0 ? DK : round16(p.dim);
   constexpr uint32_t kKeyTile = key_tile(DK, EXTENDED), kGroups = GROUPS;
-  const uint32_t bytes = (kQueryTile * (padded + 8u) + kGroups * 2u * kKeyTile * (padded + 8u + DV + 8u)) * 2u;
+  auto bytes_of = [](uint32_t width) { return (kQueryTile * (width + 8u) + kGroups * 2u * kKeyTile * (width + 8u + DV + 8u)) * 2u; };
+  const uint32_t bytes = bytes_of(padded);
   static_assert(kGroups == 1u || kGroups * (4u + DV / 2u) * 512u <= (kQueryTile * (DK + 8u) + kGroups * 2u * kKeyTile * (DK + DV + 16u)) * 2u,
                 "the groups' results take the tiles' place");
   auto kernel = attention_prompt_kernel<DK, DV, EXTENDED, GROUPS>;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes_of(DK > 0 ? DK : kWidestHead)) != cudaSuccess) {
     cudaGetLastError();
     return -1;
   }
@@ -908,15 +913,18 @@ int run_prompt(const KernelArgs& args, const RowAttentionParams& p) {
 template <int DK, int DV, bool EXTENDED, uint32_t STAGES>
 int run_decode_stages(const KernelArgs& args, const RowAttentionParams& p) {
   const uint32_t padded = DK > 0 ? DK : round16(p.dim);
-  uint32_t bytes = (16u * (padded + 8u) + kDecodeWarps * STAGES * kWarpKeys * (padded + 8u + DV + 8u)) * 2u;
-  const uint32_t merge = kDecodeWarps * record_floats<DV>() * 4u;
-  if (bytes < merge) bytes = merge;
+  auto bytes_of = [](uint32_t width) {
+    const uint32_t rings = (16u * (width + 8u) + kDecodeWarps * STAGES * kWarpKeys * (width + 8u + DV + 8u)) * 2u;
+    const uint32_t merge = kDecodeWarps * record_floats<DV>() * 4u;
+    return rings < merge ? merge : rings;
+  };
+  const uint32_t bytes = bytes_of(padded);
   const size_t heads = (size_t)p.sequences * p.kv_heads, counters = (heads * 4 + 255) / 256 * 256;
   LLMOPT_REQUIRE(p.splits <= kMostSplits, "at most 64 splits");
   LLMOPT_REQUIRE(p.splits == 1u || args.lengths[6] >= counters + heads * p.splits * record_floats<DV>() * 4,
                  "split scratch is too short");
   auto kernel = attention_decode_kernel<DK, DV, EXTENDED, STAGES>;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) {
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes_of(DK > 0 ? DK : kWidestHead)) != cudaSuccess) {
     cudaGetLastError();
     return -1;
   }
@@ -979,7 +987,7 @@ int launch_row_attention(const KernelArgs& args) {
                      args.lengths[3] >= (size_t)p.sequences * 4 && args.lengths[4] >= (size_t)p.sequences * 4,
                  "buffer is too short");
   if (rows == 0) return 0;
-  const bool vectors = e == 2 && p.dim % 8u == 0 && p.vdim % 8u == 0 && p.dim <= 256u && p.vdim <= 256u &&
+  const bool vectors = e == 2 && p.dim % 8u == 0 && p.vdim % 8u == 0 && p.dim <= kWidestHead && p.vdim <= 256u &&
                        p.query_stride % 8u == 0 && p.query_column % 8u == 0 && p.token_stride % 8u == 0 && p.key_offset % 8u == 0 && p.value_offset % 8u == 0 &&
                        ((uintptr_t)args.buffers[0] & 15u) == 0 && ((uintptr_t)args.buffers[1] & 15u) == 0;
   if (vectors) {

@@ -462,8 +462,9 @@ int launch_one(const KernelArgs& args, const GemvProblem& p) {
   if (AFFINE) shared_bytes += (size_t)p.x_rows * (p.k / 64) * sizeof(float);
   auto kernel = w4a16_gemv_kernel<NT, NMAT, EPI, AFFINE>;
   if (shared_bytes > 48 * 1024) {
-    if (shared_bytes > 200 * 1024) return fail(args, "shape needs more shared memory than one CTA has");
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared_bytes);
+    constexpr int kMost = 200 * 1024;  // of any launch: another thread's may be under way
+    if (shared_bytes > kMost) return fail(args, "shape needs more shared memory than one CTA has");
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
   }
   const uint32_t resident = (uint32_t)context_sm_count(args.ctx) * 3u;
   const uint32_t ctas = wanted < resident ? wanted : resident;

@@ -672,6 +672,8 @@ inline bool wide_forms_at_two_ctas() {
   return two;
 }
 
+constexpr size_t kSharedPerSm = 220 * 1024;  // usable shared memory of one SM
+
 template <int NT, int NMAT, int EPI, bool SMALLX, int GPW>
 bool plan_pipe(const KernelArgs& args, const GemvProblem& p, PipePlan* plan) {
   uint32_t total_tiles = 0;
@@ -682,7 +684,6 @@ bool plan_pipe(const KernelArgs& args, const GemvProblem& p, PipePlan* plan) {
   if (SMALLX) fixed_bytes += (size_t)groups * 2 * p.x_rows * 4 * 16 + 16 + (size_t)(p.x_rows * groups + 4) * sizeof(float);
   const size_t stage_bytes = (size_t)NMAT * Stage<GPW>::kBytes + 16;
   const uint32_t sms = (uint32_t)context_sm_count(args.ctx);
-  constexpr size_t kSharedPerSm = 220 * 1024;  // usable shared memory of one SM
   const uint32_t chunks_per_tile = p.k / Stage<GPW>::kChunkK;
   // a fourth resident CTA only where the kernel was compiled for it and every CTA still gets four tiles
   uint32_t most = kDenseResidency<NT, EPI> == 4 && total_tiles >= 16u * sms ? 4u : 3u;
@@ -730,7 +731,8 @@ int run_pipe(const KernelArgs& args, const GemvProblem& p, const PipePlan& plan)
     kernel = w4a16_gemv_pipe_kernel<NT, NMAT, EPI, SMALLX, GPW, kSparse>;
   else if (NT > 1 && wide_forms_at_two_ctas())
     kernel = w4a16_gemv_pipe_kernel<NT, NMAT, EPI, SMALLX, GPW, (NT > 1 ? 2 : kDense)>;
-  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.shared_bytes) != cudaSuccess) {
+  // the most that any plan asks for: another thread's launch may be under way
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSharedPerSm) != cudaSuccess) {
     cudaGetLastError();
     return -1;
   }

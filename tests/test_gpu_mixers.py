@@ -97,36 +97,75 @@ def test_fp32_products_in_tiles_of_every_width(runtime, m, n, k):
     close(results[0], x.astype(np.float64) @ w[:n].T.astype(np.float64), 1e-5, "narrow")
 
 
-def test_fp32_products_of_two_threads():
-    """One kernel of 128 and of 296 thread blocks, launched by two threads with a runtime of their own: what a launch asks an SM for is
-    nobody else's."""
+def _launches_of(kind, second, runtime):
+    """(item, output) of a kernel that takes more or less shared memory by what it is called with."""
+    from llmopt_b200 import dispatch, parameters
+    from llmopt_b200.cuda_native import Batch, DispatchItem
+
+    rng = np.random.default_rng(second)
+    nothing = empty(runtime, 16)
+    if kind == "fp32 tiles":  # 128 and 296 thread blocks
+        m, n, k, dtype = (40, 9472, 32, "float32") if second else (100, 2048, 32, "float32")
+    elif kind == "bf16 rows":
+        m, n, k, dtype = (8, 4800, 4096, "bfloat16") if second else (8, 2400, 2048, "bfloat16")
+    elif kind == "w4a16 rows":
+        k = 4096 if second else 1024
+        tensor = lambda array, dtype: dispatch.Tensor(upload(runtime, array), array.shape, dtype)
+        out = dispatch.Tensor(empty(runtime, 2 * 2048, "bfloat16"), (2, 2048), "float16")
+        commands = Batch(runtime)
+        dispatch.dispatch_w4a16_linear(dispatch.Context(runtime, batch=commands), input=tensor(rng.standard_normal((2, k)).astype(np.float16), "float16"),
+                                       weight=tensor(rng.integers(0, 256, (2048, k // 2), dtype=np.uint8), "uint8"),
+                                       scale=tensor(rng.uniform(0.01, 0.02, (2048, k // 64)).astype(np.float16), "float16"), output=out)
+        item = commands.pending[0]
+        commands.abort()
+        return item, out.buffer
+    else:  # row attention of prompts and of single tokens
+        dim, tokens = 256 if second else 136, 40 if kind == "prompts' attention" else 1
+        out = empty(runtime, tokens * dim * 2, "bfloat16")
+        query, pool = (upload(runtime, rng.standard_normal(size).astype(np.float32), "bfloat16") for size in ((tokens, 2 * dim), (64, 2 * dim)))
+        return DispatchItem("llmopt_row_attention_bf16",
+                            [query, pool, upload(runtime, np.arange(64, dtype=np.uint32)), upload(runtime, np.array([64 - tokens], np.uint32)),
+                             upload(runtime, np.zeros(1, np.uint32)), out, nothing, query],
+                            parameters.row_attention(sequences=1, tokens=tokens, heads=2, kv_heads=1, dim=dim, vdim=dim, token_stride=2 * dim,
+                                                     key_offset=0, value_offset=dim, table_stride=64, table_rows=1, pool_rows=64, sink=False,
+                                                     splits=1, scale=0.1)), out
+    x, w = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
+    out = empty(runtime, m * n)
+    return DispatchItem("llmopt_dense_linear_" + suffix(dtype), [upload(runtime, x, dtype), upload(runtime, w, dtype), nothing, nothing, out, nothing, nothing],
+                        parameters.dense_linear(m=m, n=n, k=k, split=0, has_bias=False, epilogue=None, table_rows=0, table_stride=0,
+                                                table_offset=0)), out
+
+
+@pytest.mark.parametrize("kind", ["fp32 tiles", "bf16 rows", "w4a16 rows", "prompts' attention", "a token's attention"])
+def test_launches_of_two_threads(kind):
+    """Two threads with a runtime of their own launch one kernel: what a launch asks an SM for is nobody else's."""
     import threading
 
-    from llmopt_b200 import parameters
-    from llmopt_b200.cuda_native import Batch, DispatchItem, Runtime
+    from llmopt_b200.cuda_native import Batch, Runtime
 
     start, wrong = threading.Barrier(2), []
 
-    def work(m, n, k):
+    def work(second):
         try:
             runtime = Runtime(0)
-            rng = np.random.default_rng(m)
-            x, w = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((n, k)).astype(np.float32)
-            out, nothing = empty(runtime, m * n), empty(runtime, 16)
-            item = DispatchItem("llmopt_dense_linear_f32", [upload(runtime, x), upload(runtime, w), nothing, nothing, out, nothing, nothing],
-                                parameters.dense_linear(m=m, n=n, k=k, split=0, has_bias=False, epilogue=None, table_rows=0,
-                                                        table_stride=0, table_offset=0))
-            start.wait()
-            for _ in range(30):
+            item, out = _launches_of(kind, second, runtime)
+
+            def run(count):
                 commands = Batch(runtime)
-                for _ in range(100):
+                for _ in range(count):
                     commands.dispatch_item(item)
                 commands.commit()
-            close(download(out, (m, n)), x.astype(np.float64) @ w.T.astype(np.float64), 1e-5, str(m))
-        except Exception as error:  # an assertion of another thread would go unnoticed
-            wrong.append((m, repr(error)))
+                return out.to_numpy(np.uint8)
 
-    threads = [threading.Thread(target=work, args=shape) for shape in ((100, 2048, 32), (40, 9472, 32))]
+            alone = run(1)
+            start.wait()
+            for _ in range(30):
+                assert np.array_equal(run(100), alone)
+        except Exception as error:  # an assertion of another thread would go unnoticed
+            wrong.append((second, repr(error)))
+            start.abort()
+
+    threads = [threading.Thread(target=work, args=(second,)) for second in (0, 1)]
     for thread in threads:
         thread.start()
     for thread in threads:
