@@ -261,7 +261,8 @@ dense_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
     auto of_row = [&](uint32_t parity, uint32_t of_half) -> float& { return exchange[(parity * 2u + of_half) * kTile + row]; };
     auto halves_sync = [] { asm volatile("bar.sync 1, 256;" ::: "memory"); };
     const float scale = p.scale * 1.4426950408889634f;
-    float top = kLowest, total = 0.0f;  // in units of log2 e
+    float top = kLowest;  // in units of log2 e
+    float of_halves[3u - S::kHalves] = {};  // denominators; a tile's halves apart in either form, which gives both the same bits
     bool ok = true;
     for (uint32_t tile = 0; tile < tiles; ++tile) {
       const uint32_t which = tile % S::kScores, k0 = tile * kTile + half * S::kKeys;
@@ -299,7 +300,8 @@ dense_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
       if (__any_sync(0xffffffffu, grown)) {
         const float keep = grown ? exp2_fast(top - most) : 1.0f;
         if (grown) top = most;
-        total *= keep;
+#pragma unroll
+        for (float& part : of_halves) part *= keep;
         if (tile > 0) {
           if (ALONE) {  // P V of the tile before may still be under way
             ok = __all_sync(0xffffffffu, barrier_wait(sums_full, (tile - 1u) & 1u));
@@ -334,7 +336,7 @@ dense_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
           two[1] += rounded.y;
           weights[i] = *reinterpret_cast<const uint32_t*>(&pair);
         }
-        total += two[0] + two[1];
+        of_halves[ALONE ? 0u : part / 2u] += two[0] + two[1];
         tmem_store_16(mine + part * 16u, weights);  // over scores that are in registers
       }
       // A wait names a phase by its parity, so nobody may be two phases behind: with two tiles of scores a row could be done with this
@@ -346,8 +348,9 @@ dense_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
       __syncwarp();
       if (lane == 0) barrier_arrive(weights_full);
     }
+    float total = of_halves[0] + of_halves[2u - S::kHalves];
     if (ALONE) {
-      of_row(tiles & 1u, half) = total;
+      of_row(tiles & 1u, half) = of_halves[0];
       halves_sync();
       total = of_row(tiles & 1u, 0) + of_row(tiles & 1u, 1);
     }

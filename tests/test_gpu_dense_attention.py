@@ -67,6 +67,20 @@ def test_dense_attention_tiles_of_128(runtime, oracle, b, h, kvh, ql, kl, d, cau
     assert_close_f16(got, want, label=f"dense attention d={d} q={ql} k={kl}")
 
 
+@pytest.mark.parametrize("ql,kl,d,causal,growth", [(520, 520, 64, True, 0.02), (520, 600, 128, True, 0.3), (500, 333, 128, False, 0.02)])
+def test_heads_alone_and_among_many(runtime, ql, kl, d, causal, growth):
+    """Few heads have an SM for each tile of queries, two threads a row and two tiles of scores, many share: the same bits."""
+    rng = np.random.default_rng(24)
+    q = rng.standard_normal((1, 4, ql, d)).astype(np.float16)
+    k = (rng.standard_normal((1, 2, kl, d)) * np.minimum(1.0 + growth * np.arange(kl), 12.0)[:, None]).astype(np.float16)
+    v = rng.standard_normal((1, 2, kl, d)).astype(np.float16)
+    few = _attention(runtime, q, k, v, causal=causal, scale=d ** -0.5)
+    many = _attention(runtime, *(np.tile(x, (1, 30, 1, 1)) for x in (q, k, v)), causal=causal, scale=d ** -0.5)
+    assert np.isfinite(few).all()
+    for copy in range(30):
+        assert np.array_equal(many[0, 4 * copy:4 * copy + 4].view(np.uint16), few[0].view(np.uint16))
+
+
 @pytest.mark.parametrize("b,h,kvh,ql,kl,past,d,causal,tfo,tfv", [
     (1, 3, 1, 128, 128, 0, 64, 1, 1, 0),
     (1, 2, 2, 300, 363, 63, 128, 1, 1, 1),
