@@ -5,15 +5,16 @@
 // and issues tcgen05.mma: S = Q K^T into tensor memory (128 columns), later O += P V (D columns).  Warps of rows read S and write
 // P = exp2(S - top) over it as fp16 pairs, the A operand of P V in tensor memory; V is the B operand as it lies in memory,
 // dimensions contiguous.  O stays in tensor memory; it is scaled only when a row's maximum has grown by more than 2^kSlack since it
-// was last scaled: weights of up to 2^kSlack are as exact in fp16, and the denominator adds what P V uses.
+// was last scaled: weights of up to 2^kSlack are as exact in fp16, and the denominator adds what P V uses (rescaling put off in this
+// way was published with FlashAttention-4, 2025).
 //
 // What bounds a tile is the chain from S to P (16 exponentials a cycle and SM are its floor), so two of them run side by side,
-// in one of two forms:
+// in one of two forms, of which both give the same bits:
 //  * ALONE: one CTA per SM, two threads per row, and the next tile's scores multiplied beside this tile's exponentials;
 //  * otherwise two CTAs share an SM, a thread per row.
-// Up to two and a half CTAs per SM the first is faster, where rows are short in tiles or CTAs few: us with 64 x 64 tiles on mma.sync,
-// two per SM, ALONE: 9 heads of 64, 60 tokens 7.4, 8.8, 6.4; 300 9.5, 11.7, 7.9; 2048 47.6, 39.7, 25.2; 16 heads of 128, 2048
-// tokens 75.6, 48.5, 30.4; 32 heads 1000 tokens 45, 26.1, 19.8; 1400 - , 34.7, 33.2; 1650 - , 38.1, 43.2; 2048 143, 51.0, 60.6.
+// Up to two CTAs per SM the first is faster or as fast, beyond the second, with either head size.  us, causal, back to back over six sets of
+// operands, CTAs and then two per SM, ALONE: heads of 64: 9 5.4, 5.0; 144 33.1, 25.0; 256 18.8, 17.2; 288 20.8, 19.7; 320 23.4, 25.9; 512
+// 42.5, 55.1.  Of 128: 128 21.5, 15.7; 256 22.8, 22.7; 288 25.7, 25.8; 320 28.9, 32.7; 352 31.4, 37.0; 512 49.8, 63.7.
 // K and V two tiles deep changed nothing: their way hides behind the exponentials.
 //
 // Rows beyond a head's keys or queries are zero-filled by TMA.  Every wait on an mbarrier is bounded; a wait that runs out raises
@@ -456,7 +457,7 @@ int launch_attention_dense_tc(const KernelArgs& args, const DenseParams& p) {
   for (int i = 0; i < 5; ++i)
     if (i != 3 && ((uintptr_t)args.buffers[i] & 15u)) return -1;
   const size_t ctas = (size_t)p.heads * ((p.q_len + kTile - 1u) / kTile) * p.batches;
-  const bool alone = 2u * ctas <= 5u * (size_t)context_sm_count(args.ctx);
+  const bool alone = ctas <= 2u * (size_t)context_sm_count(args.ctx);
   if (p.dim == 64u) return alone ? run<64, true>(args, p) : run<64, false>(args, p);
   return alone ? run<128, true>(args, p) : run<128, false>(args, p);
 }
