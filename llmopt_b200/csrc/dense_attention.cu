@@ -9,8 +9,8 @@
 //   nonzero byte keeps it (llmopt_attention_allowed, lib/metal_attention_source.ml:257-274).
 //
 // Kernels behind the names:
-//  * D in {64, 128} without a mask: dense_attention_tc.cu, on tcgen05.
-//  * D in {64, 128} otherwise: a flash-attention forward pass on mma.sync.m16n8k16: one CTA per 64 queries
+//  * D in {64, 128} without a mask, a positive scale and 16-byte aligned buffers: dense_attention_tc.cu, on tcgen05.
+//  * D in {64, 128} otherwise (a mask, another scale, an output aligned to 4 bytes): a flash-attention forward pass on mma.sync.m16n8k16: one CTA per 64 queries
 //    of one (batch, head), four warps of 16 query rows; K and V tiles staged in padded shared
 //    memory; S = Q K^T with K rows as the col-major B operand (ldmatrix), online softmax in
 //    fp32 per row (units of log2 e), P rounded to half before P V like the reference's SIMD
@@ -83,7 +83,7 @@ __device__ __forceinline__ void copy_async_16(void* shared_target, const void* s
 // shared memory and fetched with cp.async one tile ahead of the arithmetic; a tile every key of which
 // every query row of the warp may see (no mask, inside the causal triangle, inside k_len) skips the
 // per-element visibility test.
-template <int D, int KT>
+template <int D, int KT, bool BY_HEAD>
 __global__ void __launch_bounds__(128) dense_attention_mma_kernel(const __half* __restrict__ query,
                                                                   const __half* __restrict__ key,
                                                                   const __half* __restrict__ value,
@@ -96,8 +96,9 @@ __global__ void __launch_bounds__(128) dense_attention_mma_kernel(const __half* 
   Row* q_tile = reinterpret_cast<Row*>(dense_shared);                 // [kQueryTile]
   Row* k_tiles = q_tile + kQueryTile;                                  // [2][KT]
   Row* v_tiles = k_tiles + 2 * KT;                                     // [2][KT]
-  // the last query tiles see the most keys under a causal mask: they are scheduled first, over all heads
-  const uint32_t q0 = (gridDim.y - 1u - blockIdx.y) * kQueryTile, head = blockIdx.x, batch = blockIdx.z;
+  // the last query tiles see the most keys under a causal mask: they are scheduled first, of each head (BY_HEAD) or over all heads
+  const uint32_t q0 = (BY_HEAD ? gridDim.x - 1u - blockIdx.x : gridDim.y - 1u - blockIdx.y) * kQueryTile;
+  const uint32_t head = BY_HEAD ? blockIdx.y : blockIdx.x, batch = blockIdx.z;
   const uint32_t kv_head = head / (p.heads / p.kv_heads);
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, r = lane >> 2, c = lane & 3u;
   constexpr int kChunks = D / 8;  // 16-byte chunks per row
@@ -344,18 +345,24 @@ int launch_attention_dense(const KernelArgs& args) {
   const bool aligned = p.q_len <= 65535u * kQueryTile &&  // a grid's second dimension
                        (((uintptr_t)args.buffers[0] | (uintptr_t)args.buffers[1] | (uintptr_t)args.buffers[2]) & 15u) == 0 &&
                        ((uintptr_t)args.buffers[4] & 3u) == 0;
-  const dim3 grid(p.heads, (p.q_len + kQueryTile - 1) / kQueryTile, p.batches);
-  auto shared_bytes = [](uint32_t dim, uint32_t keys) { return (size_t)(kQueryTile + 4 * keys) * (dim + 8) * sizeof(__half); };
+  // Over all heads pays where CTAs wait for others to end, elsewhere the heads' own order is the faster; four CTAs start at once on an SM with
+  // heads of 64, two with heads of 128.  With a mask, us, by head and over all: heads of 64: 4 heads, 500 tokens (32 CTAs) 38.9, 43.3; 16, 1000
+  // (256) 74.9, 82.5; 32, 1000 (512) 77.8, 82.8; 16, 2048 (512) 110.9, 106.3; 32, 1400 (704) 108.6, 115.2; 24, 2048 (768) 142, 117;
+  // 32, 2048 (1024) 175, 130.  Of 128: 16, 1000 (256) 87.6, 96.0; 16, 1400 (352) 119.6, 130.6; 16, 1700 (432) 163, 148; 32, 1000 (512) 125, 99.
+  const uint32_t query_tiles = (p.q_len + kQueryTile - 1) / kQueryTile;
+  const size_t together = args.ctx == nullptr ? 0u : (size_t)context_sm_count(args.ctx) * (p.dim == 64u ? 4u : 2u);
+  const bool by_head = 4u * (size_t)query_tiles * p.heads * p.batches <= 5u * together;
+  const dim3 grid(by_head ? query_tiles : p.heads, by_head ? p.heads : query_tiles, p.batches);
+  auto launch = [&](auto kernel) {
+    const size_t shared = (size_t)(kQueryTile + 4 * 64) * (p.dim + 8) * sizeof(__half);
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+    launch_kernel(args, kernel, grid, dim3(128), shared, (const __half*)args.buffers[0], (const __half*)args.buffers[1],
+                  (const __half*)args.buffers[2], mask, (__half*)args.buffers[4], p);
+  };
   if (aligned && p.dim == 64) {
-    auto kernel = dense_attention_mma_kernel<64, 64>;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared_bytes(64, 64));
-    launch_kernel(args, kernel, grid, dim3(128), shared_bytes(64, 64), (const __half*)args.buffers[0],
-                  (const __half*)args.buffers[1], (const __half*)args.buffers[2], mask, (__half*)args.buffers[4], p);
+    by_head ? launch(dense_attention_mma_kernel<64, 64, true>) : launch(dense_attention_mma_kernel<64, 64, false>);
   } else if (aligned && p.dim == 128) {
-    auto kernel = dense_attention_mma_kernel<128, 64>;
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared_bytes(128, 64));
-    launch_kernel(args, kernel, grid, dim3(128), shared_bytes(128, 64), (const __half*)args.buffers[0],
-                  (const __half*)args.buffers[1], (const __half*)args.buffers[2], mask, (__half*)args.buffers[4], p);
+    by_head ? launch(dense_attention_mma_kernel<128, 64, true>) : launch(dense_attention_mma_kernel<128, 64, false>);
   } else {
     const size_t rows = (size_t)p.batches * p.heads * p.q_len;
     launch_kernel(args, dense_attention_rows_kernel, dim3((uint32_t)((rows + 7) / 8)), dim3(256), 0,

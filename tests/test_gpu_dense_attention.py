@@ -126,6 +126,41 @@ def test_values_of_masked_keys_do_not_show(runtime, b, h, kvh, ql, kl, past, d, 
     assert np.abs(got[~strange].astype(np.float64) - clean[~strange]).max() <= 10 * 2.0 ** -11
 
 
+@pytest.mark.parametrize("why", ["mask", "scale", "address"])
+@pytest.mark.parametrize("b,h,kvh,ql,kl,d,causal,tfo,tfv", [
+    (1, 3, 1, 64, 64, 64, True, True, False),      # one whole tile
+    (2, 4, 2, 65, 129, 128, True, False, True),    # one row more, cached keys, values token first
+    (1, 8, 2, 333, 400, 64, True, True, True),     # several tiles of queries, by head
+    (1, 6, 3, 260, 130, 128, True, True, False),   # keys that end before the queries
+    (1, 2, 1, 200, 90, 64, False, False, False),
+    (3, 40, 8, 250, 250, 128, True, True, True),   # more thread blocks than start at once: over all heads
+    (2, 60, 20, 389, 420, 64, True, False, False),
+])
+def test_dense_attention_beside_the_tensor_memory_form(runtime, oracle, b, h, kvh, ql, kl, d, causal, tfo, tfv, why):
+    """What a mask, a negative scale or an output that is aligned to four bytes only takes to the mma.sync kernel."""
+    from llmopt_b200 import dispatch
+    from llmopt_b200.cuda_native import Buffer
+
+    rng = np.random.default_rng(25)
+    q = rng.standard_normal((b, h, ql, d)).astype(np.float16)
+    k = rng.standard_normal((b, kvh, kl, d)).astype(np.float16)
+    v = rng.standard_normal((b, kl, kvh, d) if tfv else (b, kvh, kl, d)).astype(np.float16)
+    scale = float(np.float32((-1.0 if why == "scale" else 1.0) / np.sqrt(d)))
+    mask = (rng.random((1, 1, ql, kl)) > 0.2).astype(np.uint8) if why == "mask" else None
+    shape, shift = (b, ql, h, d) if tfo else (b, h, ql, d), 4 if why == "address" else 0
+    room = Buffer.of_array(runtime, np.full(2 * q.size + 16, 0xff, np.uint8))
+    out = room.view(shift, 2 * q.size)
+    dispatch.dispatch_attention(_ctx(runtime), causal=causal, scale=scale, query=_tensor(runtime, q), key=_tensor(runtime, k),
+                                value=_tensor(runtime, v), output=dispatch.Tensor(out, shape, "float16"),
+                                mask=None if mask is None else _tensor(runtime, mask, "bool"))
+    want = oracle.attention_dense(q, k, v, mask, causal=int(causal), scale=scale, kv_heads=kvh, token_first_output=int(tfo),
+                                  past_length=max(0, kl - ql), token_first_value=int(tfv), mask_dtype=1,
+                                  mask_batches=0 if mask is None else 1, mask_heads=1)
+    assert_close_f16(out.to_numpy(np.float16, shape), want, label=f"{why} d={d} q={ql} k={kl}")
+    rest = room.to_numpy(np.uint8)
+    assert (rest[:shift] == 0xff).all() and (rest[shift + 2 * q.size:] == 0xff).all()
+
+
 @pytest.mark.parametrize("kind", ["bool", "float16"])
 def test_dense_attention_masks(runtime, oracle, kind):
     rng = np.random.default_rng(21)
