@@ -646,6 +646,13 @@ paged_merge_kernel(const __half* __restrict__ query, const __half* __restrict__ 
 struct ClusterPlan {
   uint32_t ctas, warps;
 };
+constexpr ClusterPlan kClusterForms[] = {{2u, 4u}, {4u, 4u}, {8u, 4u}, {8u, 8u}};
+constexpr bool every_record_is_merged() {
+  for (const ClusterPlan& form : kClusterForms)
+    if (form.ctas > kMostClusterCtas) return false;
+  return true;
+}
+static_assert(every_record_is_merged(), "the merge of a cluster reads kMostClusterCtas records");
 
 template <int D, int GROUP, int CP, int WARPS, bool CLUSTER>
 int launch_split_copy(const KernelArgs& args, const PagedParams& p, uint32_t slot_batch_stride, float* scratch,
@@ -723,8 +730,7 @@ ClusterPlan pick_cluster(const KernelArgs& args, const PagedParams& p, uint32_t 
   auto cost_of = [&](float count, float share) { return fminf(count, kMostWaves) * kWave + count * share; };
   float least = kMerge + kRecord * (float)splits + cost_of(record_waves, (float)longest / (float)splits);
   ClusterPlan best = {0u, 0u};
-  const ClusterPlan forms[] = {{2u, 4u}, {4u, 4u}, {8u, 4u}, {8u, 8u}};
-  for (const ClusterPlan& form : forms) {
+  for (const ClusterPlan& form : kClusterForms) {
     const float rate = (float)form.warps / (float)kWarps;
     const float form_waves = waves(pairs * form.ctas, (size_t)((float)resident * 0.9f / rate));
     if (form.warps > (uint32_t)kWarps && form_waves > 1.0f) continue;
