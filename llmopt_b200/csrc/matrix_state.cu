@@ -669,8 +669,12 @@ __global__ void __launch_bounds__(ScanThreads<MEMORY, FORM>::kAll) scan_kernel(c
           const ulonglong2* k = reinterpret_cast<const ulonglong2*>(chunk.k[t]) + part;
           const float4 scalar = chunk.scalar[t];
           float values[kOwn];
-          if constexpr (kOwn == 2) *reinterpret_cast<float2*>(values) = *reinterpret_cast<const float2*>(&chunk.v[t][column0 % kScanColumns]);
-          else values[0] = chunk.v[t][column0 % kScanColumns];
+          if constexpr (kOwn == 2) {
+            const float2 two = *reinterpret_cast<const float2*>(&chunk.v[t][column0 % kScanColumns]);
+            values[0] = two.x, values[1] = two.y;
+          } else {
+            values[0] = chunk.v[t][column0 % kScanColumns];
+          }
           const Pair keep2 = pair_of(scalar.x, scalar.x);
           Pair kk[R4 * 2];
 #pragma unroll
