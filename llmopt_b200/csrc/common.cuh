@@ -46,6 +46,7 @@ struct KernelArgs {
   const FusedNorm* fused_norm;  // null unless the plan builder folded a norm into this dispatch
   // null unless the plan builder handed the rotary + cache pack of the new token to this (attention) dispatch
   const struct RotaryPackFusion* rotary_fusion;
+  bool in_plan;  // captured into a plan, which replays it
   bool apart;  // this launch starts when its predecessor has ended, also where overlap is allowed
 };
 

@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(kGemvWarps * 32, NT <= 4 ? 2 : 1) dense_gemv_k
       stage[2 + half] = present ? load_stream(w_high + k) : zero;
     }
   };
-  // the weights are nobody's output: their first blocks may be requested before the predecessor ends
+  // the weights are nobody's output: where the launch may start early their first blocks are requested before the predecessor ends
 #pragma unroll
   for (int s = 0; s < kGemvStages; ++s) fetch(a[s], rank * kGemvWarps + warp + s * stride);
   grid_dependency_wait();
@@ -286,12 +286,15 @@ int run_gemv(const KernelArgs& args, DenseProblem p, DenseStore store) {
     }
     auto run = [&](auto kernel) {
       const DenseTask<STORE> task(p);
-      // These start when their predecessor has ended.  Let in early they took longer than they saved, and so did the launch before
-      // them, in steps of both designs of decoders at every number of rows, us: width 2048 recurrent 8 rows 578 -> 535, 32 rows
+      // In a plan, and with 17 to 32 rows, these start when their predecessor has ended.  In steps, which are plans, they took longer
+      // than they saved when they were let in early, and so did the launch before them, us: width 2048 recurrent 8 rows 578 -> 535, 32 rows
       // 1190 -> 1105, windowed one row 340 -> 298, 8 rows 565 -> 500; width 4096 windowed 8 rows 1335 -> 1010, 32 rows 2850 -> 1990,
-      // recurrent one row 850 -> 694.  It is not that early ones share an SM: kept apart by shared memory they stay slow.
+      // recurrent one row 850 -> 694.  It is not that early ones share an SM: kept apart by shared memory they stay slow; and a plan of
+      // norms and products alone takes the same time either way.  Outside of plans a launch that waits costs 2 us: norm and product in
+      // turn, k and n 512, 8 rows 6.4 us, 4.4 early; 2048, 8 rows 9.2 and 7.7, 64 rows 17.8 and 15.9.  Prompts: recurrent 9 tokens 1641,
+      // 1608, 50 tokens 2408, 2314, windowed 50 tokens 2311, 2276; but 24 tokens 1953, 2026 and 1697, 1715.
       KernelArgs launch = args;
-      launch.apart = true;
+      launch.apart = args.in_plan || (p.m > 16u && p.m <= 32u);
       if (p.cluster == 1u) launch_kernel(launch, kernel, dim3(tiles), dim3(kGemvWarps * 32), 0, task);
       else launch_cluster_kernel(launch, kernel, dim3(tiles * p.cluster), dim3(kGemvWarps * 32), 0, p.cluster, task);
       return check_launch(args);

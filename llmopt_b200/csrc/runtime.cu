@@ -568,6 +568,7 @@ static void fill_args(Context* context, const OwnedRecord& record, const uint32_
   args.name = record.name.c_str();
   args.past_tokens_cell = is_paged_attention_name(args.name) && record.params.size() >= 16 ? past_cell : nullptr;
   args.checkpoint_cell = is_checkpoint_pack_name(args.name) && record.params.size() >= 4 ? checkpoint_cell : nullptr;
+  args.in_plan = past_cell != nullptr;
 }
 
 static int run_record(Context* context, const OwnedRecord& record, const uint32_t* past_cell,
