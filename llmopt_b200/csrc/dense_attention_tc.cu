@@ -4,17 +4,19 @@
 // A CTA owns 128 queries of one head and walks over tiles of 128 keys.  One thread brings Q, K and V by TMA (128-byte swizzle)
 // and issues tcgen05.mma: S = Q K^T into tensor memory (128 columns), later O += P V (D columns).  Warps of rows read S and write
 // P = exp2(S - top) over it as fp16 pairs, the A operand of P V in tensor memory; V is the B operand as it lies in memory,
-// dimensions contiguous.  O stays in tensor memory; it is scaled only when a row's maximum has grown by more than 2^kSlack since it
-// was last scaled: weights of up to 2^kSlack are as exact in fp16, and the denominator adds what P V uses (rescaling put off in this
-// way was published with FlashAttention-4, 2025).
+// dimensions contiguous.  O stays in tensor memory and is scaled, behind the exponentials, where a row's maximum has grown: the largest
+// weight is 1 and exact in fp16.  (Left alone until a maximum has grown by 2^8 it is rounded like any other: 2 to 8 % further from 64 bits
+// from 333 to 2048 tokens.)  The denominator adds what P V uses.  The first 16 of 64 keys have the remainder of their weight multiplied as
+// well, which lies beside the weights: with the maxima of 128 keys instead of 64 fewer weights are exact than on mma.sync, 0.35 % more error;
+// with the remainders it is 1 to 10 % less, for 2 to 10 % of the time.
 //
 // What bounds a tile is the chain from S to P (16 exponentials a cycle and SM are its floor), so two of them run side by side,
 // in one of two forms, of which both give the same bits:
 //  * ALONE: one CTA per SM, two threads per row, and the next tile's scores multiplied beside this tile's exponentials;
 //  * otherwise two CTAs share an SM, a thread per row.
-// Up to two CTAs per SM the first is faster or as fast, beyond the second, with either head size.  us, causal, back to back over six sets of
-// operands, CTAs and then two per SM, ALONE: heads of 64: 9 5.4, 5.0; 144 33.1, 25.0; 256 18.8, 17.2; 288 20.8, 19.7; 320 23.4, 25.9; 512
-// 42.5, 55.1.  Of 128: 128 21.5, 15.7; 256 22.8, 22.7; 288 25.7, 25.8; 320 28.9, 32.7; 352 31.4, 37.0; 512 49.8, 63.7.
+// Up to two CTAs per SM the first is the faster, beyond the second, with either head size.  us, causal, back to back over six sets of
+// operands, CTAs and then two per SM, ALONE: heads of 64: 9 5.7, 5.0; 144 37.5, 25.5; 256 20.9, 17.4; 288 23.1, 20.0; 320 26.0, 26.3; 352
+// 29.3, 30.7; 512 45.6, 56.6.  Of 128: 128 23.8, 17.1; 256 25.0, 23.4; 288 28.0, 26.7; 320 31.2, 33.8; 352 35.3, 38.7; 512 54.1, 66.8.
 // K and V two tiles deep changed nothing: their way hides behind the exponentials.
 //
 // Rows beyond a head's keys or queries are zero-filled by TMA.  Every wait on an mbarrier is bounded; a wait that runs out raises
@@ -33,7 +35,6 @@ namespace {
 
 constexpr uint32_t kTile = 128;      // queries, and keys of a tile
 constexpr uint32_t kBlockBytes = kTile * 128;  // 64 dimensions of 128 rows
-constexpr float kSlack = 8.0f;
 constexpr float kLowest = -1.0e30f;
 
 // Keys that some query sees; beyond, memory need not hold numbers, and TMA puts zeros there.
@@ -76,6 +77,11 @@ __device__ __forceinline__ void mma_f16_weights(uint32_t tmem_d, uint32_t tmem_a
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
       ::"r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(instruction), "r"(accumulate), "r"(0u)
       : "memory");
+}
+__device__ __forceinline__ void tmem_store_8(uint32_t address, const uint32_t (&v)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"r"(address), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
 }
 __device__ __forceinline__ void tmem_store_16(uint32_t address, const uint32_t (&v)[16]) {
   asm volatile(
@@ -236,8 +242,11 @@ dense_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
         for (uint32_t j = 0; j < kTile / 16; ++j) {
           const uint32_t half = j * 16u / S::kKeys, weights = scores + which * kTile + half * S::kKeys + (j * 16u - half * S::kKeys) / 2u;
           // bit 16: the B operand's columns are contiguous
-          mma_f16_weights(sums, weights, value_descriptor(base + S::kV + j * 2048u), instruction_descriptor(kTile, D) | (1u << 16),
-                          (tile > 0 || j > 0) ? 1u : 0u);
+          const uint32_t instruction = instruction_descriptor(kTile, D) | (1u << 16);
+          const uint64_t values = value_descriptor(base + S::kV + j * 2048u);
+          mma_f16_weights(sums, weights, values, instruction, (tile > 0 || j > 0) ? 1u : 0u);
+          if (j % 4u == 0)  // the remainders of these 16 weights
+            mma_f16_weights(sums, scores + which * kTile + half * S::kKeys + S::kKeys / 2u + (j / 4u - half) * 8u, values, instruction, 1u);
         }
         mma_commit(sums_full), ++sums_issued;
         ok = barrier_wait(sums_full, tile & 1u);  // V and the weights are read
@@ -297,31 +306,15 @@ dense_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
         halves_sync();
         most = fmaxf(most, of_row(tile & 1u, half ^ 1u));
       }
-      const bool grown = most > top + kSlack;
-      if (__any_sync(0xffffffffu, grown)) {
-        const float keep = grown ? exp2_fast(top - most) : 1.0f;
-        if (grown) top = most;
+      const bool grown = most > top;
+      const bool any = __any_sync(0xffffffffu, grown);
+      const float keep = grown ? exp2_fast(top - most) : 1.0f;
+      if (grown) top = most;
 #pragma unroll
-        for (float& part : of_halves) part *= keep;
-        if (tile > 0) {
-          if (ALONE) {  // P V of the tile before may still be under way
-            ok = __all_sync(0xffffffffu, barrier_wait(sums_full, (tile - 1u) & 1u));
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          }
-#pragma unroll 1
-          for (uint32_t part = half * (D / 32u / S::kHalves); part < (half + 1u) * (D / 32u / S::kHalves); ++part) {
-            uint32_t held[32];
-            tmem_load_32(sums + lanes + part * 32u, held);
-            tmem_wait_load();
-#pragma unroll
-            for (int i = 0; i < 32; ++i) held[i] = __float_as_uint(__uint_as_float(held[i]) * keep);
-            tmem_store_32(sums + lanes + part * 32u, held);
-          }
-        }
-      }
+      for (float& part : of_halves) part *= keep;
 #pragma unroll
       for (uint32_t part = 0; part < S::kKeys / 32u; ++part) {
-        uint32_t weights[16];
+        uint32_t weights[16], rests[8];
         float two[2] = {0.0f, 0.0f};
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
@@ -332,18 +325,38 @@ dense_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
             high = part * 32u + 2u * i + 1u < seen ? high : 0.0f;
           }
           const __half2 pair = __floats2half2_rn(low, high);
-          const float2 rounded = __half22float2(pair);
-          two[0] += rounded.x;
-          two[1] += rounded.y;
           weights[i] = *reinterpret_cast<const uint32_t*>(&pair);
+          const float2 rounded = __half22float2(pair);
+          if (part % 2u == 0 && i < 8) {
+            two[0] += low;
+            two[1] += high;
+            const __half2 rest = __floats2half2_rn(low - rounded.x, high - rounded.y);
+            rests[i] = *reinterpret_cast<const uint32_t*>(&rest);
+          } else {
+            two[0] += rounded.x;
+            two[1] += rounded.y;
+          }
         }
         of_halves[ALONE ? 0u : part / 2u] += two[0] + two[1];
         tmem_store_16(mine + part * 16u, weights);  // over scores that are in registers
+        if (part % 2u == 0) tmem_store_8(mine + S::kKeys / 2u + part / 2u * 8u, rests);
       }
       // A wait names a phase by its parity, so nobody may be two phases behind: with two tiles of scores a row could be done with this
       // tile before P V of the one before has begun (V late), which would end the wait for the last P V too early, and run
       // `weights_full` past the thread that waits for it.  tests/test_barrier_order_cpu.py goes through every order.
       if (ALONE && tile > 0) ok = barrier_wait(sums_full, (tile - 1u) & 1u) && ok;
+      if (any && tile > 0) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+        for (uint32_t part = half * (D / 32u / S::kHalves); part < (half + 1u) * (D / 32u / S::kHalves); ++part) {
+          uint32_t held[32];
+          tmem_load_32(sums + lanes + part * 32u, held);
+          tmem_wait_load();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) held[i] = __float_as_uint(__uint_as_float(held[i]) * keep);
+          tmem_store_32(sums + lanes + part * 32u, held);
+        }
+      }
       tmem_wait_store();
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
