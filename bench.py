@@ -564,7 +564,7 @@ def time_baseline_mode(runtime, peaks) -> dict:
 def time_other_kernels(runtime, peaks) -> dict:
     """Kernels of the path that no leg above times: the Q4_0-block GEMV (GGUF blocks, 18 bytes per 32
     weights) at the gate shape against the HBM peak, and the dense causal prefill attention
-    (mma.sync flash-attention forward) at 2048 tokens of the Llama-8B head geometry against the
+    (tcgen05, scores and read-outs in tensor memory) at 2048 tokens of the Llama-8B head geometry against the
     tensor peak."""
     from llmopt_b200 import kernel_bench
 
@@ -595,7 +595,7 @@ def time_other_kernels(runtime, peaks) -> dict:
     out["dense_attention_causal_2048"] = {
         "kernel": item.name, "ms": round(milliseconds, 5), "bound": "tensor", "tflops": round(flops / milliseconds / 1e9, 1),
         "frac": round(flops / milliseconds / 1e9 / peaks["bf16_tflops"], 3),
-        "note": "legacy tensor path (mma.sync), fp16, 32 query / 8 KV heads of 128", "mode": "isolated launch"}
+        "note": "tcgen05, fp16, 32 query / 8 KV heads of 128", "mode": "isolated launch"}
     del keep
     return out
 
