@@ -15,13 +15,17 @@
 //  * ALONE: one CTA per SM, two threads per row, and the next tile's scores multiplied beside this tile's exponentials;
 //  * otherwise two CTAs share an SM, a thread per row.
 // Up to two CTAs per SM the first is the faster, beyond the second, with either head size.  us, causal, back to back over six sets of
-// operands, CTAs and then two per SM, ALONE: heads of 64: 9 5.7, 5.0; 144 37.5, 25.5; 256 20.9, 17.4; 288 23.1, 20.0; 320 26.0, 26.3; 352
-// 29.3, 30.7; 512 45.6, 56.6.  Of 128: 128 23.8, 17.1; 256 25.0, 23.4; 288 28.0, 26.7; 320 31.2, 33.8; 352 35.3, 38.7; 512 54.1, 66.8.
+// operands, CTAs and then two per SM, ALONE: heads of 64: 9 5.7, 5.1; 144 38.0, 26.4; 256 21.3, 17.9; 288 23.6, 20.6; 320 26.1, 26.9; 352
+// 29.2, 31.4; 512 46.5, 59.1.  Of 128: 128 26.0, 17.0; 256 27.6, 23.9; 288 30.4, 27.3; 320 33.4, 34.4; 352 37.3, 39.4; 512 56.7, 68.4.
 // K and V two tiles deep changed nothing: their way hides behind the exponentials.
 //
-// Rows beyond a head's keys or queries are zero-filled by TMA.  Every wait on an mbarrier is bounded; a wait that runs out raises
+// P V multiplies the weight of a masked key, zero, with its value, and zero times an infinity is no number.  Queries are left out of
+// the products of 64 keys of which they see none, so a value reaches none but the queries that see it and up to 63 before, as on mma.sync.
+// Rows beyond a head's keys or queries, and keys behind the last query's, are zero-filled by TMA.  Every wait on an mbarrier is bounded; a wait that runs out raises
 // the context's device error word, and the CTA lets its copies land and its products end, frees its tensor memory and returns.
 #include <cuda.h>
+
+#include <type_traits>
 
 #include "dense_attention.cuh"
 #include "w4a16_tc_device.cuh"
@@ -70,13 +74,23 @@ __device__ __forceinline__ void tma_load_4d(uint32_t destination, const CUtensor
       ::"r"(destination), "l"(map), "r"(bar), "r"(x), "r"(row), "r"(head), "r"(batch)
       : "memory");
 }
+// LOWER: the first 64 rows (lanes) keep what they have.
+template <bool LOWER>
 __device__ __forceinline__ void mma_f16_weights(uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t instruction, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(instruction), "r"(accumulate), "r"(0u)
-      : "memory");
+  if constexpr (LOWER)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %6, %6}, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(instruction), "r"(accumulate), "r"(0xffffffffu), "r"(0u)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(b_desc), "r"(instruction), "r"(accumulate), "r"(0u)
+        : "memory");
 }
 __device__ __forceinline__ void tmem_store_8(uint32_t address, const uint32_t (&v)[8]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
@@ -117,50 +131,10 @@ __device__ __forceinline__ uint64_t value_descriptor(uint32_t shared_address) {
   return descriptor;
 }
 
-// P V multiplies a weight of zero with the value of a masked key, which makes NaN of an infinity or a NaN there.  A warp computes such
-// a row's dimensions first .. first + 32 * PARTS - 1 once more, from its visible keys alone and in the manner of the general kernel;
-// the queries are still in shared memory.  Nothing is done where the masked keys of its last tile are numbers: the row's own result it is.
-template <int D, int PARTS>
-__device__ __noinline__ void walk_row(const unsigned char* q_tile, uint32_t row, const __half* keys, const __half* values, size_t value_stride,
-                                      uint32_t seen, uint32_t multiplied, uint32_t first, float scale, __half* target) {
-  const uint32_t lane = threadIdx.x & 31u;
-  bool masked = false;
-  for (uint32_t key = seen; key < multiplied; ++key)
-#pragma unroll
-    for (int i = 0; i < PARTS; ++i)
-      masked |= !(fabsf(__half2float(values[key * value_stride + first + i * 32 + lane])) < INFINITY);
-  if (!__any_sync(0xffffffffu, masked)) return;
-  float q[D / 32], result[PARTS] = {}, top = -INFINITY, total = 0.0f;
-#pragma unroll
-  for (int i = 0; i < D / 32; ++i) {  // 128-byte swizzle
-    const uint32_t d = i * 32 + lane, at = d / 64u * kBlockBytes + row * 128u + ((d % 64u * 2u) ^ (row % 8u * 16u));
-    q[i] = __half2float(*reinterpret_cast<const __half*>(q_tile + at));
-  }
-  for (uint32_t key = 0; key < seen; ++key) {
-    float dot = 0.0f;
-#pragma unroll
-    for (int i = 0; i < D / 32; ++i) dot = fmaf(q[i], __half2float(keys[(size_t)key * D + i * 32 + lane]), dot);
-    const float score = warp_sum(dot) * scale, next = fmaxf(top, score);
-    const float keep = top == -INFINITY ? 0.0f : expf(top - next), weight = expf(score - next);
-    bool lost = true;  // every result is NaN and stays it
-#pragma unroll
-    for (int i = 0; i < PARTS; ++i) {
-      result[i] = result[i] * keep + weight * __half2float(values[key * value_stride + first + i * 32 + lane]);
-      lost = lost && isnan(result[i]);
-    }
-    total = total * keep + weight;
-    top = next;
-    if (__all_sync(0xffffffffu, lost)) break;
-  }
-#pragma unroll
-  for (int i = 0; i < PARTS; ++i) target[first + i * 32 + lane] = __float2half_rn(total == 0.0f ? 0.0f : result[i] / total);
-}
-
 template <int D, bool ALONE>
 __global__ void __launch_bounds__(Shape<D, ALONE>::kThreads, ALONE ? 1 : 2)
 dense_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                          const __grid_constant__ CUtensorMap map_v, const __half* key, const __half* value, __half* output, DenseParams p,
-                          uint32_t* error_word) {
+                          const __grid_constant__ CUtensorMap map_v, __half* output, DenseParams p, uint32_t* error_word) {
   using S = Shape<D, ALONE>;
   extern __shared__ unsigned char shared_raw[];
   grid_chain_prologue();
@@ -174,7 +148,9 @@ dense_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
   // the last query tiles see the most keys under a causal mask: they are scheduled first, over all heads
   const uint32_t q0 = (gridDim.y - 1u - blockIdx.y) * kTile, head = blockIdx.x, batch = blockIdx.z;
   const uint32_t key_end = p.causal ? min(p.k_len, min(q0 + kTile, p.q_len) + p.past_length) : p.k_len;
-  const uint32_t tiles = (key_end + kTile - 1u) / kTile;
+  // Tiles of keys begin so that 64 keys in line are the diagonal of 64 queries; the first may begin ahead of the first key.
+  const uint32_t lead = p.causal ? (64u - p.past_length % 64u) % 64u : 0u;
+  const uint32_t tiles = (key_end + lead + kTile - 1u) / kTile;
 
   if (threadIdx.x == 0) {
     barrier_init(q_full, 1);  // the expect_tx arrivals; complete by byte count
@@ -204,15 +180,16 @@ dense_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
     if (lane == 0) {
       const int32_t kv_head = (int32_t)(head / (p.heads / p.kv_heads));
       uint32_t k_issued = 0, v_issued = 0, scores_issued = 0, sums_issued = 0;
-      auto load = [&](const CUtensorMap* map, uint32_t target, uint32_t row, int32_t of_head, uint32_t bar) {
+      auto load = [&](const CUtensorMap* map, uint32_t target, int32_t row, int32_t of_head, uint32_t bar) {
         barrier_expect_tx(bar, S::kTileBytes);
 #pragma unroll
         for (uint32_t block = 0; block < S::kBlocks; ++block)
-          tma_load_4d(base + target + block * kBlockBytes, map, (int32_t)(block * 64u), (int32_t)row, of_head, (int32_t)batch, bar);
+          tma_load_4d(base + target + block * kBlockBytes, map, (int32_t)(block * 64u), row, of_head, (int32_t)batch, bar);
       };
-      load(&map_q, 0, q0, (int32_t)head, q_full);
-      load(&map_k, S::kK, 0, kv_head, k_full), ++k_issued;
-      load(&map_v, S::kV, 0, kv_head, v_full), ++v_issued;
+      auto first_key = [&](uint32_t tile) { return (int32_t)(tile * kTile) - (int32_t)lead; };
+      load(&map_q, 0, (int32_t)q0, (int32_t)head, q_full);
+      load(&map_k, S::kK, first_key(0), kv_head, k_full), ++k_issued;
+      load(&map_v, S::kV, first_key(0), kv_head, v_full), ++v_issued;
       auto multiply = [&](uint32_t tile) {  // S = Q K^T
         if (*abort_flag || !barrier_wait(k_full, tile & 1u)) return false;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -226,32 +203,45 @@ dense_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
         mma_commit(scores_full + which * 8u), ++scores_issued;
         return true;
       };
+      auto add_values = [&](uint32_t tile, uint32_t upper, auto lower) {  // O += P V of the first or last 64 keys
+        const uint32_t first = scores + tile % S::kScores * kTile;
+        const uint32_t instruction = instruction_descriptor(kTile, D) | (1u << 16);  // bit 16: the B operand's columns are contiguous
+#pragma unroll
+        for (uint32_t i = 0; i < 4; ++i) {
+          const uint32_t j = upper * 4u + i, half = upper * 64u / S::kKeys, weights = first + half * S::kKeys;
+          const uint64_t values = value_descriptor(base + S::kV + j * 2048u);
+          mma_f16_weights<decltype(lower)::value>(sums, weights + (j * 16u - half * S::kKeys) / 2u, values, instruction, (tile > 0 || j > 0) ? 1u : 0u);
+          if (i == 0)  // and the remainders of the weights
+            mma_f16_weights<decltype(lower)::value>(sums, weights + S::kKeys / 2u + (upper - half) * 8u, values, instruction, 1u);
+        }
+      };
       bool ok = barrier_wait(q_full, 0) && multiply(0);
       for (uint32_t tile = 0; tile < tiles && ok; ++tile) {
         const uint32_t which = tile % S::kScores;
         ok = barrier_wait(scores_full + which * 8u, tile / S::kScores & 1u);  // K is read
         if (!ok) break;
         if (tile + 1u < tiles) {
-          load(&map_k, S::kK, (tile + 1u) * kTile, kv_head, k_full), ++k_issued;
+          load(&map_k, S::kK, first_key(tile + 1u), kv_head, k_full), ++k_issued;
           if (ALONE) ok = multiply(tile + 1u);  // beside this tile's exponentials; its place was last read by P V of the tile before
         }
         ok = ok && !*abort_flag && barrier_wait(v_full, tile & 1u) && barrier_wait(weights_full, tile & 1u);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-        for (uint32_t j = 0; j < kTile / 16; ++j) {
-          const uint32_t half = j * 16u / S::kKeys, weights = scores + which * kTile + half * S::kKeys + (j * 16u - half * S::kKeys) / 2u;
-          // bit 16: the B operand's columns are contiguous
-          const uint32_t instruction = instruction_descriptor(kTile, D) | (1u << 16);
-          const uint64_t values = value_descriptor(base + S::kV + j * 2048u);
-          mma_f16_weights(sums, weights, values, instruction, (tile > 0 || j > 0) ? 1u : 0u);
-          if (j % 4u == 0)  // the remainders of these 16 weights
-            mma_f16_weights(sums, scores + which * kTile + half * S::kKeys + S::kKeys / 2u + (j / 4u - half) * 8u, values, instruction, 1u);
+        // zero times an infinity is no number: the first 64 queries leave 64 keys out of which they see none
+        const bool apart = p.causal && first_key(tile) + 64 > (int32_t)(q0 + p.past_length);
+        if (!apart) {
+          add_values(tile, 0, std::false_type());
+          add_values(tile, 1, std::false_type());
+        } else if (first_key(tile) <= (int32_t)(q0 + p.past_length)) {
+          add_values(tile, 0, std::false_type());
+          add_values(tile, 1, std::true_type());
+        } else {  // nobody sees the last ones
+          add_values(tile, 0, std::true_type());
         }
         mma_commit(sums_full), ++sums_issued;
         ok = barrier_wait(sums_full, tile & 1u);  // V and the weights are read
         if (ok && tile + 1u < tiles) {
-          load(&map_v, S::kV, (tile + 1u) * kTile, kv_head, v_full), ++v_issued;
+          load(&map_v, S::kV, first_key(tile + 1u), kv_head, v_full), ++v_issued;
           if (!ALONE) ok = multiply(tile + 1u);
         }
       }
@@ -285,12 +275,17 @@ dense_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       // keys below `seen` are visible to this row; all of them to the whole warp where `whole`
-      const uint32_t limit = p.causal ? min(p.k_len, query + p.past_length + 1u) : p.k_len, seen = limit > k0 ? limit - k0 : 0u;
+      const uint32_t limit = lead + (p.causal ? min(p.k_len, query + p.past_length + 1u) : p.k_len), seen = limit > k0 ? limit - k0 : 0u;
       const bool whole = __all_sync(0xffffffffu, seen >= S::kKeys);
       uint32_t raw[S::kKeys / 32u][32];
 #pragma unroll
       for (uint32_t part = 0; part < S::kKeys / 32u; ++part) tmem_load_32(mine + part * 32u, raw[part]);
       tmem_wait_load();
+      if (k0 < lead) {  // what lies ahead of the first key
+#pragma unroll
+        for (uint32_t i = 0; i < 64u; ++i)
+          if (i < lead) raw[i / 32][i % 32] = 0xff800000u;
+      }
       float four[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
       if (whole) {
 #pragma unroll
@@ -374,7 +369,6 @@ dense_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
     if (ok) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const float inverse = total == 0.0f ? 0.0f : 1.0f / total;
-      bool finite = true;
       __half* const target = output + (p.token_first_output ? (((size_t)batch * p.q_len + query) * p.heads + head) * D
                                                             : (((size_t)batch * p.heads + head) * p.q_len + query) * D);
 #pragma unroll 1
@@ -388,25 +382,13 @@ dense_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
             uint32_t words[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-              const float low = __uint_as_float(raw[i * 8 + j * 2]) * inverse, high = __uint_as_float(raw[i * 8 + j * 2 + 1]) * inverse;
-              finite = finite && fabsf(low) < INFINITY && fabsf(high) < INFINITY;
-              const __half2 pair = __floats2half2_rn(low, high);
+              const __half2 pair = __floats2half2_rn(__uint_as_float(raw[i * 8 + j * 2]) * inverse, __uint_as_float(raw[i * 8 + j * 2 + 1]) * inverse);
               words[j] = *reinterpret_cast<const uint32_t*>(&pair);
             }
             *reinterpret_cast<uint4*>(target + part * 32u + i * 8) = make_uint4(words[0], words[1], words[2], words[3]);
           }
         }
         __syncwarp();  // tcgen05.ld needs the whole warp
-      }
-      for (uint32_t left = __ballot_sync(0xffffffffu, !finite); left != 0; left &= left - 1u) {
-        barrier_wait(q_full, 0);  // over long ago; this thread has not waited for it yet
-        const uint32_t at = row - lane + (uint32_t)__ffs(left) - 1u, kv_head = head / (p.heads / p.kv_heads);
-        const uint32_t seen = p.causal ? min(p.k_len, q0 + at + p.past_length + 1u) : p.k_len, multiplied = min(seen_by_any(p), tiles * kTile);
-        const size_t head_row = (size_t)batch * p.kv_heads + kv_head;
-        const __half* const values = value + (p.token_first_value ? ((size_t)batch * p.k_len * p.kv_heads + kv_head) * D : head_row * p.k_len * D);
-        const int64_t along = p.token_first_output ? (int64_t)p.heads * D : D;  // from one row of the output to the next
-        walk_row<D, D / 32 / S::kHalves>(base_pointer, at, key + head_row * p.k_len * D, values, p.token_first_value ? (size_t)p.kv_heads * D : D,
-                                         seen, multiplied, half * (D / S::kHalves), p.scale, target + ((int64_t)at - (int64_t)row) * along);
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     }
@@ -457,7 +439,7 @@ int run(const KernelArgs& args, const DenseParams& p) {
     return -1;
   }
   launch_kernel(args, kernel, dim3(p.heads, (p.q_len + kTile - 1u) / kTile, p.batches), dim3(S::kThreads), S::kSharedBytes, map_q, map_k,
-                map_v, (const __half*)args.buffers[1], (const __half*)args.buffers[2], (__half*)args.buffers[4], p, args.ctx ? context_device_error(args.ctx) : nullptr);
+                map_v, (__half*)args.buffers[4], p, args.ctx ? context_device_error(args.ctx) : nullptr);
   return check_launch(args);
 }
 
@@ -466,7 +448,7 @@ int run(const KernelArgs& args, const DenseParams& p) {
 int launch_attention_dense_tc(const KernelArgs& args, const DenseParams& p) {
   if (!(p.scale > 0.0f)) return -1;  // the largest score is that of the largest product
   if (args.ctx == nullptr || p.mask_batches != 0 || p.batches > 65535u || p.q_len > 65535u * kTile || (p.dim != 64u && p.dim != 128u)) return -1;
-  if (p.causal && (uint64_t)p.q_len + p.past_length > 0xffffffffull) return -1;
+  if (p.causal && (uint64_t)p.q_len + p.past_length > 0x7fffff00ull) return -1;  // TMA's coordinates
   for (int i = 0; i < 5; ++i)
     if (i != 3 && ((uintptr_t)args.buffers[i] & 15u)) return -1;
   const size_t ctas = (size_t)p.heads * ((p.q_len + kTile - 1u) / kTile) * p.batches;
