@@ -10,19 +10,20 @@
 // well, which lies beside the weights: with the maxima of 128 keys instead of 64 fewer weights are exact than on mma.sync, 0.35 % more error;
 // with the remainders it is 1 to 10 % less, for 2 to 10 % of the time.
 //
-// What bounds a tile is the chain from S to P (16 exponentials a cycle and SM are its floor), so two of them run side by side,
+// What bounds a tile is the chain from S to P (no pipe is busy for more than 36 % of the time), so two of them run side by side,
 // in one of two forms, of which both give the same bits:
 //  * ALONE: one CTA per SM, two threads per row, and the next tile's scores multiplied beside this tile's exponentials;
 //  * otherwise two CTAs share an SM, a thread per row.
 // Up to two CTAs per SM the first is the faster, beyond the second, with either head size.  us, causal, back to back over six sets of
 // operands, CTAs and then two per SM, ALONE: heads of 64: 9 5.7, 5.1; 144 38.0, 26.4; 256 21.3, 17.9; 288 23.6, 20.6; 320 26.1, 26.9; 352
 // 29.2, 31.4; 512 46.5, 59.1.  Of 128: 128 26.0, 17.0; 256 27.6, 23.9; 288 30.4, 27.3; 320 33.4, 34.4; 352 37.3, 39.4; 512 56.7, 68.4.
-// K and V two tiles deep changed nothing: their way hides behind the exponentials.
+// K and V two tiles deep changed nothing: their way hides behind that chain.
 //
 // P V multiplies the weight of a masked key, zero, with its value, and zero times an infinity is no number.  Queries are left out of
 // the products of 64 keys of which they see none, so a value reaches none but the queries that see it and up to 63 before, as on mma.sync.
-// Rows beyond a head's keys or queries, and keys behind the last query's, are zero-filled by TMA.  Every wait on an mbarrier is bounded; a wait that runs out raises
-// the context's device error word, and the CTA lets its copies land and its products end, frees its tensor memory and returns.
+// Rows beyond a head's keys or queries, and keys behind the last query's, are zero-filled by TMA.  Every wait on an mbarrier is bounded;
+// a wait that runs out raises the context's device error word, and the CTA lets its copies land and its products end, frees its tensor
+// memory and returns.
 #include <cuda.h>
 
 #include <type_traits>
